@@ -922,9 +922,8 @@ Grid::~Grid() {
     cudaFree(b.packed);
     cudaFree(b.dTcTiles);
     cudaFree(b.tc64Items);
-    cudaFree(b.packed64);
-    cudaFree(b.colExp);
   }
+  if (pool_ != nullptr) cudaMemPoolDestroy(pool_);
   cudaFree(scratchSpectra_);
   cudaFree(scratchCoeffs_);
   for (auto& [N, t] : tables_) {
@@ -1044,8 +1043,7 @@ int Grid::BatchFor(int N, bool real, bool analysis, int P, int p0, int count, co
       for (int nt = 0; nt < h.nTiles; ++nt)
         b.tcTiles.push_back(make_int4(static_cast<int>(b.tcHost.size()), mt, nt, 0));
     b.tcHost.push_back(h);
-    // the FP64 emulation's tiles: 128 rows, 64 columns, 16 deep, seven
-    // slices a tile
+    // the FP64 slices' tiles: 128 rows, 64 columns, 16 deep
     Tc64Item e{};
     e.M = g.M;
     e.N = g.N;
@@ -1056,13 +1054,13 @@ int Grid::BatchFor(int N, bool real, bool analysis, int P, int p0, int count, co
     e.ldc = g.ldc;
     e.ldb = g.ldb;
     e.aPanel = b.panel64;
-    e.bPack = b.packed64Count;
+    e.bPack = b.packed64;
     e.b = g.b;
     e.c = g.c;
     e.rowExp = b.rowExps;
     e.colExp = b.colExps;
-    b.panel64 += static_cast<long long>(e.mTiles) * e.kSteps * kTc64Slices * kTcTileM * kTcTileK;
-    b.packed64Count += static_cast<long long>(e.nTiles) * e.kSteps * kTc64Slices * kTc64TileN * kTcTileK;
+    b.panel64 += static_cast<long long>(e.mTiles) * e.kSteps;
+    b.packed64 += static_cast<long long>(e.nTiles) * e.kSteps;
     b.rowExps += g.M;
     b.colExps += g.N;
     b.maxNTiles64 = std::max(b.maxNTiles64, e.nTiles);
@@ -1097,45 +1095,71 @@ int Grid::RunGemm(const Batch& b, const double* A, const double* B, double* C, b
   return SL3DGPU_OK;
 }
 
-// The FP64 contraction emulated on the tensor cores: the spin's split
-// panel for this direction made on first use, the batch's items, packed-B
-// buffer and column exponents on its first use; then B split and packed, and
-// the contraction.
+// Whether a batch's FP64 contraction runs as slice products: within the
+// exactness bound on its depth, and wider than the narrow kernels' columns.
+bool Grid::UseSlices64(const Batch& b) const {
+  if (emulateFp64) return b.maxK <= Tc64MaxK(kTc64Slices);
+  return b.maxN > kNarrowN && b.maxK <= Tc64MaxK(kTc64SlicesFull);
+}
+
+// The FP64 contraction as slice products on the tensor cores: the spin's
+// split panel for this direction made on first use, the batch's items on its
+// first use; then B split and packed into memory of this call, and the
+// contraction.
 int Grid::RunGemm64(int N, bool real, Batch& b, const double* B, double* C, bool accumulate,
                     cudaStream_t stream) {
   if (b.count == 0) return SL3DGPU_OK;
+  const int slices = emulateFp64 ? kTc64Slices : kTc64SlicesFull;
   if (dTcError_ == nullptr) {
     SL3D_CUDA(cudaMalloc(&dTcError_, sizeof(int)));
     SL3D_CUDA(ZeroIn(dTcError_, sizeof(int)));
   }
+  if (pool_ == nullptr) {
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    SL3D_CUDA(cudaGetDevice(&props.location.id));
+    SL3D_CUDA(cudaMemPoolCreate(&pool_, &props));
+    uint64_t keep = UINT64_MAX;  // kept until the grid is destroyed
+    SL3D_CUDA(cudaMemPoolSetAttribute(pool_, cudaMemPoolAttrReleaseThreshold, &keep));
+  }
   if (b.tc64Items == nullptr) {
     SL3D_CUDA(cudaMalloc(&b.tc64Items, b.tc64Host.size() * sizeof(Tc64Item)));
     SL3D_CUDA(CopyIn(b.tc64Items, b.tc64Host.data(), b.tc64Host.size() * sizeof(Tc64Item)));
-    SL3D_CUDA(cudaMalloc(&b.packed64, std::max<long long>(b.packed64Count, 1) * sizeof(uint16_t)));
-    SL3D_CUDA(cudaMalloc(&b.colExp, std::max<long long>(b.colExps, 1) * sizeof(int)));
   }
-  const std::array<int, 3> key{N, real ? 1 : 0, b.analysis ? 1 : 0};
+  const SpinTable* t = nullptr;
+  if (int st = Table(N, &t); st != SL3DGPU_OK) return st;
+  const std::array<int, 4> key{N, real ? 1 : 0, b.analysis ? 1 : 0, slices};
   auto found = panels64_.find(key);
   if (found == panels64_.end()) {
-    const SpinTable* t = nullptr;
-    if (int st = Table(N, &t); st != SL3DGPU_OK) return st;
-    Panel64 panel;
-    SL3D_CUDA(cudaMalloc(&panel.slices, std::max<long long>(b.panel64, 1) * sizeof(uint16_t)));
+    Tc64Panel panel;
+    const size_t values = static_cast<size_t>(std::max<long long>(b.panel64, 1)) * slices * kTcTileM * kTcTileK;
+    SL3D_CUDA(cudaMalloc(&panel.slices, values * sizeof(uint16_t)));
     SL3D_CUDA(cudaMalloc(&panel.rowExp, std::max<long long>(b.rowExps, 1) * sizeof(int)));
     prof::Scope scope(prof::kOther, stream);
-    LaunchPanelA64(b.items, b.tc64Items, b.count, b.maxM, b.maxATiles, t->values, panel.rowExp, panel.slices,
-                   stream);
+    LaunchPanelA64(slices, b.items, b.tc64Items, b.count, b.maxM, b.maxATiles, t->values, panel, stream);
     SL3D_CHECK_LAUNCH();
     found = panels64_.emplace(key, panel).first;
   }
+  // this call's packed tiles, then its column exponents
+  const size_t tileBytes = static_cast<size_t>(b.packed64) * slices * kTc64TileN * kTcTileK * sizeof(uint16_t);
+  void* scratch = nullptr;
+  SL3D_CUDA(cudaMallocFromPoolAsync(&scratch, tileBytes + std::max<long long>(b.colExps, 1) * sizeof(int), pool_,
+                                    stream));
+  auto* packed = static_cast<uint16_t*>(scratch);
+  auto* colExp = reinterpret_cast<int*>(static_cast<char*>(scratch) + tileBytes);
+  int status = SL3DGPU_OK;
   {
-    prof::Scope scope(prof::kStream, stream, 0.0, 8.0 * b.colExps + 2.0 * b.packed64Count);
-    LaunchPackB64(b.tc64Items, b.count, b.maxNTiles64, B, b.colExp, b.packed64, stream);
-    SL3D_CHECK_LAUNCH();
+    prof::Scope scope(prof::kStream, stream, 0.0, 8.0 * b.colExps + static_cast<double>(tileBytes));
+    LaunchPackB64(slices, b.tc64Items, b.count, b.maxNTiles64, B, colExp, packed, stream);
   }
-  prof::Scope scope(prof::kLegendre64Tc, stream, b.flops);
-  return RunGemm64Tc(b.tc64Items, b.count, b.maxMTiles, b.maxNTiles64, found->second.slices, b.packed64,
-                     found->second.rowExp, b.colExp, C, accumulate, dTcError_, stream);
+  {
+    prof::Scope scope(prof::kLegendre64Tc, stream, b.flops);
+    status = RunGemm64Tc(slices, b.items, b.tc64Items, b.count, b.maxMTiles, b.maxNTiles64, t->values, found->second,
+                         B, packed, colExp, C, accumulate, dTcError_, stream);
+  }
+  SL3D_CUDA(cudaFreeAsync(scratch, stream));
+  return status;
 }
 
 int Grid::LegendreSynthesis(int N, bool real, const double* coeffs, int P, int p0, int count,
@@ -1151,7 +1175,7 @@ int Grid::LegendreSynthesis(int N, bool real, const double* coeffs, int P, int p
     if (t->Rows(m, lmax) == 0)
       SL3D_CUDA(cudaMemsetAsync(spectra + static_cast<long long>(m - mlo) * ntheta * 2LL * count, 0,
                                 sizeof(double) * ntheta * 2 * count, stream));
-  if (emulateFp64 && b->maxK <= kTc64MaxK)
+  if (UseSlices64(*b))
     return RunGemm64(N, real, *MutableBatch(N, real, false, P, p0, count), coeffs, spectra, false, stream);
   return RunGemm(*b, t->values, coeffs, spectra, false, stream);
 }
@@ -1163,7 +1187,7 @@ int Grid::LegendreAnalysis(int N, bool real, const double* spectra, int P, int p
   if (int st = Table(N, &t); st != SL3DGPU_OK) return st;
   const Batch* b = nullptr;
   if (int st = BatchFor(N, real, true, P, p0, count, &b); st != SL3DGPU_OK) return st;
-  if (emulateFp64 && b->maxK <= kTc64MaxK)
+  if (UseSlices64(*b))
     return RunGemm64(N, real, *MutableBatch(N, real, true, P, p0, count), spectra, coeffs, accumulate, stream);
   return RunGemm(*b, t->values, spectra, coeffs, accumulate, stream);
 }

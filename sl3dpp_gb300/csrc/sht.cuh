@@ -54,11 +54,18 @@ struct GemmItem {
 struct Tc64Item {
   int M, N, K, mTiles;
   int kSteps, nTiles, ldc, ldb;
-  long long aPanel;  // BF16 values: the item's panel, [mTile][kStep][slice][128 x 16]
-  long long bPack;   // BF16 values: its packed B, [nTile][kStep][slice][64 x 16]
+  long long aPanel;  // tiles: the item's panel, [mTile][kStep] of [slice][128 x 16]
+  long long bPack;   // tiles: its packed B, [nTile][kStep] of [slice][64 x 16]
   long long b, c;    // FP64 offsets of B's source and of C
   long long rowExp;  // ints: the power-of-two exponents of its M rows of A
   long long colExp;  // ints: those of its N columns of B (per call)
+};
+
+// The table split into FP64 slices for one direction: its slice panels and
+// row exponents.
+struct Tc64Panel {
+  uint16_t* slices = nullptr;
+  int* rowExp = nullptr;
 };
 
 // A tensor-core item's host description (mirrors TcItem in tc_gemm.cuh).
@@ -75,9 +82,11 @@ class Grid {
   ~Grid();
 
   int lmax = 0, nmax = 0, band = 0, ntheta = 0, nphi = 0;
-  // The FP64 contractions emulated on the tensor cores (tc_gemm64.cu)
-  // rather than run on the FP64 units; batches deeper than the emulation's
-  // exactness bound keep the FP64 units.
+  // The FP64 contractions run as slice products on the tensor cores
+  // (tc_gemm64.cu): eight slices, at least the FP64 units' accuracy, or, with
+  // this set, seven (about 49 bits) and the rings in double-float. Batches of
+  // few columns and ones deeper than the slices' exactness bound keep the
+  // FP64 units.
   bool emulateFp64 = false;
   std::vector<double> theta, weights;  // host copies
   double* dTheta = nullptr;
@@ -157,22 +166,20 @@ class Grid {
     std::vector<int4> tcTiles;  // {item, row tile, column tile}, column tiles of a row tile adjacent
     int4* dTcTiles = nullptr;
     int maxK = 0;
-    // the FP64 emulation's form: items, extents, packed B and column
-    // exponents (made on first use)
+    // the FP64 slices' form: items (made on first use) and extents
     std::vector<Tc64Item> tc64Host;
     Tc64Item* tc64Items = nullptr;
     int maxNTiles64 = 0, maxBTiles64 = 0;
-    long long panel64 = 0, packed64Count = 0, rowExps = 0, colExps = 0;
-    uint16_t* packed64 = nullptr;
-    int* colExp = nullptr;
+    long long panel64 = 0, packed64 = 0;  // tiles of the panel and of the packed B
+    long long rowExps = 0, colExps = 0;
   };
-  // The table split for the FP64 emulation per (spin, real, direction): its
-  // slice panels and row exponents.
-  struct Panel64 {
-    uint16_t* slices = nullptr;
-    int* rowExp = nullptr;
-  };
-  std::map<std::array<int, 3>, Panel64> panels64_;
+  // The table split for the FP64 slices per (spin, real, direction, slices).
+  std::map<std::array<int, 4>, Tc64Panel> panels64_;
+  // Where a call's packed B and column exponents come from, stream-ordered:
+  // calls on several streams each have their own, and the memory stays with
+  // the grid between them.
+  cudaMemPool_t pool_ = nullptr;
+  bool UseSlices64(const Batch& b) const;
   int RunGemm64(int N, bool real, Batch& b, const double* B, double* C, bool accumulate, cudaStream_t stream);
   // The table pre-tiled for the tensor cores per (spin, real, direction).
   std::map<std::array<int, 3>, float*> panels_;

@@ -1263,7 +1263,7 @@ int Viscoelastic3DGpu::FinishStage(V3dState& out, double dt, int scheme) {
   SL3D_CUDA(cudaMemcpyAsync(out.coeffs.p, s.p, spectralComplex * sizeof(double2), cudaMemcpyDeviceToDevice, stream));
   // a tensor-core contraction that gave up waiting leaves its output
   // unspecified: the step fails rather than return it
-  if (grid->emulateFp64) SL3D_TRY(grid->TensorCoreStatus(stream));
+  SL3D_TRY(grid->TensorCoreStatus(stream));
   out.hasStrain = out.hasCoeffs = true;
   out.latFirst = lateralFirst;
   out.latEnd = lateralEnd;
@@ -3255,7 +3255,7 @@ int Viscoelastic3DGpu::StageAdjoint(V3dState& in, const V3dState& end, double dt
   }
   passAddSph = passAddTor = nullptr;
   SL3D_TRY(rc);
-  if (grid->emulateFp64) SL3D_TRY(grid->TensorCoreStatus(stream));
+  SL3D_TRY(grid->TensorCoreStatus(stream));
   if (!info.converged) {
     SetError("v3d adjoint: a stage's transposed fixed point did not converge");
     return SL3DGPU_ERR_UNCONVERGED;
@@ -3375,7 +3375,7 @@ int Viscoelastic3DGpu::TangentStage(V3dState& in, const V3dState& end, double dt
   } else {
     SL3D_TRY(Converge(*f, loadDot, info));
   }
-  if (grid->emulateFp64) SL3D_TRY(grid->TensorCoreStatus(stream));
+  SL3D_TRY(grid->TensorCoreStatus(stream));
   if (!info.converged) {
     SetError("v3d tangent: a stage's tangent solve did not converge");
     return SL3DGPU_ERR_UNCONVERGED;

@@ -86,23 +86,25 @@ int RunGemmTc(const TcItem* tcItems, const int4* tiles, int tileCount, int tileN
 // -- FP64 emulated on the tensor cores (tc_gemm64.cu) ------------------------------------
 //
 // The FP64 contraction as exact BF16 products: A's rows and B's columns are
-// scaled by powers of two to |x| < 1 and split into kTc64Slices integer
-// slices of at most 7 bits, x = sum_p s_p 2^{-7 (p + 1)} (the Ozaki
-// splitting); the slice products of each level d = p + q < kTc64Slices are
-// accumulated in FP32 by tcgen05.mma kind::f16, exactly (integers below 2^24
-// for K <= 455), and the levels are joined in FP64. About 49 bits of each
-// value enter, so the result carries FP64-level accuracy relative to
-// (row maximum) x (column maximum) x K.
-constexpr int kTc64Slices = 7;
-constexpr int kTc64TileN = 64;   // 7 accumulators of 64 columns in tensor memory
-constexpr int kTc64MaxK = 448;   // the exactness bound on the depth, with margin
+// scaled by powers of two to |x| < 1 and split into integer slices of at
+// most 7 bits, x = sum_p s_p 2^{-7 (p + 1)} (the Ozaki splitting); the slice
+// products of each level d = p + q below the slice count are accumulated in
+// FP32 by tcgen05.mma kind::f16, exactly (integers below 2^24), and the levels
+// are joined in FP64. Seven slices carry about 49 bits of each value, eight
+// 56: with eight the result is at least as accurate as the FP64 units'
+// relative to (row maximum) x (column maximum) x K.
+constexpr int kTc64Slices = 7;       // a grid that asked for the emulation
+constexpr int kTc64SlicesFull = 8;   // the default FP64 contraction
+constexpr int kTc64TileN = 64;       // up to 8 accumulators of 64 columns in tensor memory
+// The exactness bounds on the depth (455 and 409), with margin.
+__host__ __device__ constexpr int Tc64MaxK(int slices) { return slices == kTc64SlicesFull ? 400 : 448; }
 
-void LaunchPanelA64(const GemmItem* items, const Tc64Item* tcItems, int count, int maxM, int maxATiles,
-                    const double* table, int* rowExp, uint16_t* panels, cudaStream_t stream);
-void LaunchPackB64(const Tc64Item* tcItems, int count, int maxNTiles, const double* B, int* colExp,
+void LaunchPanelA64(int slices, const GemmItem* items, const Tc64Item* tcItems, int count, int maxM, int maxATiles,
+                    const double* table, const Tc64Panel& panel, cudaStream_t stream);
+void LaunchPackB64(int slices, const Tc64Item* tcItems, int count, int maxNTiles, const double* B, int* colExp,
                    uint16_t* packed, cudaStream_t stream);
-int RunGemm64Tc(const Tc64Item* tcItems, int count, int maxMTiles, int maxNTiles, const uint16_t* panels,
-                const uint16_t* packed, const int* rowExp, const int* colExp, double* C, bool accumulate,
-                int* errorFlag, cudaStream_t stream);
+int RunGemm64Tc(int slices, const GemmItem* items, const Tc64Item* tcItems, int count, int maxMTiles, int maxNTiles,
+                const double* table, const Tc64Panel& panel, const double* B, uint16_t* packed, int* colExp, double* C,
+                bool accumulate, int* errorFlag, cudaStream_t stream);
 
 }  // namespace sl3dgpu

@@ -4,36 +4,54 @@
 //
 // Splitting. Row i of A has the exponent e_i with max_k |A(i, k)| < 2^{e_i},
 // column n of B the exponent f_n likewise; x = A(i, k) 2^{-e_i} (|x| < 1) is
-// rounded to X = round(x 2^49), an integer below 2^49 read off the double's
-// bits, and X is written in balanced base-2^7 digits,
-// X = sum_{p < 7} s_p 2^{7 (6 - p)}, |s_p| <= 64 for p > 0 and |s_0| <= 128:
-// x = sum_p s_p 2^{-7 (p + 1)} to within 2^{-50}. Integer arithmetic only
-// (the FP64 units of this part are slow); the digits are exact in BF16.
+// rounded to X = round(x 2^{7 S}) for S slices, an integer read off the
+// double's bits, and X is written in balanced base-2^7 digits,
+// X = sum_{p < S} s_p 2^{7 (S - 1 - p)}, |s_p| <= 64 for p > 0 and
+// |s_0| <= 128: x = sum_p s_p 2^{-7 (p + 1)} to within 2^{-7 S - 1}. Integer
+// arithmetic only (the FP64 units of this part are slow); the digits are
+// exact in BF16.
+//
+// Two widths. S = 7 (49 bits, 28 slice products a step) serves a grid that
+// asked for the emulation; S = 8 (56 bits, 36 products) is the default FP64
+// contraction: a value within a factor eight of its row's (column's) largest
+// enters with all its 53 bits and the products below 2^-63 of the row and
+// column maxima are dropped, so that its error stays below the FP64 units'
+// own rounding (measured against quadruple precision at lmax 33 to 256, white
+// and decaying coefficients: 0.1 to 0.45 of theirs in the 2-norm). Against
+// the FP64 units' register-tiled product, bound by GB300's 1.2 TF/s FP64
+// pipe: 45 spin -2 fields at lmax 128, 1.12 ms a contraction there, 0.18 ms
+// here with the packing.
 //
 // Products. Level d = p + q gathers sum_k s_p(A) s_q(B) over p + q = d, at
 // most (d + 3) 2^12 per k in magnitude, so below 2^24 -- exact in the FP32
-// accumulator -- for K <= 455 at d = 6. The levels d < 7 are kept (28
-// products per 16-deep step) and joined exactly as integers,
-// H = acc_0 2^14 + acc_1 2^7 + acc_2 and L = acc_3 2^21 + acc_4 2^14 +
-// acc_5 2^7 + acc_6, and C(i, n) = 2^{e_i + f_n} (2^{-28} H + 2^{-56} L) is
-// rounded once to FP64 from that exact integer, by integer arithmetic.
+// accumulator -- for K <= 455 at S = 7 (d = 6) and K <= 409 at S = 8 (d = 7).
+// The levels d < S are kept and joined exactly as integers, the upper ones
+// into H, the last four into L, and C(i, n) = 2^{e_i + f_n} 2^{-7 (S + 1)}
+// (H 2^28 + L) is rounded once to FP64 from that exact integer, by integer
+// arithmetic.
+//
+// Infinities and NaN. A column of B holding one has no exponent; it is
+// marked, and its outputs are the plain FP64 sum over k from the table and B
+// themselves, as the FP64 units would give them (the packed digits of such a
+// column are not used). A wait that gives up leaves NaN in its tile.
 //
 // Kernel. One CTA of eight warps per (64-column tile, 128-row tile, item),
 // the column tiles of a row tile adjacent in the launch so that its A panel
 // is read from HBM once. One elected thread runs the K loop as the FP32
 // contraction does (tc_gemm.cu): it arms a stage's "full" mbarrier, issues
-// two TMA bulk copies (A's seven slices, 28 KB; B's, 14 KB), four stages in
-// flight, and when they have landed issues the step's tcgen05.mma kind::f16
-// into the level accumulators (tensor-memory columns 64 d .. 64 d + 63 of
-// 512) and commits them to the stage's "empty" mbarrier. B's seven slices
-// are stored as one 448-row operand, slice q in rows 64 q .. 64 q + 63, so
-// that one MMA of N = 64 c multiplies A's slice p by c consecutive slices
-// q0 .. q0 + c - 1 into the c consecutive levels p + q0 ..: the 28 products
-// of a step take 10 MMAs of N up to 256 rather than 28 of N = 64 (the same
-// tensor work, in fewer instructions for the one issuing thread). Every wait
-// has an iteration limit. The epilogue reads the seven levels with
-// tcgen05.ld, two warps per lane quarter (a column half each), joins them in
-// FP64 and stores (or adds) the rows in range.
+// two TMA bulk copies (A's S slices, 4 KB each; B's, 2 KB each), four stages
+// in flight, and when they have landed issues the step's tcgen05.mma
+// kind::f16 into the level accumulators (tensor-memory columns 64 d ..
+// 64 d + 63 of 512) and commits them to the stage's "empty" mbarrier. B's
+// slices are stored as one operand of 64 S rows, slice q in rows 64 q ..
+// 64 q + 63, so that one MMA of N = 64 c multiplies A's slice p by c
+// consecutive slices q0 .. q0 + c - 1 into the c consecutive levels
+// p + q0 ..: the 28 (36) products of a step take 10 (12) MMAs of N up to 256
+// (the same tensor work, in fewer instructions for the one issuing thread).
+// Every wait has an iteration limit. The epilogue reads the levels with
+// tcgen05.ld, two warps per lane quarter (a column half each), joins them
+// and stores (or adds) the rows in range.
+#include <climits>
 #include <cstdint>
 
 #include "profile.cuh"
@@ -42,17 +60,18 @@
 namespace sl3dgpu {
 namespace {
 
-constexpr int kSlices = kTc64Slices;
 constexpr int kTileN = kTc64TileN;
 constexpr int kStages = 4;
 constexpr int kThreads = 256;  // eight warps: two per tensor-memory lane quarter in the epilogue
 constexpr int kATile = kTcTileM * kTcTileK;  // BF16 values of one slice of an A tile: 2048 (4 KB)
 constexpr int kBTile = kTileN * kTcTileK;    // of a B tile: 1024 (2 KB)
-constexpr int kBRows = kSlices * kTileN;     // B's slices as one operand of 448 rows
 constexpr int kBSlice = kTileN * 8;          // BF16 offset of the next slice's rows (8 row groups of 64)
-constexpr uint32_t kTmemColumns = 512;       // 7 levels x 64 columns, rounded up to a power of two
+constexpr uint32_t kTmemColumns = 512;       // up to 8 levels x 64 columns
+constexpr int kNonFinite = INT_MIN;           // the exponent of a column that holds an infinity or a NaN
 
-static_assert(kSlices * kTileN <= static_cast<int>(kTmemColumns), "the levels fit in tensor memory");
+static_assert(kTc64Slices * kTileN <= static_cast<int>(kTmemColumns) &&
+                  kTc64SlicesFull * kTileN <= static_cast<int>(kTmemColumns),
+              "the levels fit in tensor memory");
 
 // Instruction descriptor of kind::f16: FP32 accumulator, BF16 A and B, both
 // K-major, N and M.
@@ -70,24 +89,31 @@ __device__ inline uint32_t Bf16Bits(int integer) { return __float_as_uint(static
 __device__ inline int ExponentAbove(unsigned long long magnitudeBits) {
   if (magnitudeBits == 0) return 0;
   const int biased = static_cast<int>(magnitudeBits >> 52);
+  if (biased == 0x7FF) return kNonFinite;
   return biased == 0 ? -1022 : biased - 1022;
 }
 
-// v (|v| < 2^e) as kSlices balanced base-2^7 digits of round(v 2^{49 - e}),
-// packed as BF16 bits.
-__device__ inline void Split(double v, int e, uint32_t (&s)[kSlices]) {
+// v (|v| < 2^e) as S balanced base-2^7 digits of round(v 2^{7 S - e}),
+// packed as BF16 bits. (A non-finite column's digits are arbitrary: its
+// outputs do not use them.)
+template <int S>
+__device__ inline void Split(double v, int e, uint32_t (&s)[S]) {
   const unsigned long long bits = static_cast<unsigned long long>(__double_as_longlong(v));
   const int biased = static_cast<int>((bits >> 52) & 0x7FF);
   const long long mantissa = static_cast<long long>(bits & ((1ULL << 52) - 1)) | (biased ? (1LL << 52) : 0LL);
-  // v = mantissa 2^{E - 52}, E <= e - 1, so X = mantissa 2^{E - e - 3}: a
-  // right shift by t >= 4, rounded to nearest
+  // v = mantissa 2^{E - 52}, E <= e - 1, so X = mantissa 2^{E - e + 7 S - 52}:
+  // a right shift by t, rounded to nearest, or a left one by at most 3 (S = 8)
   const int E = biased ? biased - 1023 : -1022;
-  const int t = e - E + 3;
+  const int t = e - E + 52 - 7 * S;
   long long X = 0;
-  if (t < 63) X = (mantissa + (1LL << (t - 1))) >> t;
+  if (7 * S < 53 || t > 0) {
+    if (t < 63) X = (mantissa + (1LL << (t - 1))) >> t;
+  } else {
+    X = mantissa << min(-t, 3);
+  }
   if (bits >> 63) X = -X;
 #pragma unroll
-  for (int p = kSlices - 1; p > 0; --p) {
+  for (int p = S - 1; p > 0; --p) {
     int r = static_cast<int>(X & 127);
     if (r >= 64) r -= 128;
     s[p] = Bf16Bits(r);
@@ -96,7 +122,7 @@ __device__ inline void Split(double v, int e, uint32_t (&s)[kSlices]) {
   s[0] = Bf16Bits(static_cast<int>(X));
 }
 
-// (H 2^28 + L) 2^(scale - 56) as a double, rounded to nearest even, by
+// (H 2^28 + L) 2^scale as a double, rounded to nearest even, by
 // integer arithmetic (the exact 128-bit integer's top 53 bits and its
 // exponent written into the bits); values outside the normal range take the
 // slow path through ldexp.
@@ -109,7 +135,7 @@ __device__ inline double JoinToDouble(long long H, long long L, int scale) {
   const int bits = top ? 128 - __clzll(top) : 64 - __clzll(low);  // the integer's bit length
   const int shift = bits - 53;
   unsigned long long mantissa;
-  int exponent = bits - 1 + scale - 56;
+  int exponent = bits - 1 + scale;
   if (shift > 0) {
     const unsigned __int128 q = m >> shift;
     const unsigned __int128 rem = m - (q << shift), half = static_cast<unsigned __int128>(1) << (shift - 1);
@@ -140,9 +166,10 @@ __device__ inline int Tile16Index(int row, int k, int rows) {
 
 // Eight consecutive-k slices of one row (s[q][p]: value q, slice p) stored as
 // one 16-byte core-matrix row per slice.
-__device__ inline void StoreSlices(uint16_t* tile, int sliceStride, int at, const uint32_t (&s)[8][kSlices]) {
+template <int S>
+__device__ inline void StoreSlices(uint16_t* tile, int sliceStride, int at, const uint32_t (&s)[8][S]) {
 #pragma unroll
-  for (int p = 0; p < kSlices; ++p) {
+  for (int p = 0; p < S; ++p) {
     uint4 v;
     v.x = s[0][p] | (s[1][p] << 16);
     v.y = s[2][p] | (s[3][p] << 16);
@@ -150,6 +177,16 @@ __device__ inline void StoreSlices(uint16_t* tile, int sliceStride, int at, cons
     v.w = s[6][p] | (s[7][p] << 16);
     *reinterpret_cast<uint4*>(tile + p * sliceStride + at) = v;
   }
+}
+
+// One output as the FP64 units sum it, for a column holding an infinity or a
+// NaN.
+__device__ __noinline__ double PlainSum(const GemmItem& g, const double* table, const double* B, int i, int n) {
+  double sum = 0.0;
+  for (int k = 0; k < g.K; ++k)
+    sum = fma(table[g.a + static_cast<long long>(i) * g.sAi + static_cast<long long>(k) * g.sAk],
+              B[g.b + static_cast<long long>(k) * g.ldb + n], sum);
+  return sum;
 }
 
 // Row exponents of A, one thread per (item, row): the maximum over the
@@ -168,6 +205,7 @@ __global__ void RowExpKernel(const GemmItem* items, const Tc64Item* tcItems, con
 }
 
 // A's panel: one thread per (item, tile, 8-deep K group, row).
+template <int S>
 __global__ void PanelA64Kernel(const GemmItem* items, const Tc64Item* tcItems, const double* table,
                                const int* rowExp, uint16_t* panels) {
   const GemmItem g = items[blockIdx.y];
@@ -182,16 +220,16 @@ __global__ void PanelA64Kernel(const GemmItem* items, const Tc64Item* tcItems, c
     const int ks = static_cast<int>(tile % it.kSteps), mt = static_cast<int>(tile / it.kSteps);
     const int i = mt * kTcTileM + r, k0 = ks * kTcTileK + 8 * kg;
     const int e = i < g.M ? rowExp[it.rowExp + i] : 0;
-    uint32_t s[8][kSlices];
+    uint32_t s[8][S];
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
       const int k = k0 + q;
       const double v = (i < g.M && k < g.K) ? table[g.a + static_cast<long long>(i) * g.sAi +
                                                     static_cast<long long>(k) * g.sAk]
                                             : 0.0;
-      Split(v, e, s[q]);
+      Split<S>(v, e, s[q]);
     }
-    StoreSlices(panels + it.aPanel + tile * kSlices * kATile, kATile, Tile16Index(r, 8 * kg, kTcTileM), s);
+    StoreSlices<S>(panels + (it.aPanel + tile) * S * kATile, kATile, Tile16Index(r, 8 * kg, kTcTileM), s);
   }
 }
 
@@ -202,6 +240,7 @@ __global__ void PanelA64Kernel(const GemmItem* items, const Tc64Item* tcItems, c
 // consecutive columns and its stores of one slice 512 contiguous bytes.
 constexpr int kPackThreads = 256, kPackLanes = kPackThreads / kTileN;
 
+template <int S>
 __global__ void __launch_bounds__(kPackThreads) PackB64Kernel(const Tc64Item* tcItems, const double* B, int* colExp,
                                                               uint16_t* packed) {
   const Tc64Item it = tcItems[blockIdx.y];
@@ -221,24 +260,28 @@ __global__ void __launch_bounds__(kPackThreads) PackB64Kernel(const Tc64Item* tc
   for (int q = 0; q < kPackLanes; ++q) mx = max(mx, largest[q][nn]);
   const int e = ExponentAbove(mx);
   if (lane == 0 && n < it.N) colExp[it.colExp + n] = e;
-  uint16_t* base = packed + it.bPack + static_cast<long long>(nt) * it.kSteps * kSlices * kBTile;
+  uint16_t* base = packed + (it.bPack + static_cast<long long>(nt) * it.kSteps) * S * kBTile;
   for (int group = lane; group < 2 * it.kSteps; group += kPackLanes) {
     const int ks = group / 2, kg = group % 2, k0 = 8 * group;
-    uint32_t s[8][kSlices];
+    uint32_t s[8][S];
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
       const int k = k0 + q;
       const double v = (n < it.N && k < it.K) ? col[static_cast<long long>(k) * it.ldb] : 0.0;
-      Split(v, e, s[q]);
+      Split<S>(v, e, s[q]);
     }
-    StoreSlices(base + static_cast<long long>(ks) * kSlices * kBTile, kBSlice, Tile16Index(nn, 8 * kg, kBRows), s);
+    StoreSlices<S>(base + static_cast<long long>(ks) * S * kBTile, kBSlice, Tile16Index(nn, 8 * kg, S * kTileN), s);
   }
 }
 
-__global__ void __launch_bounds__(kThreads) TcGemm64Kernel(const Tc64Item* tcItems, const uint16_t* panels,
-                                                           const uint16_t* packed, const int* rowExp,
-                                                           const int* colExp, double* C, bool accumulate,
-                                                           int* errorFlag) {
+template <int S>
+__global__ void __launch_bounds__(kThreads) TcGemm64Kernel(const GemmItem* items, const Tc64Item* tcItems,
+                                                           const double* table, const double* B,
+                                                           const uint16_t* panels, const uint16_t* packed,
+                                                           const int* rowExp, const int* colExp, double* C,
+                                                           bool accumulate, int* errorFlag) {
+  constexpr int kSlices = S;
+  constexpr int kBRows = kSlices * kTileN;  // B's slices as one operand
   const Tc64Item it = tcItems[blockIdx.z];
   const int nt = blockIdx.x, mt = blockIdx.y;
   if (mt >= it.mTiles || nt >= it.nTiles) return;  // the whole CTA, before any tensor-memory work
@@ -253,7 +296,9 @@ __global__ void __launch_bounds__(kThreads) TcGemm64Kernel(const Tc64Item* tcIte
   uint64_t* empty = full + kStages;
   uint32_t* tmemSlot = reinterpret_cast<uint32_t*>(empty + kStages);
   __shared__ int okShared;
-  __shared__ double rowsOut[kThreads / 32][32][17];  // each warp's 32 x 16 block, padded
+  // the epilogue's staging, each warp's 32 x 16 block padded, in the stages'
+  // memory (every MMA has read them by then)
+  auto rowsOut = reinterpret_cast<double (*)[32][17]>(tc64Smem);
   const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
 
   if (warp == 0) {
@@ -275,10 +320,11 @@ __global__ void __launch_bounds__(kThreads) TcGemm64Kernel(const Tc64Item* tcIte
   const uint32_t tmem = *tmemSlot;
 
   if (tid == 0) {
-    const uint16_t* aSrc = panels + it.aPanel + static_cast<long long>(mt) * it.kSteps * kSlices * kATile;
-    const uint16_t* bSrc = packed + it.bPack + static_cast<long long>(nt) * it.kSteps * kSlices * kBTile;
+    const uint16_t* aSrc = panels + (it.aPanel + static_cast<long long>(mt) * it.kSteps) * kSlices * kATile;
+    const uint16_t* bSrc = packed + (it.bPack + static_cast<long long>(nt) * it.kSteps) * kSlices * kBTile;
     uint32_t phaseFull[kStages] = {0, 0, 0, 0}, phaseEmpty[kStages] = {0, 0, 0, 0};
     bool ok = true;
+    int issued = 0, landed = 0;  // steps whose copies were started, and waited for
     auto issue = [&](int ks) {
       const int buf = ks % kStages;
       if (ks >= kStages) {
@@ -299,6 +345,7 @@ __global__ void __launch_bounds__(kThreads) TcGemm64Kernel(const Tc64Item* tcIte
               SmemAddr(sB + buf * kSlices * kBTile)),
           "l"(bSrc + static_cast<long long>(ks) * kSlices * kBTile), "r"(bBytes), "r"(bar)
           : "memory");
+      ++issued;
     };
     for (int ks = 0; ks < min(kStages - 1, it.kSteps); ++ks) issue(ks);
     for (int ks = 0; ks < it.kSteps && ok; ++ks) {
@@ -308,6 +355,7 @@ __global__ void __launch_bounds__(kThreads) TcGemm64Kernel(const Tc64Item* tcIte
       ok = WaitParity(SmemAddr(full + buf), phaseFull[buf]);
       phaseFull[buf] ^= 1u;
       if (!ok) break;
+      ++landed;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t aBase = SmemAddr(sA + buf * kSlices * kATile);
       const uint32_t bBase = SmemAddr(sB + buf * kSlices * kBTile);
@@ -339,15 +387,20 @@ __global__ void __launch_bounds__(kThreads) TcGemm64Kernel(const Tc64Item* tcIte
       const int last = (it.kSteps - 1) % kStages;
       ok = WaitParity(SmemAddr(empty + last), phaseEmpty[last]);
     }
+    // having given up, wait (bounded) for the copies still in flight
+    if (!ok)
+      for (int ks = landed; ks < issued; ++ks)
+        WaitParity(SmemAddr(full + ks % kStages), phaseFull[ks % kStages]);
     okShared = ok ? 1 : 0;
     if (!ok) atomicExch(errorFlag, 1);
   }
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  if (okShared) {
+  const bool good = okShared != 0;
+  {
     // Epilogue: this warp's lane quarter (32 rows) and column half, 16
-    // columns at a time, the seven levels joined as integers and rounded
-    // once to FP64.
+    // columns at a time, the levels joined as integers and rounded once to
+    // FP64.
     const int quarter = warp % 4, half = warp / 4;
     const int i = i0 + 32 * quarter + lane;
     const int e = i < it.M ? rowExp[it.rowExp + i] : 0;
@@ -377,11 +430,24 @@ __global__ void __launch_bounds__(kThreads) TcGemm64Kernel(const Tc64Item* tcIte
           long long acc[kSlices];
 #pragma unroll
           for (int d = 0; d < kSlices; ++d) acc[d] = __float2int_rn(__uint_as_float(r[d][q]));
-          const long long H = (acc[0] << 14) + (acc[1] << 7) + acc[2];
-          const long long L = (acc[3] << 21) + (acc[4] << 14) + (acc[5] << 7) + acc[6];
-          v = JoinToDouble(H, L, e + colExp[it.colExp + n0 + n]);
+          long long H = 0, L = 0;
+#pragma unroll
+          for (int d = 0; d < kSlices - 4; ++d) H += acc[d] << (7 * (kSlices - 5 - d));
+#pragma unroll
+          for (int d = kSlices - 4; d < kSlices; ++d) L += acc[d] << (7 * (kSlices - 1 - d));
+          v = JoinToDouble(H, L, e + colExp[it.colExp + n0 + n] - 7 * (kSlices + 1));
         }
         rowsOut[warp][lane][q] = v;
+      }
+      // a non-finite column among these 16 (or a wait that gave up): rare
+      const bool marked = lane < 16 && c0 + lane < nCols && colExp[it.colExp + n0 + c0 + lane] == kNonFinite;
+      const unsigned columns = __ballot_sync(0xffffffffu, marked);
+      if (!good || columns != 0) {
+        for (int q = 0; q < 16; ++q)
+          if (!good)
+            rowsOut[warp][lane][q] = __longlong_as_double(0x7FF8000000000000LL);
+          else if (((columns >> q) & 1u) && i < it.M)
+            rowsOut[warp][lane][q] = PlainSum(items[blockIdx.z], table, B, i, n0 + c0 + q);
       }
       __syncwarp();
       const int n = c0 + (lane & 15);
@@ -410,36 +476,56 @@ __global__ void __launch_bounds__(kThreads) TcGemm64Kernel(const Tc64Item* tcIte
 
 }  // namespace
 
-void LaunchPanelA64(const GemmItem* items, const Tc64Item* tcItems, int count, int maxM, int maxATiles,
-                    const double* table, int* rowExp, uint16_t* panels, cudaStream_t stream) {
-  if (count == 0) return;
-  RowExpKernel<<<dim3(static_cast<unsigned>((maxM + 127) / 128), count), 128, 0, stream>>>(items, tcItems, table,
-                                                                                          rowExp);
-  const long long perItem = static_cast<long long>(maxATiles) * 2 * kTcTileM;
-  const unsigned blocks = static_cast<unsigned>(std::min<long long>((perItem + 255) / 256, 4096));
-  PanelA64Kernel<<<dim3(blocks, count), 256, 0, stream>>>(items, tcItems, table, rowExp, panels);
-}
-
-void LaunchPackB64(const Tc64Item* tcItems, int count, int maxNTiles, const double* B, int* colExp,
-                   uint16_t* packed, cudaStream_t stream) {
-  if (count == 0 || maxNTiles == 0) return;
-  PackB64Kernel<<<dim3(static_cast<unsigned>(maxNTiles), count), kPackThreads, 0, stream>>>(tcItems, B, colExp,
-                                                                                           packed);
-}
-
-int RunGemm64Tc(const Tc64Item* tcItems, int count, int maxMTiles, int maxNTiles, const uint16_t* panels,
-                const uint16_t* packed, const int* rowExp, const int* colExp, double* C, bool accumulate,
-                int* errorFlag, cudaStream_t stream) {
-  if (count == 0 || maxMTiles == 0 || maxNTiles == 0) return SL3DGPU_OK;
-  constexpr size_t smem = static_cast<size_t>(kStages) * kSlices * (kATile + kBTile) * sizeof(uint16_t) +
+namespace {
+template <int S>
+int Run(const GemmItem* items, const Tc64Item* tcItems, int count, int maxMTiles, int maxNTiles, const double* table,
+        const Tc64Panel& panel, const double* B, uint16_t* packed, int* colExp, double* C, bool accumulate,
+        int* errorFlag, cudaStream_t stream) {
+  constexpr size_t smem = static_cast<size_t>(kStages) * S * (kATile + kBTile) * sizeof(uint16_t) +
                           2 * kStages * sizeof(uint64_t) + 16;
-  static_assert(smem <= 227 * 1024, "the stages fit in shared memory");
-  SL3D_CUDA(AllowDynamicSmem(TcGemm64Kernel));
+  static_assert(smem <= 226 * 1024, "the stages fit in shared memory");
+  static_assert(smem >= kThreads / 32 * 32 * 17 * sizeof(double), "the epilogue's staging fits in the stages");
+  SL3D_CUDA(AllowDynamicSmem(TcGemm64Kernel<S>));
   dim3 grid(static_cast<unsigned>(maxNTiles), static_cast<unsigned>(maxMTiles), static_cast<unsigned>(count));
-  TcGemm64Kernel<<<grid, kThreads, smem, stream>>>(tcItems, panels, packed, rowExp, colExp, C, accumulate,
-                                                   errorFlag);
+  TcGemm64Kernel<S><<<grid, kThreads, smem, stream>>>(items, tcItems, table, B, panel.slices, packed, panel.rowExp,
+                                                      colExp, C, accumulate, errorFlag);
   SL3D_CHECK_LAUNCH();
   return SL3DGPU_OK;
+}
+}  // namespace
+
+void LaunchPanelA64(int slices, const GemmItem* items, const Tc64Item* tcItems, int count, int maxM, int maxATiles,
+                    const double* table, const Tc64Panel& panel, cudaStream_t stream) {
+  if (count == 0) return;
+  RowExpKernel<<<dim3(static_cast<unsigned>((maxM + 127) / 128), count), 128, 0, stream>>>(items, tcItems, table,
+                                                                                          panel.rowExp);
+  const long long perItem = static_cast<long long>(maxATiles) * 2 * kTcTileM;
+  const dim3 grid(static_cast<unsigned>(std::min<long long>((perItem + 255) / 256, 4096)), count);
+  if (slices == kTc64SlicesFull)
+    PanelA64Kernel<kTc64SlicesFull><<<grid, 256, 0, stream>>>(items, tcItems, table, panel.rowExp, panel.slices);
+  else
+    PanelA64Kernel<kTc64Slices><<<grid, 256, 0, stream>>>(items, tcItems, table, panel.rowExp, panel.slices);
+}
+
+void LaunchPackB64(int slices, const Tc64Item* tcItems, int count, int maxNTiles, const double* B, int* colExp,
+                   uint16_t* packed, cudaStream_t stream) {
+  if (count == 0 || maxNTiles == 0) return;
+  const dim3 grid(static_cast<unsigned>(maxNTiles), count);
+  if (slices == kTc64SlicesFull)
+    PackB64Kernel<kTc64SlicesFull><<<grid, kPackThreads, 0, stream>>>(tcItems, B, colExp, packed);
+  else
+    PackB64Kernel<kTc64Slices><<<grid, kPackThreads, 0, stream>>>(tcItems, B, colExp, packed);
+}
+
+int RunGemm64Tc(int slices, const GemmItem* items, const Tc64Item* tcItems, int count, int maxMTiles, int maxNTiles,
+                const double* table, const Tc64Panel& panel, const double* B, uint16_t* packed, int* colExp, double* C,
+                bool accumulate, int* errorFlag, cudaStream_t stream) {
+  if (count == 0 || maxMTiles == 0 || maxNTiles == 0) return SL3DGPU_OK;
+  return slices == kTc64SlicesFull
+             ? Run<kTc64SlicesFull>(items, tcItems, count, maxMTiles, maxNTiles, table, panel, B, packed, colExp, C,
+                                    accumulate, errorFlag, stream)
+             : Run<kTc64Slices>(items, tcItems, count, maxMTiles, maxNTiles, table, panel, B, packed, colExp, C,
+                                accumulate, errorFlag, stream);
 }
 
 }  // namespace sl3dgpu
