@@ -1,5 +1,8 @@
 // Error text, version and the device-memory helpers of the sl3dgpu C ABI.
+#include <mutex>
+#include <set>
 #include <string>
+#include <utility>
 
 #include "common.cuh"
 
@@ -10,6 +13,27 @@ thread_local std::string lastError;
 }
 
 void SetError(const std::string& text) { lastError = text; }
+
+cudaError_t AllowDynamicSmemOnce(const void* kernel) {
+  static std::mutex lock;
+  static std::set<std::pair<int, const void*>> done;  // (device, kernel)
+  int device = 0;
+  if (const cudaError_t e = cudaGetDevice(&device); e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> guard(lock);
+  if (done.count({device, kernel}) != 0) return cudaSuccess;
+  int optin = 0;
+  if (const cudaError_t e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+      e != cudaSuccess)
+    return e;
+  cudaFuncAttributes a{};
+  if (const cudaError_t e = cudaFuncGetAttributes(&a, kernel); e != cudaSuccess) return e;
+  if (const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 optin - static_cast<int>(a.sharedSizeBytes));
+      e != cudaSuccess)
+    return e;
+  done.insert({device, kernel});
+  return cudaSuccess;
+}
 
 }  // namespace sl3dgpu
 

@@ -60,19 +60,12 @@ inline cudaError_t ZeroIn(void* dst, size_t bytes) {
 // leaves beside its static shared memory. The attribute is global to the
 // function, so it takes one value for every caller: host threads driving
 // problems of different sizes would otherwise race between setting it and
-// launching. Occupancy follows each launch's actual dynamic size.
+// launching. Occupancy follows each launch's actual dynamic size. Set once a
+// kernel and device: setting it at every launch cost two runtime calls each.
+cudaError_t AllowDynamicSmemOnce(const void* kernel);
 template <class F>
 inline cudaError_t AllowDynamicSmem(F* kernel) {
-  static const int optin = [] {
-    int device = 0, bytes = 0;
-    cudaGetDevice(&device);
-    cudaDeviceGetAttribute(&bytes, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
-    return bytes;
-  }();
-  cudaFuncAttributes a{};
-  if (const cudaError_t e = cudaFuncGetAttributes(&a, kernel); e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              optin - static_cast<int>(a.sharedSizeBytes));
+  return AllowDynamicSmemOnce(reinterpret_cast<const void*>(kernel));
 }
 
 constexpr int kWarp = 32;
