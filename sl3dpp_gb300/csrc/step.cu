@@ -30,7 +30,6 @@
 #include <cstring>
 #include <limits>
 #include <memory>
-#include <mutex>
 #include <string>
 #include <thread>
 #include <tuple>
@@ -183,6 +182,11 @@ class Viscoelastic3DGpu {
   std::vector<CorrectionGraph> correctionGraphs;
   Dev<CorrectionControl> correctionControl;
   bool useGraphs = true;  // SL3DGPU_NO_GRAPHS=1 keeps the loop on the host
+  // Operators driven from several host threads keep the loop on the host:
+  // building these graphs (conditional nodes) beside other threads' launches
+  // crashed in the driver's cudaGraphDestroy now and then, under a lock
+  // around every graph call too; the ensemble is as fast either way.
+  bool manyThreads = false;
   std::vector<long long> CorrectionKey(const Flavour& f) const;
   int CorrectionGraphFor(const Flavour& f, CorrectionGraph** out);
   int CaptureCorrectionBody(const Flavour& f, cudaGraphConditionalHandle handle);
@@ -2207,7 +2211,7 @@ int Viscoelastic3DGpu::Correct(const Flavour& f, double tolerance, sl3dgpu_step_
   for (; iteration < options.max_iterations; ++iteration) {
     // after the first pass (and the warm start's decision) the loop runs on
     // the device, as a CUDA graph, when it can
-    if (iteration >= 1 && !triedGraph && useGraphs && !prof::TimingOn()) {
+    if (iteration >= 1 && !triedGraph && useGraphs && !manyThreads && !prof::TimingOn()) {
       triedGraph = true;
       if (CorrectionGraphFor(f, &graph) == SL3DGPU_OK) break;
       graph = nullptr;
@@ -4344,6 +4348,8 @@ extern "C" int sl3dgpu_v3d_run_many(int count, sl3dgpu_v3d* const* ops, sl3dgpu_
   SL3D_CUDA(cudaGetDevice(&device));
   const int cores = std::max(1, static_cast<int>(std::thread::hardware_concurrency()));
   const int workers = std::max(1, std::min(count, threads > 0 ? threads : cores));
+  for (int i = 0; i < count; ++i)
+    if (ops[i] != nullptr) ops[i]->op.manyThreads = workers > 1;
   std::vector<std::string> errors(count);
   std::atomic<int> next{0};
   auto work = [&] {
@@ -4358,6 +4364,8 @@ extern "C" int sl3dgpu_v3d_run_many(int count, sl3dgpu_v3d* const* ops, sl3dgpu_
   for (int w = 1; w < workers; ++w) pool.emplace_back(work);
   work();
   for (auto& t : pool) t.join();
+  for (int i = 0; i < count; ++i)
+    if (ops[i] != nullptr) ops[i]->op.manyThreads = false;
   for (int i = 0; i < count; ++i)
     if (statuses[i] != SL3DGPU_OK) {
       SetError("v3d: run " + std::to_string(i) + ": " + errors[i]);
