@@ -59,6 +59,7 @@
 #include "step_kernels.cuh"
 #include "systems.cuh"
 #include "sealevel.cuh"
+#include "sht.cuh"
 
 namespace sl3dgpu {
 namespace {
@@ -207,7 +208,7 @@ struct SleRun {
   // field = Synthesise(f_l coefficients + add)
   int SynthesiseScaled(const double* f, const double* coeffs, double* field, const double* add = nullptr) {
     SL3D_TRY(ScaleDegrees(f, coeffs, add, 1.0, scaledLm.p));
-    return sl3dgpu_synthesise_batch(grid, scaledLm.p, 1, field, stream);
+    return SynthesiseFixed(grid, scaledLm.p, field, stream);
   }
   // out = a + c b (complex coefficients)
   int Axpy(const double* a, const double* b, double c, double* out) {
@@ -664,7 +665,7 @@ int PrepareSolve(SleWorkspace& ws, sl3dgpu_grid* grid, const sl3dgpu_sle_body* b
     // from degree 1, the l's without degree 0
     auto channel = [&](const double* field, const double* hc, const double* kc, const double* lc, int first,
                        double* degree0) -> int {
-      SL3D_TRY(sl3dgpu_expand_batch(grid, field, 1, scratch.p, s));
+      SL3D_TRY(ExpandFixed(grid, field, scratch.p, s));
       std::vector<double> hf(L + 1, 0.0), kf(L + 1, 0.0), lf(L + 1, 0.0);
       for (int l = first; l <= L; ++l) {
         hf[l] = hc[l];
@@ -690,7 +691,7 @@ int PrepareSolve(SleWorkspace& ws, sl3dgpu_grid* grid, const sl3dgpu_sle_body* b
     SL3D_TRY(run.ScaleDegrees(zeros.data(), staticSlc.p, staticSlc.p, -1.0, staticSlc.p));
     if (hasTide) SL3D_TRY(run.Axpy(staticSlc.p, forcing->tide, -1.0 / g, staticSlc.p));
     if (hasLayer) {
-      SL3D_TRY(sl3dgpu_expand_batch(grid, forcing->solid_surface_change, 1, scratch.p, s));
+      SL3D_TRY(ExpandFixed(grid, forcing->solid_surface_change, scratch.p, s));
       SL3D_TRY(run.Axpy(staticSlc.p, scratch.p, -1.0, staticSlc.p));
     }
   }
@@ -787,7 +788,7 @@ int SynthesisePatched(SleWorkspace& ws, bool patch, const double* f, bool factor
     RotationPatchKernel<<<1, 32, 0, s>>>(ws.rotation.p, run.loadLm.p, run.scaledLm.p, ws.omega.p, mode);
     SL3D_CHECK_LAUNCH();
   }
-  return sl3dgpu_synthesise_batch(run.grid, run.scaledLm.p, 1, field, s);
+  return SynthesiseFixed(run.grid, run.scaledLm.p, field, s);
 }
 
 // -- the nonlinear solve's pointwise work (src/SeaLevel.cpp:1098-1217) ----------------------------------
@@ -940,7 +941,7 @@ int SeaLevelSolve(SleWorkspace& ws, sl3dgpu_grid* grid, const sl3dgpu_sle_body* 
   // the toroidal potential is carried, whatever else is solved (:561-563)
   if (toroidal_potential != nullptr) {
     if (forcing->toroidal_response != nullptr)
-      SL3D_TRY(sl3dgpu_synthesise_batch(grid, forcing->toroidal_response, 1, toroidal_potential, s));
+      SL3D_TRY(SynthesiseFixed(grid, forcing->toroidal_response, toroidal_potential, s));
     else
       SL3D_TRY(zero(toroidal_potential));
   }
@@ -979,7 +980,7 @@ int SeaLevelSolve(SleWorkspace& ws, sl3dgpu_grid* grid, const sl3dgpu_sle_body* 
   // the seed: sigma + rho_w C s_mean, expanded
   SeedKernel<<<fb, 256, 0, s>>>(run.fieldSize, directData.p, ocean, water_density * meanSlc, run.seeded.p);
   SL3D_CHECK_LAUNCH();
-  SL3D_TRY(sl3dgpu_expand_batch(grid, run.seeded.p, 1, run.loadLm.p, s));
+  SL3D_TRY(ExpandFixed(grid, run.seeded.p, run.loadLm.p, s));
 
   SL3D_TRY(ws.ResetMixer(anderson_memory, s));
   LoadMixer& mixer = ws.mixer;
@@ -1015,7 +1016,7 @@ int SeaLevelSolve(SleWorkspace& ws, sl3dgpu_grid* grid, const sl3dgpu_sle_body* 
       }
     }
     havePrev = true;
-    SL3D_TRY(sl3dgpu_expand_batch(grid, run.newLoad.p, 1, run.newLoadLm.p, s));
+    SL3D_TRY(ExpandFixed(grid, run.newLoad.p, run.newLoadLm.p, s));
     SL3D_TRY(mixer.Update(run.loadLm.p, run.newLoadLm.p, nc, s));
     ++count;
   }
@@ -1034,7 +1035,7 @@ int SeaLevelSolve(SleWorkspace& ws, sl3dgpu_grid* grid, const sl3dgpu_sle_body* 
                                tangential_potential, 3));
   // TotalLoadCoefficients (src/Evolution3D.cpp:237-249): the direct loads and
   // the ocean's, rho_w C S of the last sea level change
-  if (total_load != nullptr) SL3D_TRY(sl3dgpu_expand_batch(grid, run.newLoad.p, 1, total_load, s));
+  if (total_load != nullptr) SL3D_TRY(ExpandFixed(grid, run.newLoad.p, total_load, s));
   double tail[4];
   SL3D_CUDA(cudaMemcpyAsync(tail, ws.shift.p, sizeof(double), cudaMemcpyDeviceToHost, s));
   SL3D_CUDA(cudaMemcpyAsync(tail + 1, ws.omega.p, 3 * sizeof(double), cudaMemcpyDeviceToHost, s));
@@ -1122,7 +1123,7 @@ int SeaLevelSolveNonlinear(SleWorkspace& ws, sl3dgpu_grid* grid, const sl3dgpu_s
   while (count < max_iterations) {
     BudgetLoadKernel<<<fb, 256, 0, s>>>(n, budget, ws.nlOcean.p, ws.nlChange.p, direct, run.newLoad.p);
     SL3D_CHECK_LAUNCH();
-    SL3D_TRY(sl3dgpu_expand_batch(grid, run.newLoad.p, 1, run.loadLm.p, s));
+    SL3D_TRY(ExpandFixed(grid, run.newLoad.p, run.loadLm.p, s));
     SL3D_TRY(SynthesisePatched(ws, su.rotating, ws.slcFactor.p, true, slcAdd, ws.nlLocal.p, 0));
     BudgetRingKernel<<<run.ntheta, kRingThreads, 0, s>>>(run.nphi, run.weights.p, budget, ws.nlOcean.p,
                                                          ws.nlLocal.p, dynamic, ws.nlRingUnbalanced.p,
@@ -1163,7 +1164,7 @@ int SeaLevelSolveNonlinear(SleWorkspace& ws, sl3dgpu_grid* grid, const sl3dgpu_s
                                tangential_potential, 3));
   if (toroidal_potential) {
     if (forcing->toroidal_response != nullptr)
-      SL3D_TRY(sl3dgpu_synthesise_batch(grid, forcing->toroidal_response, 1, toroidal_potential, s));
+      SL3D_TRY(SynthesiseFixed(grid, forcing->toroidal_response, toroidal_potential, s));
     else
       SL3D_CUDA(cudaMemsetAsync(toroidal_potential, 0, bytes, s));
   }
@@ -1177,7 +1178,7 @@ int SeaLevelSolveNonlinear(SleWorkspace& ws, sl3dgpu_grid* grid, const sl3dgpu_s
   if (load_coefficients) {
     BudgetLoadKernel<<<fb, 256, 0, s>>>(n, budget, ws.nlOcean.p, ws.nlChange.p, direct, run.newLoad.p);
     SL3D_CHECK_LAUNCH();
-    SL3D_TRY(sl3dgpu_expand_batch(grid, run.newLoad.p, 1, load_coefficients, s));
+    SL3D_TRY(ExpandFixed(grid, run.newLoad.p, load_coefficients, s));
   }
   double tail[4];
   SL3D_CUDA(cudaMemcpyAsync(tail, ws.shift.p, sizeof(double), cudaMemcpyDeviceToHost, s));

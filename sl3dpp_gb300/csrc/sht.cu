@@ -9,8 +9,10 @@
 //    c_lm = sum_j Lambda^N_lm(theta_j) G_m(theta_j).
 // The contraction is one dense matrix product per (spin, order) with the
 // batch's fields as columns, run here as a batched FP64 register-tiled GEMM;
-// the FFT is a mixed-radix (2, 3, 4, 5) Stockham transform in shared memory,
-// one warp per ring (warp-synchronous stages), several rings per CTA.
+// the FFT is a mixed-radix Stockham transform in shared memory, several rings
+// per CTA: FP64 values in block fixed point (ring_fixed.cu), in
+// double-float where the emulation was asked for (ring_df.cu), FP32 values
+// here, one warp per ring (warp-synchronous stages).
 #include <algorithm>
 #include <cstdlib>
 #include <cmath>
@@ -18,6 +20,8 @@
 #include <numeric>
 
 #include "profile.cuh"
+#include "ring_df.cuh"
+#include "ring_stages.cuh"
 #include "sht.cuh"
 #include "tc_gemm.cuh"
 
@@ -248,153 +252,6 @@ void LaunchNarrow(bool analysis, int maxM, int count, const GemmItem* items, con
 
 // -- FFT ---------------------------------------------------------------------------------
 
-template <class T2>
-struct Real;
-template <>
-struct Real<double2> {
-  using type = double;
-};
-template <>
-struct Real<float2> {
-  using type = float;
-};
-
-template <class T2>
-__device__ inline T2 Make(typename Real<T2>::type x, typename Real<T2>::type y) {
-  T2 v;
-  v.x = x;
-  v.y = y;
-  return v;
-}
-template <class T2>
-__device__ inline T2 Mul(T2 a, T2 b) {
-  return Make<T2>(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-template <class T2>
-__device__ inline T2 Add(T2 a, T2 b) {
-  return Make<T2>(a.x + b.x, a.y + b.y);
-}
-template <class T2>
-__device__ inline T2 Sub(T2 a, T2 b) {
-  return Make<T2>(a.x - b.x, a.y - b.y);
-}
-
-// A double-float value, hi + lo with |lo| <= ulp(hi) / 2 (about 48
-// significant bits): the FP64 ring transforms' arithmetic on the FP32 pipe
-// when the grid emulates FP64 (the FP64 pipe is GB300's slow one). Dekker's
-// and Knuth's error-free transformations -- TwoSum, FastTwoSum and the
-// FMA-based TwoProduct -- in their usual double-single forms: a sum's
-// error is bounded by about 2^-46 (|a| + |b|) (the "sloppy" addition, whose
-// bound is normwise, which is what a transform's error analysis uses), a
-// product's by about 2^-46 |a b|. The _rn intrinsics keep the compiler from
-// contracting the error terms into FMAs.
-struct Df {
-  float hi, lo;
-  __host__ __device__ constexpr Df() : hi(0.0f), lo(0.0f) {}
-  __host__ __device__ constexpr Df(float h, float l) : hi(h), lo(l) {}
-  // the nearest double-float of d (constant-folded for literal constants)
-  __host__ __device__ constexpr Df(double d)
-      : hi(static_cast<float>(d)), lo(static_cast<float>(d - static_cast<double>(static_cast<float>(d)))) {}
-  __host__ __device__ constexpr Df(int i) : Df(static_cast<double>(i)) {}
-  __device__ explicit operator double() const { return static_cast<double>(hi) + static_cast<double>(lo); }
-  __device__ explicit operator float() const { return __fadd_rn(hi, lo); }
-};
-struct Df2 {
-  Df x, y;
-};
-template <>
-struct Real<Df2> {
-  using type = Df;
-};
-
-// FastTwoSum of s and an error term e (|s| >= |e| or s = 0)
-__device__ inline Df Renormalise(float s, float e) {
-  const float h = __fadd_rn(s, e);
-  return Df(h, __fsub_rn(e, __fsub_rn(h, s)));
-}
-__device__ inline Df operator+(Df a, Df b) {
-  const float s = __fadd_rn(a.hi, b.hi);
-  const float bb = __fsub_rn(s, a.hi);
-  const float e = __fadd_rn(__fsub_rn(a.hi, __fsub_rn(s, bb)), __fsub_rn(b.hi, bb));  // TwoSum's error
-  return Renormalise(s, __fadd_rn(e, __fadd_rn(a.lo, b.lo)));
-}
-__device__ inline Df operator-(Df a) { return Df(-a.hi, -a.lo); }
-__device__ inline Df operator-(Df a, Df b) { return a + (-b); }
-__device__ inline Df operator*(Df a, Df b) {
-  const float p = __fmul_rn(a.hi, b.hi);
-  float e = __fmaf_rn(a.hi, b.hi, -p);  // TwoProduct's error
-  e = __fmaf_rn(a.hi, b.lo, e);
-  e = __fmaf_rn(a.lo, b.hi, e);
-  return Renormalise(p, e);
-}
-
-// A value of the storage type in the compute type, and back.
-template <class C2, class T2>
-__device__ inline C2 ToCompute(T2 v) {
-  if constexpr (std::is_same_v<C2, T2>)
-    return v;
-  else
-    return Make<C2>(typename Real<C2>::type(v.x), typename Real<C2>::type(v.y));
-}
-template <class T, class C>
-__device__ inline T ToStorage(C v) {
-  if constexpr (std::is_same_v<T, C>)
-    return v;
-  else
-    return static_cast<T>(v);
-}
-template <class T2, class C2>
-__device__ inline T2 ToStorage2(C2 v) {
-  if constexpr (std::is_same_v<T2, C2>)
-    return v;
-  else
-    return Make<T2>(ToStorage<typename Real<T2>::type>(v.x), ToStorage<typename Real<T2>::type>(v.y));
-}
-
-// The DFT of R values in registers, y_u = sum_q v_q e^{sign 2 pi i q u / R},
-// for the radices of the plans (2, 3, 4, 5), with the roots as constants.
-template <class T2, int R>
-__device__ inline void Butterfly(T2 (&v)[R], int sign) {
-  using T = typename Real<T2>::type;
-  auto I = [](T2 a) { return Make<T2>(-a.y, a.x); };  // i a
-  auto S = [](T k, T2 a) { return Make<T2>(k * a.x, k * a.y); };
-  const T sg = sign > 0 ? T(1) : T(-1);
-  if constexpr (R == 2) {
-    const T2 a = v[0], b = v[1];
-    v[0] = Add(a, b);
-    v[1] = Sub(a, b);
-  } else if constexpr (R == 3) {
-    const T2 t = Add(v[1], v[2]);
-    const T2 d = S(sg * T(0.86602540378443864676), Sub(v[1], v[2]));
-    const T2 a = Sub(v[0], S(T(0.5), t));
-    v[0] = Add(v[0], t);
-    v[1] = Add(a, I(d));
-    v[2] = Sub(a, I(d));
-  } else if constexpr (R == 4) {
-    const T2 a0 = Add(v[0], v[2]), a1 = Sub(v[0], v[2]);
-    const T2 b0 = Add(v[1], v[3]), b1 = S(sg, Sub(v[1], v[3]));
-    v[0] = Add(a0, b0);
-    v[1] = Add(a1, I(b1));
-    v[2] = Sub(a0, b0);
-    v[3] = Sub(a1, I(b1));
-  } else {
-    static_assert(R == 5, "radix");
-    const T c1 = T(0.30901699437494742410), c2 = T(-0.80901699437494742410);
-    const T s1 = T(0.95105651629515357212), s2 = T(0.58778525229247312917);
-    const T2 t1 = Add(v[1], v[4]), t2 = Add(v[2], v[3]);
-    const T2 d1 = Sub(v[1], v[4]), d2 = Sub(v[2], v[3]);
-    const T2 a1 = Add(v[0], Add(S(c1, t1), S(c2, t2)));
-    const T2 a2 = Add(v[0], Add(S(c2, t1), S(c1, t2)));
-    const T2 b1 = S(sg, Add(S(s1, d1), S(s2, d2)));
-    const T2 b2 = S(sg, Sub(S(s2, d1), S(s1, d2)));
-    v[0] = Add(v[0], Add(t1, t2));
-    v[1] = Add(a1, I(b1));
-    v[4] = Sub(a1, I(b1));
-    v[2] = Add(a2, I(b2));
-    v[3] = Sub(a2, I(b2));
-  }
-}
-
 // One Stockham stage of radix R over one ring, by one warp: butterfly idx
 // takes in[idx + q m] (q < R), twiddled by e^{sign 2 pi i q k stride / n}
 // (k = idx mod Ns; the exponent stays below n), and writes
@@ -591,17 +448,12 @@ size_t RingSmem(int n, int rings, int buffers) {
 // One CTA per (colatitude j, group of G consecutive fields p0..p0+G-1), one
 // warp per ring. The spectra [m][j][p] are read and written by the whole CTA
 // with the G fields of an order adjacent; the transforms run warp-synchronous.
-//
-// T2 is the values' type in memory, C2 the transform's arithmetic: the same
-// type, or double-float (Df2) for FP64 values under FP64 emulation.
-template <class T2, class C2, int R1, int R2>
+template <class T2, int R1, int R2>
 __global__ void __launch_bounds__(256, (R1 > 0 && sizeof(T2) == 8) ? 3 : 1)
     RingKernel(int mode, int lmax, int ntheta, int count, bool real, FftPlan plan, const T2* twGlobal,
                const double* weights, const T2* spectraIn, const void* fieldsIn,
                const typename Real<T2>::type* pointWeight, void* fieldsOut, T2* spectraOut) {
-  static_assert(sizeof(C2) == sizeof(T2), "the shared-memory layout is sized by the storage type");
   using T = typename Real<T2>::type;
-  using C = typename Real<C2>::type;
   extern __shared__ __align__(16) unsigned char ringSmem[];
   const int n = R1 > 0 ? R1 * R2 : plan.n;  // a constant in the two-stage form
   constexpr int buffers = R1 > 0 ? 1 : 2;
@@ -610,9 +462,9 @@ __global__ void __launch_bounds__(256, (R1 > 0 && sizeof(T2) == 8) ? 3 : 1)
   const long long ringStride = static_cast<long long>(buffers) * n + 1;
   const int G = blockDim.x / kWarp;
   const int warp = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
-  C2* tw = reinterpret_cast<C2*>(ringSmem);
-  C2* twB = tw + n;  // the two-stage form's stage-B twiddles
-  C2* bufs = twB + n;
+  T2* tw = reinterpret_cast<T2*>(ringSmem);
+  T2* twB = tw + n;  // the two-stage form's stage-B twiddles
+  T2* bufs = twB + n;
   // A real field's ring shares one complex transform with the next field's
   // (z = x + i y; Z_m = X_m + i Y_m, X_m = (Z_m + conj Z_{n-m}) / 2,
   // Y_m = (Z_m - conj Z_{n-m}) / 2i): a warp carries two real fields.
@@ -636,11 +488,11 @@ __global__ void __launch_bounds__(256, (R1 > 0 && sizeof(T2) == 8) ? 3 : 1)
           PrefetchL2(pointWeight + (static_cast<long long>(f) * ntheta + j) * n + k * (128 / sizeof(T)));
     }
   }
-  for (int e = threadIdx.x; e < n; e += blockDim.x) tw[e] = ToCompute<C2>(twGlobal[e]);
+  for (int e = threadIdx.x; e < n; e += blockDim.x) tw[e] = (twGlobal[e]);
   if constexpr (R1 > 0)
-    for (int e = threadIdx.x; e < n; e += blockDim.x) twB[e] = ToCompute<C2>(twGlobal[(e / R1) * (e % R1)]);
-  C2* a = bufs + ringStride * warp;  // this warp's ring
-  C2* b = buffers == 2 ? a + n : a;
+    for (int e = threadIdx.x; e < n; e += blockDim.x) twB[e] = (twGlobal[(e / R1) * (e % R1)]);
+  T2* a = bufs + ringStride * warp;  // this warp's ring
+  T2* b = buffers == 2 ? a + n : a;
   int at = 0;  // which of a, b holds the ring's current values
   // the rows of this warp's fields (the second of a real pair may not exist)
   const int f0 = p0 + perRing * warp, f1 = real ? f0 + 1 : f0;
@@ -649,22 +501,22 @@ __global__ void __launch_bounds__(256, (R1 > 0 && sizeof(T2) == 8) ? 3 : 1)
   const long long row1 = (static_cast<long long>(f1) * ntheta + j) * n;
   if (mode == kRingSynth || mode == kRingWeighted) {
     for (int e = threadIdx.x; e < G * n; e += blockDim.x)
-      bufs[ringStride * (e / n) + e % n] = Make<C2>(0, 0);
+      bufs[ringStride * (e / n) + e % n] = Make<T2>(0, 0);
     __syncthreads();
 #pragma unroll 4
     for (int e = threadIdx.x; e < mcount * rings; e += blockDim.x) {
       const int r = e % rings, mi = e / rings;
       const int m = real ? mi : mi - lmax;
       const long long at0 = (static_cast<long long>(mi) * ntheta + j) * count + p0 + perRing * r;
-      const C2 v = ToCompute<C2>(spectraIn[at0]);
-      C2* ring = bufs + ringStride * r;
+      const T2 v = (spectraIn[at0]);
+      T2* ring = bufs + ringStride * r;
       if (real) {
-        const C2 u = perRing * r + 1 < groups ? ToCompute<C2>(spectraIn[at0 + 1]) : Make<C2>(0, 0);
+        const T2 u = perRing * r + 1 < groups ? (spectraIn[at0 + 1]) : Make<T2>(0, 0);
         if (m == 0) {
-          ring[0] = Make<C2>(v.x, u.x);
+          ring[0] = Make<T2>(v.x, u.x);
         } else {
-          ring[m] = Make<C2>(v.x - u.y, v.y + u.x);      // v + i u
-          ring[n - m] = Make<C2>(v.x + u.y, u.x - v.y);  // conj(v) + i conj(u)
+          ring[m] = Make<T2>(v.x - u.y, v.y + u.x);      // v + i u
+          ring[n - m] = Make<T2>(v.x + u.y, u.x - v.y);  // conj(v) + i conj(u)
         }
       } else {
         ring[m < 0 ? m + n : m] = v;
@@ -672,25 +524,25 @@ __global__ void __launch_bounds__(256, (R1 > 0 && sizeof(T2) == 8) ? 3 : 1)
     }
     __syncthreads();
     if (warp < rings) {
-      at = RingTransform<C2, R1, R2>(a, b, plan, tw, twB, +1, lane);
-      C2* res = at ? b : a;
+      at = RingTransform<T2, R1, R2>(a, b, plan, tw, twB, +1, lane);
+      T2* res = at ? b : a;
       if (mode == kRingSynth) {
         for (int k = lane; k < n; k += kWarp) {
           if (real) {
-            static_cast<T*>(fieldsOut)[row0 + k] = ToStorage<T>(res[k].x);
-            if (second) static_cast<T*>(fieldsOut)[row1 + k] = ToStorage<T>(res[k].y);
+            static_cast<T*>(fieldsOut)[row0 + k] = (res[k].x);
+            if (second) static_cast<T*>(fieldsOut)[row1 + k] = (res[k].y);
           } else {
-            static_cast<T2*>(fieldsOut)[row0 + k] = ToStorage2<T2>(res[k]);
+            static_cast<T2*>(fieldsOut)[row0 + k] = (res[k]);
           }
         }
       } else {
         // the pointwise weights on the synthesised values
 #pragma unroll 5
         for (int k = lane; k < n; k += kWarp) {
-          const C w0 = C(pointWeight[row0 + k]);
-          const C w1 = real ? (second ? C(pointWeight[row1 + k]) : C(0)) : w0;
-          const C2 v = res[k];
-          res[k] = Make<C2>(v.x * w0, v.y * w1);
+          const T w0 = T(pointWeight[row0 + k]);
+          const T w1 = real ? (second ? T(pointWeight[row1 + k]) : T(0)) : w0;
+          const T2 v = res[k];
+          res[k] = Make<T2>(v.x * w0, v.y * w1);
         }
         __syncwarp();
       }
@@ -701,17 +553,17 @@ __global__ void __launch_bounds__(256, (R1 > 0 && sizeof(T2) == 8) ? 3 : 1)
     if (warp < rings) {
 #pragma unroll 5
       for (int k = lane; k < n; k += kWarp) {
-        C2 v;
+        T2 v;
         if (real) {
-          v = Make<C2>(C(static_cast<const T*>(fieldsIn)[row0 + k]),
-                       second ? C(static_cast<const T*>(fieldsIn)[row1 + k]) : C(0));
+          v = Make<T2>(T(static_cast<const T*>(fieldsIn)[row0 + k]),
+                       second ? T(static_cast<const T*>(fieldsIn)[row1 + k]) : T(0));
         } else {
-          v = ToCompute<C2>(static_cast<const T2*>(fieldsIn)[row0 + k]);
+          v = (static_cast<const T2*>(fieldsIn)[row0 + k]);
         }
         if (pointWeight != nullptr) {
-          const C w0 = C(pointWeight[row0 + k]);
-          const C w1 = real ? (second ? C(pointWeight[row1 + k]) : C(0)) : w0;
-          v = Make<C2>(v.x * w0, v.y * w1);
+          const T w0 = T(pointWeight[row0 + k]);
+          const T w1 = real ? (second ? T(pointWeight[row1 + k]) : T(0)) : w0;
+          v = Make<T2>(v.x * w0, v.y * w1);
         }
         a[k] = v;
       }
@@ -722,29 +574,29 @@ __global__ void __launch_bounds__(256, (R1 > 0 && sizeof(T2) == 8) ? 3 : 1)
   // has the same stage count, so the result's side is the same for all: a
   // after two transforms, the stage parity's side after one
   if (warp < rings) {
-    C2* x = at ? b : a;
-    C2* y = at ? a : b;
-    RingTransform<C2, R1, R2>(x, y, plan, tw, twB, -1, lane);
+    T2* x = at ? b : a;
+    T2* y = at ? a : b;
+    RingTransform<T2, R1, R2>(x, y, plan, tw, twB, -1, lane);
   }
   const int out = (mode == kRingWeighted || R1 > 0) ? 0 : plan.stages % 2;
   __syncthreads();
-  const C scale = C(static_cast<T>(2.0 * 3.14159265358979323846 / n * weights[j]));
+  const T scale = T(static_cast<T>(2.0 * 3.14159265358979323846 / n * weights[j]));
 #pragma unroll 4
   for (int e = threadIdx.x; e < mcount * groups; e += blockDim.x) {
     const int g = e % groups, mi = e / groups;
     const int m = real ? mi : mi - lmax;
-    const C2* ring = bufs + ringStride * (g / perRing) + (out ? n : 0);
-    C2 v;
+    const T2* ring = bufs + ringStride * (g / perRing) + (out ? n : 0);
+    T2 v;
     if (real) {
-      const C2 z = ring[m], w = ring[m == 0 ? 0 : n - m];  // Z_m and Z_{n-m}
+      const T2 z = ring[m], w = ring[m == 0 ? 0 : n - m];  // Z_m and Z_{n-m}
       // X_m = (Z_m + conj Z_{n-m}) / 2, Y_m = (Z_m - conj Z_{n-m}) / 2i
-      v = g % 2 == 0 ? Make<C2>(C(0.5) * (z.x + w.x), C(0.5) * (z.y - w.y))
-                     : Make<C2>(C(0.5) * (z.y + w.y), C(0.5) * (w.x - z.x));
+      v = g % 2 == 0 ? Make<T2>(T(0.5) * (z.x + w.x), T(0.5) * (z.y - w.y))
+                     : Make<T2>(T(0.5) * (z.y + w.y), T(0.5) * (w.x - z.x));
     } else {
       v = ring[m < 0 ? m + n : m];
     }
     spectraOut[(static_cast<long long>(mi) * ntheta + j) * count + p0 + g] =
-        ToStorage2<T2>(Make<C2>(v.x * scale, v.y * scale));
+        (Make<T2>(v.x * scale, v.y * scale));
   }
 }
 
@@ -754,16 +606,16 @@ template <class T2>
 using RingFn = void (*)(int, int, int, int, bool, FftPlan, const T2*, const double*, const T2*, const void*,
                         const typename Real<T2>::type*, void*, T2*);
 
-template <class T2, class C2 = T2>
+template <class T2>
 RingFn<T2> RingKernelFor(int n, int* buffers) {
   *buffers = 1;
   switch (n) {
-    case 800: return RingKernel<T2, C2, 25, 32>;
-    case 400: return RingKernel<T2, C2, 25, 16>;  // R1 odd: stage A's stores are bank-conflict free
-    case 50: return RingKernel<T2, C2, 5, 10>;
-    case 40: return RingKernel<T2, C2, 5, 8>;
-    case 25: return RingKernel<T2, C2, 5, 5>;
-    default: *buffers = 2; return RingKernel<T2, C2, 0, 0>;
+    case 800: return RingKernel<T2, 25, 32>;
+    case 400: return RingKernel<T2, 25, 16>;  // R1 odd: stage A's stores are bank-conflict free
+    case 50: return RingKernel<T2, 5, 10>;
+    case 40: return RingKernel<T2, 5, 8>;
+    case 25: return RingKernel<T2, 5, 5>;
+    default: *buffers = 2; return RingKernel<T2, 0, 0>;
   }
 }
 
@@ -901,6 +753,15 @@ int Grid::Create(int lmax, int nmax, double oversampling, std::unique_ptr<Grid>&
   SL3D_CUDA(CopyIn(g->dTheta, g->theta.data(), g->ntheta * sizeof(double)));
   SL3D_CUDA(CopyIn(g->dWeights, g->weights.data(), g->ntheta * sizeof(double)));
   SL3D_CUDA(CopyIn(g->dTwiddle, tw.data(), g->nphi * sizeof(double2)));
+  if (plan.stages > kFxMaxStages || !MakeFxPlan(g->nphi, &g->fxPlan)) {
+    SetError("grid: " + std::to_string(g->nphi) + " longitudes have no transform plan");
+    return SL3DGPU_ERR_ARGUMENT;
+  }
+  g->dfPlan = FxPlanOf(g->nphi, plan.radix, plan.stages);
+  std::vector<FxRoot> roots(g->nphi);
+  for (int k = 0; k < g->nphi; ++k) roots[k] = MakeFxRoot(k, g->nphi);
+  SL3D_CUDA(cudaMalloc(&g->dRoots, g->nphi * sizeof(FxRoot)));
+  SL3D_CUDA(CopyIn(g->dRoots, roots.data(), g->nphi * sizeof(FxRoot)));
   out = std::move(g);
   return SL3DGPU_OK;
 }
@@ -916,6 +777,7 @@ Grid::~Grid() {
   cudaFree(dWeights);
   cudaFree(dTwiddle);
   cudaFree(dTwiddle32);
+  cudaFree(dRoots);
   for (auto& [key, b] : batches_) {
     cudaFree(b.items);
     cudaFree(b.tcItems);
@@ -1193,33 +1055,13 @@ int Grid::LegendreAnalysis(int N, bool real, const double* spectra, int P, int p
 }
 
 namespace {
-// Under FP64 emulation the FP64 rings' transforms run in double-float on the
-// FP32 pipe, unless SL3DGPU_FP64_RINGS=1 keeps them on the FP64 pipe.
-bool DoubleFloatRings(const Grid& g) {
-  static const bool fp64 = [] {
-    const char* v = std::getenv("SL3DGPU_FP64_RINGS");
-    return v != nullptr && v[0] == '1';
-  }();
-  return g.emulateFp64 && !fp64;
-}
+// The most fields that count as a small batch (the FP64 units' rings).
+constexpr int kSmallBatch = 8;
 
 int LaunchRing(const Grid& g, int mode, bool real, int count, const double* spectraIn,
                const void* fieldsIn, const double* weight, void* fieldsOut, double* spectraOut,
-               cudaStream_t stream) {
+               cudaStream_t stream, bool fixedPoint) {
   if (count == 0) return SL3DGPU_OK;
-  int buffers = 2;
-  // double-float takes the planned stages: the two-stage form's unrolled
-  // register transforms would outgrow the instruction cache in it
-  const bool df = DoubleFloatRings(g);
-  const RingFn<double2> kernel = df ? RingKernel<double2, Df2, 0, 0> : RingKernelFor<double2>(g.nphi, &buffers);
-  // the planned stages keep two rings of 16-byte values a warp: at long
-  // rings the double-float kernel takes one CTA an SM with up to eight
-  // rings rather than two CTAs of two
-  const int rings = RingsPerCta<double2>(g.nphi, buffers, df && g.nphi > 400 ? 210 * 1024 : 100 * 1024);
-  const size_t smem = RingSmem<double2>(g.nphi, rings, buffers);
-  SL3D_CUDA(AllowDynamicSmem(kernel));
-  const int fields = real ? 2 * rings : rings;  // real fields go two to a ring
-  dim3 grid((count + fields - 1) / fields, g.ntheta);
   // algorithmic traffic: the spectra and the grid values the mode reads and writes
   const double spec = static_cast<double>(real ? g.lmax + 1 : 2 * g.lmax + 1) * g.ntheta * count * 16.0;
   const double field = static_cast<double>(g.ntheta) * g.nphi * count * (real ? 8.0 : 16.0);
@@ -1228,29 +1070,55 @@ int LaunchRing(const Grid& g, int mode, bool real, int count, const double* spec
   // a real field's transform counts half a complex one (two share a ring)
   const double ffts = static_cast<double>(g.ntheta) * count * (mode == kRingWeighted ? 2 : 1) * (real ? 0.5 : 1.0);
   prof::Scope scope(prof::kRing, stream, ffts * 5.0 * g.nphi * std::log2(static_cast<double>(g.nphi)), bytes);
-  kernel<<<grid, rings * kWarp, smem, stream>>>(mode, g.lmax, g.ntheta, count, real, g.plan, g.dTwiddle,
-                                          g.dWeights, reinterpret_cast<const double2*>(spectraIn),
-                                          fieldsIn, weight, fieldsOut,
-                                          reinterpret_cast<double2*>(spectraOut));
+  FxRingArgs a{};
+  a.mode = mode;
+  a.lmax = g.lmax;
+  a.ntheta = g.ntheta;
+  a.count = count;
+  a.real = real;
+  a.roots = g.dRoots;
+  a.twiddle = g.dTwiddle;
+  a.weights = g.dWeights;
+  a.spectraIn = reinterpret_cast<const double2*>(spectraIn);
+  a.fieldsIn = fieldsIn;
+  a.pointWeight = weight;
+  a.fieldsOut = fieldsOut;
+  a.spectraOut = reinterpret_cast<double2*>(spectraOut);
+  if (g.emulateFp64) return LaunchDfRings(g.dfPlan, a, stream);
+  // A batch of few fields is a launch's latency either way; it stays on the
+  // FP64 units, so that fields made one at a time -- the delta field and the
+  // loads a mixed run starts from -- are what they were bit for bit: where
+  // that form stops, its strain at lmax 256 is reproducible to 1e-9 only from
+  // the same bits. The sea-level solver's many single transforms ask for the
+  // fixed-point form (10 against 18 us at lmax 128).
+  if (count > kSmallBatch || fixedPoint) return LaunchFxRings(g.fxPlan, a, stream);
+  int buffers = 2;
+  const RingFn<double2> kernel = RingKernelFor<double2>(g.nphi, &buffers);
+  const int rings = RingsPerCta<double2>(g.nphi, buffers);
+  SL3D_CUDA(AllowDynamicSmem(kernel));
+  const int perCta = real ? 2 * rings : rings;  // real fields go two to a ring
+  kernel<<<dim3((count + perCta - 1) / perCta, g.ntheta), rings * kWarp, RingSmem<double2>(g.nphi, rings, buffers),
+           stream>>>(mode, g.lmax, g.ntheta, count, real, g.plan, g.dTwiddle, g.dWeights, a.spectraIn, fieldsIn,
+                     weight, fieldsOut, a.spectraOut);
   SL3D_CHECK_LAUNCH();
   return SL3DGPU_OK;
 }
 }  // namespace
 
 int Grid::RingSynthesis(bool real, const double* spectra, int count, double* fields,
-                        cudaStream_t stream) {
-  return LaunchRing(*this, kRingSynth, real, count, spectra, nullptr, nullptr, fields, nullptr, stream);
+                        cudaStream_t stream, bool fixedPoint) {
+  return LaunchRing(*this, kRingSynth, real, count, spectra, nullptr, nullptr, fields, nullptr, stream, fixedPoint);
 }
 
 int Grid::RingAnalysis(bool real, const double* fields, int count, double* spectra,
-                       cudaStream_t stream, const double* weight) {
-  return LaunchRing(*this, kRingAnalyse, real, count, nullptr, fields, weight, nullptr, spectra, stream);
+                       cudaStream_t stream, const double* weight, bool fixedPoint) {
+  return LaunchRing(*this, kRingAnalyse, real, count, nullptr, fields, weight, nullptr, spectra, stream, fixedPoint);
 }
 
 int Grid::RingWeighted(bool real, const double* spectraIn, int count, const double* weight,
                        double* spectraOut, cudaStream_t stream) {
   return LaunchRing(*this, kRingWeighted, real, count, spectraIn, nullptr, weight, nullptr, spectraOut,
-                    stream);
+                    stream, false);
 }
 
 // The spin's table (FP64; the tensor-core panels are made from it) and the
@@ -1499,7 +1367,7 @@ extern "C" int sl3dgpu_grid_colatitudes(const sl3dgpu_grid* grid, double* theta,
 namespace {
 
 int Synthesise(sl3dgpu_grid* handle, int N, bool real, const double* coeffs, int count,
-               double* fields, void* stream) {
+               double* fields, void* stream, bool fixedPoint = false) {
   if (handle == nullptr || count < 0) {
     SetError("null grid or negative count");
     return SL3DGPU_ERR_ARGUMENT;
@@ -1515,11 +1383,11 @@ int Synthesise(sl3dgpu_grid* handle, int N, bool real, const double* coeffs, int
     return st;
   if (int st = g.ToDevice(N, real, coeffs, count, dev, s); st != SL3DGPU_OK) return st;
   if (int st = g.LegendreSynthesis(N, real, dev, count, spectra, s); st != SL3DGPU_OK) return st;
-  return g.RingSynthesis(real, spectra, count, fields, s);
+  return g.RingSynthesis(real, spectra, count, fields, s, fixedPoint);
 }
 
 int Expand(sl3dgpu_grid* handle, int N, bool real, const double* fields, int count, double* coeffs,
-           void* stream) {
+           void* stream, bool fixedPoint = false) {
   if (handle == nullptr || count < 0) {
     SetError("null grid or negative count");
     return SL3DGPU_ERR_ARGUMENT;
@@ -1533,12 +1401,21 @@ int Expand(sl3dgpu_grid* handle, int N, bool real, const double* fields, int cou
                          &spectra, &dev);
       st != SL3DGPU_OK)
     return st;
-  if (int st = g.RingAnalysis(real, fields, count, spectra, s); st != SL3DGPU_OK) return st;
+  if (int st = g.RingAnalysis(real, fields, count, spectra, s, nullptr, fixedPoint); st != SL3DGPU_OK) return st;
   if (int st = g.LegendreAnalysis(N, real, spectra, count, dev, s); st != SL3DGPU_OK) return st;
   return g.FromDevice(N, real, dev, count, coeffs, s);
 }
 
 }  // namespace
+
+namespace sl3dgpu {
+int SynthesiseFixed(sl3dgpu_grid* grid, const double* coeffs, double* field, cudaStream_t stream) {
+  return Synthesise(grid, 0, true, coeffs, 1, field, stream, true);
+}
+int ExpandFixed(sl3dgpu_grid* grid, const double* field, double* coeffs, cudaStream_t stream) {
+  return Expand(grid, 0, true, field, 1, coeffs, stream, true);
+}
+}  // namespace sl3dgpu
 
 extern "C" int sl3dgpu_synthesise_spin_batch(sl3dgpu_grid* grid, int N, const double* coeffs,
                                              int count, double* fields, void* stream) {

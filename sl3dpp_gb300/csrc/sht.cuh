@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "ring_fixed.cuh"
 
 namespace sl3dgpu {
 
@@ -93,6 +94,8 @@ class Grid {
   double* dWeights = nullptr;
   double2* dTwiddle = nullptr;
   float2* dTwiddle32 = nullptr;
+  FxRoot* dRoots = nullptr;  // the fixed-point rings' roots of unity
+  FxPlan fxPlan, dfPlan;
   FftPlan plan;
 
   // The table of spin N, built on first use (device kernel).
@@ -119,11 +122,13 @@ class Grid {
                        cudaStream_t stream) {
     return LegendreAnalysis(N, real, spectra, count, 0, count, coeffs, false, stream);
   }
-  int RingSynthesis(bool real, const double* spectra, int count, double* fields, cudaStream_t stream);
+  // fixedPoint: small batches in fixed point too (larger ones always are).
+  int RingSynthesis(bool real, const double* spectra, int count, double* fields, cudaStream_t stream,
+                    bool fixedPoint = false);
   // Optional pointwise weight (a real field over the same values) applied
   // before the analysis.
   int RingAnalysis(bool real, const double* fields, int count, double* spectra, cudaStream_t stream,
-                   const double* weight = nullptr);
+                   const double* weight = nullptr, bool fixedPoint = false);
   // Synthesis, the pointwise weight and the analysis of each ring in one
   // pass through shared memory: the grid values never reach HBM.
   int RingWeighted(bool real, const double* spectraIn, int count, const double* weight,
@@ -198,6 +203,11 @@ class Grid {
   int* dTcError_ = nullptr;  // set by a tensor-core wait that gave up
   int Table32(int N, const SpinTable** out);
 };
+
+// One real field's transforms with the rings in fixed point (the sea-level
+// solver's; reference layouts).
+int SynthesiseFixed(sl3dgpu_grid* grid, const double* coeffs, double* field, cudaStream_t stream);
+int ExpandFixed(sl3dgpu_grid* grid, const double* field, double* coeffs, cudaStream_t stream);
 
 // Smallest 2^a 3^b 5^c at or above n.
 int FftFriendly(int n);
