@@ -11,8 +11,9 @@
 //    columns a rank-1 step touches, 2kl+ku+1 rows deep for LU) is staged in
 //    shared memory as a ring and streamed column by column, so each band
 //    value is read from and written to HBM once;
-//  - solves: one warp per (system, 64 right-hand sides), two adjacent
-//    columns a lane (an order's real and imaginary parts). Right-hand sides
+//  - solves: a warp per (system, 32 right-hand sides) in FP64, a column a
+//    lane, and per 64 in FP32 and LU, two adjacent columns a lane (an order's
+//    real and imaginary parts). Right-hand sides
 //    are stored row-major (dof-major, the columns fastest), so a warp's rows
 //    are coalesced; a degree's 2(l+1) real columns (its orders m >= 0) are
 //    its right-hand-side vectors. Each substitution runs in chunks of rows:
@@ -203,23 +204,13 @@ __device__ inline void CpCommit() { asm volatile("cp.async.commit_group;\n" ::: 
 __device__ inline void CpWaitAll() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
 __device__ inline void CpWaitOne() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
 
-// The solution ring's slots: in FP64 twice the depth, the Cholesky
-// substitution keeping a mirror of every slot at slot + depth so that its
-// reads need no wrap (fewer integer instructions beside the FP64 ones, which
-// bound it); in FP32 the wrapped ring alone (the mirror's larger staging cost
-// the windowed FP32 solves more than the wrap did).
-template <class T>
-__host__ __device__ constexpr int RingSlots(int depth) {
-  return sizeof(T) == sizeof(double) ? 2 * depth : depth;
-}
-
 // A solve launch's per-warp shared-memory plan.
 struct SolvePlan {
   int depth;    // ring slots: the solve's reach + 1
   int bandCap;  // band values one staged chunk holds
   template <class T>
   __host__ __device__ long long Bytes() const {
-    const long long pairs = static_cast<long long>(RingSlots<T>(depth)) * kWarp +
+    const long long pairs = static_cast<long long>(depth) * kWarp +
                             static_cast<long long>(kBuffers) * kChunk * kWarp;
     const long long b = pairs * 2 * sizeof(T) + static_cast<long long>(kBuffers) * (bandCap + kChunk) * sizeof(T) +
                         static_cast<long long>(kBuffers) * kChunk * sizeof(int);
@@ -227,8 +218,8 @@ struct SolvePlan {
   }
 };
 
-// One warp's staging: the solution ring (RingSlots x 32 lane pairs, each
-// lane's own columns; in FP64 slots depth.. mirror slots 0..), and kBuffers of band columns, right-hand-side rows (lane
+// One warp's staging: the solution ring (depth x 32 lane pairs, each lane's
+// own columns), and kBuffers of band columns, right-hand-side rows (lane
 // pairs), row scales and pivots.
 template <class T>
 struct Stage {
@@ -241,7 +232,7 @@ struct Stage {
   int bandCap;
   __device__ Stage(unsigned char* base, const SolvePlan& plan) : bandCap(plan.bandCap) {
     ring = reinterpret_cast<T2*>(base);
-    rhs = ring + static_cast<long long>(RingSlots<T>(plan.depth)) * kWarp;
+    rhs = ring + static_cast<long long>(plan.depth) * kWarp;
     band = reinterpret_cast<T*>(rhs + static_cast<long long>(kBuffers) * kChunk * kWarp);
     scale = band + static_cast<long long>(kBuffers) * plan.bandCap;
     pivot = reinterpret_cast<int*>(scale + kBuffers * kChunk);
@@ -563,10 +554,10 @@ __device__ __forceinline__ bool WindowSolve(int kd, int c, const Lane<T>& ln, co
 #undef SL3D_WINDOW_CASE
 }
 
-template <class T>
-__global__ void CholeskySolveKernel(const sl3dgpu_band_system* systems, const WorkItem* items, int itemCount,
-                                    const T* bands, T* rhs, const T* scales, SolvePlan plan, const int2* windows,
-                                    int mode) {
+__global__ void CholeskySolve32Kernel(const sl3dgpu_band_system* systems, const WorkItem* items, int itemCount,
+                                      const float* bands, float* rhs, const float* scales, SolvePlan plan,
+                                      const int2* windows, int mode) {
+  using T = float;
   using T2 = typename PairOf<T>::type;
   extern __shared__ __align__(16) unsigned char solveSmem[];
   const int warpInBlock = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
@@ -576,7 +567,6 @@ __global__ void CholeskySolveKernel(const sl3dgpu_band_system* systems, const Wo
   const WorkItem item = items[warp];
   const Lane<T> ln = LaneOf(systems[item.system], rhs, item.column, lane);
   const int n = ln.s.n, kd = ln.s.ku, ld = kd + 1, depth = plan.depth;
-  constexpr bool kMirror = RingSlots<T>(1) == 2;
   const T* ab = bands + ln.s.band;
   T2* ring = st.ring + lane;
   int lo = 0, hi = n - 1;
@@ -587,10 +577,6 @@ __global__ void CholeskySolveKernel(const sl3dgpu_band_system* systems, const Wo
   }
   T2 zero;
   zero.x = zero.y = T(0);
-  // The register form in FP32 only: FP64's solves are bound by its FP64
-  // unit, and its window's 128 registers slowed them (the mirrored ring
-  // serves them better).
-  constexpr bool kWindowForm = sizeof(T) == sizeof(float);
   WindowSet<T2> window;  // the register form's recent solutions
   if (mode == kSolveCompletion) {
     // x at rows lo .. lo + kd - 1 (stored scaled) seeds the ring
@@ -602,7 +588,6 @@ __global__ void CholeskySolveKernel(const sl3dgpu_band_system* systems, const Wo
         v.y /= f;
       }
       ring[(r % depth) * kWarp] = v;
-      if constexpr (kMirror) ring[(r % depth + depth) * kWarp] = v;
     }
   } else {
     // U^T y = b, forward: chunk c holds rows [lo + c kChunk, ...) and their
@@ -617,7 +602,7 @@ __global__ void CholeskySolveKernel(const sl3dgpu_band_system* systems, const Wo
         },
         [&](int c, int buf) {
           const int j0 = lo + c * kChunk, j1 = min(n, j0 + kChunk);
-          if (kWindowForm && c >= 2 &&
+          if (c >= 2 &&
               WindowSolve<T, true>(kd, c, ln, st, buf, ring, lo, depth, j0, j1 - j0, hi, true, window, lane))
             return;
           const T* band = st.Band(buf);
@@ -627,40 +612,10 @@ __global__ void CholeskySolveKernel(const sl3dgpu_band_system* systems, const Wo
           for (int j = j0; j < j1; ++j) {
             const T* column = band + (j - j0) * ld + kd;  // column[-t] = U(j - t, j)
             const T inv = __shfl_sync(0xffffffffu, laneInv, j - j0);
-            T2 a = j <= hi ? Start(ln, st, buf, j - j0, j, lane) : zero;
-            T2 b = zero;
-            const int reach = min(kd, j - lo);
-            if constexpr (sizeof(T) == sizeof(float)) {
-              const float2 sum = RowSum32<true>(a, column, ld, reach, ring, slot, depth);
-              const T2 y = make_float2(sum.x * inv, sum.y * inv);
-              ring[slot * kWarp] = y;
-              ln.Store(j, y);
-              slot = SlotAhead(slot, 1, depth);
-              continue;
-            }
-            // row j - t: slot + depth - t of the mirrored ring, else wrapped
-            const T2* back = ring + (slot + depth) * kWarp;
-            int t = 1;
-            for (; t + 1 <= reach; t += 2) {
-              const T u0 = column[-t], u1 = column[-t - 1];
-              const T2 y0 = kMirror ? back[-t * kWarp] : ring[SlotBack(slot, t, depth) * kWarp];
-              const T2 y1 = kMirror ? back[-(t + 1) * kWarp] : ring[SlotBack(slot, t + 1, depth) * kWarp];
-              a.x -= u0 * y0.x;
-              a.y -= u0 * y0.y;
-              b.x -= u1 * y1.x;
-              b.y -= u1 * y1.y;
-            }
-            if (t <= reach) {
-              const T u0 = column[-t];
-              const T2 y0 = kMirror ? back[-t * kWarp] : ring[SlotBack(slot, t, depth) * kWarp];
-              a.x -= u0 * y0.x;
-              a.y -= u0 * y0.y;
-            }
-            T2 y;
-            y.x = (a.x + b.x) * inv;
-            y.y = (a.y + b.y) * inv;
+            const T2 a = j <= hi ? Start(ln, st, buf, j - j0, j, lane) : zero;
+            const float2 sum = RowSum32<true>(a, column, ld, min(kd, j - lo), ring, slot, depth);
+            const T2 y = make_float2(sum.x * inv, sum.y * inv);
             ring[slot * kWarp] = y;
-            if constexpr (kMirror) ring[(slot + depth) * kWarp] = y;
             ln.Store(j, y);
             slot = SlotAhead(slot, 1, depth);
           }
@@ -681,7 +636,7 @@ __global__ void CholeskySolveKernel(const sl3dgpu_band_system* systems, const Wo
       },
       [&](int c, int buf) {
         const int i1 = top - c * kChunk, i0 = max(bottom, i1 - kChunk);
-        if (kWindowForm && c >= 2 &&
+        if (c >= 2 &&
             WindowSolve<T, false>(kd, c, ln, st, buf, ring, top - 1, depth, i1 - 1, i1 - i0, 0, rhsEnd > 0, window, lane))
           return;
         const T* band = st.Band(buf);
@@ -689,44 +644,132 @@ __global__ void CholeskySolveKernel(const sl3dgpu_band_system* systems, const Wo
         for (int i = i1 - 1; i >= i0; --i) {
           const int r = i - i0;
           const T inv = __shfl_sync(0xffffffffu, laneInv, r);
-          T2 a = rhsEnd > 0 ? st.Rhs(buf, r)[lane] : zero;
-          T2 b = zero;
-          const int reach = min(kd, n - 1 - i);
-          if constexpr (sizeof(T) == sizeof(float)) {
-            const float2 sum = RowSum32<false>(a, band + r * ld + kd, ld, reach, ring, slot, depth);
-            T2 v = make_float2(sum.x * inv, sum.y * inv);
-            ring[slot * kWarp] = v;
-            if (ln.s.scale >= 0) v = Scaled(v, st.Scale(buf, r));
-            ln.Store(i, v);
-            slot = SlotBack(slot, 1, depth);
-            continue;
-          }
-          // row i + t: slot + t of the mirrored ring, else wrapped
-          const T2* ahead = ring + slot * kWarp;
-          int t = 1;
-          for (; t + 1 <= reach; t += 2) {
-            const T u0 = band[(r + t) * ld + kd - t];  // U(i, i + t)
-            const T u1 = band[(r + t + 1) * ld + kd - t - 1];
-            const T2 y0 = kMirror ? ahead[t * kWarp] : ring[SlotAhead(slot, t, depth) * kWarp];
-            const T2 y1 = kMirror ? ahead[(t + 1) * kWarp] : ring[SlotAhead(slot, t + 1, depth) * kWarp];
-            a.x -= u0 * y0.x;
-            a.y -= u0 * y0.y;
-            b.x -= u1 * y1.x;
-            b.y -= u1 * y1.y;
-          }
-          if (t <= reach) {
-            const T u0 = band[(r + t) * ld + kd - t];
-            const T2 y0 = kMirror ? ahead[t * kWarp] : ring[SlotAhead(slot, t, depth) * kWarp];
-            a.x -= u0 * y0.x;
-            a.y -= u0 * y0.y;
-          }
-          T2 v;
-          v.x = (a.x + b.x) * inv;
-          v.y = (a.y + b.y) * inv;
+          const T2 a = rhsEnd > 0 ? st.Rhs(buf, r)[lane] : zero;
+          const float2 sum =
+              RowSum32<false>(a, band + r * ld + kd, ld, min(kd, n - 1 - i), ring, slot, depth);
+          T2 v = make_float2(sum.x * inv, sum.y * inv);
           ring[slot * kWarp] = v;
-          if constexpr (kMirror) ring[(slot + depth) * kWarp] = v;
           if (ln.s.scale >= 0) v = Scaled(v, st.Scale(buf, r));
           ln.Store(i, v);
+          slot = SlotBack(slot, 1, depth);
+        }
+      });
+}
+
+// The FP64 Cholesky solve, a column a lane: the same substitutions (two
+// partial sums a row, odd and even distances; the diagonal's reciprocal), a
+// warp a CTA, two CTAs for an item's 64 columns. GB300 issues one FP64 warp
+// instruction in 64 cycles a sub-partition whatever lanes are active, so a
+// row costs its instruction count: with two columns a lane and four warps a
+// CTA (as the FP32 solves run) a row took twice the instructions and the
+// warps filled a third of the SMs. The solution ring is mirrored (slot +
+// depth) so that its reads need no wrap. The arithmetic and its order are the
+// earlier kernel's, so the results are its bits. An lmax-128 pass's two
+// launches (spheroidal, toroidal): 2.95 -> 1.65 ms; an lmax-45 one's 1.13 ->
+// 0.61 ms.
+struct Plan64 {
+  int depth, bandCap;
+  __host__ __device__ long long Values() const {
+    return 2LL * depth * kWarp + static_cast<long long>(kBuffers) * (kChunk * kWarp + bandCap + kChunk);
+  }
+};
+
+__global__ void __launch_bounds__(kWarp) CholeskySolve64Kernel(const sl3dgpu_band_system* systems,
+                                                               const WorkItem* items, const double* bands,
+                                                               double* rhs, const double* scales, Plan64 plan) {
+  extern __shared__ __align__(16) unsigned char solve64Smem[];
+  const int lane = threadIdx.x;
+  const WorkItem item = items[blockIdx.x / 2];
+  const sl3dgpu_band_system s = systems[item.system];
+  const int first = item.column + static_cast<int>(blockIdx.x % 2) * kWarp, col = first + lane;
+  if (first >= s.nrhs) return;  // the whole warp
+  const bool live = col < s.nrhs;
+  const int n = s.n, kd = s.ku, ld = kd + 1, depth = plan.depth;
+  const double* ab = bands + s.band;
+  double* x = rhs + s.rhs + col;
+  const bool scaled = s.scale >= 0;
+  double* base = reinterpret_cast<double*>(solve64Smem);
+  double* ring = base + lane;                       // [2 depth][32]
+  double* rhsStage = base + 2LL * depth * kWarp;    // [buffer][kChunk][32]
+  double* bandStage = rhsStage + kBuffers * kChunk * kWarp;
+  double* scaleStage = bandStage + static_cast<long long>(kBuffers) * plan.bandCap;
+  // band columns [c0, c1), right-hand-side rows [r0, r1) and their scales
+  auto stage = [&](int buf, int c0, int c1, int r0, int r1) {
+    const double* src = ab + static_cast<long long>(c0) * ld;
+    double* band = bandStage + buf * plan.bandCap;
+    const int count = (c1 - c0) * ld;
+    for (int e = lane; e < count; e += kWarp) CpAsync(band + e, src + e);
+    if (live)
+      for (int r = r0; r < r1; ++r)
+        CpAsync(rhsStage + (buf * kChunk + r - r0) * kWarp + lane, x + static_cast<long long>(r) * s.nrhs);
+    if (scaled)
+      for (int r = r0 + lane; r < r1; r += kWarp) CpAsync(scaleStage + buf * kChunk + (r - r0), scales + s.scale + r);
+    CpCommit();
+  };
+  const int chunks = (n + kChunk - 1) / kChunk;
+  int slot = 0;  // the ring slot of the current row (row mod depth)
+  Pipeline(
+      chunks,
+      [&](int c) {
+        const int j0 = c * kChunk, j1 = min(n, j0 + kChunk);
+        stage(c % kBuffers, j0, j1, j0, j1);
+      },
+      [&](int c, int buf) {
+        const int j0 = c * kChunk, j1 = min(n, j0 + kChunk);
+        const double* band = bandStage + buf * plan.bandCap;
+        // the chunk's reciprocal diagonals, row j0 + k's in lane k
+        const double laneInv = lane < j1 - j0 ? 1.0 / band[lane * ld + kd] : 1.0;
+        for (int j = j0; j < j1; ++j) {
+          const double* column = band + (j - j0) * ld + kd;  // column[-t] = U(j - t, j)
+          const double inv = __shfl_sync(0xffffffffu, laneInv, j - j0);
+          double a = 0.0, b = 0.0;
+          if (live && j != s.pinned0 && j != s.pinned1) {
+            a = rhsStage[(buf * kChunk + j - j0) * kWarp + lane];
+            if (scaled) a *= scaleStage[buf * kChunk + j - j0];
+          }
+          const int reach = min(kd, j);
+          const double* back = ring + (slot + depth) * kWarp;  // row j - t at back[-t]
+          int t = 1;
+          for (; t + 1 <= reach; t += 2) {
+            a = fma(-column[-t], back[-t * kWarp], a);
+            b = fma(-column[-t - 1], back[-(t + 1) * kWarp], b);
+          }
+          if (t <= reach) a = fma(-column[-t], back[-t * kWarp], a);
+          const double y = (a + b) * inv;
+          ring[slot * kWarp] = y;
+          ring[(slot + depth) * kWarp] = y;
+          if (live) x[static_cast<long long>(j) * s.nrhs] = y;
+          slot = SlotAhead(slot, 1, depth);
+        }
+      });
+  slot = (n - 1) % depth;
+  Pipeline(
+      chunks,
+      [&](int c) {
+        const int i1 = n - c * kChunk, i0 = max(0, i1 - kChunk);
+        stage(c % kBuffers, i0, min(n, i1 + kd), i0, i1);
+      },
+      [&](int c, int buf) {
+        const int i1 = n - c * kChunk, i0 = max(0, i1 - kChunk);
+        const double* band = bandStage + buf * plan.bandCap;
+        const double laneInv = lane < i1 - i0 ? 1.0 / band[lane * ld + kd] : 1.0;  // row i0 + k's in lane k
+        for (int i = i1 - 1; i >= i0; --i) {
+          const int r = i - i0;
+          const double inv = __shfl_sync(0xffffffffu, laneInv, r);
+          double a = live ? rhsStage[(buf * kChunk + r) * kWarp + lane] : 0.0, b = 0.0;
+          const int reach = min(kd, n - 1 - i);
+          const double* ahead = ring + slot * kWarp;  // row i + t at ahead[t]
+          int t = 1;
+          for (; t + 1 <= reach; t += 2) {
+            a = fma(-band[(r + t) * ld + kd - t], ahead[t * kWarp], a);  // U(i, i + t)
+            b = fma(-band[(r + t + 1) * ld + kd - t - 1], ahead[(t + 1) * kWarp], b);
+          }
+          if (t <= reach) a = fma(-band[(r + t) * ld + kd - t], ahead[t * kWarp], a);
+          double v = (a + b) * inv;
+          ring[slot * kWarp] = v;
+          ring[(slot + depth) * kWarp] = v;
+          if (scaled) v *= scaleStage[buf * kChunk + r];
+          if (live) x[static_cast<long long>(i) * s.nrhs] = v;
           slot = SlotBack(slot, 1, depth);
         }
       });
@@ -929,7 +972,8 @@ int SolveBatch(const sl3dgpu_band_system* devSystems, const sl3dgpu_band_system*
   int warpsPerBlock = 4;
   while (warpsPerBlock > 1 && perWarp * warpsPerBlock > 100 * 1024) warpsPerBlock /= 2;
   const size_t smem = perWarp * warpsPerBlock;
-  if (smem > 200 * 1024) {
+  // the limit on the bandwidth (FP64's mirrored ring counted)
+  if (smem + (sizeof(T) == sizeof(double) ? plan.depth * kWarp * 2 * sizeof(T) : 0) > 200 * 1024) {
     SetError("band solve: the staged band exceeds shared memory");
     return SL3DGPU_ERR_ARGUMENT;
   }
@@ -947,10 +991,15 @@ int SolveBatch(const sl3dgpu_band_system* devSystems, const sl3dgpu_band_system*
     SL3D_CUDA(AllowDynamicSmem(LuSolveKernel<T>));
     LuSolveKernel<T><<<blocks, warpsPerBlock * kWarp, smem, stream>>>(devSystems, items, itemCount, bands, pivots,
                                                                      rhs, scales, plan);
+  } else if constexpr (sizeof(T) == sizeof(float)) {
+    SL3D_CUDA(AllowDynamicSmem(CholeskySolve32Kernel));
+    CholeskySolve32Kernel<<<blocks, warpsPerBlock * kWarp, smem, stream>>>(devSystems, items, itemCount, bands, rhs,
+                                                                          scales, plan, windows, mode);
   } else {
-    SL3D_CUDA(AllowDynamicSmem(CholeskySolveKernel<T>));
-    CholeskySolveKernel<T><<<blocks, warpsPerBlock * kWarp, smem, stream>>>(devSystems, items, itemCount, bands,
-                                                                           rhs, scales, plan, windows, mode);
+    const Plan64 plan64{plan.depth, plan.bandCap};
+    const size_t smem64 = static_cast<size_t>(plan64.Values()) * sizeof(double);
+    SL3D_CUDA(AllowDynamicSmem(CholeskySolve64Kernel));
+    CholeskySolve64Kernel<<<2 * itemCount, kWarp, smem64, stream>>>(devSystems, items, bands, rhs, scales, plan64);
   }
   SL3D_CHECK_LAUNCH();
   return SL3DGPU_OK;
