@@ -1,0 +1,45 @@
+// The FP64 Cholesky solves by blocks of rows (band_block.cu): a flavour's
+// factorised systems rewritten once so that a solve advances a block of rows
+// at a time.
+#pragma once
+
+#include <vector>
+
+#include "common.cuh"
+
+namespace sl3dgpu {
+
+// One system of a blocked solve.
+struct BlockSystem {
+  int n, kd, nrhs, blocks;
+  long long forward, backward;  // doubles: its blocks' coefficients, [block][(kd + B) x B]
+  long long rhs, scale;         // as sl3dgpu_band_system's
+  int second;                   // which of the two right-hand-side arrays
+};
+
+struct BlockSolver {
+  int block = 0;  // rows a block (8 or 16); 0: the row-by-row solve is the faster
+  int kd = 0;     // the largest bandwidth
+  int itemCount = 0;
+  BlockSystem* systems = nullptr;
+  int2* items = nullptr;  // (system, first column)
+  double* data = nullptr;
+  BlockSolver() = default;
+  BlockSolver(const BlockSolver&) = delete;
+  BlockSolver& operator=(const BlockSolver&) = delete;
+  ~BlockSolver() {
+    cudaFree(systems);
+    cudaFree(items);
+    cudaFree(data);
+  }
+};
+
+// Chooses the form for two lists of factorised Cholesky systems (the second
+// list's right-hand sides in the second array) and makes a blocked form's
+// coefficients from their factors.
+int BuildBlockSolver(const std::vector<sl3dgpu_band_system>& first, const std::vector<sl3dgpu_band_system>& second,
+                     const double* bands, const double* scales, BlockSolver& out, cudaStream_t stream);
+// Solves every system in place (out.block > 0).
+int RunBlockSolver(const BlockSolver& b, double* first, double* second, const double* scales, cudaStream_t stream);
+
+}  // namespace sl3dgpu

@@ -1028,6 +1028,11 @@ int Viscoelastic3DGpu::Solve(const Flavour& f) { return SolveColumns(f, rhsSph.p
 int Viscoelastic3DGpu::SolveColumns(const Flavour& f, double2* sph, double2* tor) {
   auto* sphD = reinterpret_cast<double*>(sph);
   auto* torD = reinterpret_cast<double*>(tor);
+  if (f.blocked.block > 0) {
+    SL3D_TRY(RunBlockSolver(f.blocked, sphD, torD, f.scales.p, stream));
+    return BandSolveBatch(f.dSphLu.p, f.sphLu.data(), static_cast<int>(f.sphLu.size()), f.iSphLu.p, f.nSphLu,
+                          f.bands.p, f.pivots.p, sphD, f.scales.p, 1, stream);
+  }
   SL3D_TRY(BandSolveBatch(f.dSphChol.p, f.sphChol.data(), static_cast<int>(f.sphChol.size()), f.iSphChol.p,
                           f.nSphChol, f.bands.p, f.pivots.p, sphD, f.scales.p, 0, stream));
   SL3D_TRY(BandSolveBatch(f.dSphLu.p, f.sphLu.data(), static_cast<int>(f.sphLu.size()), f.iSphLu.p, f.nSphLu,

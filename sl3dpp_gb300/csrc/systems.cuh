@@ -8,6 +8,7 @@
 
 #include <vector>
 
+#include "band_block.cuh"
 #include "common.cuh"
 #include "host/earth.hpp"
 #include "step_kernels.cuh"
@@ -92,6 +93,7 @@ struct Flavour {
   Dev<sl3dgpu_band_system> dSphChol, dSphLu, dTorChol;
   Dev<int2> iSphChol, iSphLu, iTorChol;
   int nSphChol = 0, nSphLu = 0, nTorChol = 0;
+  BlockSolver blocked;  // the Cholesky solves by blocks, where they are the faster form
   // The FP32 correction's row windows per system ({lo, hi}: the rows its
   // lateral forces reach), for the lateral node range [windowFirst, windowEnd).
   mutable int windowFirst = -1, windowEnd = -1;
