@@ -32,8 +32,8 @@
 // the 3D step (step_kernels.cu) with the reference's memory and plain start;
 // the integrals sum each ring in a fixed tree and the rings in order (the
 // grid's Integrate, SurfaceGrid.hpp:257-267); the stopping test's maxima are
-// order-free. The rotation block (RotationPatchKernel) and the conservation's
-// shift (ShiftKernel) are formed on the device; an iteration brings one
+// order-free. The rotation block (RotationPatch) and the conservation's
+// shift (ShiftAndLoadKernel) are formed on the device; an iteration brings one
 // thing to the host, the stopping test's maxima. A workspace (SleWorkspace)
 // keeps the buffers between solves on one grid, so that the coupled closure's
 // solve in every pass of a step allocates nothing.
@@ -51,6 +51,8 @@
 #include <array>
 #include <cmath>
 #include <string>
+#include <memory>
+#include <mutex>
 #include <vector>
 
 #include "common.cuh"
@@ -120,13 +122,26 @@ __global__ void SeedKernel(long long n, const double* direct, const double* ocea
   if (i < n) out[i] = direct[i] + rhoMean * ocean[i];
 }
 
-// S += shift; C S; the next load sigma_d + rho_w C S; per block the largest
-// |C S - C S_prev| and |C S| (blockIdx-ordered partials), C S kept for the next test.
-__global__ void ShiftAndLoadKernel(long long n, const double* shiftPtr, double rho, const double* direct,
+// The conservation's uniform shift, a^2 dphi sum_rings of the ring partials of
+// C S (every block forms it, in the same fixed tree), s_mean minus it over
+// the ocean's area (src/SeaLevel.cpp:655-661); S += shift; C S; the next load
+// sigma_d + rho_w C S; per block the largest |C S - C S_prev| and |C S|
+// (blockIdx-ordered partials), C S kept for the next test.
+__global__ void ShiftAndLoadKernel(long long n, const double* ringPartial, int ntheta, double scale, double meanSlc,
+                                   double perOceanArea, double* shiftOut, double rho, const double* direct,
                                    const double* ocean, double* slc, double* oceanSlc, double* newLoad, bool havePrev,
                                    double* maxima) {
   __shared__ double red[2][kRingThreads];
-  const double shift = *shiftPtr;
+  double ringSum = 0.0;
+  for (int j = threadIdx.x; j < ntheta; j += blockDim.x) ringSum += ringPartial[j];
+  for (int off = 16; off > 0; off >>= 1) ringSum += __shfl_xor_sync(0xffffffffu, ringSum, off);
+  if (threadIdx.x % 32 == 0) red[0][threadIdx.x / 32] = ringSum;
+  __syncthreads();
+  ringSum = red[0][0];
+  for (int w = 1; w < kRingThreads / 32; ++w) ringSum += red[0][w];
+  const double shift = meanSlc - scale * ringSum * perOceanArea;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *shiftOut = shift;
+  __syncthreads();
   double dmax = 0.0, smax = 0.0;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<long long>(gridDim.x) * blockDim.x) {
@@ -180,7 +195,18 @@ struct SleRun {
   double r2 = 0.0, dphi = 0.0;
   Dev<double> weights, ringPartial, maxima, loadLm, newLoadLm, scaledLm, factors;
   Dev<double> seeded, slc, oceanSlc, newLoad;
-  std::vector<double> hostRing, hostMaxima;
+  std::vector<double> hostRing;
+  // The block maxima and, from 2 kMaxBlocks on, the mixer's sums: one pinned
+  // read an iteration; then the mixer's gamma, written back.
+  double* hostMaxima = nullptr;
+  static constexpr int kSums = 2 * kMixMaxMemory;
+  double* MixerSums() { return maxima.p + 2 * kMaxBlocks; }
+  double* HostMixerSums() { return hostMaxima + 2 * kMaxBlocks; }
+  double* HostGamma() { return hostMaxima + 2 * kMaxBlocks + kSums; }
+  static size_t MaximaCount() { return 2 * kMaxBlocks + kSums; }
+  ~SleRun() {
+    if (hostMaxima != nullptr) cudaFreeHost(hostMaxima);
+  }
 
   // a^2 int a (b) dOmega, the rings in order
   int Integrate(const double* a, const double* b, double* out) {
@@ -223,7 +249,7 @@ struct SleRun {
     const int b = static_cast<int>(std::min<long long>(kMaxBlocks, (n + 255) / 256));
     MaxAbsKernel<<<b, kRingThreads, 0, stream>>>(n, a, maxima.p);
     SL3D_CHECK_LAUNCH();
-    SL3D_CUDA(cudaMemcpyAsync(hostMaxima.data(), maxima.p, 2 * b * sizeof(double), cudaMemcpyDeviceToHost, stream));
+    SL3D_CUDA(cudaMemcpyAsync(hostMaxima, maxima.p, 2 * b * sizeof(double), cudaMemcpyDeviceToHost, stream));
     SL3D_CUDA(cudaStreamSynchronize(stream));
     double m = 0.0;
     for (int i = 0; i < b; ++i) m = std::max(m, hostMaxima[2 * i + 1]);
@@ -231,17 +257,6 @@ struct SleRun {
     return SL3DGPU_OK;
   }
 };
-
-// The conservation's uniform shift on the device: a^2 dphi sum_rings of the
-// ring partials of C S, in order (the host's Integrate), then s_mean minus
-// it over the ocean's area (src/SeaLevel.cpp:655-661).
-__global__ void ShiftKernel(const double* ringPartial, int ntheta, double scale, double meanSlc, double perOceanArea,
-                            double* shift) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  double sum = 0.0;
-  for (int j = 0; j < ntheta; ++j) sum += ringPartial[j];
-  shift[0] = meanSlc - scale * sum * perOceanArea;
-}
 
 // GRDSolver::Rotation's inputs that do not change within a solve: the
 // factors of the constructor (src/SeaLevel.cpp:220-247), the static blocks
@@ -256,68 +271,83 @@ struct RotationInputs {
 };
 
 // The rotation block of the load's (2, 0), (2, 1) and (0, 0) coefficients
-// (GRDSolver::Rotation, src/SeaLevel.cpp:348-392), and the patch of a
-// scaled coefficient vector's degree-0/2 entries, on the device: mode 0 the
-// sea level change's (and the angular velocity out), 1 the displacement's,
-// 2 the potential's, 3 the tangential potential's (src/SeaLevel.cpp:625-640,
-// 714-724). One thread; the host solve's arithmetic in its order.
-__global__ void RotationPatchKernel(const RotationInputs* p, const double* load, double* out, double* omegaOut,
-                                    int mode) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// (GRDSolver::Rotation, src/SeaLevel.cpp:348-392) and the value it gives one
+// of these entries of a scaled coefficient vector: mode 0 the sea level
+// change's (and the angular velocity out), 1 the displacement's, 2 the
+// potential's, 3 the tangential potential's (src/SeaLevel.cpp:625-640,
+// 714-724). The host solve's arithmetic in its order; `value` the scaled
+// coefficient, (l, m) one of the three.
+__device__ double2 RotationPatch(const RotationInputs& p, double2 l20, double2 l21, double load0, double2 value,
+                                 int l, int m, double* omegaOut, int mode) {
   const double r2 = sqrt(2.0);
   // BlockOf of the load: (2,0) re, -sqrt2 re (2,1), sqrt2 im (2,1)
-  const double l00 = load[6], l01 = -r2 * load[8], l11 = r2 * load[9];
-  const double load0 = load[0];
-  const double grav00 = p->k2 * l00 + p->staticGrav2[0], grav01 = p->k2 * l01 + p->staticGrav2[1],
-               grav11 = p->k2 * l11 + p->staticGrav2[3];
-  const double disp00 = p->h2 * l00 + p->staticDisp2[0], disp01 = p->h2 * l01 + p->staticDisp2[1],
-               disp11 = p->h2 * l11 + p->staticDisp2[3];
-  double transverse0 = p->inertia * grav01, transverse1 = p->inertia * grav11;
-  double axial = -p->axialInertia * grav00 -
-                 p->trace * ((p->mu + p->mphi) * load0 + p->mu * p->displacementLoad0 + p->mphi * p->potentialLoad0 +
-                             p->inertiaMoment) -
-                 p->shell * (load0 + p->potentialLoad0);
-  transverse0 -= p->inverseInertiaDifference * p->angularMomentum[0];
-  transverse1 -= p->inverseInertiaDifference * p->angularMomentum[1];
-  axial += p->inversePolarInertia * p->angularMomentum[2];
+  const double l00 = l20.x, l01 = -r2 * l21.x, l11 = r2 * l21.y;
+  const double grav00 = p.k2 * l00 + p.staticGrav2[0], grav01 = p.k2 * l01 + p.staticGrav2[1],
+               grav11 = p.k2 * l11 + p.staticGrav2[3];
+  const double disp00 = p.h2 * l00 + p.staticDisp2[0], disp01 = p.h2 * l01 + p.staticDisp2[1],
+               disp11 = p.h2 * l11 + p.staticDisp2[3];
+  double transverse0 = p.inertia * grav01, transverse1 = p.inertia * grav11;
+  double axial = -p.axialInertia * grav00 -
+                 p.trace * ((p.mu + p.mphi) * load0 + p.mu * p.displacementLoad0 + p.mphi * p.potentialLoad0 +
+                            p.inertiaMoment) -
+                 p.shell * (load0 + p.potentialLoad0);
+  transverse0 -= p.inverseInertiaDifference * p.angularMomentum[0];
+  transverse1 -= p.inverseInertiaDifference * p.angularMomentum[1];
+  axial += p.inversePolarInertia * p.angularMomentum[2];
   double omega0 = 0.0, omega1 = 0.0;
-  if (p->transverse) {
-    omega0 = transverse0 / p->rotationDenominator;
-    omega1 = transverse1 / p->rotationDenominator;
+  if (p.transverse) {
+    omega0 = transverse0 / p.rotationDenominator;
+    omega1 = transverse1 / p.rotationDenominator;
   }
-  const double omega2 = axial / p->axialRotationDenominator;
-  const double c00 = p->axialRotation * omega2, c01 = p->rotation * omega0, c11 = p->rotation * omega1;
-  const double centrifugal0 = p->uniformRotation * omega2;
-  const double d00 = disp00 + p->ht2 * c00, d01 = disp01 + p->ht2 * c01, d11 = disp11 + p->ht2 * c11;
-  const double g00 = grav00 + p->kt2 * c00, g01 = grav01 + p->kt2 * c01, g11 = grav11 + p->kt2 * c11;
-  // FromBlock into out[6..9]: (2,0) = b00, (2,1) = (-b01 / sqrt2, b11 / sqrt2)
-  auto put = [&](double b00, double b01, double b11) {
-    out[6] = b00;
-    out[7] = 0.0;
-    out[8] = -b01 / r2;
-    out[9] = b11 / r2;
+  const double omega2 = axial / p.axialRotationDenominator;
+  const double c00 = p.axialRotation * omega2, c01 = p.rotation * omega0, c11 = p.rotation * omega1;
+  const double centrifugal0 = p.uniformRotation * omega2;
+  const double d00 = disp00 + p.ht2 * c00, d01 = disp01 + p.ht2 * c01, d11 = disp11 + p.ht2 * c11;
+  const double g00 = grav00 + p.kt2 * c00, g01 = grav01 + p.kt2 * c01, g11 = grav11 + p.kt2 * c11;
+  // FromBlock: (2,0) = b00, (2,1) = (-b01 / sqrt2, b11 / sqrt2)
+  auto of = [&](double b00, double b01, double b11) {
+    return m == 0 ? make_double2(b00, 0.0) : make_double2(-b01 / r2, b11 / r2);
   };
-  const double ig = 1.0 / p->g;
+  const double ig = 1.0 / p.g;
   if (mode == 0) {
-    omegaOut[0] = omega0;
-    omegaOut[1] = omega1;
-    omegaOut[2] = omega2;
-    const double s00 = -((d00 + ((g00 + c00) + p->tide2[0]) * ig) + p->layer2[0]);
-    const double s01 = -((d01 + ((g01 + c01) + p->tide2[1]) * ig) + p->layer2[1]);
-    const double s11 = -((d11 + ((g11 + c11) + p->tide2[3]) * ig) + p->layer2[3]);
-    put(s00, s01, s11);
-    out[0] -= (p->hc + (p->kc + 1.0) / p->g) * centrifugal0;
-  } else if (mode == 1) {
-    put(d00, d01, d11);
-    out[0] += p->hc * centrifugal0;
-  } else if (mode == 2) {
-    put(g00, g01, g11);
-    out[0] += p->kc * centrifugal0;
-  } else {
-    out[6] += p->lt2 * c00;
-    out[8] += -(p->lt2 * c01) / r2;
-    out[9] += (p->lt2 * c11) / r2;
+    if (l == 0) {
+      omegaOut[0] = omega0;
+      omegaOut[1] = omega1;
+      omegaOut[2] = omega2;
+      return make_double2(value.x - (p.hc + (p.kc + 1.0) / p.g) * centrifugal0, value.y);
+    }
+    return of(-((d00 + ((g00 + c00) + p.tide2[0]) * ig) + p.layer2[0]),
+              -((d01 + ((g01 + c01) + p.tide2[1]) * ig) + p.layer2[1]),
+              -((d11 + ((g11 + c11) + p.tide2[3]) * ig) + p.layer2[3]));
   }
+  if (mode == 1) return l == 0 ? make_double2(value.x + p.hc * centrifugal0, value.y) : of(d00, d01, d11);
+  if (mode == 2) return l == 0 ? make_double2(value.x + p.kc * centrifugal0, value.y) : of(g00, g01, g11);
+  if (l == 0) return value;
+  const double2 c = of(p.lt2 * c00, p.lt2 * c01, p.lt2 * c11);
+  return make_double2(value.x + c.x, value.y + c.y);
+}
+
+// out = f_l load + add over the (l, m >= 0) coefficients, the degree-0/2
+// entries patched by the rotation of the load when `rotation` is given. load
+// and out in the transforms' device layout (an order's degrees together, so
+// that no permutation stands between this and the contraction), add in the
+// reference's. One launch for what took three (scale, one-thread patch,
+// permutation).
+__global__ void ScalePatchKernel(int lmax, const double* f, const double2* load, const double2* add,
+                                 const RotationInputs* rotation, double2* out, double* omegaOut, int mode) {
+  const int m = blockIdx.y, l = m + static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
+  if (l > lmax) return;
+  auto row = [lmax](int ll, int mm) { return static_cast<long long>(mm) * (lmax + 1) - mm * (mm - 1) / 2 + ll - mm; };
+  const double2 v = load[row(l, m)];
+  double2 o = make_double2(f[l] * v.x, f[l] * v.y);
+  if (add != nullptr) {
+    const double2 a = add[static_cast<long long>(l) * (l + 1) / 2 + m];
+    o.x += a.x;
+    o.y += a.y;
+  }
+  if (rotation != nullptr && ((l == 0) || (l == 2 && m < 2)))
+    o = RotationPatch(*rotation, load[row(2, 0)], load[row(2, 1)], load[row(0, 0)].x, o, l, m, omegaOut, mode);
+  out[row(l, m)] = o;
 }
 
 // The Anderson mixer of the load coefficients (AndersonMixer::Update, the
@@ -327,7 +357,8 @@ struct LoadMixer {
   bool first = true;
   std::vector<Dev<double>> dG, dF;
   Dev<double*> dGPtr, dFPtr;
-  Dev<double> xPrev, fPrev, partial, sums, gamma, gram;  // the Gram matrix on the device
+  Dev<double> xPrev, fPrev, partial, gamma;
+  std::vector<double> gram;  // the Gram matrix
 
   int Init(int m, long long n) {
     memory = m;
@@ -346,19 +377,12 @@ struct LoadMixer {
     SL3D_CUDA(xPrev.Alloc(n));
     SL3D_CUDA(fPrev.Alloc(n));
     SL3D_CUDA(partial.Alloc(static_cast<size_t>(1024) * 2 * kMixMaxMemory));
-    SL3D_CUDA(sums.Alloc(2 * kMixMaxMemory));
     SL3D_CUDA(gamma.Alloc(kMixMaxMemory + 1));
-    SL3D_CUDA(gram.Alloc(static_cast<size_t>(memory) * memory));
-    SL3D_CUDA(ZeroIn(gram.p, static_cast<size_t>(memory) * memory * sizeof(double)));
+    gram.assign(static_cast<size_t>(memory) * memory, 0.0);
     return SL3DGPU_OK;
   }
 
-  // x <- the mixed iterate from x and its image gx
-  int Update(double* x, const double* gx, long long n, cudaStream_t stream) {
-    if (memory <= 0) {
-      SL3D_CUDA(cudaMemcpyAsync(x, gx, n * sizeof(double), cudaMemcpyDeviceToDevice, stream));
-      return SL3DGPU_OK;
-    }
+  MixerArgs Args(double* x, const double* gx, long long n) {
     MixerArgs a{};
     a.n = n;
     a.memory = memory;
@@ -369,20 +393,39 @@ struct LoadMixer {
     a.dG = dGPtr.p;
     a.dF = dFPtr.p;
     a.partial = partial.p;
-    a.blocks = static_cast<int>(std::min<long long>(1024, n));
+    // two values a thread: a block's reduction costs its FP64 shuffle sums
+    // whatever it covers (30 us with 1024 blocks at lmax 128, 5 us so)
+    a.blocks = static_cast<int>(std::min<long long>(1024, std::max<long long>(1, n / 512)));
     a.gamma = gamma.p;
+    a.slot = slot;
+    a.m = std::min(count + 1, memory);
+    return a;
+  }
+
+  // x <- the mixed iterate from x and its image gx, in two parts: the sweep's
+  // sums on the device, then, the sums read, their least squares on the host
+  // (a 5 x 5 eigenproblem: 63 us on one FP64 warp, a few here) and the mix.
+  int Sweep(double* x, const double* gx, long long n, double* sums, cudaStream_t stream) {
+    if (memory <= 0 || first) return SL3DGPU_OK;
+    LaunchMixerSweep(Args(x, gx, n), sums, stream);
+    SL3D_CHECK_LAUNCH();
+    return SL3DGPU_OK;
+  }
+  // hostGamma: pinned, kMixMaxMemory + 1 values, free until the next wait on the stream
+  int Mix(double* x, const double* gx, long long n, const double* hostSums, double* hostGamma, cudaStream_t stream) {
+    if (memory <= 0) {
+      SL3D_CUDA(cudaMemcpyAsync(x, gx, n * sizeof(double), cudaMemcpyDeviceToDevice, stream));
+      return SL3DGPU_OK;
+    }
+    const MixerArgs a = Args(x, gx, n);
     if (first) {
       LaunchMixerFirst(a, stream);
       SL3D_CHECK_LAUNCH();
       first = false;
       return SL3DGPU_OK;
     }
-    a.slot = slot;
-    a.m = std::min(count + 1, memory);
-    LaunchMixerSweep(a, sums.p, stream);
-    SL3D_CHECK_LAUNCH();
-    LaunchMixerGram(gram.p, a.m, a.slot, a.memory, sums.p, gamma.p, stream);  // one FP64 warp, no host round trip
-    SL3D_CHECK_LAUNCH();
+    hostGamma[a.m] = MixerSolve(gram.data(), a.m, slot, memory, hostSums, hostGamma) ? 1.0 : 0.0;
+    SL3D_CUDA(cudaMemcpyAsync(gamma.p, hostGamma, (a.m + 1) * sizeof(double), cudaMemcpyHostToDevice, stream));
     LaunchMixerMix(a, stream);
     SL3D_CHECK_LAUNCH();
     count = a.m;
@@ -489,8 +532,9 @@ struct SleWorkspace {
     SL3D_CUDA(run.weights.Upload(w));
     SL3D_CUDA(run.ringPartial.Alloc(ntheta));
     run.hostRing.assign(ntheta, 0.0);
-    SL3D_CUDA(run.maxima.Alloc(2 * kMaxBlocks));
-    run.hostMaxima.assign(2 * kMaxBlocks, 0.0);
+    SL3D_CUDA(run.maxima.Alloc(SleRun::MaximaCount()));
+    if (run.hostMaxima == nullptr)
+      SL3D_CUDA(cudaMallocHost(&run.hostMaxima, (SleRun::MaximaCount() + kMixMaxMemory + 1) * sizeof(double)));
     const long long nc = 2 * run.coefCount;
     for (auto* d : {&run.loadLm, &run.newLoadLm, &run.scaledLm}) SL3D_CUDA(d->Alloc(nc));
     SL3D_CUDA(run.factors.Alloc(run.lmax + 1));
@@ -515,7 +559,7 @@ struct SleWorkspace {
     return SL3DGPU_OK;
   }
   // the mixer at its plain start, with `memory` columns
-  int ResetMixer(int memory, cudaStream_t s) {
+  int ResetMixer(int memory) {
     if (mixerMemory != memory) {
       mixer = LoadMixer{};
       SL3D_TRY(mixer.Init(memory, 2 * run.coefCount));
@@ -524,8 +568,7 @@ struct SleWorkspace {
     }
     mixer.first = true;
     mixer.count = mixer.slot = 0;
-    if (memory > 0)
-      SL3D_CUDA(cudaMemsetAsync(mixer.gram.p, 0, static_cast<size_t>(memory) * memory * sizeof(double), s));
+    std::fill(mixer.gram.begin(), mixer.gram.end(), 0.0);
     return SL3DGPU_OK;
   }
 };
@@ -771,24 +814,20 @@ int PrepareSolve(SleWorkspace& ws, sl3dgpu_grid* grid, const sl3dgpu_sle_body* b
 
 // field = Synthesise(f_l L + add) of the run's load L (f on the device or the
 // host), its degree-0/2 coefficients patched first by the rotation of L when
-// `patch` (mode: RotationPatchKernel's).
+// `patch` (mode: RotationPatch's). L is in the transforms' device layout.
 int SynthesisePatched(SleWorkspace& ws, bool patch, const double* f, bool factorsOnDevice, const double* add,
                       double* field, int mode) {
   SleRun& run = ws.run;
   const cudaStream_t s = run.stream;
-  if (factorsOnDevice) {
-    ScaleDegreesKernel<<<static_cast<unsigned>((run.coefCount + 255) / 256), 256, 0, s>>>(
-        run.lmax, f, reinterpret_cast<const double2*>(run.loadLm.p), reinterpret_cast<const double2*>(add), 1.0,
-        reinterpret_cast<double2*>(run.scaledLm.p));
-    SL3D_CHECK_LAUNCH();
-  } else {
-    SL3D_TRY(run.ScaleDegrees(f, run.loadLm.p, add, 1.0, run.scaledLm.p));
+  if (!factorsOnDevice) {
+    SL3D_CUDA(cudaMemcpyAsync(run.factors.p, f, (run.lmax + 1) * sizeof(double), cudaMemcpyHostToDevice, s));
+    f = run.factors.p;
   }
-  if (patch) {
-    RotationPatchKernel<<<1, 32, 0, s>>>(ws.rotation.p, run.loadLm.p, run.scaledLm.p, ws.omega.p, mode);
-    SL3D_CHECK_LAUNCH();
-  }
-  return SynthesiseFixed(run.grid, run.scaledLm.p, field, s);
+  ScalePatchKernel<<<dim3((run.lmax + 128) / 128, run.lmax + 1), 128, 0, s>>>(
+      run.lmax, f, reinterpret_cast<const double2*>(run.loadLm.p), reinterpret_cast<const double2*>(add),
+      patch ? ws.rotation.p : nullptr, reinterpret_cast<double2*>(run.scaledLm.p), ws.omega.p, mode);
+  SL3D_CHECK_LAUNCH();
+  return SynthesiseFixed(run.grid, run.scaledLm.p, field, s, true);
 }
 
 // -- the nonlinear solve's pointwise work (src/SeaLevel.cpp:1098-1217) ----------------------------------
@@ -980,9 +1019,9 @@ int SeaLevelSolve(SleWorkspace& ws, sl3dgpu_grid* grid, const sl3dgpu_sle_body* 
   // the seed: sigma + rho_w C s_mean, expanded
   SeedKernel<<<fb, 256, 0, s>>>(run.fieldSize, directData.p, ocean, water_density * meanSlc, run.seeded.p);
   SL3D_CHECK_LAUNCH();
-  SL3D_TRY(ExpandFixed(grid, run.seeded.p, run.loadLm.p, s));
+  SL3D_TRY(ExpandFixed(grid, run.seeded.p, run.loadLm.p, s, true));
 
-  SL3D_TRY(ws.ResetMixer(anderson_memory, s));
+  SL3D_TRY(ws.ResetMixer(anderson_memory));
   LoadMixer& mixer = ws.mixer;
   double err = INFINITY;
   bool converged = false, havePrev = false;
@@ -993,14 +1032,17 @@ int SeaLevelSolve(SleWorkspace& ws, sl3dgpu_grid* grid, const sl3dgpu_sle_body* 
     SL3D_TRY(SynthesisePatched(ws, su.rotating, ws.slcFactor.p, true, slcAdd, run.slc.p, 0));
     RingSumKernel<<<run.ntheta, kRingThreads, 0, s>>>(run.nphi, run.weights.p, ocean, run.slc.p, run.ringPartial.p);
     SL3D_CHECK_LAUNCH();
-    ShiftKernel<<<1, 32, 0, s>>>(run.ringPartial.p, run.ntheta, run.r2 * run.dphi, meanSlc, perOceanArea,
-                                 ws.shift.p);
+    ShiftAndLoadKernel<<<blocks, kRingThreads, 0, s>>>(run.fieldSize, run.ringPartial.p, run.ntheta,
+                                                       run.r2 * run.dphi, meanSlc, perOceanArea, ws.shift.p,
+                                                       water_density, directData.p, ocean, run.slc.p, run.oceanSlc.p,
+                                                       run.newLoad.p, havePrev, run.maxima.p);
     SL3D_CHECK_LAUNCH();
-    ShiftAndLoadKernel<<<blocks, kRingThreads, 0, s>>>(run.fieldSize, ws.shift.p, water_density, directData.p, ocean,
-                                                       run.slc.p, run.oceanSlc.p, run.newLoad.p, havePrev,
-                                                       run.maxima.p);
-    SL3D_CHECK_LAUNCH();
-    SL3D_CUDA(cudaMemcpyAsync(run.hostMaxima.data(), run.maxima.p, 2 * blocks * sizeof(double),
+    // the next load's coefficients and the mixer's sums before the stopping
+    // test, so that one round trip brings both its maxima and the sums (their
+    // small least squares is the host's)
+    SL3D_TRY(ExpandFixed(grid, run.newLoad.p, run.newLoadLm.p, s, true));
+    SL3D_TRY(mixer.Sweep(run.loadLm.p, run.newLoadLm.p, nc, run.MixerSums(), s));
+    SL3D_CUDA(cudaMemcpyAsync(run.hostMaxima, run.maxima.p, run.MaximaCount() * sizeof(double),
                               cudaMemcpyDeviceToHost, s));
     SL3D_CUDA(cudaStreamSynchronize(s));
     if (havePrev) {
@@ -1016,8 +1058,7 @@ int SeaLevelSolve(SleWorkspace& ws, sl3dgpu_grid* grid, const sl3dgpu_sle_body* 
       }
     }
     havePrev = true;
-    SL3D_TRY(ExpandFixed(grid, run.newLoad.p, run.newLoadLm.p, s));
-    SL3D_TRY(mixer.Update(run.loadLm.p, run.newLoadLm.p, nc, s));
+    SL3D_TRY(mixer.Mix(run.loadLm.p, run.newLoadLm.p, nc, run.HostMixerSums(), run.HostGamma(), s));
     ++count;
   }
   // the sea level change is the last one formed; the other fields from the
@@ -1123,7 +1164,7 @@ int SeaLevelSolveNonlinear(SleWorkspace& ws, sl3dgpu_grid* grid, const sl3dgpu_s
   while (count < max_iterations) {
     BudgetLoadKernel<<<fb, 256, 0, s>>>(n, budget, ws.nlOcean.p, ws.nlChange.p, direct, run.newLoad.p);
     SL3D_CHECK_LAUNCH();
-    SL3D_TRY(ExpandFixed(grid, run.newLoad.p, run.loadLm.p, s));
+    SL3D_TRY(ExpandFixed(grid, run.newLoad.p, run.loadLm.p, s, true));
     SL3D_TRY(SynthesisePatched(ws, su.rotating, ws.slcFactor.p, true, slcAdd, ws.nlLocal.p, 0));
     BudgetRingKernel<<<run.ntheta, kRingThreads, 0, s>>>(run.nphi, run.weights.p, budget, ws.nlOcean.p,
                                                          ws.nlLocal.p, dynamic, ws.nlRingUnbalanced.p,
@@ -1135,7 +1176,7 @@ int SeaLevelSolveNonlinear(SleWorkspace& ws, sl3dgpu_grid* grid, const sl3dgpu_s
     BudgetUpdateKernel<<<blocks, kRingThreads, 0, s>>>(n, ws.shift.p, budget, ws.nlLocal.p, dynamic, held, ws.nlSlc.p,
                                                        ws.nlChange.p, ws.nlOcean.p, run.maxima.p);
     SL3D_CHECK_LAUNCH();
-    SL3D_CUDA(cudaMemcpyAsync(run.hostMaxima.data(), run.maxima.p, 4 * blocks * sizeof(double),
+    SL3D_CUDA(cudaMemcpyAsync(run.hostMaxima, run.maxima.p, 4 * blocks * sizeof(double),
                               cudaMemcpyDeviceToHost, s));
     SL3D_CUDA(cudaStreamSynchronize(s));
     double m[4] = {0.0, 0.0, 0.0, 0.0};
@@ -1206,13 +1247,38 @@ int Flotation(long long n, double water_density, double ice_density, const doubl
 
 using namespace sl3dgpu;
 
+namespace {
+// The workspace a solve by handle runs in: the grid's own, kept between
+// solves (its forty allocations and their release were a fifth of an lmax-128
+// solve), or, while another thread's solve holds that, one for the call. A
+// solve waits for its stream before it returns, so the next may use any stream.
+struct GridWorkspace {
+  std::unique_lock<std::mutex> held;
+  std::unique_ptr<SleWorkspace> own;
+  SleWorkspace* ws = nullptr;
+  explicit GridWorkspace(sl3dgpu_grid* grid) {
+    if (grid != nullptr) {
+      GridAttachment& a = AttachmentOf(grid);
+      held = std::unique_lock<std::mutex>(a.lock, std::try_to_lock);
+      if (held.owns_lock()) {
+        if (!a.workspace) a.workspace = std::shared_ptr<void>(new SleWorkspace, [](void* p) { delete static_cast<SleWorkspace*>(p); });
+        ws = static_cast<SleWorkspace*>(a.workspace.get());
+        return;
+      }
+    }
+    own = std::make_unique<SleWorkspace>();
+    ws = own.get();
+  }
+};
+}  // namespace
+
 extern "C" int sl3dgpu_sle_solve(sl3dgpu_grid* grid, const sl3dgpu_sle_body* body, const double* ocean,
                                  const sl3dgpu_sle_forcing* forcing, double rtol, int max_iterations,
                                  int anderson_memory, double* sea_level_change, double* displacement,
                                  double* potential, double* tangential_potential, double* toroidal_potential,
                                  sl3dgpu_sle_result* result, void* stream) {
-  SleWorkspace ws;
-  return SeaLevelSolve(ws, grid, body, ocean, forcing, rtol, max_iterations, anderson_memory, sea_level_change,
+  GridWorkspace ws(grid);
+  return SeaLevelSolve(*ws.ws, grid, body, ocean, forcing, rtol, max_iterations, anderson_memory, sea_level_change,
                        displacement, potential, tangential_potential, toroidal_potential, nullptr, result,
                        AsStream(stream));
 }
@@ -1225,8 +1291,8 @@ extern "C" int sl3dgpu_sle_solve_nonlinear(sl3dgpu_grid* grid, const sl3dgpu_sle
                                            double* toroidal_potential, double* final_sea_level,
                                            double* final_ocean_function, double* load_coefficients,
                                            sl3dgpu_sle_result* result, void* stream) {
-  SleWorkspace ws;
-  return SeaLevelSolveNonlinear(ws, grid, body, ice_density, state, forcing, rtol, max_iterations, sea_level_change,
+  GridWorkspace ws(grid);
+  return SeaLevelSolveNonlinear(*ws.ws, grid, body, ice_density, state, forcing, rtol, max_iterations, sea_level_change,
                                 displacement, potential, tangential_potential, toroidal_potential, final_sea_level,
                                 final_ocean_function, load_coefficients, result, AsStream(stream));
 }

@@ -1311,6 +1311,7 @@ using namespace sl3dgpu;
 
 struct sl3dgpu_grid {
   std::unique_ptr<Grid> grid;
+  GridAttachment attachment;
 };
 
 extern "C" int sl3dgpu_grid_create(int lmax, int nmax, double oversampling, sl3dgpu_grid** out) {
@@ -1409,12 +1410,25 @@ int Expand(sl3dgpu_grid* handle, int N, bool real, const double* fields, int cou
 }  // namespace
 
 namespace sl3dgpu {
-int SynthesiseFixed(sl3dgpu_grid* grid, const double* coeffs, double* field, cudaStream_t stream) {
-  return Synthesise(grid, 0, true, coeffs, 1, field, stream, true);
+int SynthesiseFixed(sl3dgpu_grid* grid, const double* coeffs, double* field, cudaStream_t stream, bool device) {
+  if (!device) return Synthesise(grid, 0, true, coeffs, 1, field, stream, true);
+  auto& g = *grid->grid;
+  double *spectra = nullptr, *unused = nullptr;
+  if (int st = g.Scratch(static_cast<size_t>(g.lmax + 1) * g.ntheta * 2, 0, &spectra, &unused); st != SL3DGPU_OK)
+    return st;
+  if (int st = g.LegendreSynthesis(0, true, coeffs, 1, spectra, stream); st != SL3DGPU_OK) return st;
+  return g.RingSynthesis(true, spectra, 1, field, stream, true);
 }
-int ExpandFixed(sl3dgpu_grid* grid, const double* field, double* coeffs, cudaStream_t stream) {
-  return Expand(grid, 0, true, field, 1, coeffs, stream, true);
+int ExpandFixed(sl3dgpu_grid* grid, const double* field, double* coeffs, cudaStream_t stream, bool device) {
+  if (!device) return Expand(grid, 0, true, field, 1, coeffs, stream, true);
+  auto& g = *grid->grid;
+  double *spectra = nullptr, *unused = nullptr;
+  if (int st = g.Scratch(static_cast<size_t>(g.lmax + 1) * g.ntheta * 2, 0, &spectra, &unused); st != SL3DGPU_OK)
+    return st;
+  if (int st = g.RingAnalysis(true, field, 1, spectra, stream, nullptr, true); st != SL3DGPU_OK) return st;
+  return g.LegendreAnalysis(0, true, spectra, 1, coeffs, stream);
 }
+GridAttachment& AttachmentOf(sl3dgpu_grid* grid) { return grid->attachment; }
 }  // namespace sl3dgpu
 
 extern "C" int sl3dgpu_synthesise_spin_batch(sl3dgpu_grid* grid, int N, const double* coeffs,

@@ -21,6 +21,7 @@
 #include <cstdint>
 #include <map>
 #include <memory>
+#include <mutex>
 #include <vector>
 
 #include "common.cuh"
@@ -205,9 +206,17 @@ class Grid {
 };
 
 // One real field's transforms with the rings in fixed point (the sea-level
-// solver's; reference layouts).
-int SynthesiseFixed(sl3dgpu_grid* grid, const double* coeffs, double* field, cudaStream_t stream);
-int ExpandFixed(sl3dgpu_grid* grid, const double* field, double* coeffs, cudaStream_t stream);
+// solver's), the coefficients in the reference layout or, with `device`, in
+// the transforms' own (an order's degrees together).
+int SynthesiseFixed(sl3dgpu_grid* grid, const double* coeffs, double* field, cudaStream_t stream, bool device = false);
+int ExpandFixed(sl3dgpu_grid* grid, const double* field, double* coeffs, cudaStream_t stream, bool device = false);
+
+// What another part of the library keeps with a grid handle (released with it).
+struct GridAttachment {
+  std::mutex lock;
+  std::shared_ptr<void> workspace;
+};
+GridAttachment& AttachmentOf(sl3dgpu_grid* grid);
 
 // Smallest 2^a 3^b 5^c at or above n.
 int FftFriendly(int n);
