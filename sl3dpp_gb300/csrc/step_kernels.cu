@@ -406,10 +406,9 @@ __global__ void AddLoadKernel(Geometry g, const double2* sigma, const double* un
                               const double* tideUnits, const long long* unitOffset, double2* sol) {
   const int l = blockIdx.x;
   const DegreeInfo d = g.degrees[l];
-  const int cols = l + 1;
-  const long long total = static_cast<long long>(d.sphNdof) * cols;
-  for (long long t = threadIdx.x; t < total; t += blockDim.x) {
-    const int dof = static_cast<int>(t / cols), m = static_cast<int>(t % cols);
+  const int cols = l + 1, total = d.sphNdof * cols;
+  for (int t = blockIdx.y * blockDim.x + threadIdx.x; t < total; t += gridDim.y * blockDim.x) {
+    const int dof = t / cols, m = t - dof * cols;
     double2& x = sol[d.sphRhs + t];
     if (sigma != nullptr) {
       const double2 a = sigma[l * (l + 1) / 2 + m];
@@ -580,33 +579,81 @@ __global__ void CombineKernel(long long values, long long fieldSize, const doubl
 // extrapolated guess, and a NaN in it would otherwise vanish from the
 // maxima (a NaN with its sign bit set is the largest bit pattern, and fmax
 // drops NaNs), under-reporting the change.
+//
+// FP64 instructions are the cost (19 cycles an SM each for a warp): the block
+// sums compare bit patterns, and a square is only formed where its FP32
+// estimate (the bits truncated to FP32, within 2^-18 below) reaches the
+// thread's largest so far; the maxima are the exact squares'.
+__device__ __forceinline__ float TruncatedToFloat(double v) {
+  const uint32_t h = static_cast<uint32_t>(__double2hiint(v)) & 0x7FFFFFFFu;
+  const int e = static_cast<int>(h >> 20) - 896;
+  if (e <= 0) return 0.0f;
+  if (e >= 255) return __int_as_float(0x7F800000);
+  return __uint_as_float((static_cast<uint32_t>(e) << 23) | ((h & 0xFFFFFu) << 3));
+}
+// The largest |v|^2 seen, as bits, and its estimate.
+struct LargestSquare {
+  unsigned long long bits = 0;
+  float estimate = 0.0f;
+  __device__ __forceinline__ void See(double x, double y) {
+    const float fx = TruncatedToFloat(x), fy = TruncatedToFloat(y), square = fx * fx + fy * fy;
+    // outside FP32's comfortable range every square is formed
+    if (square < estimate * 0.9999f && estimate > 1e-30f && estimate < 1e30f) return;
+    estimate = fmaxf(estimate, square);
+    bits = max(bits, static_cast<unsigned long long>(__double_as_longlong(x * x + y * y)));
+  }
+};
+
+// Three block values reduced by their bit patterns (non-negative doubles order
+// as them; the third a flag): 256 threads, the result in thread 0's.
+__device__ __forceinline__ void BlockLargest(unsigned long long& a, unsigned long long& b, unsigned& flag) {
+  __shared__ unsigned long long sa[8], sb[8];
+  __shared__ unsigned sf[8];
+  for (int off = 16; off > 0; off >>= 1) {
+    a = max(a, __shfl_xor_sync(0xffffffffu, a, off));
+    b = max(b, __shfl_xor_sync(0xffffffffu, b, off));
+    flag |= __shfl_xor_sync(0xffffffffu, flag, off);
+  }
+  if (threadIdx.x % 32 == 0) {
+    sa[threadIdx.x / 32] = a;
+    sb[threadIdx.x / 32] = b;
+    sf[threadIdx.x / 32] = flag;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0)
+    for (int w = 1; w < 8; ++w) {
+      a = max(a, sa[w]);
+      b = max(b, sb[w]);
+      flag |= sf[w];
+    }
+}
+
 template <class T2>
-__global__ void RelativeChangeKernel(const T2* next, const T2* now, long long n, double* partial) {
+__global__ void __launch_bounds__(256) RelativeChangeKernel(const T2* next, const T2* now, long long n,
+                                                            double* partial) {
   using T = typename Scalar<T2>::type;
-  __shared__ double s0[256], s1[256], s2[256];
-  T scale = 0, diff = 0;
-  bool finite = true;
+  unsigned long long scaleBits = 0, diffBits = 0;
+  unsigned flag = 0;  // a non-finite value
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
   if constexpr (sizeof(T) == sizeof(double)) {
-    // FP64: the finiteness test and the maxima on the bits (a square is
-    // never negative, and non-negative doubles order as their bit patterns),
-    // so that only the squares and differences use GB300's small FP64 unit
-    unsigned long long scaleBits = 0, diffBits = 0, nonFinite = 0;
-    constexpr unsigned long long kExp = 0x7ff0000000000000ull;
+    LargestSquare largest, change;
+    unsigned nonFinite = 0;
+    const uint32_t kExp = 0x7ff00000u;
+    auto bad = [kExp](double v) {
+      return static_cast<unsigned>((static_cast<uint32_t>(__double2hiint(v)) & kExp) == kExp);
+    };
     for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n; i += stride) {
       const T2 a = next[i], b = now[i];
-      const unsigned long long ax = __double_as_longlong(a.x), ay = __double_as_longlong(a.y);
-      const unsigned long long bx = __double_as_longlong(b.x), by = __double_as_longlong(b.y);
-      nonFinite |= static_cast<unsigned long long>((ax & kExp) == kExp) | static_cast<unsigned long long>((ay & kExp) == kExp) |
-                   static_cast<unsigned long long>((bx & kExp) == kExp) | static_cast<unsigned long long>((by & kExp) == kExp);
-      const double dx = a.x - b.x, dy = a.y - b.y;
-      scaleBits = max(scaleBits, static_cast<unsigned long long>(__double_as_longlong(a.x * a.x + a.y * a.y)));
-      diffBits = max(diffBits, static_cast<unsigned long long>(__double_as_longlong(dx * dx + dy * dy)));
+      nonFinite |= bad(a.x) | bad(a.y) | bad(b.x) | bad(b.y);
+      largest.See(a.x, a.y);
+      change.See(a.x - b.x, a.y - b.y);
     }
-    scale = __longlong_as_double(static_cast<long long>(scaleBits));
-    diff = __longlong_as_double(static_cast<long long>(diffBits));
-    finite = nonFinite == 0;
+    scaleBits = largest.bits;
+    diffBits = change.bits;
+    flag = nonFinite;
   } else {
+    T scale = 0, diff = 0;
+    bool finite = true;
     for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n; i += stride) {
       const T2 a = next[i], b = now[i];
       finite = finite && (a.x - a.x == T(0)) && (a.y - a.y == T(0)) && (b.x - b.x == T(0)) && (b.y - b.y == T(0));
@@ -614,50 +661,31 @@ __global__ void RelativeChangeKernel(const T2* next, const T2* now, long long n,
       const T dx = a.x - b.x, dy = a.y - b.y;
       diff = fmax(diff, dx * dx + dy * dy);
     }
+    scaleBits = static_cast<unsigned long long>(__double_as_longlong(static_cast<double>(scale)));
+    diffBits = static_cast<unsigned long long>(__double_as_longlong(static_cast<double>(diff)));
+    flag = finite ? 0u : 1u;
   }
-  s0[threadIdx.x] = static_cast<double>(scale);
-  s1[threadIdx.x] = static_cast<double>(diff);
-  s2[threadIdx.x] = finite ? 1.0 : 0.0;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w /= 2) {
-    if (threadIdx.x < w) {
-      s0[threadIdx.x] = fmax(s0[threadIdx.x], s0[threadIdx.x + w]);
-      s1[threadIdx.x] = fmax(s1[threadIdx.x], s1[threadIdx.x + w]);
-      s2[threadIdx.x] = fmin(s2[threadIdx.x], s2[threadIdx.x + w]);
-    }
-    __syncthreads();
-  }
+  BlockLargest(scaleBits, diffBits, flag);
   if (threadIdx.x == 0) {
-    partial[blockIdx.x * 3 + 0] = s0[0];
-    partial[blockIdx.x * 3 + 1] = s1[0];
-    partial[blockIdx.x * 3 + 2] = s2[0];
+    partial[blockIdx.x * 3 + 0] = __longlong_as_double(static_cast<long long>(scaleBits));
+    partial[blockIdx.x * 3 + 1] = __longlong_as_double(static_cast<long long>(diffBits));
+    partial[blockIdx.x * 3 + 2] = flag ? 0.0 : 1.0;
   }
 }
 
-__global__ void ReduceMaxKernel(const double* partial, int count, double* result) {
-  __shared__ double s0[256], s1[256], s2[256];
-  double a = 0.0, b = 0.0, c = 1.0;
+__global__ void __launch_bounds__(256) ReduceMaxKernel(const double* partial, int count, double* result) {
+  unsigned long long a = 0, b = 0;
+  unsigned flag = 0;
   for (int i = threadIdx.x; i < count; i += blockDim.x) {
-    a = fmax(a, partial[3 * i]);
-    b = fmax(b, partial[3 * i + 1]);
-    c = fmin(c, partial[3 * i + 2]);
+    a = max(a, static_cast<unsigned long long>(__double_as_longlong(partial[3 * i])));
+    b = max(b, static_cast<unsigned long long>(__double_as_longlong(partial[3 * i + 1])));
+    flag |= __double_as_longlong(partial[3 * i + 2]) == 0 ? 1u : 0u;
   }
-  s0[threadIdx.x] = a;
-  s1[threadIdx.x] = b;
-  s2[threadIdx.x] = c;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w /= 2) {
-    if (threadIdx.x < w) {
-      s0[threadIdx.x] = fmax(s0[threadIdx.x], s0[threadIdx.x + w]);
-      s1[threadIdx.x] = fmax(s1[threadIdx.x], s1[threadIdx.x + w]);
-      s2[threadIdx.x] = fmin(s2[threadIdx.x], s2[threadIdx.x + w]);
-    }
-    __syncthreads();
-  }
+  BlockLargest(a, b, flag);
   if (threadIdx.x == 0) {
-    result[0] = s0[0];
-    result[1] = s1[0];
-    result[2] = s2[0];
+    result[0] = __longlong_as_double(static_cast<long long>(a));
+    result[1] = __longlong_as_double(static_cast<long long>(b));
+    result[2] = flag ? 0.0 : 1.0;
   }
 }
 
@@ -1096,15 +1124,21 @@ namespace {
 // Orders a block of the chunked maps takes: the most (up to 32) whose
 // shared-memory rows fit a budget that leaves room for two blocks an SM.
 constexpr size_t kChunkSmemBudget = 110 * 1024;
-inline int ChunkOrders(size_t bytesPerOrder, size_t fixedBytes) {
-  int mc = 32;
-  while (mc > 1 && fixedBytes + bytesPerOrder * mc > kChunkSmemBudget) mc /= 2;
-  return mc;
-}
 inline int ChunkBlocks(int lmax, int mc) {  // sum over l <= lmax of (floor(l / mc) + 1)
   long long blocks = 0;
   for (int l = 0; l <= lmax; ++l) blocks += l / mc + 1;
   return static_cast<int>(blocks);
+}
+
+// Orders a block: what the budget holds, and fewer where that would leave SMs
+// idle (blocks for two an SM, while a block keeps some 128 nodes' work): at
+// lmax 32 the strain's 34 blocks of 32 orders took 112 us on the FP64 unit.
+constexpr int kChunkBlocks = 2 * 152;
+inline int ChunkOrders(size_t bytesPerOrder, size_t fixedBytes, int lmax, int nodes) {
+  int mc = 32;
+  while (mc > 1 && fixedBytes + bytesPerOrder * mc > kChunkSmemBudget) mc /= 2;
+  while (mc > 1 && ChunkBlocks(lmax, mc) < kChunkBlocks && mc / 2 * nodes >= 128) mc /= 2;
+  return mc;
 }
 
 template <class T2, int MC>
@@ -1125,7 +1159,7 @@ void StrainWith(const Geometry& g, const T2* solSph, const T2* solTor, T2* spect
 template <class T2>
 void Forces(const Geometry& g, const T2* spectral, T2* rhsSph, T2* rhsTor, cudaStream_t stream) {
   prof::Scope scope(prof::kForce, stream);
-  switch (ChunkOrders(static_cast<size_t>(6) * (g.P | 1) * sizeof(T2), 0)) {
+  switch (ChunkOrders(static_cast<size_t>(6) * (g.P | 1) * sizeof(T2), 0, g.lmax, g.P)) {
     case 32: return ForcesWith<T2, 32>(g, spectral, rhsSph, rhsTor, stream);
     case 16: return ForcesWith<T2, 16>(g, spectral, rhsSph, rhsTor, stream);
     case 8: return ForcesWith<T2, 8>(g, spectral, rhsSph, rhsTor, stream);
@@ -1140,7 +1174,7 @@ void Strain(const Geometry& g, const T2* solSph, const T2* solTor, T2* spectral,
             cudaStream_t stream) {
   prof::Scope scope(prof::kStrain, stream);
   const size_t globals = static_cast<size_t>(std::max(g.maxGlobals, 1));
-  switch (ChunkOrders(globals * 3 * sizeof(T2), globals * sizeof(T2))) {
+  switch (ChunkOrders(globals * 3 * sizeof(T2), globals * sizeof(T2), g.lmax, g.P)) {
     case 32: return StrainWith<T2, 32>(g, solSph, solTor, spectral, add, stream);
     case 16: return StrainWith<T2, 16>(g, solSph, solTor, spectral, add, stream);
     case 8: return StrainWith<T2, 8>(g, solSph, solTor, spectral, add, stream);
@@ -1187,7 +1221,9 @@ void LaunchAddLoad(const Geometry& g, const double2* sigma, const double* units,
                    double2* solSph, cudaStream_t stream, const double2* tide, const double* tideUnits) {
   if (sigma == nullptr && tide == nullptr) return;
   prof::Scope scope(prof::kOther, stream);
-  AddLoadKernel<<<g.lmax + 1, 256, 0, stream>>>(g, sigma, units, tide, tideUnits, unitOffset, solSph);
+  // several blocks a degree: a degree's values are some thousands
+  AddLoadKernel<<<dim3(g.lmax + 1, g.lmax < 128 ? 16 : 8), 256, 0, stream>>>(g, sigma, units, tide, tideUnits,
+                                                                            unitOffset, solSph);
 }
 
 void LaunchSurface(const Geometry& g, const double2* solSph, const double2* solTor, int component, double2* out,

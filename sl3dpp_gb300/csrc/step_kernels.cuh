@@ -7,6 +7,8 @@
 
 #include <vector>
 
+#include <cstdint>
+
 #include <cuda_bf16.h>
 
 #include "common.cuh"
