@@ -474,6 +474,9 @@ __global__ void __launch_bounds__(256, (R1 > 0 && sizeof(T2) == 8) ? 3 : 1)
   const int groups = min(G * perRing, count - p0);  // fields of this CTA
   const int rings = (groups + perRing - 1) / perRing;
   const int mcount = real ? lmax + 1 : 2 * lmax + 1;
+  // divisions by the CTA's rings and fields as multiplications (the spectra's
+  // elements are many and the integer division was most of their cost)
+  const uint32_t byRings = 0xFFFFFFFFu / rings + 1u, byGroups = 0xFFFFFFFFu / groups + 1u;
   if (mode == kRingSynth || mode == kRingWeighted) {
     // ask L2 for this CTA's spectra (one line an order) and, weighted, for
     // the rings' point weights (read after the synthesis): their DRAM
@@ -500,12 +503,11 @@ __global__ void __launch_bounds__(256, (R1 > 0 && sizeof(T2) == 8) ? 3 : 1)
   const long long row0 = (static_cast<long long>(f0) * ntheta + j) * n;
   const long long row1 = (static_cast<long long>(f1) * ntheta + j) * n;
   if (mode == kRingSynth || mode == kRingWeighted) {
-    for (int e = threadIdx.x; e < G * n; e += blockDim.x)
-      bufs[ringStride * (e / n) + e % n] = Make<T2>(0, 0);
+    for (int k = lane; k < n; k += kWarp) a[k] = Make<T2>(0, 0);  // this warp's ring (the first of its buffers)
     __syncthreads();
 #pragma unroll 4
     for (int e = threadIdx.x; e < mcount * rings; e += blockDim.x) {
-      const int r = e % rings, mi = e / rings;
+      const int mi = rings > 1 ? static_cast<int>(FxDivide(static_cast<uint32_t>(e), byRings)) : e, r = e - mi * rings;
       const int m = real ? mi : mi - lmax;
       const long long at0 = (static_cast<long long>(mi) * ntheta + j) * count + p0 + perRing * r;
       const T2 v = (spectraIn[at0]);
@@ -583,7 +585,7 @@ __global__ void __launch_bounds__(256, (R1 > 0 && sizeof(T2) == 8) ? 3 : 1)
   const T scale = T(static_cast<T>(2.0 * 3.14159265358979323846 / n * weights[j]));
 #pragma unroll 4
   for (int e = threadIdx.x; e < mcount * groups; e += blockDim.x) {
-    const int g = e % groups, mi = e / groups;
+    const int mi = groups > 1 ? static_cast<int>(FxDivide(static_cast<uint32_t>(e), byGroups)) : e, g = e - mi * groups;
     const int m = real ? mi : mi - lmax;
     const T2* ring = bufs + ringStride * (g / perRing) + (out ? n : 0);
     T2 v;

@@ -131,7 +131,61 @@ __global__ void PackBKernel(const TcItem* tcItems, int tileN, const float* B, fl
 // gone, and B is read at 4 bytes a value.
 constexpr int kPackWarps = 4;  // warps 6 .. 9, a step each in turn
 constexpr int kPersistentThreads = 32 * (6 + kPackWarps);
-constexpr int kPackChunk = 16;  // (column, group) items a lane loads before it stores (64 reads in flight)
+constexpr int kPackChunk = 16;  // (column, 4-deep group) items a lane loads before it stores (64 reads in flight)
+
+// One bulk copy into shared memory, counted on `bar`.
+__device__ __forceinline__ void CopyTile(uint32_t to, const float* from, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(to),
+               "l"(from), "r"(bytes), "r"(bar)
+               : "memory");
+}
+
+// A step's 16 x tileN slice of B, split into TF32 parts and stored in the
+// stage's tile: a lane's columns are lane + 32 j (j < J, tileN <= 32 J), so
+// that an item's place needs no division (the index arithmetic was three
+// quarters of the packing warps' instructions). The first chunk's values are
+// loaded before `wait`. False when `wait` gave up. The MMA issue sets the
+// kernel's pace: its lane waits 30 of 100 cycles for a stage, and a 16-deep
+// step's four TF32 MMAs take about 1070 cycles.
+template <int J, class Wait>
+__device__ __forceinline__ bool PackStep(const float* from, int ldb, int columns, int depth, int tileN, float* out,
+                                         int lane, Wait wait) {
+  constexpr int kGroups = kPackChunk / J;  // 4-deep groups a chunk
+#pragma unroll
+  for (int first = 0; first < kTcTileK / 4; first += kGroups) {
+    float v[kGroups][J][4];
+#pragma unroll
+    for (int gr = 0; gr < kGroups; ++gr)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int k = 4 * (first + gr) + q;
+        const float* row = from + static_cast<long long>(k) * ldb + lane;
+#pragma unroll
+        for (int j = 0; j < J; ++j)
+          v[gr][j][q] = (lane + 32 * j < columns && k < depth) ? __ldg(row + 32 * j) : 0.0f;
+      }
+    if (first == 0 && !wait()) return false;
+#pragma unroll
+    for (int gr = 0; gr < kGroups; ++gr)
+#pragma unroll
+      for (int j = 0; j < J; ++j) {
+        const int nn = lane + 32 * j;
+        if (nn >= tileN) continue;
+        float4 hi, lo;
+        hi.x = RoundTf32(v[gr][j][0]);
+        hi.y = RoundTf32(v[gr][j][1]);
+        hi.z = RoundTf32(v[gr][j][2]);
+        hi.w = RoundTf32(v[gr][j][3]);
+        lo.x = v[gr][j][0] - hi.x;
+        lo.y = v[gr][j][1] - hi.y;
+        lo.z = v[gr][j][2] - hi.z;
+        lo.w = v[gr][j][3] - hi.w;
+        *reinterpret_cast<float4*>(out + TileIndex(nn, 4 * (first + gr), 2 * tileN)) = hi;
+        *reinterpret_cast<float4*>(out + TileIndex(tileN + nn, 4 * (first + gr), 2 * tileN)) = lo;
+      }
+  }
+  return true;
+}
 
 __global__ void __launch_bounds__(kPersistentThreads, 1)
     TcGemmKernel(const TcItem* tcItems, const int4* tiles, int tileCount, int tileN, int stages,
@@ -194,6 +248,11 @@ __global__ void __launch_bounds__(kPersistentThreads, 1)
       const TcItem it = tcItems[tile.x];
       const float* aSrc = panels + it.aPanel + static_cast<long long>(tile.y) * it.kSteps * 2 * kATileFloats;
       const float* bSrc = packed + it.bPack + static_cast<long long>(tile.z) * it.kSteps * 2 * bTileFloats;
+      // A tile's rows past the item's are not copied (their products are not
+      // stored): a quarter of the table's tiles at lmax 256, whose 385
+      // colatitudes fill one row of their fourth tile
+      const int rowGroups = min(kTcTileM, it.M - tile.y * kTcTileM + 7) / 8;
+      const uint32_t aTile = 2 * kTcTileK / 4 * 128u * rowGroups;
       for (int ks = 0; ks < it.kSteps; ++ks, ++g) {
         const int slot = static_cast<int>(g % stages);
         const long long round = g / stages;
@@ -204,13 +263,17 @@ __global__ void __launch_bounds__(kPersistentThreads, 1)
         if (abortFlag) break;
         const uint32_t bar = SmemAddr(full + slot);
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
-                     "r"(rawB != nullptr ? aBytes : aBytes + bBytes)
+                     "r"(rawB != nullptr ? aTile : aTile + bBytes)
                      : "memory");
-        asm volatile(
-            "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                SmemAddr(sA + slot * 2 * kATileFloats)),
-            "l"(aSrc + static_cast<long long>(ks) * 2 * kATileFloats), "r"(aBytes), "r"(bar)
-            : "memory");
+        const float* aFrom = aSrc + static_cast<long long>(ks) * 2 * kATileFloats;
+        if (rowGroups == kTcTileM / 8) {
+          CopyTile(SmemAddr(sA + slot * 2 * kATileFloats), aFrom, aBytes, bar);
+        } else {
+          // the 8-row groups in range of each part's 4-deep K groups
+          for (int q = 0; q < 2 * kTcTileK / 4; ++q)
+            CopyTile(SmemAddr(sA + slot * 2 * kATileFloats + q * kTcTileM * 4), aFrom + q * kTcTileM * 4,
+                     rowGroups * 128u, bar);
+        }
         if (rawB == nullptr)
           asm volatile(
               "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
@@ -315,61 +378,29 @@ __global__ void __launch_bounds__(kPersistentThreads, 1)
     // stores any (its loads overlap)
     if (rawB != nullptr) {
       const int packer = warp - 6;
-      const int groups = kTcTileK / 4;
       long long g = 0;
       bool ok = true;
       for (int t = blockIdx.x; t < tileCount && !abortFlag && ok; t += gridDim.x) {
         const int4 tile = tiles[t];
         const TcItem it = tcItems[tile.x];
         const int nBase = tile.z * tileN;
-        const int items = tileN * groups;
         for (int ks = 0; ks < it.kSteps; ++ks, ++g) {
           if (static_cast<int>(g % kPackWarps) != packer) continue;
           const int slot = static_cast<int>(g % stages);
           const long long round = g / stages;
           float* out = sB + slot * 2 * bTileFloats;
+          const float* from = rawB + it.b + static_cast<long long>(ks) * kTcTileK * it.ldb + nBase;
+          const int columns = min(tileN, it.N - nBase), depth = min(kTcTileK, it.K - ks * kTcTileK);
           // B's values are read before the slot is waited for (they go to
           // registers): their global latency overlaps the wait
-          bool waited = false;
-          for (int first = 0; first < items; first += 32 * kPackChunk) {
-            float v[kPackChunk][4];
-#pragma unroll
-            for (int j = 0; j < kPackChunk; ++j) {
-              const int item = first + lane + 32 * j;
-              const int nn = item % tileN, grp = item / tileN;
-              const int n = nBase + nn, k0 = ks * kTcTileK + 4 * grp;
-              const bool in = item < items && n < it.N;
-#pragma unroll
-              for (int q = 0; q < 4; ++q)
-                v[j][q] = (in && k0 + q < it.K) ? __ldg(rawB + it.b + static_cast<long long>(k0 + q) * it.ldb + n)
-                                                : 0.0f;
-            }
-            if (!waited) {
-              waited = true;
-              if (round > 0 && !WaitParity(SmemAddr(empty + slot), static_cast<uint32_t>((round - 1) & 1))) {
-                ok = false;
-                break;
-              }
-              if (abortFlag) break;
-            }
-#pragma unroll
-            for (int j = 0; j < kPackChunk; ++j) {
-              const int item = first + lane + 32 * j;
-              if (item >= items) break;
-              const int nn = item % tileN, grp = item / tileN;
-              float4 hi, lo;
-              hi.x = RoundTf32(v[j][0]);
-              hi.y = RoundTf32(v[j][1]);
-              hi.z = RoundTf32(v[j][2]);
-              hi.w = RoundTf32(v[j][3]);
-              lo.x = v[j][0] - hi.x;
-              lo.y = v[j][1] - hi.y;
-              lo.z = v[j][2] - hi.z;
-              lo.w = v[j][3] - hi.w;
-              *reinterpret_cast<float4*>(out + TileIndex(nn, 4 * grp, 2 * tileN)) = hi;
-              *reinterpret_cast<float4*>(out + TileIndex(tileN + nn, 4 * grp, 2 * tileN)) = lo;
-            }
-          }
+          auto wait = [&] {
+            if (round > 0 && !WaitParity(SmemAddr(empty + slot), static_cast<uint32_t>((round - 1) & 1))) ok = false;
+            return ok && !abortFlag;
+          };
+          if (tileN <= 128)
+            ok = PackStep<4>(from, it.ldb, columns, depth, tileN, out, lane, wait) && ok;
+          else
+            ok = PackStep<8>(from, it.ldb, columns, depth, tileN, out, lane, wait) && ok;
           if (!ok || abortFlag) break;
           // the stores visible to the tensor cores before the stage is full
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
