@@ -907,7 +907,7 @@ int Grid::BatchFor(int N, bool real, bool analysis, int P, int p0, int count, co
       for (int nt = 0; nt < h.nTiles; ++nt)
         b.tcTiles.push_back(make_int4(static_cast<int>(b.tcHost.size()), mt, nt, 0));
     b.tcHost.push_back(h);
-    // the FP64 slices' tiles: 128 rows, 64 columns, 16 deep
+    // the FP64 slices' tiles: 128 rows, 32 columns, 16 deep
     Tc64Item e{};
     e.M = g.M;
     e.N = g.N;

@@ -52,12 +52,12 @@ struct GemmItem {
 };
 
 // One item of the FP64 contraction emulated on the tensor cores: 128-row
-// tiles of A, 64-column tiles of B, 16-deep steps.
+// tiles of A, 32-column tiles of B, 16-deep steps.
 struct Tc64Item {
   int M, N, K, mTiles;
   int kSteps, nTiles, ldc, ldb;
   long long aPanel;  // tiles: the item's panel, [mTile][kStep] of [slice][128 x 16]
-  long long bPack;   // tiles: its packed B, [nTile][kStep] of [slice][64 x 16]
+  long long bPack;   // tiles: its packed B, [nTile][kStep] of [slice][32 x 16]
   long long b, c;    // FP64 offsets of B's source and of C
   long long rowExp;  // ints: the power-of-two exponents of its M rows of A
   long long colExp;  // ints: those of its N columns of B (per call)

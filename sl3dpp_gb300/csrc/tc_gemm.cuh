@@ -95,7 +95,7 @@ int RunGemmTc(const TcItem* tcItems, const int4* tiles, int tileCount, int tileN
 // relative to (row maximum) x (column maximum) x K.
 constexpr int kTc64Slices = 7;       // a grid that asked for the emulation
 constexpr int kTc64SlicesFull = 8;   // the default FP64 contraction
-constexpr int kTc64TileN = 64;       // up to 8 accumulators of 64 columns in tensor memory
+constexpr int kTc64TileN = 32;       // up to 8 accumulators of 32 columns in half of tensor memory
 // The exactness bounds on the depth (455 and 409), with margin.
 __host__ __device__ constexpr int Tc64MaxK(int slices) { return slices == kTc64SlicesFull ? 400 : 448; }
 

@@ -35,22 +35,22 @@
 // themselves, as the FP64 units would give them (the packed digits of such a
 // column are not used). A wait that gives up leaves NaN in its tile.
 //
-// Kernel. One CTA of eight warps per (64-column tile, 128-row tile, item),
-// the column tiles of a row tile adjacent in the launch so that its A panel
-// is read from HBM once. One elected thread runs the K loop as the FP32
-// contraction does (tc_gemm.cu): it arms a stage's "full" mbarrier, issues
-// two TMA bulk copies (A's S slices, 4 KB each; B's, 2 KB each), four stages
-// in flight, and when they have landed issues the step's tcgen05.mma
-// kind::f16 into the level accumulators (tensor-memory columns 64 d ..
-// 64 d + 63 of 512) and commits them to the stage's "empty" mbarrier. B's
-// slices are stored as one operand of 64 S rows, slice q in rows 64 q ..
-// 64 q + 63, so that one MMA of N = 64 c multiplies A's slice p by c
-// consecutive slices q0 .. q0 + c - 1 into the c consecutive levels
-// p + q0 ..: the 28 (36) products of a step take 10 (12) MMAs of N up to 256
-// (the same tensor work, in fewer instructions for the one issuing thread).
-// Every wait has an iteration limit. The epilogue reads the levels with
-// tcgen05.ld, two warps per lane quarter (a column half each), joins them
-// and stores (or adds) the rows in range.
+// Kernel. One CTA of eight warps per (32-column tile, 128-row tile, item),
+// two an SM, so that one's epilogue runs beside the other's products (with 64
+// columns the levels filled tensor memory and every CTA's epilogue, a third
+// to a half of its time, left the tensor pipe idle); the column tiles of a row
+// tile are adjacent in the launch so that its A panel is read from HBM once.
+// One elected thread runs the K loop as the FP32 contraction does
+// (tc_gemm.cu): it arms a stage's "full" mbarrier, issues two TMA bulk copies
+// (A's S slices, 4 KB each; B's, 1 KB each), and when they have landed issues
+// the step's tcgen05.mma kind::f16 into the level accumulators
+// (tensor-memory columns 32 d .. 32 d + 31 of 256) and commits them to the
+// stage's "empty" mbarrier. B's slices are stored as one operand of 32 S rows,
+// slice q in rows 32 q .. 32 q + 31, so that one MMA of N = 32 (S - p)
+// multiplies A's slice p by the slices 0 .. S - 1 - p into the consecutive
+// levels p ..: a step takes S MMAs. Every wait has an iteration limit. The
+// epilogue reads the levels with tcgen05.ld, two warps per lane quarter (a
+// column half each), joins them and stores (or adds) the rows in range.
 #include <climits>
 #include <cstdint>
 
@@ -61,12 +61,12 @@ namespace sl3dgpu {
 namespace {
 
 constexpr int kTileN = kTc64TileN;
-constexpr int kStages = 4;
+constexpr int kStages = 2;     // a CTA; two CTAs an SM
 constexpr int kThreads = 256;  // eight warps: two per tensor-memory lane quarter in the epilogue
 constexpr int kATile = kTcTileM * kTcTileK;  // BF16 values of one slice of an A tile: 2048 (4 KB)
-constexpr int kBTile = kTileN * kTcTileK;    // of a B tile: 1024 (2 KB)
-constexpr int kBSlice = kTileN * 8;          // BF16 offset of the next slice's rows (8 row groups of 64)
-constexpr uint32_t kTmemColumns = 512;       // up to 8 levels x 64 columns
+constexpr int kBTile = kTileN * kTcTileK;    // of a B tile: 512 (1 KB)
+constexpr int kBSlice = kTileN * 8;          // BF16 offset of the next slice's rows (4 row groups of 64)
+constexpr uint32_t kTmemColumns = 256;       // up to 8 levels x 32 columns: two CTAs an SM
 constexpr int kNonFinite = INT_MIN;           // the exponent of a column that holds an infinity or a NaN
 
 static_assert(kTc64Slices * kTileN <= static_cast<int>(kTmemColumns) &&
@@ -234,8 +234,8 @@ __global__ void PanelA64Kernel(const GemmItem* items, const Tc64Item* tcItems, c
 }
 
 // B's column exponents and packed slices, one CTA of 256 threads per
-// (column tile, item): 64 columns x 4 lanes along k. The exponents first
-// (each lane's maximum over its k, then over the four lanes), then the
+// (column tile, item): 32 columns x 8 lanes along k. The exponents first
+// (each lane's maximum over its k, then over the eight lanes), then the
 // slices, 8-deep k groups in turn; a warp's reads of one k are 32
 // consecutive columns and its stores of one slice 512 contiguous bytes.
 constexpr int kPackThreads = 256, kPackLanes = kPackThreads / kTileN;
@@ -275,7 +275,7 @@ __global__ void __launch_bounds__(kPackThreads) PackB64Kernel(const Tc64Item* tc
 }
 
 template <int S>
-__global__ void __launch_bounds__(kThreads) TcGemm64Kernel(const GemmItem* items, const Tc64Item* tcItems,
+__global__ void __launch_bounds__(kThreads, 2) TcGemm64Kernel(const GemmItem* items, const Tc64Item* tcItems,
                                                            const double* table, const double* B,
                                                            const uint16_t* panels, const uint16_t* packed,
                                                            const int* rowExp, const int* colExp, double* C,
@@ -322,7 +322,7 @@ __global__ void __launch_bounds__(kThreads) TcGemm64Kernel(const GemmItem* items
   if (tid == 0) {
     const uint16_t* aSrc = panels + (it.aPanel + static_cast<long long>(mt) * it.kSteps) * kSlices * kATile;
     const uint16_t* bSrc = packed + (it.bPack + static_cast<long long>(nt) * it.kSteps) * kSlices * kBTile;
-    uint32_t phaseFull[kStages] = {0, 0, 0, 0}, phaseEmpty[kStages] = {0, 0, 0, 0};
+    uint32_t phaseFull[kStages] = {}, phaseEmpty[kStages] = {};
     bool ok = true;
     int issued = 0, landed = 0;  // steps whose copies were started, and waited for
     auto issue = [&](int ks) {
@@ -360,23 +360,19 @@ __global__ void __launch_bounds__(kThreads) TcGemm64Kernel(const GemmItem* items
       const uint32_t aBase = SmemAddr(sA + buf * kSlices * kATile);
       const uint32_t bBase = SmemAddr(sB + buf * kSlices * kBTile);
       constexpr uint32_t aLbo = kTcTileM * 16, bLbo = kBRows * 16, sbo = 128;
-      // A's slice p against B's slices q0 .. q0 + c - 1 (c <= 4, N = 64 c),
-      // levels p + q0 .. p + q0 + c - 1; p = 0 writes every level first.
+      // A's slice p against B's slices 0 .. S - 1 - p (N = 32 (S - p)), levels
+      // p .. S - 1; p = 0 writes every level first.
 #pragma unroll
       for (int p = 0; p < kSlices; ++p) {
         const uint64_t dA = Descriptor(aBase + p * kATile * 2, aLbo, sbo);
+        const uint64_t dB = Descriptor(bBase, bLbo, sbo);
         const uint32_t enable = (ks > 0 || p > 0) ? 1u : 0u;
-#pragma unroll
-        for (int q0 = 0; q0 < kSlices - p; q0 += 4) {
-          const int c = min(4, kSlices - p - q0);
-          const uint64_t dB = Descriptor(bBase + q0 * kBSlice * 2, bLbo, sbo);
-          asm volatile(
-              "{\n\t.reg .pred r;\n\t"
-              "setp.ne.b32 r, %4, 0;\n\t"
-              "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, r;\n\t}" ::"r"(tmem + (p + q0) * kTileN),
-              "l"(dA), "l"(dB), "r"(InstrDescriptorBf16(c * kTileN, kTcTileM)), "r"(enable)
-              : "memory");
-        }
+        asm volatile(
+            "{\n\t.reg .pred r;\n\t"
+            "setp.ne.b32 r, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, r;\n\t}" ::"r"(tmem + p * kTileN),
+            "l"(dA), "l"(dB), "r"(InstrDescriptorBf16((kSlices - p) * kTileN, kTcTileM)), "r"(enable)
+            : "memory");
       }
       asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                        SmemAddr(empty + buf))
