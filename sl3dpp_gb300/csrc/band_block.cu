@@ -164,6 +164,136 @@ __global__ void __launch_bounds__(kBlockWarps* kWarp) BlockSolveKernel(const Blo
   }
 }
 
+// The FP32 solves over row windows (the mixed form's corrections), the same
+// recurrence: four columns a lane, so that a coefficient read from shared
+// memory serves four products. FP32 chains are short; what bounded the
+// row-by-row kernel was its instructions a row at a few warps an SM. A
+// correction pass's solves: lmax 64 97 -> 28 us, lmax 128 157 -> 54 us.
+template <int B>
+__global__ void __launch_bounds__(kBlockWarps* kWarp) BlockSolve32Kernel(const BlockSystem* systems, const int2* items,
+                                                                        int firstCount, const float* data,
+                                                                        float* first, float* second,
+                                                                        const float* scales, const int2* windowsFirst,
+                                                                        const int2* windowsSecond, int maxKd) {
+  constexpr int C = kWarp / B;  // groups of four columns a warp
+  extern __shared__ __align__(16) unsigned char block32Smem[];
+  const int2 item = items[blockIdx.x];
+  const BlockSystem s = systems[item.x];
+  const int2 range = item.x < firstCount ? windowsFirst[item.x] : windowsSecond[item.x - firstCount];
+  const int n = s.n, kd = s.kd, values = (kd + B) * B;
+  const int lo = min(max(range.x, 0), n), hi = min(range.y, n - 1);
+  const int b0 = lo / B, steps = s.blocks - b0;
+  if (lo >= n) return;
+  const int W = ((maxKd + B - 1) / B + 1) * B;
+  const int warp = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
+  const int r = lane % B, c = lane / B;
+  const int col = item.y + (warp * C + c) * 4;
+  const bool live0 = col < s.nrhs, live1 = col + 2 < s.nrhs;  // column pairs (nrhs is even)
+  float* stages = reinterpret_cast<float*>(block32Smem);
+  const int stageValues = (maxKd + B) * B;
+  float4* window = reinterpret_cast<float4*>(stages + kBlockStages * stageValues) + warp * (W + B) * C;
+  float4* input = window + W * C;
+  float* x = (s.second ? second : first) + s.rhs + col;
+  const long long nrhs = s.nrhs;
+  const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+
+  auto stage = [&](const float* from, int slot) {
+    float* to = stages + slot * stageValues;
+    for (int e = threadIdx.x; e < values / 4; e += kBlockWarps * kWarp) {
+      const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(to + 4 * e));
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(from + 4 * e) : "memory");
+    }
+  };
+  auto commit = [] { asm volatile("cp.async.commit_group;\n" ::: "memory"); };
+  auto load = [&](int row) {
+    float4 v = zero;
+    if (live0) {
+      const float2 p = *reinterpret_cast<const float2*>(x + row * nrhs);
+      v.x = p.x;
+      v.y = p.y;
+    }
+    if (live1) {
+      const float2 p = *reinterpret_cast<const float2*>(x + row * nrhs + 2);
+      v.z = p.x;
+      v.w = p.y;
+    }
+    return v;
+  };
+
+  for (int direction = 0; direction < 2; ++direction) {
+    const bool forward = direction == 0;
+    const float* coefficients = data + (forward ? s.forward : s.backward);
+    const int last = forward ? hi : n - 1;  // forward rows above hi are zero and not read
+    auto blockOf = [&](int step) { return forward ? b0 + step : s.blocks - 1 - step; };
+    __syncthreads();
+    for (int q = 0; q < kBlockStages - 1; ++q) {
+      if (q < steps) stage(coefficients + static_cast<long long>(blockOf(q)) * values, q);
+      commit();
+    }
+    for (int e = lane; e < W * C; e += kWarp) window[e] = zero;
+    int row = blockOf(0) * B + r;
+    float4 next = row >= lo && row <= last ? load(row) : zero;
+    __syncwarp();
+    for (int step = 0; step < steps; ++step) {
+      asm volatile("cp.async.wait_group %0;\n" ::"n"(kBlockStages - 2) : "memory");
+      __syncthreads();
+      const int ahead = step + kBlockStages - 1;
+      if (ahead < steps) stage(coefficients + static_cast<long long>(blockOf(ahead)) * values, ahead % kBlockStages);
+      commit();
+      const float* N = stages + (step % kBlockStages) * stageValues + r;
+      const float* M = N + kd * B;
+      const int j0 = blockOf(step) * B;
+      row = j0 + r;
+      input[r * C + c] = next;
+      if (step + 1 < steps) {
+        const int later = blockOf(step + 1) * B + r;
+        next = later >= lo && later <= last ? load(later) : zero;
+      }
+      __syncwarp();
+      float4 sum = zero;
+#pragma unroll
+      for (int k = 0; k < B; ++k) {
+        const float m = M[k * B];
+        const float4 v = input[k * C + c];
+        sum.x = fmaf(m, v.x, sum.x);
+        sum.y = fmaf(m, v.y, sum.y);
+        sum.z = fmaf(m, v.z, sum.z);
+        sum.w = fmaf(m, v.w, sum.w);
+      }
+      int at = forward ? j0 % W : (j0 + B - 1) % W;
+#pragma unroll 4
+      for (int t = 0; t < kd; ++t) {
+        at = forward ? (at == 0 ? W - 1 : at - 1) : (at == W - 1 ? 0 : at + 1);
+        const float m = -N[t * B];
+        const float4 v = window[at * C + c];
+        sum.x = fmaf(m, v.x, sum.x);
+        sum.y = fmaf(m, v.y, sum.y);
+        sum.z = fmaf(m, v.z, sum.z);
+        sum.w = fmaf(m, v.w, sum.w);
+      }
+      __syncwarp();
+      window[(row % W) * C + c] = sum;
+      __syncwarp();
+      if (row >= lo && row < n) {
+        const float f = !forward && s.scale >= 0 ? scales[s.scale + row] : 1.0f;
+        if (live0) *reinterpret_cast<float2*>(x + row * nrhs) = make_float2(sum.x * f, sum.y * f);
+        if (live1) *reinterpret_cast<float2*>(x + row * nrhs + 2) = make_float2(sum.z * f, sum.w * f);
+      }
+    }
+  }
+}
+
+__global__ void RoundKernel(const double* in, long long n, float* out) {
+  const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
+  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n; i += stride)
+    out[i] = static_cast<float>(in[i]);
+}
+
+size_t BlockSmem32(int B, int kd) {
+  const int W = ((kd + B - 1) / B + 1) * B, C = kWarp / B;
+  return sizeof(float) * (static_cast<size_t>(kBlockStages) * (kd + B) * B + static_cast<size_t>(kBlockWarps) * (W + B) * C * 4);
+}
+
 size_t BlockSmem(int B, int kd) {
   const int W = ((kd + B - 1) / B + 1) * B, C = kWarp / B;
   return sizeof(double) * (static_cast<size_t>(kBlockStages) * (kd + B) * B + static_cast<size_t>(kBlockWarps) * (W + B) * C);
@@ -190,7 +320,7 @@ void AddBlocks(const sl3dgpu_band_system& s, int B, SolveCost& c) {
 }  // namespace
 
 int BuildBlockSolver(const std::vector<sl3dgpu_band_system>& first, const std::vector<sl3dgpu_band_system>& second,
-                     const double* bands, const double* scales, BlockSolver& out, cudaStream_t stream) {
+                     const double* bands, const double* scales, bool fp32, BlockSolver& out, cudaStream_t stream) {
   out.block = 0;
   SolveCost rows[2], blocks8, blocks16;
   for (int which = 0; which < 2; ++which)
@@ -205,7 +335,8 @@ int BuildBlockSolver(const std::vector<sl3dgpu_band_system>& first, const std::v
   if (first.empty() || byRows <= std::min(blocks8.Cycles(), blocks16.Cycles())) return SL3DGPU_OK;
   std::vector<BlockSystem> systems;
   std::vector<sl3dgpu_band_system> bandSystems;
-  std::vector<int2> items;
+  std::vector<int2> items, items32;
+  bool even = true;  // the FP32 form takes columns in pairs
   long long values = 0;
   int maxBlocks = 0;
   for (int which = 0; which < 2; ++which)
@@ -224,6 +355,9 @@ int BuildBlockSolver(const std::vector<sl3dgpu_band_system>& first, const std::v
       b.second = which;
       for (int c = 0; c < s.nrhs; c += kBlockWarps * kWarp / B)
         items.push_back(make_int2(static_cast<int>(systems.size()), c));
+      for (int c = 0; c < s.nrhs; c += 4 * kBlockWarps * kWarp / B)
+        items32.push_back(make_int2(static_cast<int>(systems.size()), c));
+      even = even && s.nrhs % 2 == 0 && s.rhs % 2 == 0;
       out.kd = std::max(out.kd, b.kd);
       maxBlocks = std::max(maxBlocks, b.blocks);
       systems.push_back(b);
@@ -231,8 +365,12 @@ int BuildBlockSolver(const std::vector<sl3dgpu_band_system>& first, const std::v
     }
   if (BlockSmem(B, out.kd) > 200 * 1024) return SL3DGPU_OK;
   // the longest systems first
-  std::stable_sort(items.begin(), items.end(),
-                   [&](const int2& a, const int2& b) { return systems[a.x].n * systems[a.x].kd > systems[b.x].n * systems[b.x].kd; });
+  auto longer = [&](const int2& a, const int2& b) {
+    return systems[a.x].n * systems[a.x].kd > systems[b.x].n * systems[b.x].kd;
+  };
+  std::stable_sort(items.begin(), items.end(), longer);
+  std::stable_sort(items32.begin(), items32.end(), longer);
+  out.firstCount = static_cast<int>(first.size());
   out.itemCount = static_cast<int>(items.size());
   SL3D_CUDA(cudaMalloc(&out.systems, systems.size() * sizeof(BlockSystem)));
   SL3D_CUDA(cudaMalloc(&out.items, items.size() * sizeof(int2)));
@@ -254,6 +392,15 @@ int BuildBlockSolver(const std::vector<sl3dgpu_band_system>& first, const std::v
   }
   cudaFree(device);
   SL3D_CUDA(e);
+  if (fp32 && even) {
+    out.itemCount32 = static_cast<int>(items32.size());
+    SL3D_CUDA(cudaMalloc(&out.items32, items32.size() * sizeof(int2)));
+    SL3D_CUDA(cudaMalloc(&out.data32, values * sizeof(float)));
+    SL3D_CUDA(CopyIn(out.items32, items32.data(), items32.size() * sizeof(int2)));
+    RoundKernel<<<1216, 256, 0, stream>>>(out.data, values, out.data32);
+    SL3D_CHECK_LAUNCH();
+    SL3D_CUDA(cudaStreamSynchronize(stream));
+  }
   out.block = B;
   return SL3DGPU_OK;
 }
@@ -269,6 +416,23 @@ int RunBlockSolver(const BlockSolver& b, double* first, double* second, const do
     SL3D_CUDA(AllowDynamicSmem(BlockSolveKernel<16>));
     BlockSolveKernel<16><<<b.itemCount, kBlockWarps * kWarp, smem, stream>>>(b.systems, b.items, b.data, first, second,
                                                                              scales, b.kd);
+  }
+  SL3D_CHECK_LAUNCH();
+  return SL3DGPU_OK;
+}
+
+int RunBlockSolver32(const BlockSolver& b, float* first, float* second, const float* scales, const int2* windowsFirst,
+                     const int2* windowsSecond, cudaStream_t stream) {
+  const size_t smem = BlockSmem32(b.block, b.kd);
+  prof::Scope scope(prof::kBandSolve32, stream);
+  if (b.block == 8) {
+    SL3D_CUDA(AllowDynamicSmem(BlockSolve32Kernel<8>));
+    BlockSolve32Kernel<8><<<b.itemCount32, kBlockWarps * kWarp, smem, stream>>>(
+        b.systems, b.items32, b.firstCount, b.data32, first, second, scales, windowsFirst, windowsSecond, b.kd);
+  } else {
+    SL3D_CUDA(AllowDynamicSmem(BlockSolve32Kernel<16>));
+    BlockSolve32Kernel<16><<<b.itemCount32, kBlockWarps * kWarp, smem, stream>>>(
+        b.systems, b.items32, b.firstCount, b.data32, first, second, scales, windowsFirst, windowsSecond, b.kd);
   }
   SL3D_CHECK_LAUNCH();
   return SL3DGPU_OK;

@@ -24,6 +24,12 @@ struct BlockSolver {
   BlockSystem* systems = nullptr;
   int2* items = nullptr;  // (system, first column)
   double* data = nullptr;
+  // the FP32 form (the mixed form's correction solves): the coefficients
+  // rounded, and its items (more columns a CTA)
+  int firstCount = 0;  // systems of the first list
+  int itemCount32 = 0;
+  int2* items32 = nullptr;
+  float* data32 = nullptr;
   BlockSolver() = default;
   BlockSolver(const BlockSolver&) = delete;
   BlockSolver& operator=(const BlockSolver&) = delete;
@@ -31,6 +37,8 @@ struct BlockSolver {
     cudaFree(systems);
     cudaFree(items);
     cudaFree(data);
+    cudaFree(items32);
+    cudaFree(data32);
   }
 };
 
@@ -38,8 +46,14 @@ struct BlockSolver {
 // list's right-hand sides in the second array) and makes a blocked form's
 // coefficients from their factors.
 int BuildBlockSolver(const std::vector<sl3dgpu_band_system>& first, const std::vector<sl3dgpu_band_system>& second,
-                     const double* bands, const double* scales, BlockSolver& out, cudaStream_t stream);
+                     const double* bands, const double* scales, bool fp32, BlockSolver& out, cudaStream_t stream);
 // Solves every system in place (out.block > 0).
 int RunBlockSolver(const BlockSolver& b, double* first, double* second, const double* scales, cudaStream_t stream);
+
+// The FP32 solves over row windows (windowsFirst, windowsSecond: {lo, hi} a
+// system, the right-hand side zero outside): rows lo .. n - 1 of both
+// substitutions, as BandSolveWindowF's (which completes the rows below).
+int RunBlockSolver32(const BlockSolver& b, float* first, float* second, const float* scales, const int2* windowsFirst,
+                     const int2* windowsSecond, cudaStream_t stream);
 
 }  // namespace sl3dgpu

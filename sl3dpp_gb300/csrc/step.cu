@@ -1995,12 +1995,16 @@ int Viscoelastic3DGpu::Pass32(const Flavour& f, const float2* e, float2* next) {
   SL3D_CHECK_LAUNCH();
   LaunchForces(geoL, analysedL.p, rhsSph32.p, rhsTor32.p, stream);
   SL3D_CHECK_LAUNCH();
-  SL3D_TRY(BandSolveWindowF(f.dSphChol.p, f.sphChol.data(), static_cast<int>(f.sphChol.size()), f.iSphChol.p,
-                            f.nSphChol, f.bands32.p, sph, f.scales32.p, f.wSphChol.p, false, stream));
+  if (f.blocked.itemCount32 > 0) {
+    SL3D_TRY(RunBlockSolver32(f.blocked, sph, tor, f.scales32.p, f.wSphChol.p, f.wTorChol.p, stream));
+  } else {
+    SL3D_TRY(BandSolveWindowF(f.dSphChol.p, f.sphChol.data(), static_cast<int>(f.sphChol.size()), f.iSphChol.p,
+                              f.nSphChol, f.bands32.p, sph, f.scales32.p, f.wSphChol.p, false, stream));
+    SL3D_TRY(BandSolveWindowF(f.dTorChol.p, f.torChol.data(), static_cast<int>(f.torChol.size()), f.iTorChol.p,
+                              f.nTorChol, f.bands32.p, tor, f.scales32.p, f.wTorChol.p, false, stream));
+  }
   SL3D_TRY(BandSolveBatchF(f.dSphLu.p, f.sphLu.data(), static_cast<int>(f.sphLu.size()), f.iSphLu.p, f.nSphLu,
                            f.bands32.p, f.pivots.p, sph, f.scales32.p, 1, stream));
-  SL3D_TRY(BandSolveWindowF(f.dTorChol.p, f.torChol.data(), static_cast<int>(f.torChol.size()), f.iTorChol.p,
-                            f.nTorChol, f.bands32.p, tor, f.scales32.p, f.wTorChol.p, false, stream));
   LaunchStrain(geoL, rhsSph32.p, rhsTor32.p, next, stream, rL.p);  // B e + r
   SL3D_CHECK_LAUNCH();
   return SL3DGPU_OK;

@@ -163,7 +163,7 @@ int BuildSystems(const SystemsInput& in, Flavour& f) {
   SL3D_TRY(upload(f.sphChol, f.dSphChol, f.iSphChol, f.nSphChol));
   SL3D_TRY(upload(f.sphLu, f.dSphLu, f.iSphLu, f.nSphLu));
   SL3D_TRY(upload(f.torChol, f.dTorChol, f.iTorChol, f.nTorChol));
-  SL3D_TRY(BuildBlockSolver(f.sphChol, f.torChol, f.bands.p, f.scales.p, f.blocked, stream));
+  SL3D_TRY(BuildBlockSolver(f.sphChol, f.torChol, f.bands.p, f.scales.p, in.fp32, f.blocked, stream));
   // The load units K^-1 Load per degree (AddUnitChannels' cached responses).
   // The tide channel's, K^-1 Tide with the degree's power (degree 0 the
   // spherical mean of a centrifugal change, power 2: Viscoelastic3D.cpp:1049).
