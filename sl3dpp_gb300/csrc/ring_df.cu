@@ -91,19 +91,21 @@ __global__ void __launch_bounds__(kDfThreads, 2) DfRingKernel(const __grid_const
   const int n = plan.n, tid = threadIdx.x, T = blockDim.x;
   Df2* tw = reinterpret_cast<Df2*>(dfSmem);
   Df2* bufs = tw + n;  // [ring][2][n], a value between the rings' (their banks apart)
-  const int perRing = A.real ? 2 : 1;
-  const int j = blockIdx.y, f0 = blockIdx.x * G * perRing;
-  const int mcount = A.real ? A.lmax + 1 : 2 * A.lmax + 1;
+  int px;  // this CTA among its part's
+  const FxRingPart& Q = FxPartOf(A, px);
+  const int perRing = Q.real ? 2 : 1;
+  const int j = blockIdx.y, f0 = px * G * perRing;
+  const int mcount = Q.real ? A.lmax + 1 : 2 * A.lmax + 1;
   const int g = tid % G, lead = tid / G, step = T / G;
   const int fa = f0 + g * perRing;
-  const bool live = fa < A.count, second = A.real && fa + 1 < A.count;
+  const bool live = fa < A.count, second = Q.real && fa + 1 < A.count;
   const long long rows = static_cast<long long>(A.ntheta) * n;  // a field's values
   Df2* ring = bufs + g * (2 * n + 1);
   const Df zero(0.0f, 0.0f);
   const Df2 zero2 = Make<Df2>(zero, zero);
   for (int e = tid; e < n; e += T) tw[e] = FromDouble2(A.twiddle[e]);
   int at = 0;
-  const double2* in = A.spectraIn + static_cast<long long>(j) * A.count + fa;
+  const double2* in = Q.spectraIn + static_cast<long long>(j) * A.count + fa;
   const long long order = static_cast<long long>(A.ntheta) * A.count;
   if (A.mode != kDfAnalyse) {
     const int zeros = n - (2 * A.lmax + 1);  // the orders beyond lmax
@@ -111,7 +113,7 @@ __global__ void __launch_bounds__(kDfThreads, 2) DfRingKernel(const __grid_const
 #pragma unroll 4
     for (int mi = lead; mi < mcount; mi += step) {
       const Df2 v = live ? FromDouble2(in[mi * order]) : zero2;
-      if (!A.real) {
+      if (!Q.real) {
         const int m = mi - A.lmax;
         ring[m < 0 ? m + n : m] = v;
       } else {
@@ -131,23 +133,23 @@ __global__ void __launch_bounds__(kDfThreads, 2) DfRingKernel(const __grid_const
       if (f >= A.count) break;
       Df2* res = bufs + r * (2 * n + 1) + at * n;
       const long long row = static_cast<long long>(f) * rows + static_cast<long long>(j) * n, next = row + rows;
-      const bool two = A.real && f + 1 < A.count;
+      const bool two = Q.real && f + 1 < A.count;
       if (A.mode == kDfWeighted) {
 #pragma unroll 2
         for (int k = tid; k < n; k += T) {
           const Df w0 = FromDouble(A.pointWeight[row + k]);
-          const Df w1 = A.real ? (two ? FromDouble(A.pointWeight[next + k]) : zero) : w0;
+          const Df w1 = Q.real ? (two ? FromDouble(A.pointWeight[next + k]) : zero) : w0;
           const Df2 v = res[k];
           res[k] = Make<Df2>(v.x * w0, v.y * w1);
         }
-      } else if (A.real) {
-        auto* out = static_cast<double*>(A.fieldsOut);
+      } else if (Q.real) {
+        auto* out = static_cast<double*>(Q.fieldsOut);
         for (int k = tid; k < n; k += T) {
           out[row + k] = ToDouble(res[k].x);
           if (two) out[next + k] = ToDouble(res[k].y);
         }
       } else {
-        auto* out = static_cast<double2*>(A.fieldsOut);
+        auto* out = static_cast<double2*>(Q.fieldsOut);
         for (int k = tid; k < n; k += T) out[row + k] = make_double2(ToDouble(res[k].x), ToDouble(res[k].y));
       }
     }
@@ -157,19 +159,19 @@ __global__ void __launch_bounds__(kDfThreads, 2) DfRingKernel(const __grid_const
       const int f = f0 + r * perRing;
       Df2* to = bufs + r * (2 * n + 1);
       const long long row = static_cast<long long>(f) * rows + static_cast<long long>(j) * n, next = row + rows;
-      const bool one = f < A.count, two = A.real && f + 1 < A.count;
+      const bool one = f < A.count, two = Q.real && f + 1 < A.count;
 #pragma unroll 2
       for (int k = tid; k < n; k += T) {
         Df2 v = zero2;
         if (one) {
-          if (A.real)
-            v = Make<Df2>(FromDouble(static_cast<const double*>(A.fieldsIn)[row + k]),
-                          two ? FromDouble(static_cast<const double*>(A.fieldsIn)[next + k]) : zero);
+          if (Q.real)
+            v = Make<Df2>(FromDouble(static_cast<const double*>(Q.fieldsIn)[row + k]),
+                          two ? FromDouble(static_cast<const double*>(Q.fieldsIn)[next + k]) : zero);
           else
-            v = FromDouble2(static_cast<const double2*>(A.fieldsIn)[row + k]);
+            v = FromDouble2(static_cast<const double2*>(Q.fieldsIn)[row + k]);
           if (A.pointWeight != nullptr) {
             const Df w0 = FromDouble(A.pointWeight[row + k]);
-            const Df w1 = A.real ? (two ? FromDouble(A.pointWeight[next + k]) : zero) : w0;
+            const Df w1 = Q.real ? (two ? FromDouble(A.pointWeight[next + k]) : zero) : w0;
             v = Make<Df2>(v.x * w0, v.y * w1);
           }
         }
@@ -181,10 +183,10 @@ __global__ void __launch_bounds__(kDfThreads, 2) DfRingKernel(const __grid_const
   if (!live) return;
   const Df scale = FromDouble(2.0 * 3.14159265358979323846 / n * A.weights[j]), half(0.5);
   const Df2* res = ring + at * n;
-  double2* out = A.spectraOut + static_cast<long long>(j) * A.count + fa;
+  double2* out = Q.spectraOut + static_cast<long long>(j) * A.count + fa;
 #pragma unroll 2
   for (int mi = lead; mi < mcount; mi += step) {
-    if (!A.real) {
+    if (!Q.real) {
       const int m = mi - A.lmax;
       const Df2 v = res[m < 0 ? m + n : m];
       out[mi * order] = make_double2(ToDouble(v.x * scale), ToDouble(v.y * scale));
@@ -202,11 +204,11 @@ __global__ void __launch_bounds__(kDfThreads, 2) DfRingKernel(const __grid_const
 
 }  // namespace
 
-int LaunchDfRings(const FxPlan& plan, const FxRingArgs& args, cudaStream_t stream) {
+int LaunchDfRings(const FxPlan& plan, FxRingArgs args, cudaStream_t stream) {
   if (args.count == 0) return SL3DGPU_OK;
   const int n = plan.n;
   // Rings a CTA as the fixed-point kernel takes them: up to eight, two CTAs an SM.
-  const int rings = args.real ? (args.count + 1) / 2 : args.count;
+  const int rings = FxRings(args);
   auto bytes = [n](int g) { return (n + static_cast<size_t>(g) * (2 * n + 1)) * 16; };
   int G = 1;
   while (G < kDfMaxRings && G < rings && bytes(2 * G) <= 115300) G *= 2;
@@ -217,7 +219,7 @@ int LaunchDfRings(const FxPlan& plan, const FxRingArgs& args, cudaStream_t strea
   int T = 64;
   while (T < kDfThreads && T < G * n / 4) T *= 2;
   SL3D_CUDA(AllowDynamicSmem(DfRingKernel));
-  DfRingKernel<<<dim3((rings + G - 1) / G, args.ntheta), T, bytes(G), stream>>>(plan, args, G);
+  DfRingKernel<<<dim3(FxBlocks(args, G), args.ntheta), T, bytes(G), stream>>>(plan, args, G);
   SL3D_CHECK_LAUNCH();
   return SL3DGPU_OK;
 }

@@ -161,6 +161,6 @@ __host__ __device__ inline double ToDouble(Df v) {
 
 // The ring passes in double-float (the fixed-point ones' interface); the plan
 // has the radices 4, 2, 3, 5.
-int LaunchDfRings(const FxPlan& plan, const FxRingArgs& args, cudaStream_t stream);
+int LaunchDfRings(const FxPlan& plan, FxRingArgs args, cudaStream_t stream);
 
 }  // namespace sl3dgpu

@@ -79,15 +79,16 @@ __device__ __noinline__ double2* Ring64(double2* a, double2* b, const FxPlan& pl
 }
 
 // The CTA's rings in FP64 from the inputs again.
-__device__ __noinline__ void Rings64(const FxPlan& plan, const FxRingArgs& A, double2* bufs, int G) {
-  const int n = plan.n, perRing = A.real ? 2 : 1, j = blockIdx.y;
-  const int mcount = A.real ? A.lmax + 1 : 2 * A.lmax + 1;
+__device__ __noinline__ void Rings64(const FxPlan& plan, const FxRingArgs& A, const FxRingPart& Q, int x,
+                                      double2* bufs, int G) {
+  const int n = plan.n, perRing = Q.real ? 2 : 1, j = blockIdx.y;
+  const int mcount = Q.real ? A.lmax + 1 : 2 * A.lmax + 1;
   const int lane = threadIdx.x % kWarp;
   const double scale = 2.0 * 3.14159265358979323846 / n * A.weights[j];
   for (int g = threadIdx.x / kWarp; g < G; g += blockDim.x / kWarp) {
-    const int f0 = (blockIdx.x * G + g) * perRing;
+    const int f0 = (x * G + g) * perRing;
     if (f0 >= A.count) break;
-    const bool second = A.real && f0 + 1 < A.count;
+    const bool second = Q.real && f0 + 1 < A.count;
     const long long row0 = (static_cast<long long>(f0) * A.ntheta + j) * n, row1 = row0 + static_cast<long long>(A.ntheta) * n;
     double2* a = bufs + static_cast<long long>(g) * 2 * n;
     double2* b = a + n;
@@ -96,13 +97,13 @@ __device__ __noinline__ void Rings64(const FxPlan& plan, const FxRingArgs& A, do
       __syncwarp();
       for (int mi = lane; mi < mcount; mi += kWarp) {
         const long long at = (static_cast<long long>(mi) * A.ntheta + j) * A.count + f0;
-        const double2 v = A.spectraIn[at];
-        if (!A.real) {
+        const double2 v = Q.spectraIn[at];
+        if (!Q.real) {
           const int m = mi - A.lmax;
           a[m < 0 ? m + n : m] = v;
           continue;
         }
-        const double2 u = second ? A.spectraIn[at + 1] : make_double2(0.0, 0.0);
+        const double2 u = second ? Q.spectraIn[at + 1] : make_double2(0.0, 0.0);
         if (mi == 0) {
           a[0] = make_double2(v.x, u.x);
         } else {
@@ -114,11 +115,11 @@ __device__ __noinline__ void Rings64(const FxPlan& plan, const FxRingArgs& A, do
       double2* res = Ring64(a, b, plan, A.twiddle, 1, lane);
       if (A.mode == kFxSynth) {
         for (int k = lane; k < n; k += kWarp) {
-          if (A.real) {
-            static_cast<double*>(A.fieldsOut)[row0 + k] = res[k].x;
-            if (second) static_cast<double*>(A.fieldsOut)[row1 + k] = res[k].y;
+          if (Q.real) {
+            static_cast<double*>(Q.fieldsOut)[row0 + k] = res[k].x;
+            if (second) static_cast<double*>(Q.fieldsOut)[row1 + k] = res[k].y;
           } else {
-            static_cast<double2*>(A.fieldsOut)[row0 + k] = res[k];
+            static_cast<double2*>(Q.fieldsOut)[row0 + k] = res[k];
           }
         }
         continue;
@@ -126,16 +127,16 @@ __device__ __noinline__ void Rings64(const FxPlan& plan, const FxRingArgs& A, do
       b = res == a ? b : a;
       a = res;
       for (int k = lane; k < n; k += kWarp) {
-        const double w0 = A.pointWeight[row0 + k], w1 = A.real ? (second ? A.pointWeight[row1 + k] : 0.0) : w0;
+        const double w0 = A.pointWeight[row0 + k], w1 = Q.real ? (second ? A.pointWeight[row1 + k] : 0.0) : w0;
         a[k] = make_double2(a[k].x * w0, a[k].y * w1);
       }
     } else {
       for (int k = lane; k < n; k += kWarp) {
-        double2 v = A.real ? make_double2(static_cast<const double*>(A.fieldsIn)[row0 + k],
-                                          second ? static_cast<const double*>(A.fieldsIn)[row1 + k] : 0.0)
-                           : static_cast<const double2*>(A.fieldsIn)[row0 + k];
+        double2 v = Q.real ? make_double2(static_cast<const double*>(Q.fieldsIn)[row0 + k],
+                                          second ? static_cast<const double*>(Q.fieldsIn)[row1 + k] : 0.0)
+                           : static_cast<const double2*>(Q.fieldsIn)[row0 + k];
         if (A.pointWeight != nullptr) {
-          const double w0 = A.pointWeight[row0 + k], w1 = A.real ? (second ? A.pointWeight[row1 + k] : 0.0) : w0;
+          const double w0 = A.pointWeight[row0 + k], w1 = Q.real ? (second ? A.pointWeight[row1 + k] : 0.0) : w0;
           v = make_double2(v.x * w0, v.y * w1);
         }
         a[k] = v;
@@ -145,15 +146,15 @@ __device__ __noinline__ void Rings64(const FxPlan& plan, const FxRingArgs& A, do
     const double2* res = Ring64(a, b, plan, A.twiddle, -1, lane);
     for (int mi = lane; mi < mcount; mi += kWarp) {
       const long long at = (static_cast<long long>(mi) * A.ntheta + j) * A.count + f0;
-      if (!A.real) {
+      if (!Q.real) {
         const int m = mi - A.lmax;
         const double2 z = res[m < 0 ? m + n : m];
-        A.spectraOut[at] = make_double2(z.x * scale, z.y * scale);
+        Q.spectraOut[at] = make_double2(z.x * scale, z.y * scale);
         continue;
       }
       const double2 z = res[mi], w = res[mi == 0 ? 0 : n - mi];
-      A.spectraOut[at] = make_double2(0.5 * (z.x + w.x) * scale, 0.5 * (z.y - w.y) * scale);
-      if (second) A.spectraOut[at + 1] = make_double2(0.5 * (z.y + w.y) * scale, 0.5 * (w.x - z.x) * scale);
+      Q.spectraOut[at] = make_double2(0.5 * (z.x + w.x) * scale, 0.5 * (z.y - w.y) * scale);
+      if (second) Q.spectraOut[at + 1] = make_double2(0.5 * (z.y + w.y) * scale, 0.5 * (w.x - z.x) * scale);
     }
   }
 }
@@ -241,12 +242,14 @@ __global__ void __launch_bounds__(kFxThreads, 2) FxRingKernel(const __grid_const
   const int n = plan.n, tid = threadIdx.x, T = blockDim.x;
   FxRoot* roots = reinterpret_cast<FxRoot*>(fxSmem);
   Fx2* bufs = reinterpret_cast<Fx2*>(roots + n);  // [ring][2][n], a value between the rings' (their banks apart)
-  const int perRing = A.real ? 2 : 1;
-  const int j = blockIdx.y, f0 = blockIdx.x * G * perRing;
-  const int mcount = A.real ? A.lmax + 1 : 2 * A.lmax + 1;
+  int px;  // this CTA among its part's
+  const FxRingPart& Q = FxPartOf(A, px);
+  const int perRing = Q.real ? 2 : 1;
+  const int j = blockIdx.y, f0 = px * G * perRing;
+  const int mcount = Q.real ? A.lmax + 1 : 2 * A.lmax + 1;
   const int g = tid % G, lead = tid / G, step = T / G;  // this thread's ring, and its share of the ring's values
   const int fa = f0 + g * perRing;                      // its (first) field
-  const bool live = fa < A.count, second = A.real && fa + 1 < A.count;
+  const bool live = fa < A.count, second = Q.real && fa + 1 < A.count;
   const long long row0 = (static_cast<long long>(fa) * A.ntheta + j) * n;
   const long long row1 = row0 + static_cast<long long>(A.ntheta) * n;
   Fx2* ring = bufs + g * (2 * n + 1);
@@ -261,15 +264,15 @@ __global__ void __launch_bounds__(kFxThreads, 2) FxRingKernel(const __grid_const
   auto seen = [&](unsigned long long bits) { emax = max(emax, static_cast<uint32_t>(FxExponent(bits))); };
   const bool synth = A.mode != kFxAnalyse;
   if (synth) {
-    const double2* in = A.spectraIn + static_cast<long long>(j) * A.count + fa;
+    const double2* in = Q.spectraIn + static_cast<long long>(j) * A.count + fa;
     const long long order = static_cast<long long>(A.ntheta) * A.count;
-    const int zeros = A.real ? n - (2 * A.lmax + 1) : n - mcount;  // the orders beyond lmax
+    const int zeros = Q.real ? n - (2 * A.lmax + 1) : n - mcount;  // the orders beyond lmax
     for (int k = lead; k < zeros; k += step) ring[A.lmax + 1 + k] = Fx2{0, 0};
 #pragma unroll 4
     for (int mi = lead; mi < mcount; mi += step) {
       const double2 v = live ? in[mi * order] : make_double2(0.0, 0.0);
       ulonglong2 a = make_ulonglong2(Bits(v.x), Bits(v.y));
-      if (!A.real) {
+      if (!Q.real) {
         const int m = mi - A.lmax;
         raw[m < 0 ? m + n : m] = a;
       } else {
@@ -293,13 +296,13 @@ __global__ void __launch_bounds__(kFxThreads, 2) FxRingKernel(const __grid_const
     for (int k = lead; k < n; k += step) {
       double2 v = make_double2(0.0, 0.0);
       if (live) {
-        if (A.real)
-          v = make_double2(static_cast<const double*>(A.fieldsIn)[row0 + k],
-                           second ? static_cast<const double*>(A.fieldsIn)[row1 + k] : 0.0);
+        if (Q.real)
+          v = make_double2(static_cast<const double*>(Q.fieldsIn)[row0 + k],
+                           second ? static_cast<const double*>(Q.fieldsIn)[row1 + k] : 0.0);
         else
-          v = static_cast<const double2*>(A.fieldsIn)[row0 + k];
+          v = static_cast<const double2*>(Q.fieldsIn)[row0 + k];
         if (A.pointWeight != nullptr) {
-          const double w0 = A.pointWeight[row0 + k], w1 = A.real ? (second ? A.pointWeight[row1 + k] : 0.0) : w0;
+          const double w0 = A.pointWeight[row0 + k], w1 = Q.real ? (second ? A.pointWeight[row1 + k] : 0.0) : w0;
           v = make_double2(v.x * w0, v.y * w1);
         }
       }
@@ -317,7 +320,7 @@ __global__ void __launch_bounds__(kFxThreads, 2) FxRingKernel(const __grid_const
   if (e0 > 0) {
     if (synth) {
       for (int mi = lead; mi < mcount; mi += step) {
-        if (!A.real) {
+        if (!Q.real) {
           const int m = mi - A.lmax;
           const ulonglong2 a = raw[m < 0 ? m + n : m];
           sum += FxMagnitude(a.x, e0) + FxMagnitude(a.y, e0);
@@ -339,13 +342,13 @@ __global__ void __launch_bounds__(kFxThreads, 2) FxRingKernel(const __grid_const
   }
   sum = OverRing(sum, shared, G, Sum);
   if (fallback) {  // uniform: set before the barriers above
-    Rings64(plan, A, reinterpret_cast<double2*>(bufs), G);
+    Rings64(plan, A, Q, px, reinterpret_cast<double2*>(bufs), G);
     return;
   }
   // a real pair's order m enters twice, at m and n - m
-  int scale = FxScaleOf(e0, sum) - (synth && A.real ? 1 : 0);
+  int scale = FxScaleOf(e0, sum) - (synth && Q.real ? 1 : 0);
   const int first = plan.stages > 0 ? plan.radix[0] : n;
-  const int room = e0 > 0 && plan.stages > 0 ? FxRoom(e0, scale, synth && A.real) : 0;
+  const int room = e0 > 0 && plan.stages > 0 ? FxRoom(e0, scale, synth && Q.real) : 0;
   const int head = FxHeadAt(room, first);
   if (lead == 0) {
     ringScale[g] = scale;
@@ -354,7 +357,7 @@ __global__ void __launch_bounds__(kFxThreads, 2) FxRingKernel(const __grid_const
   // To fixed point in place; the forward sum's sign by swapping the parts.
   if (synth) {
     for (int mi = lead; mi < mcount; mi += step) {
-      if (!A.real) {
+      if (!Q.real) {
         const int m = mi - A.lmax;
         const int at = m < 0 ? m + n : m;
         const ulonglong2 a = raw[at];
@@ -387,8 +390,8 @@ __global__ void __launch_bounds__(kFxThreads, 2) FxRingKernel(const __grid_const
       const Fx2* res = bufs + r * (2 * n + 1) + at * n;
       const int sc = ringScale[r];
       const long long row = (static_cast<long long>(f) * A.ntheta + j) * n;
-      if (A.real) {
-        auto* out = static_cast<double*>(A.fieldsOut);
+      if (Q.real) {
+        auto* out = static_cast<double*>(Q.fieldsOut);
         const bool two = f + 1 < A.count;
         const long long next = row + static_cast<long long>(A.ntheta) * n;
         for (int k = tid; k < n; k += T) {
@@ -396,7 +399,7 @@ __global__ void __launch_bounds__(kFxThreads, 2) FxRingKernel(const __grid_const
           if (two) out[next + k] = FxTo(res[k].y, sc);
         }
       } else {
-        auto* out = static_cast<double2*>(A.fieldsOut);
+        auto* out = static_cast<double2*>(Q.fieldsOut);
         for (int k = tid; k < n; k += T) out[row + k] = make_double2(FxTo(res[k].x, sc), FxTo(res[k].y, sc));
       }
     }
@@ -425,7 +428,7 @@ __global__ void __launch_bounds__(kFxThreads, 2) FxRingKernel(const __grid_const
         FxSplit(FxFrom(Bits(A.pointWeight[row0 + k]), wscale), wh, wl);
         FxSplit(v.x, vh, vl);
         a = FxProduct(vh, vl, wh, wl);
-        if (A.real) FxSplit(second ? FxFrom(Bits(A.pointWeight[row1 + k]), wscale) : 0, wh, wl);
+        if (Q.real) FxSplit(second ? FxFrom(Bits(A.pointWeight[row1 + k]), wscale) : 0, wh, wl);
         FxSplit(v.y, vh, vl);
         b = FxProduct(vh, vl, wh, wl);
       }
@@ -434,7 +437,7 @@ __global__ void __launch_bounds__(kFxThreads, 2) FxRingKernel(const __grid_const
     }
     total = OverRing(total, shared, G, Sum);
     if (fallback) {  // uniform, as above
-      Rings64(plan, A, reinterpret_cast<double2*>(bufs), G);
+      Rings64(plan, A, Q, px, reinterpret_cast<double2*>(bufs), G);
       return;
     }
     // the sum is below 2^61 after a shift down by `whole`, each value before it
@@ -464,11 +467,11 @@ __global__ void __launch_bounds__(kFxThreads, 2) FxRingKernel(const __grid_const
     return FxTo(FxProduct(h, l, fh, fl), outScale);
   };
   const Fx2* res = ring + at * n;
-  double2* out = A.spectraOut + static_cast<long long>(j) * A.count + fa;
+  double2* out = Q.spectraOut + static_cast<long long>(j) * A.count + fa;
   const long long order = static_cast<long long>(A.ntheta) * A.count;
 #pragma unroll 2
   for (int mi = lead; mi < mcount; mi += step) {
-    if (!A.real) {
+    if (!Q.real) {
       const int m = mi - A.lmax;
       const Fx2 z = res[m < 0 ? m + n : m];
       out[mi * order] = make_double2(scaled(z.y), scaled(z.x));
@@ -556,12 +559,12 @@ bool MakeFxPlan(int n, FxPlan* plan) {
   return true;
 }
 
-int LaunchFxRings(const FxPlan& plan, const FxRingArgs& args, cudaStream_t stream) {
+int LaunchFxRings(const FxPlan& plan, FxRingArgs args, cudaStream_t stream) {
   if (args.count == 0) return SL3DGPU_OK;
   const int n = plan.n;
   // Rings a CTA: up to eight, two CTAs an SM while that leaves them two
   // (twiddles and two buffers a ring: 115 KB at four rings of 800).
-  const int rings = args.real ? (args.count + 1) / 2 : args.count;
+  const int rings = FxRings(args);
   auto bytes = [n](int g) { return (n + static_cast<size_t>(g) * (2 * n + 1)) * 16; };
   int G = 1;
   while (G < kFxMaxRings && G < rings && bytes(2 * G) <= 115300) G *= 2;
@@ -572,7 +575,7 @@ int LaunchFxRings(const FxPlan& plan, const FxRingArgs& args, cudaStream_t strea
   int T = 64;  // a power of two: a multiple of G
   while (T < kFxThreads && T < G * n / 8) T *= 2;
   SL3D_CUDA(AllowDynamicSmem(FxRingKernel));
-  FxRingKernel<<<dim3((rings + G - 1) / G, args.ntheta), T, bytes(G), stream>>>(plan, args, G);
+  FxRingKernel<<<dim3(FxBlocks(args, G), args.ntheta), T, bytes(G), stream>>>(plan, args, G);
   SL3D_CHECK_LAUNCH();
   return SL3DGPU_OK;
 }

@@ -297,19 +297,50 @@ __host__ __device__ inline double FxTo(long long X, int scale) {
 
 // The ring passes on FP64 values (Grid::RingSynthesis, RingAnalysis and
 // RingWeighted): `mode` 0 spectra -> fields, 1 fields (times a weight) ->
-// spectra, 2 spectra -> weighted fields -> spectra.
-struct FxRingArgs {
-  int mode, lmax, ntheta, count;
+// spectra, 2 spectra -> weighted fields -> spectra. One launch takes up to
+// three batches of `count` fields (a tensor's spin components), spin (complex)
+// or real, under the same point weights.
+struct FxRingPart {
   bool real;
-  const FxRoot* roots;       // n
-  const double2* twiddle;    // n, for the rings that fall back to FP64
-  const double* weights;     // per colatitude
   const double2* spectraIn;  // [order][colatitude][field]
   const void* fieldsIn;      // [field][colatitude][longitude]
-  const double* pointWeight;
   void* fieldsOut;
   double2* spectraOut;
 };
-int LaunchFxRings(const FxPlan& plan, const FxRingArgs& args, cudaStream_t stream);
+struct FxRingArgs {
+  int mode, lmax, ntheta, count;
+  const FxRoot* roots;     // n
+  const double2* twiddle;  // n, FP64 (the double-float rings', and the rings that fall back to FP64)
+  const double* weights;   // per colatitude
+  const double* pointWeight;
+  int parts;
+  FxRingPart part[3];
+  int blocks[3];  // CTAs of each part along x (the launch fills them)
+};
+// This CTA's part, and its place among the part's CTAs.
+__device__ __forceinline__ const FxRingPart& FxPartOf(const FxRingArgs& a, int& x) {
+  x = static_cast<int>(blockIdx.x);
+  int p = 0;
+  while (p + 1 < a.parts && x >= a.blocks[p]) x -= a.blocks[p++];
+  return a.part[p];
+}
+// The parts' CTAs at G rings each; their sum.
+inline int FxBlocks(FxRingArgs& a, int G) {
+  int total = 0;
+  for (int p = 0; p < a.parts; ++p) {
+    const int rings = a.part[p].real ? (a.count + 1) / 2 : a.count;  // real fields go two to a ring
+    a.blocks[p] = (rings + G - 1) / G;
+    total += a.blocks[p];
+  }
+  return total;
+}
+// The most rings of a part.
+inline int FxRings(const FxRingArgs& a) {
+  int rings = 1;
+  for (int p = 0; p < a.parts; ++p)
+    rings = rings > (a.part[p].real ? (a.count + 1) / 2 : a.count) ? rings : (a.part[p].real ? (a.count + 1) / 2 : a.count);
+  return rings;
+}
+int LaunchFxRings(const FxPlan& plan, FxRingArgs args, cudaStream_t stream);
 
 }  // namespace sl3dgpu

@@ -427,6 +427,14 @@ __device__ inline void PrefetchL2(const void* p) { asm volatile("prefetch.global
 // memory.
 enum RingMode { kRingSynth = 0, kRingAnalyse = 1, kRingWeighted = 2 };
 
+// A launch over a tensor's three components (weighted rings): the CTAs along x
+// of a complex component, and the values between the components' spectra;
+// zero for a launch over one batch.
+struct RingParts {
+  int blocks = 0;
+  long long stride = 0;
+};
+
 // Rings per CTA (one warp each) so that a CTA's shared memory (the twiddles
 // and the rings' buffers: two for the planned stages, one for the two-stage
 // form, which works in place) stays near 100 KB.
@@ -452,7 +460,7 @@ template <class T2, int R1, int R2>
 __global__ void __launch_bounds__(256, (R1 > 0 && sizeof(T2) == 8) ? 3 : 1)
     RingKernel(int mode, int lmax, int ntheta, int count, bool real, FftPlan plan, const T2* twGlobal,
                const double* weights, const T2* spectraIn, const void* fieldsIn,
-               const typename Real<T2>::type* pointWeight, void* fieldsOut, T2* spectraOut) {
+               const typename Real<T2>::type* pointWeight, void* fieldsOut, T2* spectraOut, RingParts parts) {
   using T = typename Real<T2>::type;
   extern __shared__ __align__(16) unsigned char ringSmem[];
   const int n = R1 > 0 ? R1 * R2 : plan.n;  // a constant in the two-stage form
@@ -468,9 +476,18 @@ __global__ void __launch_bounds__(256, (R1 > 0 && sizeof(T2) == 8) ? 3 : 1)
   // A real field's ring shares one complex transform with the next field's
   // (z = x + i y; Z_m = X_m + i Y_m, X_m = (Z_m + conj Z_{n-m}) / 2,
   // Y_m = (Z_m - conj Z_{n-m}) / 2i): a warp carries two real fields.
+  int x = blockIdx.x;
+  if (parts.blocks > 0) {
+    // a tensor's component: two complex ones, then the real one
+    const int c = min(x / parts.blocks, 2);
+    x -= c * parts.blocks;
+    spectraIn += c * parts.stride;
+    spectraOut += c * parts.stride;
+    real = c == 2;
+  }
   const int perRing = real ? 2 : 1;
   const int j = blockIdx.y;
-  const int p0 = blockIdx.x * G * perRing;
+  const int p0 = x * G * perRing;
   const int groups = min(G * perRing, count - p0);  // fields of this CTA
   const int rings = (groups + perRing - 1) / perRing;
   const int mcount = real ? lmax + 1 : 2 * lmax + 1;
@@ -606,7 +623,7 @@ __global__ void __launch_bounds__(256, (R1 > 0 && sizeof(T2) == 8) ? 3 : 1)
 // for the sizes it is built for, else the plan's stages.
 template <class T2>
 using RingFn = void (*)(int, int, int, int, bool, FftPlan, const T2*, const double*, const T2*, const void*,
-                        const typename Real<T2>::type*, void*, T2*);
+                        const typename Real<T2>::type*, void*, T2*, RingParts);
 
 template <class T2>
 RingFn<T2> RingKernelFor(int n, int* buffers) {
@@ -833,46 +850,59 @@ int Grid::BatchFor(int N, bool real, bool analysis, int P, int p0, int count, co
     *out = &found->second;
     return SL3DGPU_OK;
   }
-  const SpinTable* t = nullptr;
-  if (int st = Table(N, &t); st != SL3DGPU_OK) return st;
   std::vector<GemmItem> items;
-  const int mlo = real ? 0 : -lmax;
-  const long long base = real ? t->rowOffset[lmax] : 0;
   Batch b;
-  for (int m = mlo; m <= lmax; ++m) {
-    const int rows = t->Rows(m, lmax);
-    if (rows == 0) continue;
-    const int mi = m - mlo;
-    GemmItem it{};
-    if (!analysis) {
-      it.M = ntheta;
-      it.N = 2 * count;
-      it.K = rows;
+  const int components = N == kTriple ? 3 : 1;
+  for (int c = 0; c < components; ++c) {
+    Part part;
+    part.N = N == kTriple ? c - 2 : N;
+    part.real = N == kTriple ? c == 2 : real;
+    part.first = static_cast<int>(items.size());
+    const SpinTable* t = nullptr;
+    if (int st = Table(part.N, &t); st != SL3DGPU_OK) return st;
+    const int mlo = part.real ? 0 : -lmax;
+    const long long base = part.real ? t->rowOffset[lmax] : 0;
+    // a triple's component among the coefficients' and the spectra's (doubles)
+    const long long coeffs = N == kTriple ? 2 * TripleRows(c) * P : 0;
+    const long long spectra = N == kTriple ? 2 * TripleStride(count) * c : 0;
+    for (int m = mlo; m <= lmax; ++m) {
+      const int rows = t->Rows(m, lmax);
+      if (rows == 0) continue;
+      const int mi = m - mlo;
+      const long long lm = coeffs + (t->rowOffset[m + lmax] - base) * 2LL * P + 2LL * p0;
+      const long long ring = spectra + static_cast<long long>(mi) * ntheta * 2LL * count;
+      GemmItem it{};
+      it.table = c;
       it.a = static_cast<long long>(t->rowOffset[m + lmax]) * ntheta;
-      it.b = (t->rowOffset[m + lmax] - base) * 2LL * P + 2LL * p0;
-      it.c = static_cast<long long>(mi) * ntheta * 2LL * count;
-      it.sAi = 1;
-      it.sAk = ntheta;
-      it.ldb = 2 * P;
-      it.ldc = 2 * count;
-    } else {
-      it.M = rows;
       it.N = 2 * count;
-      it.K = ntheta;
-      it.a = static_cast<long long>(t->rowOffset[m + lmax]) * ntheta;
-      it.b = static_cast<long long>(mi) * ntheta * 2LL * count;
-      it.c = (t->rowOffset[m + lmax] - base) * 2LL * P + 2LL * p0;
-      it.sAi = ntheta;
-      it.sAk = 1;
-      it.ldb = 2 * count;
-      it.ldc = 2 * P;
+      if (!analysis) {
+        it.M = ntheta;
+        it.K = rows;
+        it.b = lm;
+        it.c = ring;
+        it.sAi = 1;
+        it.sAk = ntheta;
+        it.ldb = 2 * P;
+        it.ldc = 2 * count;
+      } else {
+        it.M = rows;
+        it.K = ntheta;
+        it.b = ring;
+        it.c = lm;
+        it.sAi = ntheta;
+        it.sAk = 1;
+        it.ldb = 2 * count;
+        it.ldc = 2 * P;
+      }
+      b.maxM = std::max(b.maxM, it.M);
+      b.maxN = std::max(b.maxN, it.N);
+      b.maxK = std::max(b.maxK, it.K);
+      b.flops += 2.0 * it.M * it.N * it.K;
+      b.outputs += static_cast<double>(it.M) * it.N;
+      items.push_back(it);
     }
-    b.maxM = std::max(b.maxM, it.M);
-    b.maxN = std::max(b.maxN, it.N);
-    b.maxK = std::max(b.maxK, it.K);
-    b.flops += 2.0 * it.M * it.N * it.K;
-    b.outputs += static_cast<double>(it.M) * it.N;
-    items.push_back(it);
+    part.count = static_cast<int>(items.size()) - part.first;
+    b.parts.push_back(part);
   }
   b.count = static_cast<int>(items.size());
   b.analysis = analysis;
@@ -959,6 +989,16 @@ int Grid::RunGemm(const Batch& b, const double* A, const double* B, double* C, b
   return SL3DGPU_OK;
 }
 
+// The FP64 tables of a batch's parts.
+int Grid::Tables(const Batch& b, Tc64Tables* out) {
+  for (size_t c = 0; c < b.parts.size(); ++c) {
+    const SpinTable* t = nullptr;
+    if (int st = Table(b.parts[c].N, &t); st != SL3DGPU_OK) return st;
+    out->of[c] = t->values;
+  }
+  return SL3DGPU_OK;
+}
+
 // Whether a batch's FP64 contraction runs as slice products: within the
 // exactness bound on its depth, and wider than the narrow kernels' columns.
 bool Grid::UseSlices64(const Batch& b) const {
@@ -991,8 +1031,8 @@ int Grid::RunGemm64(int N, bool real, Batch& b, const double* B, double* C, bool
     SL3D_CUDA(cudaMalloc(&b.tc64Items, b.tc64Host.size() * sizeof(Tc64Item)));
     SL3D_CUDA(CopyIn(b.tc64Items, b.tc64Host.data(), b.tc64Host.size() * sizeof(Tc64Item)));
   }
-  const SpinTable* t = nullptr;
-  if (int st = Table(N, &t); st != SL3DGPU_OK) return st;
+  Tc64Tables tables;
+  if (int st = Tables(b, &tables); st != SL3DGPU_OK) return st;
   const std::array<int, 4> key{N, real ? 1 : 0, b.analysis ? 1 : 0, slices};
   auto found = panels64_.find(key);
   if (found == panels64_.end()) {
@@ -1000,9 +1040,12 @@ int Grid::RunGemm64(int N, bool real, Batch& b, const double* B, double* C, bool
     const size_t values = static_cast<size_t>(std::max<long long>(b.panel64, 1)) * slices * kTcTileM * kTcTileK;
     SL3D_CUDA(cudaMalloc(&panel.slices, values * sizeof(uint16_t)));
     SL3D_CUDA(cudaMalloc(&panel.rowExp, std::max<long long>(b.rowExps, 1) * sizeof(int)));
-    prof::Scope scope(prof::kOther, stream);
-    LaunchPanelA64(slices, b.items, b.tc64Items, b.count, b.maxM, b.maxATiles, t->values, panel, stream);
-    SL3D_CHECK_LAUNCH();
+    for (size_t c = 0; c < b.parts.size(); ++c) {
+      prof::Scope scope(prof::kOther, stream);
+      LaunchPanelA64(slices, b.items + b.parts[c].first, b.tc64Items + b.parts[c].first, b.parts[c].count, b.maxM,
+                     b.maxATiles, tables.of[c], panel, stream);
+      SL3D_CHECK_LAUNCH();
+    }
     found = panels64_.emplace(key, panel).first;
   }
   // this call's packed tiles, then its column exponents
@@ -1019,7 +1062,7 @@ int Grid::RunGemm64(int N, bool real, Batch& b, const double* B, double* C, bool
   }
   {
     prof::Scope scope(prof::kLegendre64Tc, stream, b.flops);
-    status = RunGemm64Tc(slices, b.items, b.tc64Items, b.count, b.maxMTiles, b.maxNTiles64, t->values, found->second,
+    status = RunGemm64Tc(slices, b.items, b.tc64Items, b.count, b.maxMTiles, b.maxNTiles64, tables, found->second,
                          B, packed, colExp, C, accumulate, dTcError_, stream);
   }
   SL3D_CUDA(cudaFreeAsync(scratch, stream));
@@ -1057,35 +1100,38 @@ int Grid::LegendreAnalysis(int N, bool real, const double* spectra, int P, int p
 }
 
 namespace {
+int LaunchRingWeightedF(Grid& g, int parts, bool real, const float* spectraIn, int count, const float* weight,
+                        float* spectraOut, cudaStream_t stream);
+
 // The most fields that count as a small batch (the FP64 units' rings).
 constexpr int kSmallBatch = 8;
 
-int LaunchRing(const Grid& g, int mode, bool real, int count, const double* spectraIn,
-               const void* fieldsIn, const double* weight, void* fieldsOut, double* spectraOut,
-               cudaStream_t stream, bool fixedPoint) {
+int LaunchRings(const Grid& g, int mode, int count, int parts, const FxRingPart* part, const double* weight,
+                cudaStream_t stream, bool fixedPoint) {
   if (count == 0) return SL3DGPU_OK;
-  // algorithmic traffic: the spectra and the grid values the mode reads and writes
-  const double spec = static_cast<double>(real ? g.lmax + 1 : 2 * g.lmax + 1) * g.ntheta * count * 16.0;
-  const double field = static_cast<double>(g.ntheta) * g.nphi * count * (real ? 8.0 : 16.0);
-  const double wbytes = weight ? static_cast<double>(g.ntheta) * g.nphi * count * 8.0 : 0.0;
-  const double bytes = mode == kRingWeighted ? 2 * spec + wbytes : spec + field + wbytes;
-  // a real field's transform counts half a complex one (two share a ring)
-  const double ffts = static_cast<double>(g.ntheta) * count * (mode == kRingWeighted ? 2 : 1) * (real ? 0.5 : 1.0);
-  prof::Scope scope(prof::kRing, stream, ffts * 5.0 * g.nphi * std::log2(static_cast<double>(g.nphi)), bytes);
   FxRingArgs a{};
   a.mode = mode;
   a.lmax = g.lmax;
   a.ntheta = g.ntheta;
   a.count = count;
-  a.real = real;
   a.roots = g.dRoots;
   a.twiddle = g.dTwiddle;
   a.weights = g.dWeights;
-  a.spectraIn = reinterpret_cast<const double2*>(spectraIn);
-  a.fieldsIn = fieldsIn;
   a.pointWeight = weight;
-  a.fieldsOut = fieldsOut;
-  a.spectraOut = reinterpret_cast<double2*>(spectraOut);
+  a.parts = parts;
+  double ffts = 0.0, bytes = 0.0;
+  for (int p = 0; p < parts; ++p) {
+    a.part[p] = part[p];
+    // algorithmic traffic: the spectra and the grid values the mode reads and
+    // writes; a real field's transform counts half a complex one (two share a ring)
+    const bool real = part[p].real;
+    const double spec = static_cast<double>(real ? g.lmax + 1 : 2 * g.lmax + 1) * g.ntheta * count * 16.0;
+    const double field = static_cast<double>(g.ntheta) * g.nphi * count * (real ? 8.0 : 16.0);
+    const double wbytes = weight ? static_cast<double>(g.ntheta) * g.nphi * count * 8.0 : 0.0;
+    bytes += mode == kRingWeighted ? 2 * spec + wbytes : spec + field + wbytes;
+    ffts += static_cast<double>(g.ntheta) * count * (mode == kRingWeighted ? 2 : 1) * (real ? 0.5 : 1.0);
+  }
+  prof::Scope scope(prof::kRing, stream, ffts * 5.0 * g.nphi * std::log2(static_cast<double>(g.nphi)), bytes);
   if (g.emulateFp64) return LaunchDfRings(g.dfPlan, a, stream);
   // A batch of few fields is a launch's latency either way; it stays on the
   // FP64 units, so that fields made one at a time -- the delta field and the
@@ -1098,14 +1144,110 @@ int LaunchRing(const Grid& g, int mode, bool real, int count, const double* spec
   const RingFn<double2> kernel = RingKernelFor<double2>(g.nphi, &buffers);
   const int rings = RingsPerCta<double2>(g.nphi, buffers);
   SL3D_CUDA(AllowDynamicSmem(kernel));
-  const int perCta = real ? 2 * rings : rings;  // real fields go two to a ring
-  kernel<<<dim3((count + perCta - 1) / perCta, g.ntheta), rings * kWarp, RingSmem<double2>(g.nphi, rings, buffers),
-           stream>>>(mode, g.lmax, g.ntheta, count, real, g.plan, g.dTwiddle, g.dWeights, a.spectraIn, fieldsIn,
-                     weight, fieldsOut, a.spectraOut);
-  SL3D_CHECK_LAUNCH();
+  for (int p = 0; p < parts; ++p) {
+    const FxRingPart& q = part[p];
+    const int perCta = q.real ? 2 * rings : rings;  // real fields go two to a ring
+    kernel<<<dim3((count + perCta - 1) / perCta, g.ntheta), rings * kWarp, RingSmem<double2>(g.nphi, rings, buffers),
+             stream>>>(mode, g.lmax, g.ntheta, count, q.real, g.plan, g.dTwiddle, g.dWeights, q.spectraIn, q.fieldsIn,
+                       weight, q.fieldsOut, q.spectraOut, RingParts{});
+    SL3D_CHECK_LAUNCH();
+  }
   return SL3DGPU_OK;
 }
+
+int LaunchRing(const Grid& g, int mode, bool real, int count, const double* spectraIn,
+               const void* fieldsIn, const double* weight, void* fieldsOut, double* spectraOut,
+               cudaStream_t stream, bool fixedPoint) {
+  const FxRingPart part{real, reinterpret_cast<const double2*>(spectraIn), fieldsIn, fieldsOut,
+                        reinterpret_cast<double2*>(spectraOut)};
+  return LaunchRings(g, mode, count, 1, &part, weight, stream, fixedPoint);
+}
 }  // namespace
+
+// -- a tensor's three components ------------------------------------------------------------
+
+int Grid::RingSynthesis3(const double* spectra, int count, double2* f0, double2* f1, double* fr, cudaStream_t stream) {
+  const auto* s = reinterpret_cast<const double2*>(spectra);
+  const long long stride = TripleStride(count);
+  const FxRingPart parts[3] = {{false, s, nullptr, f0, nullptr},
+                               {false, s + stride, nullptr, f1, nullptr},
+                               {true, s + 2 * stride, nullptr, fr, nullptr}};
+  return LaunchRings(*this, kRingSynth, count, 3, parts, nullptr, stream, false);
+}
+
+int Grid::RingAnalysis3(const double2* f0, const double2* f1, const double* fr, int count, double* spectra,
+                        cudaStream_t stream, const double* weight) {
+  auto* s = reinterpret_cast<double2*>(spectra);
+  const long long stride = TripleStride(count);
+  const FxRingPart parts[3] = {{false, nullptr, f0, nullptr, s},
+                               {false, nullptr, f1, nullptr, s + stride},
+                               {true, nullptr, fr, nullptr, s + 2 * stride}};
+  return LaunchRings(*this, kRingAnalyse, count, 3, parts, weight, stream, false);
+}
+
+int Grid::RingWeighted3(const double* spectraIn, int count, const double* weight, double* spectraOut,
+                        cudaStream_t stream) {
+  const auto* in = reinterpret_cast<const double2*>(spectraIn);
+  auto* out = reinterpret_cast<double2*>(spectraOut);
+  const long long stride = TripleStride(count);
+  FxRingPart parts[3];
+  for (int c = 0; c < 3; ++c) parts[c] = {c == 2, in + c * stride, nullptr, nullptr, out + c * stride};
+  return LaunchRings(*this, kRingWeighted, count, 3, parts, weight, stream, false);
+}
+
+int Grid::LegendreSynthesis3(const double* coeffs, int P, int p0, int count, double* spectra, cudaStream_t stream) {
+  if (count == 0) return SL3DGPU_OK;
+  const Batch* b = nullptr;
+  if (int st = BatchFor(kTriple, false, false, P, p0, count, &b); st != SL3DGPU_OK) return st;
+  if (UseSlices64(*b))
+    return RunGemm64(kTriple, false, *MutableBatch(kTriple, false, false, P, p0, count), coeffs, spectra, false,
+                     stream);
+  for (int c = 0; c < 3; ++c)
+    if (int st = LegendreSynthesis(c - 2, c == 2, coeffs + 2 * TripleRows(c) * P, P, p0, count,
+                                   spectra + 2 * TripleStride(count) * c, stream);
+        st != SL3DGPU_OK)
+      return st;
+  return SL3DGPU_OK;
+}
+
+int Grid::LegendreAnalysis3(const double* spectra, int P, int p0, int count, double* coeffs, bool accumulate,
+                            cudaStream_t stream) {
+  if (count == 0) return SL3DGPU_OK;
+  const Batch* b = nullptr;
+  if (int st = BatchFor(kTriple, false, true, P, p0, count, &b); st != SL3DGPU_OK) return st;
+  if (UseSlices64(*b))
+    return RunGemm64(kTriple, false, *MutableBatch(kTriple, false, true, P, p0, count), spectra, coeffs, accumulate,
+                     stream);
+  for (int c = 0; c < 3; ++c)
+    if (int st = LegendreAnalysis(c - 2, c == 2, spectra + 2 * TripleStride(count) * c, P, p0, count,
+                                  coeffs + 2 * TripleRows(c) * P, accumulate, stream);
+        st != SL3DGPU_OK)
+      return st;
+  return SL3DGPU_OK;
+}
+
+int Grid::LegendreSynthesis3F(const float* coeffs, int count, float* spectra, cudaStream_t stream) {
+  if (count == 0) return SL3DGPU_OK;
+  const SpinTable* t = nullptr;
+  if (int st = Table32(0, &t); st != SL3DGPU_OK) return st;
+  Batch* b = MutableBatch(kTriple, false, false, count, 0, count);
+  if (b == nullptr) return SL3DGPU_ERR_CUDA;
+  return RunGemmF(kTriple, false, *b, coeffs, spectra, false, stream);
+}
+
+int Grid::LegendreAnalysis3F(const float* spectra, int count, float* coeffs, cudaStream_t stream) {
+  if (count == 0) return SL3DGPU_OK;
+  const SpinTable* t = nullptr;
+  if (int st = Table32(0, &t); st != SL3DGPU_OK) return st;
+  Batch* b = MutableBatch(kTriple, false, true, count, 0, count);
+  if (b == nullptr) return SL3DGPU_ERR_CUDA;
+  return RunGemmF(kTriple, false, *b, spectra, coeffs, false, stream);
+}
+
+int Grid::RingWeighted3F(const float* spectraIn, int count, const float* weight, float* spectraOut,
+                         cudaStream_t stream) {
+  return LaunchRingWeightedF(*this, 3, false, spectraIn, count, weight, spectraOut, stream);
+}
 
 int Grid::RingSynthesis(bool real, const double* spectra, int count, double* fields,
                         cudaStream_t stream, bool fixedPoint) {
@@ -1159,13 +1301,16 @@ int Grid::RunGemmF(int N, bool real, Batch& b, const float* B, float* C, bool ac
   const std::array<int, 3> key{N, real ? 1 : 0, b.analysis ? 1 : 0};
   auto found = panels_.find(key);
   if (found == panels_.end()) {
-    const SpinTable* t = nullptr;
-    if (int st = Table(N, &t); st != SL3DGPU_OK) return st;
+    Tc64Tables tables;
+    if (int st = Tables(b, &tables); st != SL3DGPU_OK) return st;
     float* panel = nullptr;
     SL3D_CUDA(cudaMalloc(&panel, std::max<long long>(b.panelFloats, 1) * sizeof(float)));
-    prof::Scope scope(prof::kOther, stream);
-    LaunchPanelA(b.items, items, b.count, b.maxATiles, t->values, panel, stream);
-    SL3D_CHECK_LAUNCH();
+    for (size_t c = 0; c < b.parts.size(); ++c) {
+      prof::Scope scope(prof::kOther, stream);
+      LaunchPanelA(b.items + b.parts[c].first, items + b.parts[c].first, b.parts[c].count, b.maxATiles, tables.of[c],
+                   panel, stream);
+      SL3D_CHECK_LAUNCH();
+    }
     found = panels_.emplace(key, panel).first;
   }
   // B split and packed inside the contraction (B and C never overlap here:
@@ -1235,27 +1380,44 @@ int Grid::LegendreAnalysisF(int N, bool real, const float* spectra, int P, int p
 
 int Grid::RingWeightedF(bool real, const float* spectraIn, int count, const float* weight, float* spectraOut,
                         cudaStream_t stream) {
+  return LaunchRingWeightedF(*this, 1, real, spectraIn, count, weight, spectraOut, stream);
+}
+
+namespace {
+// The FP32 weighted rings of one batch, or (parts 3) of a tensor's components.
+int LaunchRingWeightedF(Grid& g, int parts, bool real, const float* spectraIn, int count, const float* weight,
+                        float* spectraOut, cudaStream_t stream) {
   if (count == 0) return SL3DGPU_OK;
   const SpinTable* t = nullptr;
-  if (int st = Table32(0, &t); st != SL3DGPU_OK) return st;  // makes the FP32 twiddles
+  if (int st = g.Table32(0, &t); st != SL3DGPU_OK) return st;  // makes the FP32 twiddles
   int buffers = 2;
-  const RingFn<float2> kernel = RingKernelFor<float2>(nphi, &buffers);
-  const int rings = RingsPerCta<float2>(nphi, buffers);
-  const size_t smem = RingSmem<float2>(nphi, rings, buffers);
+  const RingFn<float2> kernel = RingKernelFor<float2>(g.nphi, &buffers);
+  const int rings = RingsPerCta<float2>(g.nphi, buffers);
+  const size_t smem = RingSmem<float2>(g.nphi, rings, buffers);
   SL3D_CUDA(AllowDynamicSmem(kernel));
-  const int fields = real ? 2 * rings : rings;  // real fields go two to a ring
-  dim3 grid((count + fields - 1) / fields, ntheta);
-  const double spec = static_cast<double>(real ? lmax + 1 : 2 * lmax + 1) * ntheta * count * 8.0;
-  const double wbytes = static_cast<double>(ntheta) * nphi * count * 4.0;
-  prof::Scope scope(prof::kRing32, stream,
-                    (real ? 1.0 : 2.0) * ntheta * count * 5.0 * nphi * std::log2(static_cast<double>(nphi)),
-                    2 * spec + wbytes);
-  kernel<<<grid, rings * kWarp, smem, stream>>>(kRingWeighted, lmax, ntheta, count, real, plan, dTwiddle32,
-                                                  dWeights, reinterpret_cast<const float2*>(spectraIn), nullptr,
-                                                  weight, nullptr, reinterpret_cast<float2*>(spectraOut));
+  auto blocks = [&](bool re) { return (count + (re ? 2 * rings : rings) - 1) / (re ? 2 * rings : rings); };
+  RingParts p{};
+  int x = blocks(real);
+  if (parts == 3) {
+    p.blocks = blocks(false);
+    p.stride = g.TripleStride(count);
+    x = 2 * p.blocks + blocks(true);
+  }
+  double flops = 0.0, bytes = 0.0;
+  for (int c = 0; c < parts; ++c) {
+    const bool re = parts == 3 ? c == 2 : real;
+    bytes += 2.0 * (re ? g.lmax + 1 : 2 * g.lmax + 1) * g.ntheta * count * 8.0 +
+             static_cast<double>(g.ntheta) * g.nphi * count * 4.0;
+    flops += (re ? 1.0 : 2.0) * g.ntheta * count * 5.0 * g.nphi * std::log2(static_cast<double>(g.nphi));
+  }
+  prof::Scope scope(prof::kRing32, stream, flops, bytes);
+  kernel<<<dim3(x, g.ntheta), rings * kWarp, smem, stream>>>(
+      kRingWeighted, g.lmax, g.ntheta, count, real, g.plan, g.dTwiddle32, g.dWeights,
+      reinterpret_cast<const float2*>(spectraIn), nullptr, weight, nullptr, reinterpret_cast<float2*>(spectraOut), p);
   SL3D_CHECK_LAUNCH();
   return SL3DGPU_OK;
 }
+}  // namespace
 
 int Grid::ToDevice(int N, bool real, const double* ref, int count, double* dev,
                    cudaStream_t stream) {

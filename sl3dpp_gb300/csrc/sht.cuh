@@ -46,7 +46,8 @@ struct SpinTable {
 };
 
 struct GemmItem {
-  int M, N, K, pad;
+  int M, N, K;
+  int table;  // which of its batch's tables A is in
   long long a, b, c;
   int sAi, sAk, ldb, ldc;
 };
@@ -61,6 +62,11 @@ struct Tc64Item {
   long long b, c;    // FP64 offsets of B's source and of C
   long long rowExp;  // ints: the power-of-two exponents of its M rows of A
   long long colExp;  // ints: those of its N columns of B (per call)
+};
+
+// A batch's FP64 tables (a tensor's three spins, or one).
+struct Tc64Tables {
+  const double* of[3] = {nullptr, nullptr, nullptr};
 };
 
 // The table split into FP64 slices for one direction: its slice panels and
@@ -147,6 +153,29 @@ class Grid {
   int RingWeightedF(bool real, const float* spectraIn, int count, const float* weight, float* spectraOut,
                     cudaStream_t stream);
 
+  // The same for a tensor's three components at once, spins -2 and -1 and the
+  // real spin 0, in one launch each where the one-component calls would take
+  // three: coefficients the components' rows one after another
+  // ([row][P] each), spectra theirs ([m][j][count] each, TripleStride(count)
+  // complex values apart). One launch fills the SMs at small sizes and has
+  // one last wave at large ones. lmax >= 2, so every order of every component
+  // has degrees.
+  long long TripleStride(int count) const { return static_cast<long long>(2 * lmax + 1) * ntheta * count; }
+  // Complex values a triple's spectra take.
+  static long long TripleSize(int lmax, int ntheta, int count) {
+    return (2LL * (2 * lmax + 1) + lmax + 1) * ntheta * count;
+  }
+  int LegendreSynthesis3(const double* coeffs, int P, int p0, int count, double* spectra, cudaStream_t stream);
+  int LegendreAnalysis3(const double* spectra, int P, int p0, int count, double* coeffs, bool accumulate,
+                        cudaStream_t stream);
+  int RingSynthesis3(const double* spectra, int count, double2* f0, double2* f1, double* fr, cudaStream_t stream);
+  int RingAnalysis3(const double2* f0, const double2* f1, const double* fr, int count, double* spectra,
+                    cudaStream_t stream, const double* weight = nullptr);
+  int RingWeighted3(const double* spectraIn, int count, const double* weight, double* spectraOut, cudaStream_t stream);
+  int LegendreSynthesis3F(const float* coeffs, int count, float* spectra, cudaStream_t stream);
+  int LegendreAnalysis3F(const float* spectra, int count, float* coeffs, cudaStream_t stream);
+  int RingWeighted3F(const float* spectraIn, int count, const float* weight, float* spectraOut, cudaStream_t stream);
+
   // Reference layout <-> device layout permutations.
   int ToDevice(int N, bool real, const double* ref, int count, double* dev, cudaStream_t stream);
   int FromDevice(int N, bool real, const double* dev, int count, double* ref, cudaStream_t stream);
@@ -156,7 +185,16 @@ class Grid {
 
  private:
   std::map<int, SpinTable> tables_;
+  // The components a batch's contraction covers: a spin's, or a tensor's three
+  // (N = kTriple), each an item range with its own table.
+  static constexpr int kTriple = 1000;
+  struct Part {
+    int N = 0;
+    bool real = false;
+    int first = 0, count = 0;  // items
+  };
   struct Batch {
+    std::vector<Part> parts;
     GemmItem* items = nullptr;
     int count = 0, maxM = 0, maxN = 0;
     bool analysis = false;
@@ -186,6 +224,11 @@ class Grid {
   // the grid between them.
   cudaMemPool_t pool_ = nullptr;
   bool UseSlices64(const Batch& b) const;
+  int Tables(const Batch& b, Tc64Tables* out);
+  // The complex rows before a triple's component, and its spin.
+  long long TripleRows(int component) const {
+    return component == 0 ? 0 : component == 1 ? SpinRows(-2) : SpinRows(-2) + SpinRows(-1);
+  }
   int RunGemm64(int N, bool real, Batch& b, const double* B, double* C, bool accumulate, cudaStream_t stream);
   // The table pre-tiled for the tensor cores per (spin, real, direction).
   std::map<std::array<int, 3>, float*> panels_;
@@ -202,6 +245,9 @@ class Grid {
   // panel (made on first use), B packed, the contraction.
   int RunGemmF(int N, bool real, Batch& b, const float* B, float* C, bool accumulate, cudaStream_t stream);
   int* dTcError_ = nullptr;  // set by a tensor-core wait that gave up
+
+ public:
+  // The spin's table, with the FP32 twiddles made.
   int Table32(int N, const SpinTable** out);
 };
 

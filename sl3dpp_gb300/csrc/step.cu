@@ -733,7 +733,7 @@ int Viscoelastic3DGpu::Create(const sl3dgpu_layer* layers, int nlayers, const sl
   SL3D_CUDA(rhsSph.Alloc(rhsSphComplex));
   SL3D_CUDA(rhsTor.Alloc(std::max<long long>(rhsTorComplex, 1)));
   for (auto* b : {&s, &sNext, &fixedS, &analysed, &analysedStart}) SL3D_CUDA(b->Alloc(spectralComplex));
-  const size_t spectra = static_cast<size_t>(2 * L + 1) * grid->ntheta * P;
+  const size_t spectra = static_cast<size_t>(Grid::TripleSize(L, grid->ntheta, P));  // a tensor's three components
   SL3D_CUDA(spectraA.Alloc(spectra));
   SL3D_CUDA(spectraB.Alloc(spectra));
   if (!staticMode) {
@@ -889,51 +889,25 @@ int Viscoelastic3DGpu::FlavourOf(int scheme, double dt, Flavour** out) {
 // -- transforms over the nodes ----------------------------------------------------------------------
 
 int Viscoelastic3DGpu::Synthesise(const double2* spectral, GridTensor& out) {
-  const auto* base = reinterpret_cast<const double*>(spectral);
-  auto* spectra = reinterpret_cast<double*>(spectraA.p);
-  SL3D_TRY(grid->LegendreSynthesis(-2, false, base, P, 0, P, spectra, stream));
-  SL3D_TRY(grid->RingSynthesis(false, spectra, P, reinterpret_cast<double*>(out.c0.p), stream));
-  SL3D_TRY(grid->LegendreSynthesis(-1, false, base + 2 * rows0 * P, P, 0, P, spectra, stream));
-  SL3D_TRY(grid->RingSynthesis(false, spectra, P, reinterpret_cast<double*>(out.c1.p), stream));
-  SL3D_TRY(grid->LegendreSynthesis(0, true, base + 2 * (rows0 + rows1) * P, P, 0, P, spectra, stream));
-  return grid->RingSynthesis(true, spectra, P, out.r.p, stream);
+  return SynthesiseRange(spectral, out, 0, P);
 }
 
-int Viscoelastic3DGpu::Analyse(const GridTensor& in, double2* spectral) {
-  auto* base = reinterpret_cast<double*>(spectral);
-  auto* spectra = reinterpret_cast<double*>(spectraA.p);
-  SL3D_TRY(grid->RingAnalysis(false, reinterpret_cast<const double*>(in.c0.p), P, spectra, stream));
-  SL3D_TRY(grid->LegendreAnalysis(-2, false, spectra, P, 0, P, base, false, stream));
-  SL3D_TRY(grid->RingAnalysis(false, reinterpret_cast<const double*>(in.c1.p), P, spectra, stream));
-  SL3D_TRY(grid->LegendreAnalysis(-1, false, spectra, P, 0, P, base + 2 * rows0 * P, false, stream));
-  SL3D_TRY(grid->RingAnalysis(true, in.r.p, P, spectra, stream));
-  return grid->LegendreAnalysis(0, true, spectra, P, 0, P, base + 2 * (rows0 + rows1) * P, false, stream);
-}
+int Viscoelastic3DGpu::Analyse(const GridTensor& in, double2* spectral) { return AnalyseRange(in, spectral, 0, P); }
 
 int Viscoelastic3DGpu::SynthesiseRange(const double2* spectral, GridTensor& out, int p0, int count) {
   if (count <= 0) return SL3DGPU_OK;
-  const auto* base = reinterpret_cast<const double*>(spectral);
   auto* spectra = reinterpret_cast<double*>(spectraA.p);
   const long long off = p0 * fieldSize;
-  SL3D_TRY(grid->LegendreSynthesis(-2, false, base, P, p0, count, spectra, stream));
-  SL3D_TRY(grid->RingSynthesis(false, spectra, count, reinterpret_cast<double*>(out.c0.p + off), stream));
-  SL3D_TRY(grid->LegendreSynthesis(-1, false, base + 2 * rows0 * P, P, p0, count, spectra, stream));
-  SL3D_TRY(grid->RingSynthesis(false, spectra, count, reinterpret_cast<double*>(out.c1.p + off), stream));
-  SL3D_TRY(grid->LegendreSynthesis(0, true, base + 2 * (rows0 + rows1) * P, P, p0, count, spectra, stream));
-  return grid->RingSynthesis(true, spectra, count, out.r.p + off, stream);
+  SL3D_TRY(grid->LegendreSynthesis3(reinterpret_cast<const double*>(spectral), P, p0, count, spectra, stream));
+  return grid->RingSynthesis3(spectra, count, out.c0.p + off, out.c1.p + off, out.r.p + off, stream);
 }
 
 int Viscoelastic3DGpu::AnalyseRange(const GridTensor& in, double2* spectral, int p0, int count) {
   if (count <= 0) return SL3DGPU_OK;
-  auto* base = reinterpret_cast<double*>(spectral);
   auto* spectra = reinterpret_cast<double*>(spectraA.p);
   const long long off = p0 * fieldSize;
-  SL3D_TRY(grid->RingAnalysis(false, reinterpret_cast<const double*>(in.c0.p + off), count, spectra, stream));
-  SL3D_TRY(grid->LegendreAnalysis(-2, false, spectra, P, p0, count, base, false, stream));
-  SL3D_TRY(grid->RingAnalysis(false, reinterpret_cast<const double*>(in.c1.p + off), count, spectra, stream));
-  SL3D_TRY(grid->LegendreAnalysis(-1, false, spectra, P, p0, count, base + 2 * rows0 * P, false, stream));
-  SL3D_TRY(grid->RingAnalysis(true, in.r.p + off, count, spectra, stream));
-  return grid->LegendreAnalysis(0, true, spectra, P, p0, count, base + 2 * (rows0 + rows1) * P, false, stream);
+  SL3D_TRY(grid->RingAnalysis3(in.c0.p + off, in.c1.p + off, in.r.p + off, count, spectra, stream));
+  return grid->LegendreAnalysis3(spectra, P, p0, count, reinterpret_cast<double*>(spectral), false, stream);
 }
 
 // The nodes a state holds on the grid follow the operator's lateral range;
@@ -990,35 +964,21 @@ SpectralMemoryArgs Viscoelastic3DGpu::SpectralArgs(int scheme, double dt, const 
 int Viscoelastic3DGpu::AnalyseWeighted(const GridTensor& in, const double* w, double2* spectral) {
   const int p0 = lateralFirst, count = lateralEnd - lateralFirst;
   if (count <= 0) return SL3DGPU_OK;
-  auto* base = reinterpret_cast<double*>(spectral);
   auto* spectra = reinterpret_cast<double*>(spectraA.p);
   const long long off = p0 * fieldSize;
-  SL3D_TRY(grid->RingAnalysis(false, reinterpret_cast<const double*>(in.c0.p + off), count, spectra, stream, w + off));
-  SL3D_TRY(grid->LegendreAnalysis(-2, false, spectra, P, p0, count, base, true, stream));
-  SL3D_TRY(grid->RingAnalysis(false, reinterpret_cast<const double*>(in.c1.p + off), count, spectra, stream, w + off));
-  SL3D_TRY(grid->LegendreAnalysis(-1, false, spectra, P, p0, count, base + 2 * rows0 * P, true, stream));
-  SL3D_TRY(grid->RingAnalysis(true, in.r.p + off, count, spectra, stream, w + off));
-  return grid->LegendreAnalysis(0, true, spectra, P, p0, count, base + 2 * (rows0 + rows1) * P, true, stream);
+  SL3D_TRY(grid->RingAnalysis3(in.c0.p + off, in.c1.p + off, in.r.p + off, count, spectra, stream, w + off));
+  return grid->LegendreAnalysis3(spectra, P, p0, count, reinterpret_cast<double*>(spectral), true, stream);
 }
 
 // Analyse(W Synthesise(strain)) over the lateral nodes, added onto out.
 int Viscoelastic3DGpu::WeightedPass(const double2* strain, double2* out) {
   const int p0 = lateralFirst, count = lateralEnd - lateralFirst;
   if (count <= 0) return SL3DGPU_OK;
-  const auto* in = reinterpret_cast<const double*>(strain);
-  auto* o = reinterpret_cast<double*>(out);
   auto* a = reinterpret_cast<double*>(spectraA.p);
   auto* b = reinterpret_cast<double*>(spectraB.p);
-  const double* w = weight.p + p0 * fieldSize;
-  const long long offs[3] = {0, 2 * rows0 * P, 2 * (rows0 + rows1) * P};
-  const int spins[3] = {-2, -1, 0};
-  for (int c = 0; c < 3; ++c) {
-    const bool real = c == 2;
-    SL3D_TRY(grid->LegendreSynthesis(spins[c], real, in + offs[c], P, p0, count, a, stream));
-    SL3D_TRY(grid->RingWeighted(real, a, count, w, b, stream));
-    SL3D_TRY(grid->LegendreAnalysis(spins[c], real, b, P, p0, count, o + offs[c], true, stream));
-  }
-  return SL3DGPU_OK;
+  SL3D_TRY(grid->LegendreSynthesis3(reinterpret_cast<const double*>(strain), P, p0, count, a, stream));
+  SL3D_TRY(grid->RingWeighted3(a, count, weight.p + p0 * fieldSize, b, stream));
+  return grid->LegendreAnalysis3(b, P, p0, count, reinterpret_cast<double*>(out), true, stream);
 }
 
 // -- a pass --------------------------------------------------------------------------------------------
@@ -1941,18 +1901,9 @@ int Viscoelastic3DGpu::PrepareLateral() {
 int Viscoelastic3DGpu::WeightedPass32(const float2* strain, float2* out) {
   const int p0 = lateralFirst, count = lateralEnd - lateralFirst;
   if (count <= 0) return SL3DGPU_OK;
-  const auto* in = reinterpret_cast<const float*>(strain);
-  auto* o = reinterpret_cast<float*>(out);
-  const float* w = weight32.p + p0 * fieldSize;
-  const long long offs[3] = {0, 2 * rows0 * count, 2 * (rows0 + rows1) * count};
-  const int spins[3] = {-2, -1, 0};
-  for (int c = 0; c < 3; ++c) {
-    const bool real = c == 2;
-    SL3D_TRY(grid->LegendreSynthesisF(spins[c], real, in + offs[c], count, 0, count, spectra32A.p, stream));
-    SL3D_TRY(grid->RingWeightedF(real, spectra32A.p, count, w, spectra32B.p, stream));
-    SL3D_TRY(grid->LegendreAnalysisF(spins[c], real, spectra32B.p, count, 0, count, o + offs[c], false, stream));
-  }
-  return SL3DGPU_OK;
+  SL3D_TRY(grid->LegendreSynthesis3F(reinterpret_cast<const float*>(strain), count, spectra32A.p, stream));
+  SL3D_TRY(grid->RingWeighted3F(spectra32A.p, count, weight32.p + p0 * fieldSize, spectra32B.p, stream));
+  return grid->LegendreAnalysis3F(spectra32B.p, count, reinterpret_cast<float*>(out), stream);
 }
 
 // The flavour's per-system row windows for the current lateral range: a

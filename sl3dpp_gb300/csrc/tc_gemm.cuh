@@ -104,7 +104,7 @@ void LaunchPanelA64(int slices, const GemmItem* items, const Tc64Item* tcItems, 
 void LaunchPackB64(int slices, const Tc64Item* tcItems, int count, int maxNTiles, const double* B, int* colExp,
                    uint16_t* packed, cudaStream_t stream);
 int RunGemm64Tc(int slices, const GemmItem* items, const Tc64Item* tcItems, int count, int maxMTiles, int maxNTiles,
-                const double* table, const Tc64Panel& panel, const double* B, uint16_t* packed, int* colExp, double* C,
-                bool accumulate, int* errorFlag, cudaStream_t stream);
+                const Tc64Tables& tables, const Tc64Panel& panel, const double* B, uint16_t* packed, int* colExp,
+                double* C, bool accumulate, int* errorFlag, cudaStream_t stream);
 
 }  // namespace sl3dgpu

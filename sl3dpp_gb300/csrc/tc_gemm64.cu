@@ -276,7 +276,7 @@ __global__ void __launch_bounds__(kPackThreads) PackB64Kernel(const Tc64Item* tc
 
 template <int S>
 __global__ void __launch_bounds__(kThreads, 2) TcGemm64Kernel(const GemmItem* items, const Tc64Item* tcItems,
-                                                           const double* table, const double* B,
+                                                           const Tc64Tables tables, const double* B,
                                                            const uint16_t* panels, const uint16_t* packed,
                                                            const int* rowExp, const int* colExp, double* C,
                                                            bool accumulate, int* errorFlag) {
@@ -443,7 +443,7 @@ __global__ void __launch_bounds__(kThreads, 2) TcGemm64Kernel(const GemmItem* it
           if (!good)
             rowsOut[warp][lane][q] = __longlong_as_double(0x7FF8000000000000LL);
           else if (((columns >> q) & 1u) && i < it.M)
-            rowsOut[warp][lane][q] = PlainSum(items[blockIdx.z], table, B, i, n0 + c0 + q);
+            rowsOut[warp][lane][q] = PlainSum(items[blockIdx.z], tables.of[items[blockIdx.z].table], B, i, n0 + c0 + q);
       }
       __syncwarp();
       const int n = c0 + (lane & 15);
@@ -474,7 +474,7 @@ __global__ void __launch_bounds__(kThreads, 2) TcGemm64Kernel(const GemmItem* it
 
 namespace {
 template <int S>
-int Run(const GemmItem* items, const Tc64Item* tcItems, int count, int maxMTiles, int maxNTiles, const double* table,
+int Run(const GemmItem* items, const Tc64Item* tcItems, int count, int maxMTiles, int maxNTiles, const Tc64Tables& tables,
         const Tc64Panel& panel, const double* B, uint16_t* packed, int* colExp, double* C, bool accumulate,
         int* errorFlag, cudaStream_t stream) {
   constexpr size_t smem = static_cast<size_t>(kStages) * S * (kATile + kBTile) * sizeof(uint16_t) +
@@ -483,7 +483,7 @@ int Run(const GemmItem* items, const Tc64Item* tcItems, int count, int maxMTiles
   static_assert(smem >= kThreads / 32 * 32 * 17 * sizeof(double), "the epilogue's staging fits in the stages");
   SL3D_CUDA(AllowDynamicSmem(TcGemm64Kernel<S>));
   dim3 grid(static_cast<unsigned>(maxNTiles), static_cast<unsigned>(maxMTiles), static_cast<unsigned>(count));
-  TcGemm64Kernel<S><<<grid, kThreads, smem, stream>>>(items, tcItems, table, B, panel.slices, packed, panel.rowExp,
+  TcGemm64Kernel<S><<<grid, kThreads, smem, stream>>>(items, tcItems, tables, B, panel.slices, packed, panel.rowExp,
                                                       colExp, C, accumulate, errorFlag);
   SL3D_CHECK_LAUNCH();
   return SL3DGPU_OK;
@@ -514,13 +514,13 @@ void LaunchPackB64(int slices, const Tc64Item* tcItems, int count, int maxNTiles
 }
 
 int RunGemm64Tc(int slices, const GemmItem* items, const Tc64Item* tcItems, int count, int maxMTiles, int maxNTiles,
-                const double* table, const Tc64Panel& panel, const double* B, uint16_t* packed, int* colExp, double* C,
-                bool accumulate, int* errorFlag, cudaStream_t stream) {
+                const Tc64Tables& tables, const Tc64Panel& panel, const double* B, uint16_t* packed, int* colExp,
+                double* C, bool accumulate, int* errorFlag, cudaStream_t stream) {
   if (count == 0 || maxMTiles == 0 || maxNTiles == 0) return SL3DGPU_OK;
   return slices == kTc64SlicesFull
-             ? Run<kTc64SlicesFull>(items, tcItems, count, maxMTiles, maxNTiles, table, panel, B, packed, colExp, C,
+             ? Run<kTc64SlicesFull>(items, tcItems, count, maxMTiles, maxNTiles, tables, panel, B, packed, colExp, C,
                                     accumulate, errorFlag, stream)
-             : Run<kTc64Slices>(items, tcItems, count, maxMTiles, maxNTiles, table, panel, B, packed, colExp, C,
+             : Run<kTc64Slices>(items, tcItems, count, maxMTiles, maxNTiles, tables, panel, B, packed, colExp, C,
                                 accumulate, errorFlag, stream);
 }
 
