@@ -780,29 +780,41 @@ __global__ void MixerSweepKernel(MixerArgsT<T> a) {
 #pragma unroll
   for (int i = 0; i < M; ++i) dF[i] = a.dF[i];
   for (long long at = begin + threadIdx.x; at < end; at += blockDim.x) {
-    const T xs = a.x[at], gs = a.gx[at];
+    // every load of the turn before its first use
+    const T xs = a.x[at], gs = a.gx[at], xp = a.xPrev[at], fp = a.fPrev[at];
+    H history[M + 1];
+#pragma unroll
+    for (int i = 0; i < M; ++i)
+      if (i < m && i != slot) history[i] = dF[i][at];
     const T f = gs - xs;
-    const T dx = xs - a.xPrev[at];
-    const H dfStored = ToHistory(f - a.fPrev[at], dFs);
+    const T dx = xs - xp;
+    const H dfStored = ToHistory(f - fp, dFs);
     dFs[at] = dfStored;
-    dGs[at] = ToHistory(dx + (f - a.fPrev[at]), dGs);
+    dGs[at] = ToHistory(dx + (f - fp), dGs);
     a.xPrev[at] = xs;
     a.fPrev[at] = f;
     // the new column as stored, so that the Gram matrix is the stored vectors'
     const A df = static_cast<A>(FromHistory(dfStored));
 #pragma unroll
     for (int i = 0; i < M; ++i) {
-      if (i >= m) break;
-      const A di = i == slot ? df : static_cast<A>(FromHistory(dF[i][at]));
-      col[i] += di * df;
-      gam[i] += di * static_cast<A>(f);
+      if (i < m) {
+        const A di = i == slot ? df : static_cast<A>(FromHistory(history[i]));
+        col[i] += di * df;
+        gam[i] += di * static_cast<A>(f);
+      }
     }
   }
   MixerBlockPartials<M>(col, gam, a.partial);
 }
 
 // Two values a thread (FP32 iterate, BF16 history): the same sweep as
-// MixerSweepKernel<float, M> with 8-byte and 4-byte accesses.
+// MixerSweepKernel<float, M> with 8-byte and 4-byte accesses. DRAM bounds it,
+// once enough is in flight: the loads of kMixAhead of a thread's turns are
+// issued together, the histories' predicated on the live count rather than
+// behind its branches (a wait each); sums in the turns' order. At lmax 256
+// (18 million values, 8 columns) a sweep and a mix together went from 360 to
+// 160 us.
+constexpr int kMixAhead = 2;
 template <int M>
 __global__ void MixerSweepPairsKernel(MixerArgsT<float> a) {
   int m = M, slot = a.slot;
@@ -825,22 +837,41 @@ __global__ void MixerSweepPairsKernel(MixerArgsT<float> a) {
   const __nv_bfloat162* dF[M + 1];
 #pragma unroll
   for (int i = 0; i < M; ++i) dF[i] = reinterpret_cast<const __nv_bfloat162*>(a.dF[i]);
-  for (long long at = begin + threadIdx.x; at < end; at += blockDim.x) {
-    const float2 xs = x[at], gs = gx[at], xp = xPrev[at], fp = fPrev[at];
-    const float2 f = make_float2(gs.x - xs.x, gs.y - xs.y);
-    const float2 dfRaw = make_float2(f.x - fp.x, f.y - fp.y);
-    const __nv_bfloat162 dfStored = __floats2bfloat162_rn(dfRaw.x, dfRaw.y);
-    dFs[at] = dfStored;
-    dGs[at] = __floats2bfloat162_rn(xs.x - xp.x + dfRaw.x, xs.y - xp.y + dfRaw.y);
-    xPrev[at] = xs;
-    fPrev[at] = f;
-    const float2 df = __bfloat1622float2(dfStored);
+  for (long long first = begin + threadIdx.x; first < end; first += kMixAhead * kMixThreads) {
+    float2 xs[kMixAhead], gs[kMixAhead], xp[kMixAhead], fp[kMixAhead];
+    __nv_bfloat162 history[kMixAhead][M + 1];
 #pragma unroll
-    for (int i = 0; i < M; ++i) {
-      if (i >= m) break;
-      const float2 di = i == slot ? df : __bfloat1622float2(dF[i][at]);
-      col[i] += di.x * df.x + di.y * df.y;
-      gam[i] += di.x * f.x + di.y * f.y;
+    for (int u = 0; u < kMixAhead; ++u) {
+      const long long at = first + u * kMixThreads;
+      if (at >= end) continue;
+      xs[u] = x[at];
+      gs[u] = gx[at];
+      xp[u] = xPrev[at];
+      fp[u] = fPrev[at];
+#pragma unroll
+      for (int i = 0; i < M; ++i)
+        if (i < m && i != slot) history[u][i] = dF[i][at];
+    }
+#pragma unroll
+    for (int u = 0; u < kMixAhead; ++u) {
+      const long long at = first + u * kMixThreads;
+      if (at >= end) continue;
+      const float2 f = make_float2(gs[u].x - xs[u].x, gs[u].y - xs[u].y);
+      const float2 dfRaw = make_float2(f.x - fp[u].x, f.y - fp[u].y);
+      const __nv_bfloat162 dfStored = __floats2bfloat162_rn(dfRaw.x, dfRaw.y);
+      dFs[at] = dfStored;
+      dGs[at] = __floats2bfloat162_rn(xs[u].x - xp[u].x + dfRaw.x, xs[u].y - xp[u].y + dfRaw.y);
+      xPrev[at] = xs[u];
+      fPrev[at] = f;
+      const float2 df = __bfloat1622float2(dfStored);
+#pragma unroll
+      for (int i = 0; i < M; ++i) {
+        if (i < m) {
+          const float2 di = i == slot ? df : __bfloat1622float2(history[u][i]);
+          col[i] += di.x * df.x + di.y * df.y;
+          gam[i] += di.x * f.x + di.y * f.y;
+        }
+      }
     }
   }
   MixerBlockPartials<M>(col, gam, a.partial);
@@ -882,12 +913,13 @@ __global__ void MixerMixKernel(MixerArgsT<T> a) {
   }
   for (long long at = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; at < a.n; at += stride) {
     A value = a.gx[at];
-    if (ok)
+    typename MixerArgsT<T>::H history[M + 1];
 #pragma unroll
-      for (int i = 0; i < M; ++i) {
-        if (i >= m) break;
-        value -= g[i] * static_cast<A>(FromHistory(dG[i][at]));
-      }
+    for (int i = 0; i < M; ++i)
+      if (ok && i < m) history[i] = dG[i][at];
+#pragma unroll
+    for (int i = 0; i < M; ++i)
+      if (ok && i < m) value -= g[i] * static_cast<A>(FromHistory(history[i]));
     a.x[at] = static_cast<T>(value);
   }
 }
@@ -911,17 +943,34 @@ __global__ void MixerMixPairsKernel(MixerArgsT<float> a) {
   }
   auto* x = reinterpret_cast<float2*>(a.x);
   auto* gx = reinterpret_cast<const float2*>(a.gx);
-  for (long long at = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; at < pairs; at += stride) {
-    float2 v = gx[at];
-    if (ok)
+  for (long long first = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; first < pairs;
+       first += kMixAhead * stride) {
+    // as in the sweep: the loads of a thread's next turns together
+    float2 v[kMixAhead];
+    __nv_bfloat162 history[kMixAhead][M + 1];
+#pragma unroll
+    for (int u = 0; u < kMixAhead; ++u) {
+      const long long at = first + u * stride;
+      if (at >= pairs) continue;
+      v[u] = gx[at];
+#pragma unroll
+      for (int i = 0; i < M; ++i)
+        if (ok && i < m) history[u][i] = dG[i][at];
+    }
+#pragma unroll
+    for (int u = 0; u < kMixAhead; ++u) {
+      const long long at = first + u * stride;
+      if (at >= pairs) continue;
 #pragma unroll
       for (int i = 0; i < M; ++i) {
-        if (i >= m) break;
-        const float2 d = __bfloat1622float2(dG[i][at]);
-        v.x -= g[i] * d.x;
-        v.y -= g[i] * d.y;
+        if (ok && i < m) {
+          const float2 d = __bfloat1622float2(history[u][i]);
+          v[u].x -= g[i] * d.x;
+          v[u].y -= g[i] * d.y;
+        }
       }
-    x[at] = v;
+      x[at] = v[u];
+    }
   }
 }
 
