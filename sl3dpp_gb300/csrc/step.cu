@@ -108,6 +108,8 @@ class Viscoelastic3DGpu {
   Geometry geo{};
   Dev<int> dNodeElement, dNodeQ, dElemFirstNode, dSphMap, dTorMap;
   Dev<double> dNodeR, dElemJac, dValue, dDeriv, dWeight;
+  Dev<double> dRadii64;  // Geometry::radii64/radii32
+  Dev<float> dRadii32;
   Dev<double> dCoef64;  // the node coefficient tables (Geometry::coef64/coef32)
   Dev<float> dCoef32;
   Dev<DegreeInfo> dDegrees;
@@ -678,6 +680,8 @@ int Viscoelastic3DGpu::Create(const sl3dgpu_layer* layers, int nlayers, const sl
   SL3D_CUDA(dNodeElement.Upload(nodeElement));
   SL3D_CUDA(dNodeQ.Upload(nodeQ));
   SL3D_CUDA(dNodeR.Upload(nodeR));
+  SL3D_CUDA(dRadii64.Upload(NodeRadii<double>(nodeR)));
+  SL3D_CUDA(dRadii32.Upload(NodeRadii<float>(nodeR)));
   SL3D_CUDA(dElemFirstNode.Upload(elemFirstNode));
   SL3D_CUDA(dElemJac.Upload(elemJac));
   SL3D_CUDA(dValue.Upload(pts.value));
@@ -704,6 +708,8 @@ int Viscoelastic3DGpu::Create(const sl3dgpu_layer* layers, int nlayers, const sl
       geo.coef64[w] = dCoef64.p + w * plane;
       geo.coef32[w] = dCoef32.p + w * plane;
     }
+    geo.radii64 = dRadii64.p;
+    geo.radii32 = dRadii32.p;
   }
 
   {
@@ -1881,6 +1887,8 @@ int Viscoelastic3DGpu::PrepareLateral() {
   geoL.nodeElement = dNodeElement.p + p0;
   geoL.nodeQ = dNodeQ.p + p0;
   geoL.nodeR = dNodeR.p + p0;
+  geoL.radii64 = dRadii64.p + static_cast<long long>(kRadii) * p0;
+  geoL.radii32 = dRadii32.p + static_cast<long long>(kRadii) * p0;
   for (int w = 0; w < 4; ++w) {
     geoL.coef64[w] = geo.coef64[w] + static_cast<long long>(p0) * geo.ngll;
     geoL.coef32[w] = geo.coef32[w] + static_cast<long long>(p0) * geo.ngll;

@@ -84,6 +84,36 @@ __device__ inline const float* Coef<float>(const Geometry& g, int which) {
   return g.coef32[which];
 }
 
+template <class T>
+__device__ inline const T* Radii(const Geometry& g);
+template <>
+__device__ inline const double* Radii<double>(const Geometry& g) {
+  return g.radii64;
+}
+template <>
+__device__ inline const float* Radii<float>(const Geometry& g) {
+  return g.radii32;
+}
+
+// x / d rounded to nearest from d's rounded reciprocal y: a quotient and its
+// exact remainder, whose share corrects it (Markstein's division). A division
+// proper costs about ten instructions, six a point in the strain; FP64 ones
+// are 19 cycles an SM each. In FP64 one correction leaves the rounding wrong
+// for one value in 2^52; in FP32, where that would be one in 2^23, a second
+// leaves none. Zeros, subnormals and non-finite values as x y.
+__device__ inline double DivideBy(double x, double d, double y) {
+  const double q = x * y;
+  const uint32_t e = (static_cast<uint32_t>(__double2hiint(q)) >> 20) & 0x7FFu;
+  return e - 1u >= 0x7FEu ? q : fma(fma(-q, d, x), y, q);
+}
+__device__ inline float DivideBy(float x, float d, float y) {
+  float q = x * y;
+  const uint32_t e = (__float_as_uint(q) >> 23) & 0xFFu;
+  if (e - 1u >= 0xFEu) return q;
+  q = fmaf(fmaf(-q, d, x), y, q);
+  return fmaf(fmaf(-q, d, x), y, q);
+}
+
 template <class T2>
 struct Rows {
   T2 u, v, w, du, dv, dw;
@@ -169,7 +199,7 @@ __global__ void ForceChunkKernel(Geometry g, const T2* spectral, T2* rhsSph, T2*
       A[0] = c0[Row0(g, l, m) * g.P + p];
       A[4] = CScale(sign, CConj(c0[Row0(g, l, -m) * g.P + p]));
     }
-    const Rows<T2> rows = ForceRows<T2>(l, A, static_cast<T>(g.nodeR[p]));
+    const Rows<T2> rows = ForceRows<T2>(l, A, Radii<T>(g)[kRadii * p]);
     T2* s = rowsS + static_cast<long long>(mi) * pPad + (p - d.firstNode);
     const long long k = static_cast<long long>(MC) * pPad;
     s[0] = rows.u;
@@ -219,10 +249,26 @@ __global__ void ForceChunkKernel(Geometry g, const T2* spectral, T2* rhsSph, T2*
   }
 }
 
+// The rows of a chunk's orders in the spin components, [spin row][order]:
+// spin -2 at m and -m, spin -1 at m and -m, the real spin 0 (-1 where the
+// component has none).
+template <int MC>
+__device__ inline void ChunkRows(const Geometry& g, int l, int m0, int mc, int (&rows)[5][MC]) {
+  for (int t = threadIdx.x; t < 5 * MC; t += blockDim.x) {
+    const int which = t / MC, mi = t % MC, m = which % 2 ? -(m0 + mi) : m0 + mi;
+    long long row = -1;
+    if (mi < mc) row = which == 4 ? RowR(g, l, m0 + mi) : which >= 2 ? (l >= 1 ? Row1(g, l, m) : -1) : (l >= 2 ? Row0(g, l, m) : -1);
+    rows[which][mi] = static_cast<int>(row);
+  }
+}
+
 // StrainOf (AddStrainOfSolution + DeviatoricComponents, SpinComponents.hpp:
 // 53-72, + Scatter with the -m twins from the derived components): the
 // degree's U, V, W at the carrying elements' GLL nodes, then per memory node
 // the five deviatoric components; `add` (the same layout), when given, added.
+// In FP64 the arithmetic bounds it (some 120 instructions a point), in FP32
+// the loads' latency. At lmax 128, 175 nodes: 338 -> 234 us in FP64 with the
+// divisions by reciprocals and `add` loaded first, about 50 -> 32 in FP32.
 template <class T2, int MC>
 __global__ void StrainChunkKernel(Geometry g, const T2* solSph, const T2* solTor, T2* spectral, const T2* add) {
   using T = typename Scalar<T2>::type;
@@ -240,8 +286,10 @@ __global__ void StrainChunkKernel(Geometry g, const T2* solSph, const T2* solTor
   const bool any = d.firstNode < g.P;
   if (any) {
     const int globals = d.lastGlobal - d.firstGlobal + 1;
-    for (int t = threadIdx.x; t < globals * mc; t += blockDim.x) {
-      const int mi = t % mc, gn = d.firstGlobal + t / mc, m = m0 + mi;
+#pragma unroll 4
+    for (int t = threadIdx.x; t < globals * MC; t += blockDim.x) {
+      const int mi = t % MC, gn = d.firstGlobal + t / MC, m = m0 + mi;
+      if (mi >= mc) continue;
       const int dU = g.sphMap[d.sphMap + 2LL * gn], dV = g.sphMap[d.sphMap + 2LL * gn + 1];
       T2* v = vals + static_cast<long long>(gn - d.firstGlobal) * kRow + mi;
       v[0] = dU >= 0 ? solSph[d.sphRhs + static_cast<long long>(dU) * cols + m] : Cx<T2>(0, 0);
@@ -254,21 +302,32 @@ __global__ void StrainChunkKernel(Geometry g, const T2* solSph, const T2* solTor
       v[2 * MC] = W;
     }
   }
+  __shared__ int rowAt[5][MC];
+  ChunkRows<MC>(g, l, m0, mc, rowAt);
   __syncthreads();
   const int n = g.ngll;
   const T zeta2 = l * (l + T(1)), zeta = sqrt(zeta2);
   const T s2 = T(1.41421356237309504880);
-  auto put = [&](T2* base, long long at, T2 v) {
-    const long long i = (base - spectral) + at;
-    spectral[i] = add != nullptr ? CAdd(v, add[i]) : v;
-  };
+  const T top = T(0.5) * zeta * sqrt(zeta2 - T(2));  // not used below degree 2
   for (int t = threadIdx.x; t < mc * g.P; t += blockDim.x) {
     const int mi = t / g.P, p = t % g.P, m = m0 + mi;
     const T sign = (m % 2 == 0) ? T(1) : T(-1);
+    // spin -2 at m and -m, spin -1 at m and -m, spin 0; what is added to them
+    // asked for before anything else, so that its latency runs under the sums
+    const bool live[5] = {l >= 2, l >= 2 && m > 0, l >= 1, l >= 1 && m > 0, true};
+    T2* const base[5] = {c0, c0, c1, c1, cr};
+    long long at[5];
+    T2 before[5];
+#pragma unroll
+    for (int c = 0; c < 5; ++c) {
+      at[c] = (base[c] - spectral) + static_cast<long long>(rowAt[c][mi]) * g.P + p;
+      if (add != nullptr && live[c]) before[c] = add[at[c]];
+    }
     T2 A[5] = {Cx<T2>(0, 0), Cx<T2>(0, 0), Cx<T2>(0, 0), Cx<T2>(0, 0), Cx<T2>(0, 0)};
     if (any && p >= d.firstNode) {
       const int e = g.nodeElement[p];
-      const T r = static_cast<T>(g.nodeR[p]);
+      const T* radii = Radii<T>(g) + static_cast<long long>(kRadii) * p;
+      const T r = radii[0], by3r = radii[1], byDen = radii[2], byR = radii[3];
       const T* sValue = Coef<T>(g, kStrainValue) + p * n;
       const T* sDeriv = Coef<T>(g, kStrainDeriv) + p * n;
       T2 U = Cx<T2>(0, 0), V = Cx<T2>(0, 0), W = Cx<T2>(0, 0), rdU = Cx<T2>(0, 0), rdV = Cx<T2>(0, 0),
@@ -285,31 +344,25 @@ __global__ void StrainChunkKernel(Geometry g, const T2* solSph, const T2* solTor
         rdW = CAdd(rdW, CScale(b, v[2 * MC]));
       }
       const T2 t2 = CAdd(CSub(rdU, U), CScale(T(0.5) * zeta2, V));
-      A[2] = Cx<T2>(t2.x / (T(3) * r), t2.y / (T(3) * r));
+      A[4] = Cx<T2>(DivideBy(t2.x, T(3) * r, by3r), DivideBy(t2.y, T(3) * r, by3r));
       if (l >= 1) {
         const T2 tangential = CAdd(CSub(rdV, V), U);
         const T2 twist = CSub(W, rdW);
         const T den = T(2) * s2 * r;
         const T2 a1 = CScale(zeta, CAdd(tangential, CI(twist)));
         const T2 a3 = CScale(zeta, CSub(tangential, CI(twist)));
-        A[1] = Cx<T2>(a1.x / den, a1.y / den);
-        A[3] = Cx<T2>(a3.x / den, a3.y / den);
+        A[2] = Cx<T2>(DivideBy(a1.x, den, byDen), DivideBy(a1.y, den, byDen));
+        A[3] = CScale(sign, CConj(Cx<T2>(DivideBy(a3.x, den, byDen), DivideBy(a3.y, den, byDen))));
       }
       if (l >= 2) {
-        const T factor = T(0.5) * zeta * sqrt(zeta2 - T(2)) / r;
+        const T factor = DivideBy(top, r, byR);
         A[0] = CScale(factor, CSub(V, CI(W)));
-        A[4] = CScale(factor, CAdd(V, CI(W)));
+        A[1] = CScale(sign, CConj(CScale(factor, CAdd(V, CI(W)))));
       }
     }
-    if (l >= 2) {
-      put(c0, Row0(g, l, m) * g.P + p, A[0]);
-      if (m > 0) put(c0, Row0(g, l, -m) * g.P + p, CScale(sign, CConj(A[4])));
-    }
-    if (l >= 1) {
-      put(c1, Row1(g, l, m) * g.P + p, A[1]);
-      if (m > 0) put(c1, Row1(g, l, -m) * g.P + p, CScale(sign, CConj(A[3])));
-    }
-    put(cr, RowR(g, l, m) * g.P + p, A[2]);
+#pragma unroll
+    for (int c = 0; c < 5; ++c)
+      if (live[c]) spectral[at[c]] = add != nullptr ? CAdd(A[c], before[c]) : A[c];
   }
 }
 
@@ -1173,6 +1226,10 @@ namespace {
 // Orders a block of the chunked maps takes: the most (up to 32) whose
 // shared-memory rows fit a budget that leaves room for two blocks an SM.
 constexpr size_t kChunkSmemBudget = 110 * 1024;
+// The FP32 force, bound by its loads' latency, runs with more blocks an SM (at
+// lmax 256, 55 nodes: 108 -> 85 us with 16 orders a block, 42 KB, for 32); the
+// FP64 force, bound by its arithmetic, loses with fewer orders a block.
+constexpr size_t kForce32SmemBudget = 61 * 1024;
 inline int ChunkBlocks(int lmax, int mc) {  // sum over l <= lmax of (floor(l / mc) + 1)
   long long blocks = 0;
   for (int l = 0; l <= lmax; ++l) blocks += l / mc + 1;
@@ -1183,9 +1240,10 @@ inline int ChunkBlocks(int lmax, int mc) {  // sum over l <= lmax of (floor(l / 
 // idle (blocks for two an SM, while a block keeps some 128 nodes' work): at
 // lmax 32 the strain's 34 blocks of 32 orders took 112 us on the FP64 unit.
 constexpr int kChunkBlocks = 2 * 152;
-inline int ChunkOrders(size_t bytesPerOrder, size_t fixedBytes, int lmax, int nodes) {
+inline int ChunkOrders(size_t bytesPerOrder, size_t fixedBytes, int lmax, int nodes,
+                       size_t budget = kChunkSmemBudget) {
   int mc = 32;
-  while (mc > 1 && fixedBytes + bytesPerOrder * mc > kChunkSmemBudget) mc /= 2;
+  while (mc > 1 && fixedBytes + bytesPerOrder * mc > budget) mc /= 2;
   while (mc > 1 && ChunkBlocks(lmax, mc) < kChunkBlocks && mc / 2 * nodes >= 128) mc /= 2;
   return mc;
 }
@@ -1208,7 +1266,8 @@ void StrainWith(const Geometry& g, const T2* solSph, const T2* solTor, T2* spect
 template <class T2>
 void Forces(const Geometry& g, const T2* spectral, T2* rhsSph, T2* rhsTor, cudaStream_t stream) {
   prof::Scope scope(prof::kForce, stream);
-  switch (ChunkOrders(static_cast<size_t>(6) * (g.P | 1) * sizeof(T2), 0, g.lmax, g.P)) {
+  switch (ChunkOrders(static_cast<size_t>(6) * (g.P | 1) * sizeof(T2), 0, g.lmax, g.P,
+                      sizeof(T2) == sizeof(float2) ? kForce32SmemBudget : kChunkSmemBudget)) {
     case 32: return ForcesWith<T2, 32>(g, spectral, rhsSph, rhsTor, stream);
     case 16: return ForcesWith<T2, 16>(g, spectral, rhsSph, rhsTor, stream);
     case 8: return ForcesWith<T2, 8>(g, spectral, rhsSph, rhsTor, stream);

@@ -52,9 +52,25 @@ struct Geometry {
   // [kForceValue] jac w_q r_p Value(q_p, i); [kForceDeriv] w_q Deriv(q_p, i) r_p.
   const double* coef64[4];
   const float* coef32[4];
+  // Per memory node kRadii values: r, then the reciprocals (rounded to
+  // nearest) of 3 r, 2 sqrt(2) r and r, the strain's divisors, as the kernels
+  // compute these in either precision.
+  const double* radii64;
+  const float* radii32;
   int maxGlobals;  // the most global nodes a degree's carrying elements span (shared-memory sizing)
 };
 enum NodeCoefficient { kStrainValue = 0, kStrainDeriv = 1, kForceValue = 2, kForceDeriv = 3 };
+constexpr int kRadii = 4;
+template <class T>
+std::vector<T> NodeRadii(const std::vector<double>& nodeR) {
+  const T s2 = T(1.41421356237309504880);
+  std::vector<T> out;
+  for (double radius : nodeR) {
+    const T r = static_cast<T>(radius);
+    out.insert(out.end(), {r, T(1) / (T(3) * r), T(1) / (T(2) * s2 * r), T(1) / r});
+  }
+  return out;
+}
 // The node coefficient tables of a geometry, host FP64 (4 x P x ngll).
 std::vector<double> NodeCoefficients(int P, int ngll, const std::vector<int>& nodeElement,
                                      const std::vector<int>& nodeQ, const std::vector<double>& nodeR,
