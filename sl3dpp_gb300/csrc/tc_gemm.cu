@@ -144,9 +144,7 @@ __device__ __forceinline__ void CopyTile(uint32_t to, const float* from, uint32_
 // stage's tile: a lane's columns are lane + 32 j (j < J, tileN <= 32 J), so
 // that an item's place needs no division (the index arithmetic was three
 // quarters of the packing warps' instructions). The first chunk's values are
-// loaded before `wait`. False when `wait` gave up. The MMA issue sets the
-// kernel's pace: its lane waits 30 of 100 cycles for a stage, and a 16-deep
-// step's four TF32 MMAs take about 1070 cycles.
+// loaded before `wait`. False when `wait` gave up.
 template <int J, class Wait>
 __device__ __forceinline__ bool PackStep(const float* from, int ldb, int columns, int depth, int tileN, float* out,
                                          int lane, Wait wait) {
@@ -186,6 +184,49 @@ __device__ __forceinline__ bool PackStep(const float* from, int ldb, int columns
   }
   return true;
 }
+
+// The place of a CTA's step in the ring of stages, advanced a step at a time
+// (a remainder by the stage count, 64-bit and a run-time value, took longer
+// than the step's MMAs).
+struct RingPlace {
+  int slot = 0;
+  uint32_t round = 0;
+  __device__ __forceinline__ void Next(int stages) {
+    if (++slot == stages) {
+      slot = 0;
+      ++round;
+    }
+  }
+};
+
+// A CTA's tiles t = blockIdx.x, + gridDim.x, ...: the next tile's item and the
+// one after's description are asked for a tile ahead, so that no role waits
+// for the two dependent reads between tiles.
+struct TileWalk {
+  const int4* tiles;
+  const TcItem* items;
+  int t, count;
+  int4 tile, ahead;
+  TcItem it, itAhead;
+  __device__ __forceinline__ TileWalk(const int4* tiles_, const TcItem* items_, int count_)
+      : tiles(tiles_), items(items_), t(blockIdx.x), count(count_) {
+    if (t >= count) return;
+    tile = tiles[t];
+    it = items[tile.x];
+    ahead = tiles[min(t + static_cast<int>(gridDim.x), count - 1)];
+  }
+  __device__ __forceinline__ bool Live() const { return t < count; }
+  // before a tile's steps
+  __device__ __forceinline__ void Fetch() {
+    itAhead = items[ahead.x];
+  }
+  __device__ __forceinline__ void Next() {
+    t += gridDim.x;
+    tile = ahead;
+    it = itAhead;
+    ahead = tiles[min(t + static_cast<int>(gridDim.x), count - 1)];
+  }
+};
 
 __global__ void __launch_bounds__(kPersistentThreads, 1)
     TcGemmKernel(const TcItem* tcItems, const int4* tiles, int tileCount, int tileN, int stages,
@@ -243,9 +284,11 @@ __global__ void __launch_bounds__(kPersistentThreads, 1)
   if (warp == 0 && lane == 0) {
     // -- producer --------------------------------------------------------------
     long long g = 0;
-    for (int t = blockIdx.x; t < tileCount && !abortFlag; t += gridDim.x) {
-      const int4 tile = tiles[t];
-      const TcItem it = tcItems[tile.x];
+    RingPlace at;
+    for (TileWalk walk(tiles, tcItems, tileCount); walk.Live() && !abortFlag; walk.Next()) {
+      walk.Fetch();
+      const int4 tile = walk.tile;
+      const TcItem it = walk.it;
       const float* aSrc = panels + it.aPanel + static_cast<long long>(tile.y) * it.kSteps * 2 * kATileFloats;
       const float* bSrc = packed + it.bPack + static_cast<long long>(tile.z) * it.kSteps * 2 * bTileFloats;
       // A tile's rows past the item's are not copied (their products are not
@@ -253,10 +296,9 @@ __global__ void __launch_bounds__(kPersistentThreads, 1)
       // colatitudes fill one row of their fourth tile
       const int rowGroups = min(kTcTileM, it.M - tile.y * kTcTileM + 7) / 8;
       const uint32_t aTile = 2 * kTcTileK / 4 * 128u * rowGroups;
-      for (int ks = 0; ks < it.kSteps; ++ks, ++g) {
-        const int slot = static_cast<int>(g % stages);
-        const long long round = g / stages;
-        if (round > 0 && !WaitParity(SmemAddr(empty + slot), static_cast<uint32_t>((round - 1) & 1))) {
+      for (int ks = 0; ks < it.kSteps; ++ks, ++g, at.Next(stages)) {
+        const int slot = at.slot;
+        if (at.round > 0 && !WaitParity(SmemAddr(empty + slot), (at.round - 1) & 1)) {
           giveUp();
           break;
         }
@@ -288,12 +330,13 @@ __global__ void __launch_bounds__(kPersistentThreads, 1)
       WaitParity(SmemAddr(full + static_cast<int>(q % stages)), static_cast<uint32_t>((q / stages) & 1));
   } else if (warp == 1 && lane == 0) {
     // -- MMA issue ---------------------------------------------------------------
-    long long g = 0;
+    RingPlace at;
     int local = 0;
     bool issued = false;
-    for (int t = blockIdx.x; t < tileCount && !abortFlag; t += gridDim.x, ++local) {
-      const int4 tile = tiles[t];
-      const TcItem it = tcItems[tile.x];
+    for (TileWalk walk(tiles, tcItems, tileCount); walk.Live() && !abortFlag; walk.Next(), ++local) {
+      walk.Fetch();
+      const int4 tile = walk.tile;
+      const TcItem it = walk.it;
       const int nCols = min(tileN, it.N - tile.z * tileN);
       const uint32_t idesc = InstrDescriptor((nCols + 15) / 16 * 16, kTcTileM);
       const uint32_t idescPair = InstrDescriptor(2 * tileN, kTcTileM);
@@ -306,9 +349,9 @@ __global__ void __launch_bounds__(kPersistentThreads, 1)
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t d = tmem + acc * accColumns;
       bool ok = true;
-      for (int ks = 0; ks < it.kSteps; ++ks, ++g) {
-        const int slot = static_cast<int>(g % stages);
-        if (!WaitParity(SmemAddr(full + slot), static_cast<uint32_t>((g / stages) & 1)) || abortFlag) {
+      for (int ks = 0; ks < it.kSteps; ++ks, at.Next(stages)) {
+        const int slot = at.slot;
+        if (!WaitParity(SmemAddr(full + slot), at.round & 1) || abortFlag) {
           ok = false;
           break;
         }
@@ -378,23 +421,25 @@ __global__ void __launch_bounds__(kPersistentThreads, 1)
     // stores any (its loads overlap)
     if (rawB != nullptr) {
       const int packer = warp - 6;
-      long long g = 0;
+      int turn = 0;  // the step's place among the packing warps
+      RingPlace at;
       bool ok = true;
-      for (int t = blockIdx.x; t < tileCount && !abortFlag && ok; t += gridDim.x) {
-        const int4 tile = tiles[t];
-        const TcItem it = tcItems[tile.x];
+      for (TileWalk walk(tiles, tcItems, tileCount); walk.Live() && !abortFlag && ok; walk.Next()) {
+        walk.Fetch();
+        const int4 tile = walk.tile;
+        const TcItem it = walk.it;
         const int nBase = tile.z * tileN;
-        for (int ks = 0; ks < it.kSteps; ++ks, ++g) {
-          if (static_cast<int>(g % kPackWarps) != packer) continue;
-          const int slot = static_cast<int>(g % stages);
-          const long long round = g / stages;
+        for (int ks = 0; ks < it.kSteps; ++ks, at.Next(stages), turn = (turn + 1) % kPackWarps) {
+          if (turn != packer) continue;
+          const int slot = at.slot;
+          const uint32_t round = at.round;
           float* out = sB + slot * 2 * bTileFloats;
           const float* from = rawB + it.b + static_cast<long long>(ks) * kTcTileK * it.ldb + nBase;
           const int columns = min(tileN, it.N - nBase), depth = min(kTcTileK, it.K - ks * kTcTileK);
           // B's values are read before the slot is waited for (they go to
           // registers): their global latency overlaps the wait
           auto wait = [&] {
-            if (round > 0 && !WaitParity(SmemAddr(empty + slot), static_cast<uint32_t>((round - 1) & 1))) ok = false;
+            if (round > 0 && !WaitParity(SmemAddr(empty + slot), (round - 1) & 1)) ok = false;
             return ok && !abortFlag;
           };
           if (tileN <= 128)
