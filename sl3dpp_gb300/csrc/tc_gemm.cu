@@ -2,7 +2,7 @@
 //
 // A persistent, warp-specialised kernel (TcGemmKernel, below): a TMA
 // producer lane fills a ring of shared-memory stages (the A tile's high and
-// low TF32 parts, 16 KB; B's, 2 x tileN x 64 B, split and packed there by two
+// low TF32 parts, 16 KB; B's, 2 x tileN x 64 B, split and packed there by six
 // warps from B's source), an MMA lane issues each
 // 16-deep step's tcgen05.mma kind::tf32 into one of two TMEM accumulators,
 // and four epilogue warps drain the other. B's high and low parts form one
@@ -129,7 +129,10 @@ __global__ void PackBKernel(const TcItem* tcItems, int tileN, const float* B, fl
 // cores' (async) proxy and arrive on the stage's "full" barrier beside the
 // producer's A copy -- the packing pass and its round trip through HBM are
 // gone, and B is read at 4 bytes a value.
-constexpr int kPackWarps = 4;  // warps 6 .. 9, a step each in turn
+// Warps 6 .. 11, a step each in turn; never more than the ring's stages, so that
+// no warp waits for a stage that an earlier step has yet to fill (a wait tells
+// only odd rounds from even ones).
+constexpr int kPackWarps = 6;
 constexpr int kPersistentThreads = 32 * (6 + kPackWarps);
 constexpr int kPackChunk = 16;  // (column, 4-deep group) items a lane loads before it stores (64 reads in flight)
 
@@ -416,11 +419,11 @@ __global__ void __launch_bounds__(kPersistentThreads, 1)
     }
   } else if (warp >= 6) {
     // -- B's split and pack, in shared memory: packing warp p takes the
-    // steps g = p, p + kPackWarps, ..., so that kPackWarps steps' reads are in
+    // steps g = p, p + packers, ..., so that that many steps' reads are in
     // flight; a lane loads all its items' values before it converts and
     // stores any (its loads overlap)
-    if (rawB != nullptr) {
-      const int packer = warp - 6;
+    const int packer = warp - 6, packers = min(kPackWarps, stages);
+    if (rawB != nullptr && packer < packers) {
       int turn = 0;  // the step's place among the packing warps
       RingPlace at;
       bool ok = true;
@@ -429,7 +432,7 @@ __global__ void __launch_bounds__(kPersistentThreads, 1)
         const int4 tile = walk.tile;
         const TcItem it = walk.it;
         const int nBase = tile.z * tileN;
-        for (int ks = 0; ks < it.kSteps; ++ks, at.Next(stages), turn = (turn + 1) % kPackWarps) {
+        for (int ks = 0; ks < it.kSteps; ++ks, at.Next(stages), turn = turn + 1 < packers ? turn + 1 : 0) {
           if (turn != packer) continue;
           const int slot = at.slot;
           const uint32_t round = at.round;
