@@ -170,13 +170,31 @@ __global__ void __launch_bounds__(256) GemmKernel(const GemmItem* items, const T
 // spend 64 columns of FP64 FMAs on them, and FP64 is GB300's slow pipe. These
 // kernels do only the N columns and stream the table once.
 
+//
+// With a RefLayout the coefficients are read and written in the reference
+// layout, so that a call of a few fields has no permutation launch of its own:
+// at lmax 32, one field, a synthesis and an analysis are four launches, not
+// six.
+
 constexpr int kNarrowN = 16;
+
+struct RefLayout {
+  bool real;
+  int N, mlo;      // the order of item 0 (the items are the orders in turn, none without degrees)
+  long long rows;  // complex coefficients a field
+  // The place of order m's row-th degree among a field's coefficients.
+  __device__ __forceinline__ long long At(int item, int row) const {
+    const int m = mlo + item, l = max(abs(m), abs(N)) + row;
+    return real ? static_cast<long long>(l) * (l + 1) / 2 + m : static_cast<long long>(l) * l - N * N + l + m;
+  }
+};
 
 // Analysis (A row-major in k, sAk = 1): one warp per output row, the lanes
 // over k (coalesced reads of the row), a shuffle sum at the end.
-template <int NT>
+template <int NT, bool kRef>
 __global__ void __launch_bounds__(256) GemmRowsNarrowKernel(const GemmItem* items, const double* A,
-                                                            const double* B, double* C, bool accumulate) {
+                                                            const double* B, double* C, bool accumulate,
+                                                            RefLayout ref) {
   const GemmItem it = items[blockIdx.y];
   const int lane = threadIdx.x & 31;
   const int i = blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -196,6 +214,13 @@ __global__ void __launch_bounds__(256) GemmRowsNarrowKernel(const GemmItem* item
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) acc[n] += __shfl_xor_sync(0xffffffffu, acc[n], off);
   if (lane != 0) return;
+  if constexpr (kRef) {
+    double* c = C + 2 * ref.At(blockIdx.y, i);
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+      if (n < it.N) c[2 * (n / 2) * ref.rows + n % 2] = acc[n];
+    return;
+  }
   double* c = C + it.c + static_cast<long long>(i) * it.ldc;
 #pragma unroll
   for (int n = 0; n < NT; ++n)
@@ -205,9 +230,10 @@ __global__ void __launch_bounds__(256) GemmRowsNarrowKernel(const GemmItem* item
 // Synthesis (A column-major in i, sAi = 1): 32 output rows a block, one a
 // lane (coalesced reads down the table's columns), k split over the eight
 // warps and the partial sums added in shared memory.
-template <int NT>
+template <int NT, bool kRef>
 __global__ void __launch_bounds__(256) GemmColsNarrowKernel(const GemmItem* items, const double* A,
-                                                            const double* B, double* C, bool accumulate) {
+                                                            const double* B, double* C, bool accumulate,
+                                                            RefLayout ref) {
   __shared__ double part[8][NT][32];
   const GemmItem it = items[blockIdx.y];
   const int lane = threadIdx.x & 31, group = threadIdx.x >> 5;
@@ -220,10 +246,10 @@ __global__ void __launch_bounds__(256) GemmColsNarrowKernel(const GemmItem* item
 #pragma unroll 4
     for (int k = group; k < it.K; k += 8) {
       const double av = a[static_cast<long long>(k) * it.sAk];
-      const double* bk = b + static_cast<long long>(k) * it.ldb;
+      const double* bk = kRef ? B + 2 * ref.At(blockIdx.y, k) : b + static_cast<long long>(k) * it.ldb;
 #pragma unroll
       for (int n = 0; n < NT; ++n)
-        if (n < it.N) acc[n] = fma(av, bk[n], acc[n]);
+        if (n < it.N) acc[n] = fma(av, bk[kRef ? 2 * (n / 2) * ref.rows + n % 2 : n], acc[n]);
     }
   }
 #pragma unroll
@@ -241,13 +267,27 @@ __global__ void __launch_bounds__(256) GemmColsNarrowKernel(const GemmItem* item
   }
 }
 
-template <int NT>
+template <int NT, bool kRef>
 void LaunchNarrow(bool analysis, int maxM, int count, const GemmItem* items, const double* A, const double* B,
-                  double* C, bool accumulate, cudaStream_t stream) {
+                  double* C, bool accumulate, const RefLayout& ref, cudaStream_t stream) {
   if (analysis)
-    GemmRowsNarrowKernel<NT><<<dim3((maxM + 7) / 8, count), 256, 0, stream>>>(items, A, B, C, accumulate);
+    GemmRowsNarrowKernel<NT, kRef><<<dim3((maxM + 7) / 8, count), 256, 0, stream>>>(items, A, B, C, accumulate, ref);
   else
-    GemmColsNarrowKernel<NT><<<dim3((maxM + 31) / 32, count), 256, 0, stream>>>(items, A, B, C, accumulate);
+    GemmColsNarrowKernel<NT, kRef><<<dim3((maxM + 31) / 32, count), 256, 0, stream>>>(items, A, B, C, accumulate,
+                                                                                     ref);
+}
+
+template <bool kRef>
+void Narrow(int columns, bool analysis, int maxM, int count, const GemmItem* items, const double* A, const double* B,
+            double* C, bool accumulate, const RefLayout& ref, cudaStream_t stream) {
+  if (columns <= 2)
+    LaunchNarrow<2, kRef>(analysis, maxM, count, items, A, B, C, accumulate, ref, stream);
+  else if (columns <= 4)
+    LaunchNarrow<4, kRef>(analysis, maxM, count, items, A, B, C, accumulate, ref, stream);
+  else if (columns <= 8)
+    LaunchNarrow<8, kRef>(analysis, maxM, count, items, A, B, C, accumulate, ref, stream);
+  else
+    LaunchNarrow<16, kRef>(analysis, maxM, count, items, A, B, C, accumulate, ref, stream);
 }
 
 // -- FFT ---------------------------------------------------------------------------------
@@ -972,14 +1012,7 @@ int Grid::RunGemm(const Batch& b, const double* A, const double* B, double* C, b
   // the batch's items all have the direction's layout: analysis sAk = 1,
   // synthesis sAi = 1 (BatchFor)
   if (b.maxN <= kNarrowN) {
-    if (b.maxN <= 2)
-      LaunchNarrow<2>(b.analysis, b.maxM, b.count, b.items, A, B, C, accumulate, stream);
-    else if (b.maxN <= 4)
-      LaunchNarrow<4>(b.analysis, b.maxM, b.count, b.items, A, B, C, accumulate, stream);
-    else if (b.maxN <= 8)
-      LaunchNarrow<8>(b.analysis, b.maxM, b.count, b.items, A, B, C, accumulate, stream);
-    else
-      LaunchNarrow<16>(b.analysis, b.maxM, b.count, b.items, A, B, C, accumulate, stream);
+    Narrow<false>(b.maxN, b.analysis, b.maxM, b.count, b.items, A, B, C, accumulate, {}, stream);
     SL3D_CHECK_LAUNCH();
     return SL3DGPU_OK;
   }
@@ -1067,6 +1100,23 @@ int Grid::RunGemm64(int N, bool real, Batch& b, const double* B, double* C, bool
   }
   SL3D_CUDA(cudaFreeAsync(scratch, stream));
   return status;
+}
+
+int Grid::LegendreInReferenceLayout(int N, bool real, bool analysis, const double* in, int count, double* out,
+                                    cudaStream_t stream, bool* done) {
+  *done = false;
+  if (count == 0 || 2 * count > kNarrowN) return SL3DGPU_OK;
+  const SpinTable* t = nullptr;
+  if (int st = Table(N, &t); st != SL3DGPU_OK) return st;
+  const Batch* b = nullptr;
+  if (int st = BatchFor(N, real, analysis, count, 0, count, &b); st != SL3DGPU_OK) return st;
+  if (UseSlices64(*b) || b->count != (real ? lmax + 1 : 2 * lmax + 1)) return SL3DGPU_OK;
+  RefLayout ref{real, N, real ? 0 : -lmax, real ? RealRows() : SpinRows(N)};
+  prof::Scope scope(analysis ? prof::kLegendreAnalysis : prof::kLegendreSynthesis, stream, b->flops);
+  Narrow<true>(b->maxN, analysis, b->maxM, b->count, b->items, t->values, in, out, false, ref, stream);
+  SL3D_CHECK_LAUNCH();
+  *done = true;
+  return SL3DGPU_OK;
 }
 
 int Grid::LegendreSynthesis(int N, bool real, const double* coeffs, int P, int p0, int count,
@@ -1546,8 +1596,13 @@ int Synthesise(sl3dgpu_grid* handle, int N, bool real, const double* coeffs, int
                          &spectra, &dev);
       st != SL3DGPU_OK)
     return st;
-  if (int st = g.ToDevice(N, real, coeffs, count, dev, s); st != SL3DGPU_OK) return st;
-  if (int st = g.LegendreSynthesis(N, real, dev, count, spectra, s); st != SL3DGPU_OK) return st;
+  bool done = false;
+  if (int st = g.LegendreInReferenceLayout(N, real, false, coeffs, count, spectra, s, &done); st != SL3DGPU_OK)
+    return st;
+  if (!done) {
+    if (int st = g.ToDevice(N, real, coeffs, count, dev, s); st != SL3DGPU_OK) return st;
+    if (int st = g.LegendreSynthesis(N, real, dev, count, spectra, s); st != SL3DGPU_OK) return st;
+  }
   return g.RingSynthesis(real, spectra, count, fields, s, fixedPoint);
 }
 
@@ -1567,6 +1622,9 @@ int Expand(sl3dgpu_grid* handle, int N, bool real, const double* fields, int cou
       st != SL3DGPU_OK)
     return st;
   if (int st = g.RingAnalysis(real, fields, count, spectra, s, nullptr, fixedPoint); st != SL3DGPU_OK) return st;
+  bool done = false;
+  if (int st = g.LegendreInReferenceLayout(N, real, true, spectra, count, coeffs, s, &done); st != SL3DGPU_OK || done)
+    return st;
   if (int st = g.LegendreAnalysis(N, real, spectra, count, dev, s); st != SL3DGPU_OK) return st;
   return g.FromDevice(N, real, dev, count, coeffs, s);
 }

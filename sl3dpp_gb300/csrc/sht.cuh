@@ -176,6 +176,12 @@ class Grid {
   int LegendreAnalysis3F(const float* spectra, int count, float* coeffs, cudaStream_t stream);
   int RingWeighted3F(const float* spectraIn, int count, const float* weight, float* spectraOut, cudaStream_t stream);
 
+  // The Legendre sum between the reference layout's coefficients and the
+  // spectra, where one kernel does both (few fields on the FP64 units, every
+  // order with degrees); `done` says whether.
+  int LegendreInReferenceLayout(int N, bool real, bool analysis, const double* in, int count, double* out,
+                                cudaStream_t stream, bool* done);
+
   // Reference layout <-> device layout permutations.
   int ToDevice(int N, bool real, const double* ref, int count, double* dev, cudaStream_t stream);
   int FromDevice(int N, bool real, const double* dev, int count, double* ref, cudaStream_t stream);
