@@ -514,7 +514,18 @@ __device__ inline void StageWeights(int scheme, double h, double& e, double& alp
   }
 }
 
+// The reference model's share of a node's weight, 1 - phi_1(h_0) of its branch.
+__device__ inline double ReferenceBeta(const WeightsArgs& a, long long t) {
+  const double h0 = a.dt * a.itauRef[t];
+  if (a.scheme == 1) return 1.0 - 1.0 / (1.0 + h0);
+  return 1.0 - Phi1(h0, exp(-h0));
+}
+extern __shared__ double referenceBetas[];  // [branch][node], made once a block
+
 __global__ void WeightsKernel(WeightsArgs a) {
+  const int entries = a.branches * static_cast<int>(a.values / a.fieldSize);
+  for (int t = threadIdx.x; t < entries; t += blockDim.x) referenceBetas[t] = ReferenceBeta(a, t);
+  __syncthreads();
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
   const int P = static_cast<int>(a.values / a.fieldSize);
   for (long long x = a.begin + blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; x < a.end;
@@ -526,14 +537,7 @@ __global__ void WeightsKernel(WeightsArgs a) {
     for (int k = 0; k < a.branches; ++k) {
       const double itauRef = a.itauRef[static_cast<long long>(k) * P + node];
       const double mu = a.muBranch[static_cast<long long>(k) * P + node];
-      const double h0 = a.dt * itauRef;
-      double refBeta;
-      if (a.scheme == 1) {
-        refBeta = 1.0 - 1.0 / (1.0 + h0);
-      } else {
-        const double e0 = exp(-h0);
-        refBeta = 1.0 - Phi1(h0, e0);
-      }
+      const double refBeta = referenceBetas[k * P + node];
       const double h = a.dt * (itauRef * a.factor[x]);
       double ew, aw, bw;
       if (a.scheme == 1) {
@@ -1043,7 +1047,20 @@ void ForMemory(int m, F&& f) {
 
 __device__ inline bool NonLateral(int p, int pLat0, int pLat1) { return p < pLat0 || p >= pLat1; }
 
+// A stage's weights (e, alpha, beta) depend on the node and the branch alone,
+// and an exponential with its quotients is some sixty FP64 instructions: each
+// block makes them once, [branch][node], instead of every value making its own
+// (all streaming kernels of a mixed run at lmax 256: 36 -> 30 ms). 48 bytes a
+// node with two branches, half of what the force kernel keeps of a node.
+extern __shared__ double nodeTable[];
+
+__device__ inline void MakeStageTable(const SpectralMemoryArgs& a) {
+  for (int t = threadIdx.x; t < a.branches * a.P; t += blockDim.x)
+    StageWeights(a.scheme, a.dt * a.itauRef[t], nodeTable[3 * t], nodeTable[3 * t + 1], nodeTable[3 * t + 2]);
+  __syncthreads();
+}
 __global__ void SpectralStartKernel(SpectralMemoryArgs a) {
+  MakeStageTable(a);
   const long long total = a.rows * a.P;
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total; i += stride) {
@@ -1052,8 +1069,8 @@ __global__ void SpectralStartKernel(SpectralMemoryArgs a) {
     const double2 s0 = a.s[i];
     double2 fixed = C(0, 0);
     for (int k = 0; k < a.branches; ++k) {
-      double e, alpha, beta;
-      StageWeights(a.scheme, a.dt * a.itauRef[static_cast<long long>(k) * a.P + p], e, alpha, beta);
+      const double* weights = nodeTable + 3 * (k * a.P + p);
+      const double e = weights[0], alpha = weights[1];
       const double2 m = a.in[k][i];
       const double2 o = C(e * m.x + alpha * s0.x, e * m.y + alpha * s0.y);
       a.out[k][i] = o;
@@ -1065,6 +1082,7 @@ __global__ void SpectralStartKernel(SpectralMemoryArgs a) {
 }
 
 __global__ void SpectralAdvanceKernel(SpectralMemoryArgs a) {
+  MakeStageTable(a);
   const long long total = a.rows * a.P;
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
   for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < total; i += stride) {
@@ -1072,8 +1090,7 @@ __global__ void SpectralAdvanceKernel(SpectralMemoryArgs a) {
     if (!NonLateral(p, a.pLat0, a.pLat1)) continue;
     const double2 s1 = a.s[i];
     for (int k = 0; k < a.branches; ++k) {
-      double e, alpha, beta;
-      StageWeights(a.scheme, a.dt * a.itauRef[static_cast<long long>(k) * a.P + p], e, alpha, beta);
+      const double beta = nodeTable[3 * (k * a.P + p) + 2];
       const double2 m = a.out[k][i];
       a.out[k][i] = C(m.x + beta * s1.x, m.y + beta * s1.y);
     }
@@ -1219,6 +1236,9 @@ int StreamBlocks(long long values) {
   const long long b = (values + 255) / 256;
   return static_cast<int>(b < 152 * 32 ? (b > 0 ? b : 1) : 152 * 32);
 }
+// Blocks that make a table first: what runs at once (a thread makes a few
+// entries, for tens of values).
+int TableBlocks(long long values) { return std::min(StreamBlocks(values), 152 * 6); }
 
 }  // namespace
 
@@ -1344,18 +1364,24 @@ void LaunchSurface(const Geometry& g, const double2* solSph, const double2* solT
 void LaunchWeights(const WeightsArgs& a, cudaStream_t stream) {
   prof::Scope scope(prof::kStream, stream, 0.0, (a.end - a.begin) * (8.0 + a.branches * 96.0 + 40.0 + 48.0));
   if (a.end <= a.begin) return;
-  WeightsKernel<<<StreamBlocks(a.end - a.begin), 256, 0, stream>>>(a);
+  const size_t table = static_cast<size_t>(a.branches) * (a.values / a.fieldSize) * sizeof(double);
+  AllowDynamicSmem(WeightsKernel);
+  WeightsKernel<<<TableBlocks(a.end - a.begin), 256, table, stream>>>(a);
 }
 
 void LaunchSpectralStart(const SpectralMemoryArgs& a, cudaStream_t stream) {
   const long long n = a.rows * a.P;
   prof::Scope scope(prof::kStream, stream, 0.0, n * (16.0 + a.branches * 32.0 + 16.0));
-  SpectralStartKernel<<<StreamBlocks(n), 256, 0, stream>>>(a);
+  const size_t table = static_cast<size_t>(a.branches) * a.P * 3 * sizeof(double);
+  AllowDynamicSmem(SpectralStartKernel);
+  SpectralStartKernel<<<TableBlocks(n), 256, table, stream>>>(a);
 }
 void LaunchSpectralAdvance(const SpectralMemoryArgs& a, cudaStream_t stream) {
   const long long n = a.rows * a.P;
   prof::Scope scope(prof::kStream, stream, 0.0, n * (16.0 + a.branches * 32.0));
-  SpectralAdvanceKernel<<<StreamBlocks(n), 256, 0, stream>>>(a);
+  const size_t table = static_cast<size_t>(a.branches) * a.P * 3 * sizeof(double);
+  AllowDynamicSmem(SpectralAdvanceKernel);
+  SpectralAdvanceKernel<<<TableBlocks(n), 256, table, stream>>>(a);
 }
 void LaunchSpectralSum(const SpectralMemoryArgs& a, cudaStream_t stream) {
   const long long n = a.rows * a.P;
