@@ -120,10 +120,13 @@ void sl3dgpu_grid_destroy(sl3dgpu_grid* grid);
 int sl3dgpu_grid_shape(const sl3dgpu_grid* grid, int* ntheta, int* nphi);
 /* SurfaceGrid::LMax (SurfaceGrid.hpp): the grid's degree bound, -1 for a null grid. */
 int sl3dgpu_grid_lmax(const sl3dgpu_grid* grid);
-/* The grid's FP64 Legendre contractions: 0 on the FP64 units, 1 emulated on
- * the tensor cores (seven BF16 slices a value under a power-of-two scale per
- * row and column, exact FP32 products, levels joined in FP64: about 49 bits
- * of each operand; depths beyond 448 stay on the FP64 units). */
+/* The grid's FP64 transforms. Both forms run the Legendre contractions on the
+ * tensor cores (BF16 slices of each value under a power-of-two scale per row
+ * and column, exact FP32 products, levels joined exactly): 0 with eight slices,
+ * an error below the FP64 units' own rounding, and FP64-accurate rings; 1 with
+ * seven (about 49 bits of each operand) and the rings in double-float. Depths
+ * beyond 400 (448) and, in form 0, calls of up to eight fields stay on the
+ * FP64 units. */
 int sl3dgpu_grid_set_fp64_emulation(sl3dgpu_grid* grid, int on);
 /* Host copies of the colatitudes and their Gauss-Legendre weights. */
 int sl3dgpu_grid_colatitudes(const sl3dgpu_grid* grid, double* theta, double* weights);
@@ -138,8 +141,7 @@ int sl3dgpu_expand_spin_batch(sl3dgpu_grid* grid, int N, const double* fields, i
  * the contraction inside Synthesise/Expand), in the device layouts: spin-N
  * coefficients [row][count] complex (rows in (m, l) order, m from -lmax, or
  * m >= 0 for a real spin-0 field) <-> spectra [m][colatitude][count]
- * complex. fp32 = 0: FP64 (the FP64 units, or the tensor-core emulation the
- * grid is set to); 1: FP32 buffers through the 3xTF32 tensor-core
+ * complex. fp32 = 0: FP64 (in the form the grid is set to); 1: FP32 buffers through the 3xTF32 tensor-core
  * contraction of the mixed form's correction passes. */
 int sl3dgpu_legendre_device(sl3dgpu_grid* grid, int N, int real, int analysis, int fp32, const void* in,
                             int count, void* out, void* stream);
@@ -306,8 +308,8 @@ typedef struct sl3dgpu_v3d_options {
   int warm_start;           /* 0: each step starts from the previous strain (the reference's start);
                                1: also guesses 2 s_n - s_{n-1}, the mixed form's FP32 correction
                                starting from it (the FP64 form tries it as a first pass) */
-  int fp64_emulation;       /* 0: the FP64 Legendre contractions on the FP64 units; 1: emulated on
-                               the tensor cores (sl3dgpu_grid_set_fp64_emulation) */
+  int fp64_emulation;       /* the FP64 transforms: 0 with the FP64 units' accuracy, 1 at about 49 bits
+                               (sl3dgpu_grid_set_fp64_emulation) */
   int correction_memory;    /* mixed form: the FP32 correction's Anderson history, 0..16; 0 takes
                                anderson_memory */
 } sl3dgpu_v3d_options;

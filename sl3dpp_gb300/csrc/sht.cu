@@ -1156,6 +1156,16 @@ int LaunchRingWeightedF(Grid& g, int parts, bool real, const float* spectraIn, i
 // The most fields that count as a small batch (the FP64 units' rings).
 constexpr int kSmallBatch = 8;
 
+// A grid that asked for the emulation transforms its rings in double-float on
+// the FP32 pipe, unless SL3DGPU_FP64_RINGS=1 asks for FP64 accuracy there.
+bool DoubleFloatRings() {
+  static const bool fp64 = [] {
+    const char* v = std::getenv("SL3DGPU_FP64_RINGS");
+    return v != nullptr && v[0] == '1';
+  }();
+  return !fp64;
+}
+
 int LaunchRings(const Grid& g, int mode, int count, int parts, const FxRingPart* part, const double* weight,
                 cudaStream_t stream, bool fixedPoint) {
   if (count == 0) return SL3DGPU_OK;
@@ -1182,7 +1192,7 @@ int LaunchRings(const Grid& g, int mode, int count, int parts, const FxRingPart*
     ffts += static_cast<double>(g.ntheta) * count * (mode == kRingWeighted ? 2 : 1) * (real ? 0.5 : 1.0);
   }
   prof::Scope scope(prof::kRing, stream, ffts * 5.0 * g.nphi * std::log2(static_cast<double>(g.nphi)), bytes);
-  if (g.emulateFp64) return LaunchDfRings(g.dfPlan, a, stream);
+  if (g.emulateFp64 && DoubleFloatRings()) return LaunchDfRings(g.dfPlan, a, stream);
   // A batch of few fields is a launch's latency either way; it stays on the
   // FP64 units, so that fields made one at a time -- the delta field and the
   // loads a mixed run starts from -- are what they were bit for bit: where

@@ -523,7 +523,7 @@ int Viscoelastic3DGpu::Create(const sl3dgpu_layer* layers, int nlayers, const sl
     return SL3DGPU_ERR_ARGUMENT;
   }
   if (opt.fp64_emulation != 0 && opt.fp64_emulation != 1) {
-    SetError("v3d: fp64_emulation 0 (the FP64 units) or 1 (the tensor cores)");
+    SetError("v3d: fp64_emulation 0 (the FP64 units' accuracy) or 1 (about 49 bits)");
     return SL3DGPU_ERR_ARGUMENT;
   }
   if (opt.correction_memory < 0 || opt.correction_memory > kMixMaxMemory) {
