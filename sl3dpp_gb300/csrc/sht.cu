@@ -685,56 +685,59 @@ __global__ void CastKernel(const double* in, long long n, float* out) {
 
 // -- layout permutations -------------------------------------------------------------------
 
-__global__ void ToDeviceKernel(int lmax, int N, bool real, int count, const int* rowOffset,
-                               const double2* ref, double2* dev) {
-  const long long rows = real ? static_cast<long long>(lmax + 1) * (lmax + 2) / 2
-                              : static_cast<long long>(lmax + 1) * (lmax + 1) - N * N;
-  const long long t = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
-  if (t >= rows * count) return;
-  const int p = static_cast<int>(t / rows);
-  const long long i = t % rows;
-  int l, m;
-  if (real) {
-    l = static_cast<int>((sqrt(8.0 * i + 1.0) - 1.0) * 0.5);
-    while (static_cast<long long>(l) * (l + 1) / 2 > i) --l;
-    while (static_cast<long long>(l + 1) * (l + 2) / 2 <= i) ++l;
-    m = static_cast<int>(i - static_cast<long long>(l) * (l + 1) / 2);
-  } else {
-    const long long q = i + N * N;
-    l = static_cast<int>(sqrt(static_cast<double>(q)));
-    while (static_cast<long long>(l) * l > q) --l;
-    while (static_cast<long long>(l + 1) * (l + 1) <= q) ++l;
-    m = static_cast<int>(q - static_cast<long long>(l) * l) - l;
-  }
-  const int l0 = max(abs(m), abs(N));
-  const long long row = rowOffset[m + lmax] - (real ? rowOffset[lmax] : 0) + (l - l0);
-  dev[row * count + p] = ref[t];
-}
+// Reference layout [field][coefficient] <-> device layout [row][field], whose
+// rows are the coefficients in another order: a tile of 32 coefficients by 32
+// fields through shared memory, so that both sides are read and written in
+// runs, and a coefficient's row is found once, not once a field (55 spin -1
+// fields at lmax 256: 70 us a copy value by value, 22 so, 17 at the copy
+// bandwidth).
+constexpr int kPermuteTile = 32;
 
-__global__ void FromDeviceKernel(int lmax, int N, bool real, int count, const int* rowOffset,
-                                 const double2* dev, double2* ref) {
+template <bool kToDevice>
+__global__ void __launch_bounds__(256) PermuteKernel(int lmax, int N, bool real, int count, const int* rowOffset,
+                                                     const double2* in, double2* out) {
+  __shared__ double2 tile[kPermuteTile][kPermuteTile + 1];  // [coefficient][field]
+  __shared__ long long rowAt[kPermuteTile];
   const long long rows = real ? static_cast<long long>(lmax + 1) * (lmax + 2) / 2
                               : static_cast<long long>(lmax + 1) * (lmax + 1) - N * N;
-  const long long t = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
-  if (t >= rows * count) return;
-  const int p = static_cast<int>(t / rows);
-  const long long i = t % rows;
-  int l, m;
-  if (real) {
-    l = static_cast<int>((sqrt(8.0 * i + 1.0) - 1.0) * 0.5);
-    while (static_cast<long long>(l) * (l + 1) / 2 > i) --l;
-    while (static_cast<long long>(l + 1) * (l + 2) / 2 <= i) ++l;
-    m = static_cast<int>(i - static_cast<long long>(l) * (l + 1) / 2);
-  } else {
-    const long long q = i + N * N;
-    l = static_cast<int>(sqrt(static_cast<double>(q)));
-    while (static_cast<long long>(l) * l > q) --l;
-    while (static_cast<long long>(l + 1) * (l + 1) <= q) ++l;
-    m = static_cast<int>(q - static_cast<long long>(l) * l) - l;
+  const long long i0 = static_cast<long long>(blockIdx.x) * kPermuteTile;
+  const int p0 = blockIdx.y * kPermuteTile;
+  const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
+  if (warp == 0 && i0 + lane < rows) {
+    const long long i = i0 + lane;
+    int l, m;
+    if (real) {
+      l = static_cast<int>((sqrtf(8.0f * i + 1.0f) - 1.0f) * 0.5f);  // a guess; the loops settle it
+      while (static_cast<long long>(l) * (l + 1) / 2 > i) --l;
+      while (static_cast<long long>(l + 1) * (l + 2) / 2 <= i) ++l;
+      m = static_cast<int>(i - static_cast<long long>(l) * (l + 1) / 2);
+    } else {
+      const long long q = i + N * N;
+      l = static_cast<int>(sqrtf(static_cast<float>(q)));
+      while (static_cast<long long>(l) * l > q) --l;
+      while (static_cast<long long>(l + 1) * (l + 1) <= q) ++l;
+      m = static_cast<int>(q - static_cast<long long>(l) * l) - l;
+    }
+    rowAt[lane] = rowOffset[m + lmax] - (real ? rowOffset[lmax] : 0) + (l - max(abs(m), abs(N)));
   }
-  const int l0 = max(abs(m), abs(N));
-  const long long row = rowOffset[m + lmax] - (real ? rowOffset[lmax] : 0) + (l - l0);
-  ref[t] = dev[row * count + p];
+  __syncthreads();
+  const int coefficients = static_cast<int>(min(static_cast<long long>(kPermuteTile), rows - i0));
+  const int fields = min(kPermuteTile, count - p0);
+  for (int t = warp; t < kPermuteTile; t += 8) {
+    if (kToDevice) {  // a field's coefficients
+      if (t < fields && lane < coefficients) tile[lane][t] = in[(p0 + t) * rows + i0 + lane];
+    } else {  // a coefficient's fields
+      if (t < coefficients && lane < fields) tile[t][lane] = in[rowAt[t] * count + p0 + lane];
+    }
+  }
+  __syncthreads();
+  for (int t = warp; t < kPermuteTile; t += 8) {
+    if (kToDevice) {
+      if (t < coefficients && lane < fields) out[rowAt[t] * count + p0 + lane] = tile[t][lane];
+    } else {
+      if (t < fields && lane < coefficients) out[(p0 + t) * rows + i0 + lane] = tile[lane][t];
+    }
+  }
 }
 
 void GaussLegendre(int n, std::vector<double>& x, std::vector<double>& w) {
@@ -1479,6 +1482,13 @@ int LaunchRingWeightedF(Grid& g, int parts, bool real, const float* spectraIn, i
 }
 }  // namespace
 
+namespace {
+dim3 PermuteGrid(long long rows, int count) {
+  return dim3(static_cast<unsigned>((rows + kPermuteTile - 1) / kPermuteTile),
+              static_cast<unsigned>((count + kPermuteTile - 1) / kPermuteTile));
+}
+}  // namespace
+
 int Grid::ToDevice(int N, bool real, const double* ref, int count, double* dev,
                    cudaStream_t stream) {
   const SpinTable* t = nullptr;
@@ -1486,7 +1496,7 @@ int Grid::ToDevice(int N, bool real, const double* ref, int count, double* dev,
   const long long total = (real ? RealRows() : SpinRows(N)) * count;
   if (total == 0) return SL3DGPU_OK;
   prof::Scope scope(prof::kOther, stream);
-  ToDeviceKernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, stream>>>(
+  PermuteKernel<true><<<PermuteGrid(total / count, count), 256, 0, stream>>>(
       lmax, N, real, count, t->dRowOffset, reinterpret_cast<const double2*>(ref),
       reinterpret_cast<double2*>(dev));
   SL3D_CHECK_LAUNCH();
@@ -1500,7 +1510,7 @@ int Grid::FromDevice(int N, bool real, const double* dev, int count, double* ref
   const long long total = (real ? RealRows() : SpinRows(N)) * count;
   if (total == 0) return SL3DGPU_OK;
   prof::Scope scope(prof::kOther, stream);
-  FromDeviceKernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, stream>>>(
+  PermuteKernel<false><<<PermuteGrid(total / count, count), 256, 0, stream>>>(
       lmax, N, real, count, t->dRowOffset, reinterpret_cast<const double2*>(dev),
       reinterpret_cast<double2*>(ref));
   SL3D_CHECK_LAUNCH();
