@@ -19,8 +19,8 @@
 // own rounding (measured against quadruple precision at lmax 33 to 256, white
 // and decaying coefficients: 0.1 to 0.45 of theirs in the 2-norm). Against
 // the FP64 units' register-tiled product, bound by GB300's 1.2 TF/s FP64
-// pipe: 45 spin -2 fields at lmax 128, 1.12 ms a contraction there, 0.18 ms
-// here with the packing.
+// pipe: 45 spin -2 fields at lmax 128, 1.12 ms a contraction there; both
+// transforms of these fields, rings included, take 0.50 ms here.
 //
 // Products. Level d = p + q gathers sum_k s_p(A) s_q(B) over p + q = d, at
 // most (d + 3) 2^12 per k in magnitude, so below 2^24 -- exact in the FP32
@@ -80,9 +80,14 @@ __host__ __device__ constexpr uint32_t InstrDescriptorBf16(int n, int m) {
          (static_cast<uint32_t>(m >> 4) << 24);
 }
 
-// The BF16 bits of an integer of magnitude at most 256 (exact: its float has
-// at most eight significant bits, all in the upper half).
-__device__ inline uint32_t Bf16Bits(int integer) { return __float_as_uint(static_cast<float>(integer)) >> 16; }
+// The float of an integer of magnitude at most 256, whose upper half is its BF16
+// (exact: at most eight significant bits). The integer goes in as the low bits
+// of 1.5 2^23: the conversion instruction runs at a quarter of the rate.
+__device__ inline uint32_t FloatBits(int integer) {
+  return __float_as_uint(__uint_as_float(0x4B400000u + static_cast<uint32_t>(integer)) - 12582912.0f);
+}
+// The upper halves of two floats, the first lowest.
+__device__ inline uint32_t UpperHalves(uint32_t a, uint32_t b) { return __byte_perm(a, b, 0x7632); }
 
 // The exponent e with |v| < 2^e for the largest |v| of a set, from the
 // largest magnitude's bits (0 for zero; subnormals count as below 2^-1022).
@@ -94,7 +99,7 @@ __device__ inline int ExponentAbove(unsigned long long magnitudeBits) {
 }
 
 // v (|v| < 2^e) as S balanced base-2^7 digits of round(v 2^{7 S - e}),
-// packed as BF16 bits. (A non-finite column's digits are arbitrary: its
+// as their floats' bits. (A non-finite column's digits are arbitrary: its
 // outputs do not use them.)
 template <int S>
 __device__ inline void Split(double v, int e, uint32_t (&s)[S]) {
@@ -116,10 +121,10 @@ __device__ inline void Split(double v, int e, uint32_t (&s)[S]) {
   for (int p = S - 1; p > 0; --p) {
     int r = static_cast<int>(X & 127);
     if (r >= 64) r -= 128;
-    s[p] = Bf16Bits(r);
+    s[p] = FloatBits(r);
     X = (X - r) >> 7;
   }
-  s[0] = Bf16Bits(static_cast<int>(X));
+  s[0] = FloatBits(static_cast<int>(X));
 }
 
 // (H 2^28 + L) 2^scale as a double, rounded to nearest even, by
@@ -164,19 +169,24 @@ __device__ inline int Tile16Index(int row, int k, int rows) {
   return (k >> 3) * (rows * 8) + (row >> 3) * 64 + (row & 7) * 8 + (k & 7);
 }
 
-// Eight consecutive-k slices of one row (s[q][p]: value q, slice p) stored as
-// one 16-byte core-matrix row per slice.
-template <int S>
-__device__ inline void StoreSlices(uint16_t* tile, int sliceStride, int at, const uint32_t (&s)[8][S]) {
+// Eight consecutive values of one row split and stored as one 16-byte
+// core-matrix row per slice; two values at a time, so that their digits are
+// joined in pairs as they are made and not sixty-four registers later.
+template <int S, class Value>
+__device__ inline void StoreSplit(uint16_t* tile, int sliceStride, int at, int e, Value value) {
+  uint32_t words[4][S];
 #pragma unroll
-  for (int p = 0; p < S; ++p) {
-    uint4 v;
-    v.x = s[0][p] | (s[1][p] << 16);
-    v.y = s[2][p] | (s[3][p] << 16);
-    v.z = s[4][p] | (s[5][p] << 16);
-    v.w = s[6][p] | (s[7][p] << 16);
-    *reinterpret_cast<uint4*>(tile + p * sliceStride + at) = v;
+  for (int q = 0; q < 4; ++q) {
+    uint32_t a[S], b[S];
+    Split<S>(value(2 * q), e, a);
+    Split<S>(value(2 * q + 1), e, b);
+#pragma unroll
+    for (int p = 0; p < S; ++p) words[q][p] = UpperHalves(a[p], b[p]);
   }
+#pragma unroll
+  for (int p = 0; p < S; ++p)
+    *reinterpret_cast<uint4*>(tile + p * sliceStride + at) =
+        make_uint4(words[0][p], words[1][p], words[2][p], words[3][p]);
 }
 
 // One output as the FP64 units sum it, for a column holding an infinity or a
@@ -220,16 +230,12 @@ __global__ void PanelA64Kernel(const GemmItem* items, const Tc64Item* tcItems, c
     const int ks = static_cast<int>(tile % it.kSteps), mt = static_cast<int>(tile / it.kSteps);
     const int i = mt * kTcTileM + r, k0 = ks * kTcTileK + 8 * kg;
     const int e = i < g.M ? rowExp[it.rowExp + i] : 0;
-    uint32_t s[8][S];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
+    StoreSplit<S>(panels + (it.aPanel + tile) * S * kATile, kATile, Tile16Index(r, 8 * kg, kTcTileM), e, [&](int q) {
       const int k = k0 + q;
-      const double v = (i < g.M && k < g.K) ? table[g.a + static_cast<long long>(i) * g.sAi +
-                                                    static_cast<long long>(k) * g.sAk]
-                                            : 0.0;
-      Split<S>(v, e, s[q]);
-    }
-    StoreSlices<S>(panels + (it.aPanel + tile) * S * kATile, kATile, Tile16Index(r, 8 * kg, kTcTileM), s);
+      return (i < g.M && k < g.K)
+                 ? table[g.a + static_cast<long long>(i) * g.sAi + static_cast<long long>(k) * g.sAk]
+                 : 0.0;
+    });
   }
 }
 
@@ -238,10 +244,13 @@ __global__ void PanelA64Kernel(const GemmItem* items, const Tc64Item* tcItems, c
 // (each lane's maximum over its k, then over the eight lanes), then the
 // slices, 8-deep k groups in turn; a warp's reads of one k are 32
 // consecutive columns and its stores of one slice 512 contiguous bytes.
+// Latency bounds it, and so the threads an SM holds: at 64 registers, four CTAs
+// (92 fields at lmax 64 for three spins, 37 -> 32 us; reading a group ahead
+// took 98 registers and 51 us).
 constexpr int kPackThreads = 256, kPackLanes = kPackThreads / kTileN;
 
 template <int S>
-__global__ void __launch_bounds__(kPackThreads) PackB64Kernel(const Tc64Item* tcItems, const double* B, int* colExp,
+__global__ void __launch_bounds__(kPackThreads, 4) PackB64Kernel(const Tc64Item* tcItems, const double* B, int* colExp,
                                                               uint16_t* packed) {
   const Tc64Item it = tcItems[blockIdx.y];
   const int nt = blockIdx.x;
@@ -263,14 +272,14 @@ __global__ void __launch_bounds__(kPackThreads) PackB64Kernel(const Tc64Item* tc
   uint16_t* base = packed + (it.bPack + static_cast<long long>(nt) * it.kSteps) * S * kBTile;
   for (int group = lane; group < 2 * it.kSteps; group += kPackLanes) {
     const int ks = group / 2, kg = group % 2, k0 = 8 * group;
-    uint32_t s[8][S];
+    double v[8];
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
       const int k = k0 + q;
-      const double v = (n < it.N && k < it.K) ? col[static_cast<long long>(k) * it.ldb] : 0.0;
-      Split<S>(v, e, s[q]);
+      v[q] = (n < it.N && k < it.K) ? col[static_cast<long long>(k) * it.ldb] : 0.0;
     }
-    StoreSlices<S>(base + static_cast<long long>(ks) * S * kBTile, kBSlice, Tile16Index(nn, 8 * kg, S * kTileN), s);
+    StoreSplit<S>(base + static_cast<long long>(ks) * S * kBTile, kBSlice, Tile16Index(nn, 8 * kg, S * kTileN), e,
+                  [&](int q) { return v[q]; });
   }
 }
 
