@@ -7,7 +7,9 @@
 // additions, so the same transform in 64-bit integers under one scale a
 // ring (ring_fixed.cuh) does a fraction of the work, and its error is below
 // the FP64 transform's (measured against quadruple precision on white and
-// decaying spectra, 72 to 800 longitudes).
+// decaying spectra, 72 to 800 longitudes). Both transforms of 45 spin -2 fields
+// at lmax 128 went from 1.28 to 0.63 ms with it, the rings from the larger
+// part of that to half.
 //
 // How. One CTA per (colatitude, G consecutive fields; G a power of two so that
 // a thread's values belong to one ring). The raw FP64 bits go to shared

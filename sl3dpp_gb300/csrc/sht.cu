@@ -1037,6 +1037,9 @@ int Grid::Tables(const Batch& b, Tc64Tables* out) {
 
 // Whether a batch's FP64 contraction runs as slice products: within the
 // exactness bound on its depth, and wider than the narrow kernels' columns.
+// Up to eight fields stay on the FP64 units: a contraction of so few is latency
+// either way (one field at lmax 128: 11 us, one launch; the slices are two),
+// and the fields a mixed run starts from keep their bits.
 bool Grid::UseSlices64(const Batch& b) const {
   if (emulateFp64) return b.maxK <= Tc64MaxK(kTc64Slices);
   return b.maxN > kNarrowN && b.maxK <= Tc64MaxK(kTc64SlicesFull);
