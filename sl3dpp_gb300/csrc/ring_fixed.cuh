@@ -11,6 +11,7 @@
 #pragma once
 
 #include <cstdint>
+#include <vector>
 
 #include "common.cuh"
 
@@ -51,8 +52,8 @@ __host__ __device__ inline uint32_t FxDivide(uint32_t x, uint32_t magic) {
 bool MakeFxPlan(int n, FxPlan* plan);
 // The plan of given radices (their product n).
 FxPlan FxPlanOf(int n, const int* radices, int stages);
-// e^{2 pi i k / n} in Q62.
-FxRoot MakeFxRoot(int k, int n);
+// e^{2 pi i k / n} in Q62, k < n.
+std::vector<FxRoot> MakeFxRoots(int n);
 
 __host__ __device__ inline long long FxProduct(int ah, int al, int wh, int wl) {
   const long long p = static_cast<long long>(ah) * wl + (1LL << 29) + static_cast<long long>(al) * wh;

@@ -820,8 +820,7 @@ int Grid::Create(int lmax, int nmax, double oversampling, std::unique_ptr<Grid>&
     return SL3DGPU_ERR_ARGUMENT;
   }
   g->dfPlan = FxPlanOf(g->nphi, plan.radix, plan.stages);
-  std::vector<FxRoot> roots(g->nphi);
-  for (int k = 0; k < g->nphi; ++k) roots[k] = MakeFxRoot(k, g->nphi);
+  const std::vector<FxRoot> roots = MakeFxRoots(g->nphi);
   SL3D_CUDA(cudaMalloc(&g->dRoots, g->nphi * sizeof(FxRoot)));
   SL3D_CUDA(CopyIn(g->dRoots, roots.data(), g->nphi * sizeof(FxRoot)));
   out = std::move(g);
