@@ -1084,6 +1084,8 @@ int Grid::RunGemm64(int N, bool real, Batch& b, const double* B, double* C, bool
                      b.maxATiles, tables.of[c], panel, stream);
       SL3D_CHECK_LAUNCH();
     }
+    // finished before a call on another stream can find it (once a panel, as Table waits)
+    SL3D_CUDA(cudaStreamSynchronize(stream));
     found = panels64_.emplace(key, panel).first;
   }
   // this call's packed tiles, then its column exponents
@@ -1376,6 +1378,7 @@ int Grid::RunGemmF(int N, bool real, Batch& b, const float* B, float* C, bool ac
                    panel, stream);
       SL3D_CHECK_LAUNCH();
     }
+    SL3D_CUDA(cudaStreamSynchronize(stream));  // as RunGemm64's
     found = panels_.emplace(key, panel).first;
   }
   // B split and packed inside the contraction (B and C never overlap here:
