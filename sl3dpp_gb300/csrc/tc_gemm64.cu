@@ -106,15 +106,17 @@ __device__ inline void Split(double v, int e, uint32_t (&s)[S]) {
   const unsigned long long bits = static_cast<unsigned long long>(__double_as_longlong(v));
   const int biased = static_cast<int>((bits >> 52) & 0x7FF);
   const long long mantissa = static_cast<long long>(bits & ((1ULL << 52) - 1)) | (biased ? (1LL << 52) : 0LL);
-  // v = mantissa 2^{E - 52}, E <= e - 1, so X = mantissa 2^{E - e + 7 S - 52}:
-  // a right shift by t, rounded to nearest, or a left one by at most 3 (S = 8)
+  // v = mantissa 2^{E - 52}, so X = mantissa 2^{E - e + 7 S - 52}: a right
+  // shift by t, rounded to nearest, or with S = 8 a left one, by at most 3 where
+  // E <= e - 1, and by 4 in a row (column) of subnormal values, whose E and e
+  // are both -1022 and whose mantissas are below 2^52
   const int E = biased ? biased - 1023 : -1022;
   const int t = e - E + 52 - 7 * S;
   long long X = 0;
   if (7 * S < 53 || t > 0) {
     if (t < 63) X = (mantissa + (1LL << (t - 1))) >> t;
   } else {
-    X = mantissa << min(-t, 3);
+    X = mantissa << min(-t, 4);
   }
   if (bits >> 63) X = -X;
 #pragma unroll
