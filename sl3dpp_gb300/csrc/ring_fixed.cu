@@ -229,6 +229,13 @@ __device__ __forceinline__ unsigned long long Bits(double v) {
   return static_cast<unsigned long long>(__double_as_longlong(v));
 }
 
+// A value's exponent among its ring's: 0 for zero alone, a subnormal value
+// counting as 1, so that a ring (or its weights) of nothing larger takes the
+// FP64 form.
+__device__ __forceinline__ uint32_t RingExponent(unsigned long long bits) {
+  return max(static_cast<uint32_t>(FxExponent(bits)), (bits << 1) != 0 ? 1u : 0u);
+}
+
 // Whether an exponent keeps a ring's scale inside the FP64 range (a ring of
 // zeros has none).
 __device__ __forceinline__ bool FxCarries(uint32_t emax) {
@@ -263,7 +270,7 @@ __global__ void __launch_bounds__(kFxThreads, 2) FxRingKernel(const __grid_const
   // order m at m and the second field's at n - m (order 0 of both at 0).
   // Only this thread's own entries until the transform.
   uint32_t emax = 0;
-  auto seen = [&](unsigned long long bits) { emax = max(emax, static_cast<uint32_t>(FxExponent(bits))); };
+  auto seen = [&](unsigned long long bits) { emax = max(emax, RingExponent(bits)); };
   const bool synth = A.mode != kFxAnalyse;
   if (synth) {
     const double2* in = Q.spectraIn + static_cast<long long>(j) * A.count + fa;
@@ -414,8 +421,8 @@ __global__ void __launch_bounds__(kFxThreads, 2) FxRingKernel(const __grid_const
     uint32_t wmax = 0;
     if (live)
       for (int k = lead; k < n; k += step) {
-        wmax = max(wmax, static_cast<uint32_t>(FxExponent(Bits(A.pointWeight[row0 + k]))));
-        if (second) wmax = max(wmax, static_cast<uint32_t>(FxExponent(Bits(A.pointWeight[row1 + k]))));
+        wmax = max(wmax, RingExponent(Bits(A.pointWeight[row0 + k])));
+        if (second) wmax = max(wmax, RingExponent(Bits(A.pointWeight[row1 + k])));
       }
     wmax = OverRing(wmax, shared, G, Most);
     if (!FxCarries(wmax) || (wmax > 0 && e0 > 0 && !FxCarries(static_cast<uint32_t>(max(1, e0 + static_cast<int>(wmax) - 1023)))))

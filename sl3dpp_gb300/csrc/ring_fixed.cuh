@@ -266,7 +266,7 @@ __host__ __device__ inline long long FxFrom(unsigned long long bits, int scale) 
     X = mantissa << shift;
   else
     X = shift < -54 ? 0 : (mantissa + (1LL << (-shift - 1))) >> -shift;
-  if (e == 0) X = 0;  // zero (subnormal values are below any ring's unit but a subnormal ring's)
+  if (e == 0) X = 0;  // zero, or subnormal: below the unit of any ring held in fixed point
   return bits >> 63 ? -X : X;
 }
 // X 2^-scale as a double, rounded to nearest.
