@@ -53,10 +53,18 @@ __device__ double WignerStart(int N, int m, double c, double s) {
     return v;
   }
   const int l = A;
-  const double fact[5] = {1.0, 1.0, 2.0, 6.0, 24.0};
-  double v = sqrt(fact[2 * l] / (fact[l + m] * fact[l - m]));
-  for (int k = 0; k < l - m; ++k) v *= c;
-  for (int k = 0; k < l + m; ++k) v *= s;
+  double v = 1.0;
+  if (l <= 2) {
+    const double fact[5] = {1.0, 1.0, 2.0, 6.0, 24.0};
+    v = sqrt(fact[2 * l] / (fact[l + m] * fact[l - m]));
+    for (int k = 0; k < l - m; ++k) v *= c;
+    for (int k = 0; k < l + m; ++k) v *= s;
+  } else {
+    // sqrt(binomial(2 l, r)) (c s)^r factor by factor, then the rest of the larger power
+    const int r = l - M, q = l + M;
+    for (int k = 1; k <= r; ++k) v *= sqrt((q + k) / static_cast<double>(k)) * c * s;
+    for (int k = 0; k < 2 * M; ++k) v *= m > 0 ? s : c;
+  }
   if ((l + m) % 2 != 0) v = -v;
   return v;
 }
