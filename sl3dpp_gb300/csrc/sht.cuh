@@ -18,6 +18,7 @@
 #pragma once
 
 #include <array>
+#include <climits>
 #include <cstdint>
 #include <map>
 #include <memory>
@@ -194,7 +195,7 @@ class Grid {
   std::map<int, SpinTable> tables_;
   // The components a batch's contraction covers: a spin's, or a tensor's three
   // (N = kTriple), each an item range with its own table.
-  static constexpr int kTriple = 1000;
+  static constexpr int kTriple = INT_MAX;  // no grid has this spin
   struct Part {
     int N = 0;
     bool real = false;

@@ -38,3 +38,21 @@ def test_gpu_basis_functions(gpu, N):
             want = math.sqrt((2 * l + 1) / (4 * math.pi)) * _wigner(l, m, N, grid.theta)
             got = fields[grid.SpinIndex(N, l, m)]
             assert np.max(np.abs(got - want)) < 1e-13, (l, m)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("count", [1, 12])
+def test_gpu_spin_1000(gpu, count):
+    """A spin as large as a grid of degree 1000 has, whose only degree is its
+    lowest. Its basis functions are orthogonal under the quadrature; each value
+    is a product of up to 2000 roundings, so a round trip is within 1e-11."""
+    import torch
+
+    from sl3dpp_gb300.grid import SurfaceGrid
+
+    lmax = N = 1000
+    grid = SurfaceGrid(lmax, N, 1.0)
+    c = torch.randn(count * grid.SpinCoefficientSize(N), dtype=torch.complex128, device=gpu,
+                    generator=torch.Generator(device=gpu).manual_seed(N))
+    back = grid.ExpandSpinBatch(N, grid.SynthesiseSpinBatch(N, c, count), count)
+    assert float((back - c).abs().max()) < 1e-11 * float(c.abs().max())
