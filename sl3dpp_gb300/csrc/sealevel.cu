@@ -552,7 +552,7 @@ struct SleWorkspace {
   }
   // the nonlinear solve's buffers (on its first use on the grid)
   int PrepareNonlinear() {
-    if (nlOcean.p != nullptr) return SL3DGPU_OK;
+    if (nlRingOcean.p != nullptr) return SL3DGPU_OK;  // the last of them
     for (auto* d : {&nlOcean, &nlChange, &nlSlc, &nlLocal}) SL3D_CUDA(d->Alloc(run.fieldSize));
     SL3D_CUDA(nlRingUnbalanced.Alloc(run.ntheta));
     SL3D_CUDA(nlRingOcean.Alloc(run.ntheta));
@@ -561,6 +561,7 @@ struct SleWorkspace {
   // the mixer at its plain start, with `memory` columns
   int ResetMixer(int memory) {
     if (mixerMemory != memory) {
+      mixerMemory = -1;  // until its buffers are there
       mixer = LoadMixer{};
       SL3D_TRY(mixer.Init(memory, 2 * run.coefCount));
       mixerMemory = memory;
@@ -1248,28 +1249,24 @@ int Flotation(long long n, double water_density, double ice_density, const doubl
 using namespace sl3dgpu;
 
 namespace {
-// The workspace a solve by handle runs in: the grid's own, kept between
-// solves (its forty allocations and their release were a fifth of an lmax-128
-// solve), or, while another thread's solve holds that, one for the call. A
-// solve waits for its stream before it returns, so the next may use any stream.
-struct GridWorkspace {
-  std::unique_lock<std::mutex> held;
-  std::unique_ptr<SleWorkspace> own;
-  SleWorkspace* ws = nullptr;
-  explicit GridWorkspace(sl3dgpu_grid* grid) {
-    if (grid != nullptr) {
-      GridAttachment& a = AttachmentOf(grid);
-      held = std::unique_lock<std::mutex>(a.lock, std::try_to_lock);
-      if (held.owns_lock()) {
-        if (!a.workspace) a.workspace = std::shared_ptr<void>(new SleWorkspace, [](void* p) { delete static_cast<SleWorkspace*>(p); });
-        ws = static_cast<SleWorkspace*>(a.workspace.get());
-        return;
-      }
-    }
-    own = std::make_unique<SleWorkspace>();
-    ws = own.get();
+// A solve by handle, in the grid's own workspace, kept between solves (its forty
+// allocations and their release were a fifth of an lmax-128 solve). A solve has
+// waited for its stream when it returns, a failed one here, so the next may use
+// any stream; solves of several threads on one grid take turns.
+template <class Solve>
+int WithGridWorkspace(sl3dgpu_grid* grid, cudaStream_t stream, Solve solve) {
+  if (grid == nullptr) {
+    SetError("sle: null argument");
+    return SL3DGPU_ERR_ARGUMENT;
   }
-};
+  GridAttachment& a = AttachmentOf(grid);
+  std::lock_guard<std::mutex> held(a.lock);
+  if (!a.workspace)
+    a.workspace = std::shared_ptr<void>(new SleWorkspace, [](void* p) { delete static_cast<SleWorkspace*>(p); });
+  const int status = solve(*static_cast<SleWorkspace*>(a.workspace.get()));
+  if (status != SL3DGPU_OK) cudaStreamSynchronize(stream);
+  return status;
+}
 }  // namespace
 
 extern "C" int sl3dgpu_sle_solve(sl3dgpu_grid* grid, const sl3dgpu_sle_body* body, const double* ocean,
@@ -1277,10 +1274,11 @@ extern "C" int sl3dgpu_sle_solve(sl3dgpu_grid* grid, const sl3dgpu_sle_body* bod
                                  int anderson_memory, double* sea_level_change, double* displacement,
                                  double* potential, double* tangential_potential, double* toroidal_potential,
                                  sl3dgpu_sle_result* result, void* stream) {
-  GridWorkspace ws(grid);
-  return SeaLevelSolve(*ws.ws, grid, body, ocean, forcing, rtol, max_iterations, anderson_memory, sea_level_change,
-                       displacement, potential, tangential_potential, toroidal_potential, nullptr, result,
-                       AsStream(stream));
+  return WithGridWorkspace(grid, AsStream(stream), [&](SleWorkspace& ws) {
+    return SeaLevelSolve(ws, grid, body, ocean, forcing, rtol, max_iterations, anderson_memory, sea_level_change,
+                         displacement, potential, tangential_potential, toroidal_potential, nullptr, result,
+                         AsStream(stream));
+  });
 }
 
 extern "C" int sl3dgpu_sle_solve_nonlinear(sl3dgpu_grid* grid, const sl3dgpu_sle_body* body, double ice_density,
@@ -1291,10 +1289,11 @@ extern "C" int sl3dgpu_sle_solve_nonlinear(sl3dgpu_grid* grid, const sl3dgpu_sle
                                            double* toroidal_potential, double* final_sea_level,
                                            double* final_ocean_function, double* load_coefficients,
                                            sl3dgpu_sle_result* result, void* stream) {
-  GridWorkspace ws(grid);
-  return SeaLevelSolveNonlinear(*ws.ws, grid, body, ice_density, state, forcing, rtol, max_iterations, sea_level_change,
-                                displacement, potential, tangential_potential, toroidal_potential, final_sea_level,
-                                final_ocean_function, load_coefficients, result, AsStream(stream));
+  return WithGridWorkspace(grid, AsStream(stream), [&](SleWorkspace& ws) {
+    return SeaLevelSolveNonlinear(ws, grid, body, ice_density, state, forcing, rtol, max_iterations, sea_level_change,
+                                  displacement, potential, tangential_potential, toroidal_potential, final_sea_level,
+                                  final_ocean_function, load_coefficients, result, AsStream(stream));
+  });
 }
 
 extern "C" int sl3dgpu_sle_flotation(long long n, double water_density, double ice_density, const double* ice,

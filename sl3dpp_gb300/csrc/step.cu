@@ -1974,6 +1974,7 @@ int Viscoelastic3DGpu::Mixer32Reset() {
   if (memory <= 0) return SL3DGPU_OK;
   const size_t n = 2 * compactComplex;
   if (mixer32Memory != memory || mixer32Size != n) {
+    mixer32Memory = 0;  // until its buffers are there
     dG32.resize(memory);
     dF32.resize(memory);
     std::vector<__nv_bfloat16*> gp(memory), fp(memory);

@@ -57,8 +57,10 @@ struct Dev {
   cudaError_t Alloc(size_t count) {
     cudaFree(p);
     p = nullptr;
-    n = count;
-    return cudaMalloc(&p, std::max<size_t>(count, 1) * sizeof(T));
+    n = 0;  // what a failed allocation leaves
+    const cudaError_t e = cudaMalloc(&p, std::max<size_t>(count, 1) * sizeof(T));
+    if (e == cudaSuccess) n = count;
+    return e;
   }
   cudaError_t Upload(const std::vector<T>& v) {
     if (cudaError_t e = Alloc(v.size()); e != cudaSuccess) return e;
