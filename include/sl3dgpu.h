@@ -113,7 +113,11 @@ int sl3dgpu_band_cholesky_solve_noalloc(const double* ab, int n, int kd, double*
 /* ---- the surface grid (include/sl3dpp/SurfaceGrid.hpp:58-287) ---------------
  * A Gauss-Legendre grid for degrees to lmax and spins to nmax, oversampled
  * by `oversampling` (band L' = ceil(oversampling lmax): L' + 1 colatitudes,
- * the smallest 2^a 3^b 5^c >= 2 L' + 1 longitudes from zero). */
+ * the smallest 2^a 3^b 5^c >= 2 L' + 1 longitudes from zero).
+ * Several host threads may call one grid. Its synthesis and expansion calls
+ * share the grid's scratch, so those on different streams are to be ordered by
+ * the caller; sl3dgpu_legendre_device uses none and may overlap on any streams.
+ * The sea-level solves on one grid take turns. */
 typedef struct sl3dgpu_grid sl3dgpu_grid;
 int sl3dgpu_grid_create(int lmax, int nmax, double oversampling, sl3dgpu_grid** out);
 void sl3dgpu_grid_destroy(sl3dgpu_grid* grid);

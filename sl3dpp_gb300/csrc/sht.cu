@@ -1559,6 +1559,7 @@ using namespace sl3dgpu;
 struct sl3dgpu_grid {
   std::unique_ptr<Grid> grid;
   GridAttachment attachment;
+  std::mutex calls;  // held while a call looks up or makes the grid's tables, batches and panels and launches
 };
 
 extern "C" int sl3dgpu_grid_create(int lmax, int nmax, double oversampling, sl3dgpu_grid** out) {
@@ -1597,6 +1598,7 @@ extern "C" int sl3dgpu_grid_set_fp64_emulation(sl3dgpu_grid* grid, int on) {
     SetError("grid: null handle, or fp64 emulation not 0 or 1");
     return SL3DGPU_ERR_ARGUMENT;
   }
+  std::lock_guard<std::mutex> held(grid->calls);
   grid->grid->emulateFp64 = on != 0;
   return SL3DGPU_OK;
 }
@@ -1620,6 +1622,7 @@ int Synthesise(sl3dgpu_grid* handle, int N, bool real, const double* coeffs, int
     SetError("null grid or negative count");
     return SL3DGPU_ERR_ARGUMENT;
   }
+  std::lock_guard<std::mutex> held(handle->calls);
   auto& g = *handle->grid;
   const cudaStream_t s = AsStream(stream);
   const size_t mcount = real ? g.lmax + 1 : 2 * g.lmax + 1;
@@ -1645,6 +1648,7 @@ int Expand(sl3dgpu_grid* handle, int N, bool real, const double* fields, int cou
     SetError("null grid or negative count");
     return SL3DGPU_ERR_ARGUMENT;
   }
+  std::lock_guard<std::mutex> held(handle->calls);
   auto& g = *handle->grid;
   const cudaStream_t s = AsStream(stream);
   const size_t mcount = real ? g.lmax + 1 : 2 * g.lmax + 1;
@@ -1667,6 +1671,7 @@ int Expand(sl3dgpu_grid* handle, int N, bool real, const double* fields, int cou
 namespace sl3dgpu {
 int SynthesiseFixed(sl3dgpu_grid* grid, const double* coeffs, double* field, cudaStream_t stream, bool device) {
   if (!device) return Synthesise(grid, 0, true, coeffs, 1, field, stream, true);
+  std::lock_guard<std::mutex> held(grid->calls);
   auto& g = *grid->grid;
   double *spectra = nullptr, *unused = nullptr;
   if (int st = g.Scratch(static_cast<size_t>(g.lmax + 1) * g.ntheta * 2, 0, &spectra, &unused); st != SL3DGPU_OK)
@@ -1676,6 +1681,7 @@ int SynthesiseFixed(sl3dgpu_grid* grid, const double* coeffs, double* field, cud
 }
 int ExpandFixed(sl3dgpu_grid* grid, const double* field, double* coeffs, cudaStream_t stream, bool device) {
   if (!device) return Expand(grid, 0, true, field, 1, coeffs, stream, true);
+  std::lock_guard<std::mutex> held(grid->calls);
   auto& g = *grid->grid;
   double *spectra = nullptr, *unused = nullptr;
   if (int st = g.Scratch(static_cast<size_t>(g.lmax + 1) * g.ntheta * 2, 0, &spectra, &unused); st != SL3DGPU_OK)
@@ -1702,6 +1708,7 @@ extern "C" int sl3dgpu_legendre_device(sl3dgpu_grid* grid, int N, int real, int 
     SetError("legendre: null grid, negative count, or a real field of nonzero spin");
     return SL3DGPU_ERR_ARGUMENT;
   }
+  std::lock_guard<std::mutex> held(grid->calls);
   auto& g = *grid->grid;
   const cudaStream_t s = AsStream(stream);
   if (fp32) {
