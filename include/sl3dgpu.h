@@ -117,7 +117,12 @@ int sl3dgpu_band_cholesky_solve_noalloc(const double* ab, int n, int kd, double*
  * Several host threads may call one grid. Its synthesis and expansion calls
  * share the grid's scratch, so those on different streams are to be ordered by
  * the caller; sl3dgpu_legendre_device uses none and may overlap on any streams.
- * The sea-level solves on one grid take turns. */
+ * The sea-level solves on one grid take turns.
+ * The tensor-core contractions' waits are bounded. One that gives up leaves NaN
+ * in its outputs (FP32: unspecified values) and a mark that the next call on
+ * the grid finds once the kernel has ended: that call does nothing but return
+ * SL3DGPU_ERR_WAIT, once. A step of an operator reads its own grid's mark
+ * before it returns. */
 typedef struct sl3dgpu_grid sl3dgpu_grid;
 int sl3dgpu_grid_create(int lmax, int nmax, double oversampling, sl3dgpu_grid** out);
 void sl3dgpu_grid_destroy(sl3dgpu_grid* grid);

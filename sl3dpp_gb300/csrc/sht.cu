@@ -836,7 +836,7 @@ int Grid::Create(int lmax, int nmax, double oversampling, std::unique_ptr<Grid>&
 }
 
 Grid::~Grid() {
-  cudaFree(dTcError_);
+  if (giveUp_ != nullptr) cudaFreeHost(giveUp_);
   for (auto& [key, panel] : panels_) cudaFree(panel);
   for (auto& [key, panel] : panels64_) {
     cudaFree(panel.slices);
@@ -1060,10 +1060,8 @@ int Grid::RunGemm64(int N, bool real, Batch& b, const double* B, double* C, bool
                     cudaStream_t stream) {
   if (b.count == 0) return SL3DGPU_OK;
   const int slices = emulateFp64 ? kTc64Slices : kTc64SlicesFull;
-  if (dTcError_ == nullptr) {
-    SL3D_CUDA(cudaMalloc(&dTcError_, sizeof(int)));
-    SL3D_CUDA(ZeroIn(dTcError_, sizeof(int)));
-  }
+  int* giveUp = nullptr;
+  if (int st = GiveUpFlag(&giveUp); st != SL3DGPU_OK) return st;
   if (pool_ == nullptr) {
     cudaMemPoolProps props{};
     props.allocType = cudaMemAllocationTypePinned;
@@ -1111,7 +1109,7 @@ int Grid::RunGemm64(int N, bool real, Batch& b, const double* B, double* C, bool
   {
     prof::Scope scope(prof::kLegendre64Tc, stream, b.flops);
     status = RunGemm64Tc(slices, b.items, b.tc64Items, b.count, b.maxMTiles, b.maxNTiles64, tables, found->second,
-                         B, packed, colExp, C, accumulate, dTcError_, stream);
+                         B, packed, colExp, C, accumulate, giveUp, stream);
   }
   SL3D_CUDA(cudaFreeAsync(scratch, stream));
   return status;
@@ -1360,10 +1358,8 @@ int Grid::Table32(int N, const SpinTable** out) {
 int Grid::RunGemmF(int N, bool real, Batch& b, const float* B, float* C, bool accumulate, cudaStream_t stream) {
   if (b.count == 0) return SL3DGPU_OK;
   static_assert(sizeof(TcItemHost) == sizeof(TcItem), "host and device tensor-core items agree");
-  if (dTcError_ == nullptr) {
-    SL3D_CUDA(cudaMalloc(&dTcError_, sizeof(int)));
-    SL3D_CUDA(ZeroIn(dTcError_, sizeof(int)));
-  }
+  int* giveUp = nullptr;
+  if (int st = GiveUpFlag(&giveUp); st != SL3DGPU_OK) return st;
   if (b.tcItems == nullptr) {
     SL3D_CUDA(cudaMalloc(&b.tcItems, b.tcHost.size() * sizeof(TcItem)));
     SL3D_CUDA(CopyIn(b.tcItems, b.tcHost.data(), b.tcHost.size() * sizeof(TcItem)));
@@ -1407,7 +1403,7 @@ int Grid::RunGemmF(int N, bool real, Batch& b, const float* B, float* C, bool ac
                     4.0 * b.panelFloats + (separatePack ? 4.0 : 2.0) * b.packedFloats * b.maxMTiles +
                         4.0 * b.outputs);
   return RunGemmTc(items, b.dTcTiles, static_cast<int>(b.tcTiles.size()), b.tileN, found->second, b.packed,
-                   separatePack ? nullptr : B, C, accumulate, dTcError_, stream);
+                   separatePack ? nullptr : B, C, accumulate, giveUp, stream);
 }
 
 Grid::Batch* Grid::MutableBatch(int N, bool real, bool analysis, int P, int p0, int count) {
@@ -1416,17 +1412,26 @@ Grid::Batch* Grid::MutableBatch(int N, bool real, bool analysis, int P, int p0, 
   return const_cast<Batch*>(b);
 }
 
-int Grid::TensorCoreStatus(cudaStream_t stream) {
-  if (dTcError_ == nullptr) return SL3DGPU_OK;
-  int flag = 0;
-  SL3D_CUDA(cudaMemcpyAsync(&flag, dTcError_, sizeof(int), cudaMemcpyDeviceToHost, stream));
-  SL3D_CUDA(cudaStreamSynchronize(stream));
-  if (flag != 0) {
-    SL3D_CUDA(cudaMemsetAsync(dTcError_, 0, sizeof(int), stream));
-    SetError("a tensor-core contraction gave up waiting for its completion");
-    return SL3DGPU_ERR_WAIT;
+int Grid::GiveUpFlag(int** flag) {
+  if (giveUp_ == nullptr) {
+    SL3D_CUDA(cudaMallocHost(&giveUp_, sizeof(int)));
+    *giveUp_ = 0;
   }
+  *flag = giveUp_;
   return SL3DGPU_OK;
+}
+
+int Grid::TensorCoreStatus() {
+  if (giveUp_ == nullptr || *static_cast<volatile int*>(giveUp_) == 0) return SL3DGPU_OK;
+  *giveUp_ = 0;
+  SetError("a tensor-core contraction gave up waiting for its completion");
+  return SL3DGPU_ERR_WAIT;
+}
+
+int Grid::TensorCoreStatus(cudaStream_t stream) {
+  if (giveUp_ == nullptr) return SL3DGPU_OK;
+  SL3D_CUDA(cudaStreamSynchronize(stream));
+  return TensorCoreStatus();
 }
 
 int Grid::LegendreSynthesisF(int N, bool real, const float* coeffs, int P, int p0, int count, float* spectra,
@@ -1624,6 +1629,7 @@ int Synthesise(sl3dgpu_grid* handle, int N, bool real, const double* coeffs, int
   }
   std::lock_guard<std::mutex> held(handle->calls);
   auto& g = *handle->grid;
+  if (int st = g.TensorCoreStatus(); st != SL3DGPU_OK) return st;  // an earlier call's
   const cudaStream_t s = AsStream(stream);
   const size_t mcount = real ? g.lmax + 1 : 2 * g.lmax + 1;
   const size_t rows = real ? g.RealRows() : g.SpinRows(N);
@@ -1650,6 +1656,7 @@ int Expand(sl3dgpu_grid* handle, int N, bool real, const double* fields, int cou
   }
   std::lock_guard<std::mutex> held(handle->calls);
   auto& g = *handle->grid;
+  if (int st = g.TensorCoreStatus(); st != SL3DGPU_OK) return st;  // an earlier call's
   const cudaStream_t s = AsStream(stream);
   const size_t mcount = real ? g.lmax + 1 : 2 * g.lmax + 1;
   const size_t rows = real ? g.RealRows() : g.SpinRows(N);
@@ -1690,6 +1697,7 @@ int ExpandFixed(sl3dgpu_grid* grid, const double* field, double* coeffs, cudaStr
   return g.LegendreAnalysis(0, true, spectra, 1, coeffs, stream);
 }
 GridAttachment& AttachmentOf(sl3dgpu_grid* grid) { return grid->attachment; }
+Grid& GridOf(sl3dgpu_grid* grid) { return *grid->grid; }
 }  // namespace sl3dgpu
 
 extern "C" int sl3dgpu_synthesise_spin_batch(sl3dgpu_grid* grid, int N, const double* coeffs,
@@ -1710,6 +1718,7 @@ extern "C" int sl3dgpu_legendre_device(sl3dgpu_grid* grid, int N, int real, int 
   }
   std::lock_guard<std::mutex> held(grid->calls);
   auto& g = *grid->grid;
+  if (int st = g.TensorCoreStatus(); st != SL3DGPU_OK) return st;  // an earlier call's
   const cudaStream_t s = AsStream(stream);
   if (fp32) {
     return analysis ? g.LegendreAnalysisF(N, real != 0, static_cast<const float*>(in), count, 0, count,

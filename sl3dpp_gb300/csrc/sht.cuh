@@ -146,9 +146,13 @@ class Grid {
   // correction passes): FP32 copies of the table and twiddles, made once.
   int LegendreSynthesisF(int N, bool real, const float* coeffs, int P, int p0, int count, float* spectra,
                          cudaStream_t stream);
-  // Whether a tensor-core contraction gave up waiting since the last call
-  // (reads and clears the device flag; synchronises the stream).
+  // Whether a tensor-core contraction gave up waiting (SL3DGPU_ERR_WAIT, once):
+  // in the work of `stream` and before (synchronises it), or in what has ended
+  // so far, which costs a read of host memory.
   int TensorCoreStatus(cudaStream_t stream);
+  int TensorCoreStatus();
+  // The flag those waits set, made on first use.
+  int GiveUpFlag(int** flag);
   int LegendreAnalysisF(int N, bool real, const float* spectra, int P, int p0, int count, float* coeffs,
                         bool accumulate, cudaStream_t stream);
   int RingWeightedF(bool real, const float* spectraIn, int count, const float* weight, float* spectraOut,
@@ -252,7 +256,7 @@ class Grid {
   // The FP32 contraction on the tensor cores (tc_gemm.cu): the spin's table
   // panel (made on first use), B packed, the contraction.
   int RunGemmF(int N, bool real, Batch& b, const float* B, float* C, bool accumulate, cudaStream_t stream);
-  int* dTcError_ = nullptr;  // set by a tensor-core wait that gave up
+  int* giveUp_ = nullptr;  // set by a tensor-core wait that gave up (pinned)
 
  public:
   // The spin's table, with the FP32 twiddles made.
@@ -271,6 +275,7 @@ struct GridAttachment {
   std::shared_ptr<void> workspace;
 };
 GridAttachment& AttachmentOf(sl3dgpu_grid* grid);
+Grid& GridOf(sl3dgpu_grid* grid);
 
 // Smallest 2^a 3^b 5^c at or above n.
 int FftFriendly(int n);

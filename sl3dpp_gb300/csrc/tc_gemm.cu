@@ -283,7 +283,7 @@ __global__ void __launch_bounds__(kPersistentThreads, 1)
   const uint32_t tmem = *tmemSlot;
   auto giveUp = [&] {
     abortFlag = 1;
-    atomicExch(errorFlag, 1);
+    ReportGiveUp(errorFlag);
   };
 
   if (warp == 0 && lane == 0) {
@@ -417,7 +417,7 @@ __global__ void __launch_bounds__(kPersistentThreads, 1)
       asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                        SmemAddr(drain))
                    : "memory");
-      if (!WaitParity(SmemAddr(drain), 0)) atomicExch(errorFlag, 1);
+      if (!WaitParity(SmemAddr(drain), 0)) ReportGiveUp(errorFlag);
     }
   } else if (warp >= 6) {
     // -- B's split and pack, in shared memory: packing warp p takes the

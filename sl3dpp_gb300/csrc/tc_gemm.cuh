@@ -53,6 +53,13 @@ __device__ inline bool WaitParity(uint32_t bar, uint32_t phase) {
   return false;
 }
 
+// The flag of a wait that gave up, in pinned host memory: seen by the host once
+// the kernel has ended.
+__device__ inline void ReportGiveUp(int* flag) {
+  *static_cast<volatile int*>(flag) = 1;
+  __threadfence_system();
+}
+
 constexpr int kTcTileM = 128;  // rows per tile (the MMA's M)
 constexpr int kTcTileK = 16;   // K per tile (two 8-deep MMA slices)
 constexpr int kTcMaxTileN = 256;
@@ -74,7 +81,7 @@ void LaunchPanelA(const GemmItem* items, const TcItem* tcItems, int count, int m
 void LaunchPackB(const TcItem* tcItems, int count, int maxTiles, int tileN, const float* B, float* packed,
                  cudaStream_t stream);
 // The contraction over a tile list ({item, row tile, column tile} per
-// entry), persistent CTAs, one per SM. errorFlag: a device int set non-zero
+// entry), persistent CTAs, one per SM. errorFlag: a pinned host int set non-zero
 // if a completion wait gives up (the launch then leaves C unspecified and
 // the caller reports it).
 // rawB non-null: B is split and packed inside the kernel from its source

@@ -399,7 +399,7 @@ __global__ void __launch_bounds__(kThreads, 2) TcGemm64Kernel(const GemmItem* it
       for (int ks = landed; ks < issued; ++ks)
         WaitParity(SmemAddr(full + ks % kStages), phaseFull[ks % kStages]);
     okShared = ok ? 1 : 0;
-    if (!ok) atomicExch(errorFlag, 1);
+    if (!ok) ReportGiveUp(errorFlag);
   }
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
