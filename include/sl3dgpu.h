@@ -13,6 +13,14 @@
  * at l(l+1)/2 + m (include/sl3dpp/SurfaceGrid.hpp:110-118, 191-200); grid
  * values colatitude-major. Batched device calls keep right-hand sides
  * row-major (dof-major, columns fastest), the layout the kernels coalesce on.
+ *
+ * Threads. Several host threads may call the library, each on its own handles.
+ * The mixed form's correction loop is a CUDA graph where its thread is the only
+ * one inside the library, and the host's loop, with the same results, beside
+ * others: the driver did not bear these graphs' making beside other threads'
+ * calls. A call may wait the moment that another thread makes or launches one.
+ * The library sees its own calls only: where other threads make CUDA calls of
+ * their own meanwhile, SL3DGPU_NO_GRAPHS=1 keeps the loop on the host.
  */
 #ifndef SL3DGPU_H
 #define SL3DGPU_H

@@ -4,6 +4,7 @@
 #include <string>
 #include <utility>
 
+#include "call_gate.cuh"
 #include "common.cuh"
 
 namespace sl3dgpu {
@@ -42,6 +43,7 @@ extern "C" const char* sl3dgpu_last_error(void) { return sl3dgpu::lastError.c_st
 extern "C" const char* sl3dgpu_version(void) { return "sl3dgpu 0.1 (sm_103a)"; }
 
 extern "C" int sl3dgpu_device_alloc(long long bytes, void** out) {
+  const sl3dgpu::LibraryCall inside;
   if (out == nullptr || bytes < 0) {
     sl3dgpu::SetError("device_alloc: an output pointer and bytes >= 0");
     return SL3DGPU_ERR_ARGUMENT;
@@ -53,11 +55,13 @@ extern "C" int sl3dgpu_device_alloc(long long bytes, void** out) {
 }
 
 extern "C" int sl3dgpu_device_free(void* p) {
+  const sl3dgpu::LibraryCall inside;
   if (p != nullptr) SL3D_CUDA(cudaFree(p));
   return SL3DGPU_OK;
 }
 
 extern "C" int sl3dgpu_device_copy(void* dst, const void* src, long long bytes) {
+  const sl3dgpu::LibraryCall inside;
   if (bytes < 0 || (bytes > 0 && (dst == nullptr || src == nullptr))) {
     sl3dgpu::SetError("device_copy: two pointers and bytes >= 0");
     return SL3DGPU_ERR_ARGUMENT;

@@ -29,6 +29,7 @@
 #include <utility>
 #include <vector>
 
+#include "call_gate.cuh"
 #include "common.cuh"
 #include "profile.cuh"
 
@@ -1094,6 +1095,7 @@ struct DeviceScratch {
 }  // namespace
 
 extern "C" int sl3dgpu_band_cholesky_factor(double* ab, int n, int kd) {
+  const LibraryCall inside;
   if (n < 0 || kd < 0) {
     SetError("negative order or bandwidth");
     return SL3DGPU_ERR_ARGUMENT;
@@ -1171,6 +1173,7 @@ int SolveHost(const double* ab, size_t bandSize, const int* pivots, int n, int k
 }  // namespace
 
 extern "C" int sl3dgpu_band_cholesky_solve(const double* ab, int n, int kd, double* b, int nrhs) {
+  const LibraryCall inside;
   if (n < 0 || kd < 0 || nrhs < 0) {
     SetError("negative order, bandwidth or column count");
     return SL3DGPU_ERR_ARGUMENT;
@@ -1179,6 +1182,7 @@ extern "C" int sl3dgpu_band_cholesky_solve(const double* ab, int n, int kd, doub
 }
 
 extern "C" int sl3dgpu_band_lu_factor(double* ab, int n, int kl, int ku, int* pivots) {
+  const LibraryCall inside;
   if (n < 0 || kl < 0 || ku < 0) {
     SetError("negative order or bandwidth");
     return SL3DGPU_ERR_ARGUMENT;
@@ -1212,6 +1216,7 @@ extern "C" int sl3dgpu_band_lu_factor(double* ab, int n, int kl, int ku, int* pi
 
 extern "C" int sl3dgpu_band_lu_solve(const double* ab, int n, int kl, int ku, const int* pivots,
                                      double* b, int nrhs) {
+  const LibraryCall inside;
   if (n < 0 || kl < 0 || ku < 0 || nrhs < 0) {
     SetError("negative order, bandwidth or column count");
     return SL3DGPU_ERR_ARGUMENT;
@@ -1223,6 +1228,7 @@ extern "C" int sl3dgpu_band_factor_batch(const sl3dgpu_band_system* dev_systems,
                                          const sl3dgpu_band_system* host_systems, int count,
                                          double* bands, int* pivots, int* info, int lu,
                                          void* stream) {
+  const LibraryCall inside;
   return BandFactorBatch(dev_systems, host_systems, count, bands, pivots, info, lu,
                          AsStream(stream));
 }
@@ -1232,6 +1238,7 @@ extern "C" int sl3dgpu_band_solve_batch(const sl3dgpu_band_system* dev_systems,
                                         const int* dev_items, int item_count, const double* bands,
                                         const int* pivots, double* rhs, const double* scales,
                                         int lu, void* stream) {
+  const LibraryCall inside;
   return BandSolveBatch(dev_systems, host_systems, count, reinterpret_cast<const int2*>(dev_items),
                         item_count, bands, pivots, rhs, scales, lu, AsStream(stream));
 }
@@ -1241,6 +1248,7 @@ extern "C" int sl3dgpu_band_solve_batch_f32(const sl3dgpu_band_system* dev_syste
                                             const int* dev_items, int item_count, const float* bands,
                                             float* rhs, const float* scales, const int* dev_windows,
                                             int mode, void* stream) {
+  const LibraryCall inside;
   const auto* items = reinterpret_cast<const int2*>(dev_items);
   const auto* windows = reinterpret_cast<const int2*>(dev_windows);
   if (mode == 0)

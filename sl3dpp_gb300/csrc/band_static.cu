@@ -18,6 +18,7 @@
 #include <mutex>
 #include <vector>
 
+#include "call_gate.cuh"
 #include "common.cuh"
 
 namespace sl3dgpu {
@@ -96,6 +97,7 @@ using namespace sl3dgpu;
 
 extern "C" int sl3dgpu_band_cholesky_solve_noalloc(const double* ab, int n, int kd, double* b, int nrhs,
                                                    void* stream) {
+  const LibraryCall inside;
   if (n < 0 || kd < 0 || nrhs < 0) {
     SetError("negative order, bandwidth or column count");
     return SL3DGPU_ERR_ARGUMENT;

@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "assemble.cuh"
+#include "call_gate.cuh"
 #include "common.cuh"
 #include "host/earth.hpp"
 
@@ -71,6 +72,7 @@ int AssembleOne(sl3dgpu_degree& h, bool& positive, std::vector<double>& luBand) 
 
 extern "C" int sl3dgpu_degree_create(const sl3dgpu_layer* layers, int nlayers, int ngll, int l, double eps,
                                      int toroidal, sl3dgpu_degree** out) {
+  const LibraryCall inside;
   if (layers == nullptr || nlayers <= 0 || out == nullptr || ngll < 2 || l < 0 || (toroidal && l < 1) ||
       !(eps > 0.0)) {
     SetError("degree: layers, ngll >= 2, l >= 0 (>= 1 toroidal) and eps > 0");
@@ -136,7 +138,10 @@ extern "C" int sl3dgpu_degree_create(const sl3dgpu_layer* layers, int nlayers, i
   return SL3DGPU_OK;
 }
 
-extern "C" void sl3dgpu_degree_destroy(sl3dgpu_degree* h) { delete h; }
+extern "C" void sl3dgpu_degree_destroy(sl3dgpu_degree* h) {
+  const LibraryCall inside;
+  delete h;
+}
 
 extern "C" int sl3dgpu_degree_dof_count(const sl3dgpu_degree* h) { return h ? h->n : SL3DGPU_ERR_ARGUMENT; }
 
@@ -184,6 +189,7 @@ extern "C" int sl3dgpu_degree_tide(const sl3dgpu_degree* h, int power, double* o
 }
 
 extern "C" int sl3dgpu_degree_band(const sl3dgpu_degree* h, double* out) {
+  const LibraryCall inside;
   if (h == nullptr || out == nullptr) {
     SetError("degree: null argument");
     return SL3DGPU_ERR_ARGUMENT;
@@ -193,6 +199,7 @@ extern "C" int sl3dgpu_degree_band(const sl3dgpu_degree* h, double* out) {
 }
 
 extern "C" int sl3dgpu_degree_apply(const sl3dgpu_degree* h, const double* x, int nrhs, double* y) {
+  const LibraryCall inside;
   if (h == nullptr || x == nullptr || y == nullptr || nrhs < 0) {
     SetError("degree: null argument or negative nrhs");
     return SL3DGPU_ERR_ARGUMENT;
@@ -216,6 +223,7 @@ extern "C" int sl3dgpu_degree_apply(const sl3dgpu_degree* h, const double* x, in
 }
 
 extern "C" int sl3dgpu_degree_solve(const sl3dgpu_degree* h, double* b, int nrhs) {
+  const LibraryCall inside;
   if (h == nullptr || b == nullptr || nrhs < 0) {
     SetError("degree: null argument or negative nrhs");
     return SL3DGPU_ERR_ARGUMENT;

@@ -4,6 +4,7 @@
 #include <mutex>
 #include <vector>
 
+#include "call_gate.cuh"
 #include "common.cuh"
 #include "profile.cuh"
 
@@ -167,5 +168,11 @@ int FmaPeak(double* gflops, int iters) {
 
 }  // namespace
 
-extern "C" int sl3dgpu_fp64_fma_peak(double* gflops) { return FmaPeak<double>(gflops, 4096); }
-extern "C" int sl3dgpu_fp32_fma_peak(double* gflops) { return FmaPeak<float>(gflops, 32768); }
+extern "C" int sl3dgpu_fp64_fma_peak(double* gflops) {
+  const LibraryCall inside;
+  return FmaPeak<double>(gflops, 4096);
+}
+extern "C" int sl3dgpu_fp32_fma_peak(double* gflops) {
+  const LibraryCall inside;
+  return FmaPeak<float>(gflops, 32768);
+}

@@ -55,6 +55,7 @@
 #include <mutex>
 #include <vector>
 
+#include "call_gate.cuh"
 #include "common.cuh"
 #include "profile.cuh"
 #include "sl3dgpu.h"
@@ -1274,6 +1275,7 @@ extern "C" int sl3dgpu_sle_solve(sl3dgpu_grid* grid, const sl3dgpu_sle_body* bod
                                  int anderson_memory, double* sea_level_change, double* displacement,
                                  double* potential, double* tangential_potential, double* toroidal_potential,
                                  sl3dgpu_sle_result* result, void* stream) {
+  const LibraryCall inside;
   return WithGridWorkspace(grid, AsStream(stream), [&](SleWorkspace& ws) {
     return SeaLevelSolve(ws, grid, body, ocean, forcing, rtol, max_iterations, anderson_memory, sea_level_change,
                          displacement, potential, tangential_potential, toroidal_potential, nullptr, result,
@@ -1289,6 +1291,7 @@ extern "C" int sl3dgpu_sle_solve_nonlinear(sl3dgpu_grid* grid, const sl3dgpu_sle
                                            double* toroidal_potential, double* final_sea_level,
                                            double* final_ocean_function, double* load_coefficients,
                                            sl3dgpu_sle_result* result, void* stream) {
+  const LibraryCall inside;
   return WithGridWorkspace(grid, AsStream(stream), [&](SleWorkspace& ws) {
     return SeaLevelSolveNonlinear(ws, grid, body, ice_density, state, forcing, rtol, max_iterations, sea_level_change,
                                   displacement, potential, tangential_potential, toroidal_potential, final_sea_level,
@@ -1299,5 +1302,6 @@ extern "C" int sl3dgpu_sle_solve_nonlinear(sl3dgpu_grid* grid, const sl3dgpu_sle
 extern "C" int sl3dgpu_sle_flotation(long long n, double water_density, double ice_density, const double* ice,
                                      const double* sea_level, const unsigned char* forced_land,
                                      double* ocean_function, void* stream) {
+  const LibraryCall inside;
   return Flotation(n, water_density, ice_density, ice, sea_level, forced_land, ocean_function, AsStream(stream));
 }

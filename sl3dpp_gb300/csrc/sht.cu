@@ -19,6 +19,7 @@
 #include <cstring>
 #include <numeric>
 
+#include "call_gate.cuh"
 #include "profile.cuh"
 #include "ring_df.cuh"
 #include "ring_stages.cuh"
@@ -1568,6 +1569,7 @@ struct sl3dgpu_grid {
 };
 
 extern "C" int sl3dgpu_grid_create(int lmax, int nmax, double oversampling, sl3dgpu_grid** out) {
+  const LibraryCall inside;
   if (out == nullptr) {
     SetError("null output handle");
     return SL3DGPU_ERR_ARGUMENT;
@@ -1578,7 +1580,10 @@ extern "C" int sl3dgpu_grid_create(int lmax, int nmax, double oversampling, sl3d
   return SL3DGPU_OK;
 }
 
-extern "C" void sl3dgpu_grid_destroy(sl3dgpu_grid* grid) { delete grid; }
+extern "C" void sl3dgpu_grid_destroy(sl3dgpu_grid* grid) {
+  const LibraryCall inside;
+  delete grid;
+}
 
 extern "C" int sl3dgpu_grid_lmax(const sl3dgpu_grid* grid) {
   if (grid == nullptr) {
@@ -1599,6 +1604,7 @@ extern "C" int sl3dgpu_grid_shape(const sl3dgpu_grid* grid, int* ntheta, int* np
 }
 
 extern "C" int sl3dgpu_grid_set_fp64_emulation(sl3dgpu_grid* grid, int on) {
+  const LibraryCall inside;
   if (grid == nullptr || (on != 0 && on != 1)) {
     SetError("grid: null handle, or fp64 emulation not 0 or 1");
     return SL3DGPU_ERR_ARGUMENT;
@@ -1702,16 +1708,19 @@ Grid& GridOf(sl3dgpu_grid* grid) { return *grid->grid; }
 
 extern "C" int sl3dgpu_synthesise_spin_batch(sl3dgpu_grid* grid, int N, const double* coeffs,
                                              int count, double* fields, void* stream) {
+  const LibraryCall inside;
   return Synthesise(grid, N, false, coeffs, count, fields, stream);
 }
 
 extern "C" int sl3dgpu_expand_spin_batch(sl3dgpu_grid* grid, int N, const double* fields,
                                          int count, double* coeffs, void* stream) {
+  const LibraryCall inside;
   return Expand(grid, N, false, fields, count, coeffs, stream);
 }
 
 extern "C" int sl3dgpu_legendre_device(sl3dgpu_grid* grid, int N, int real, int analysis, int fp32, const void* in,
                                        int count, void* out, void* stream) {
+  const LibraryCall inside;
   if (grid == nullptr || count < 0 || (real && N != 0)) {
     SetError("legendre: null grid, negative count, or a real field of nonzero spin");
     return SL3DGPU_ERR_ARGUMENT;
@@ -1734,10 +1743,12 @@ extern "C" int sl3dgpu_legendre_device(sl3dgpu_grid* grid, int N, int real, int 
 
 extern "C" int sl3dgpu_synthesise_batch(sl3dgpu_grid* grid, const double* coeffs, int count,
                                         double* fields, void* stream) {
+  const LibraryCall inside;
   return Synthesise(grid, 0, true, coeffs, count, fields, stream);
 }
 
 extern "C" int sl3dgpu_expand_batch(sl3dgpu_grid* grid, const double* fields, int count,
                                     double* coeffs, void* stream) {
+  const LibraryCall inside;
   return Expand(grid, 0, true, fields, count, coeffs, stream);
 }

@@ -30,12 +30,14 @@
 #include <cstring>
 #include <limits>
 #include <memory>
+#include <optional>
 #include <string>
 #include <thread>
 #include <tuple>
 #include <vector>
 
 #include "assemble.cuh"
+#include "call_gate.cuh"
 #include "host/earth.hpp"
 #include "profile.cuh"
 #include "sealevel.cuh"
@@ -184,11 +186,8 @@ class Viscoelastic3DGpu {
   std::vector<CorrectionGraph> correctionGraphs;
   Dev<CorrectionControl> correctionControl;
   bool useGraphs = true;  // SL3DGPU_NO_GRAPHS=1 keeps the loop on the host
-  // Operators driven from several host threads keep the loop on the host:
-  // building these graphs (conditional nodes) beside other threads' launches
-  // crashed in the driver's cudaGraphDestroy now and then, under a lock
-  // around every graph call too; the ensemble is as fast either way.
-  bool manyThreads = false;
+  // Made, launched and destroyed only while no other host thread is in the
+  // library (call_gate.cuh); beside one the loop stays on the host.
   std::vector<long long> CorrectionKey(const Flavour& f) const;
   int CorrectionGraphFor(const Flavour& f, CorrectionGraph** out);
   int CaptureCorrectionBody(const Flavour& f, cudaGraphConditionalHandle handle);
@@ -328,8 +327,7 @@ class Viscoelastic3DGpu {
                    double* objective, sl3dgpu_step_info* infos);
 
   ~Viscoelastic3DGpu() {
-    for (auto& g : correctionGraphs)
-      if (g.exec) cudaGraphExecDestroy(g.exec);
+    for (auto& g : correctionGraphs) RetireGraph(g.exec);
     if (hostResult) cudaFreeHost(hostResult);
     if (hostMix) cudaFreeHost(hostMix);
     if (stream) cudaStreamDestroy(stream);
@@ -2142,7 +2140,7 @@ int Viscoelastic3DGpu::CorrectionGraphFor(const Flavour& f, CorrectionGraph** ou
   if (cudaGraphInstantiate(&exec, graph, 0) != cudaSuccess) return fail(SL3DGPU_ERR_CUDA);
   cudaGraphDestroy(graph);
   if (correctionGraphs.size() >= 4) {
-    cudaGraphExecDestroy(correctionGraphs.front().exec);
+    RetireGraph(correctionGraphs.front().exec);
     correctionGraphs.erase(correctionGraphs.begin());
   }
   correctionGraphs.push_back(CorrectionGraph{key, exec, launches});
@@ -2176,16 +2174,21 @@ int Viscoelastic3DGpu::Correct(const Flavour& f, double tolerance, sl3dgpu_step_
   bool fresh = false;  // the solutions in rhs*32 are the pass of the final e
   bool triedGraph = false;
   CorrectionGraph* graph = nullptr;
+  std::optional<Alone> alone;  // from the graph's making until it is launched
   int iteration = 0;
   for (; iteration < options.max_iterations; ++iteration) {
     // after the first pass (and the warm start's decision) the loop runs on
     // the device, as a CUDA graph, when it can
-    if (iteration >= 1 && !triedGraph && useGraphs && !manyThreads && !prof::TimingOn()) {
+    if (iteration >= 1 && !triedGraph && useGraphs && !prof::TimingOn()) {
       triedGraph = true;
-      if (CorrectionGraphFor(f, &graph) == SL3DGPU_OK) break;
-      graph = nullptr;
-      useGraphs = false;  // the capture was refused: the host loop carries on
-      cudaGetLastError();
+      alone.emplace();
+      if (*alone) {
+        if (CorrectionGraphFor(f, &graph) == SL3DGPU_OK) break;
+        graph = nullptr;
+        useGraphs = false;  // the capture was refused: the host loop carries on
+        cudaGetLastError();
+      }
+      alone.reset();
     }
     SL3D_TRY(Pass32(f, eL.p, eNextL.p));
     ++info.correction_passes;
@@ -2248,6 +2251,7 @@ int Viscoelastic3DGpu::Correct(const Flavour& f, double tolerance, sl3dgpu_step_
     const size_t head = offsetof(CorrectionControl, history);
     SL3D_CUDA(cudaMemcpyAsync(correctionControl.p, &c, head, cudaMemcpyHostToDevice, stream));
     SL3D_CUDA(cudaGraphLaunch(graph->exec, stream));
+    alone.reset();
     SL3D_CUDA(cudaMemcpyAsync(&c, correctionControl.p, sizeof(CorrectionControl), cudaMemcpyDeviceToHost, stream));
     SL3D_CUDA(cudaStreamSynchronize(stream));
     const int passes = c.historyCount;
@@ -3761,6 +3765,7 @@ struct sl3dgpu_v3d_state {
 
 extern "C" int sl3dgpu_v3d_create(const sl3dgpu_layer* layers, int nlayers, const sl3dgpu_v3d_options* options,
                                   sl3dgpu_v3d** out) {
+  const LibraryCall inside;
   if (layers == nullptr || options == nullptr || out == nullptr) {
     SetError("v3d: null argument");
     return SL3DGPU_ERR_ARGUMENT;
@@ -3771,7 +3776,10 @@ extern "C" int sl3dgpu_v3d_create(const sl3dgpu_layer* layers, int nlayers, cons
   return SL3DGPU_OK;
 }
 
-extern "C" void sl3dgpu_v3d_destroy(sl3dgpu_v3d* h) { delete h; }
+extern "C" void sl3dgpu_v3d_destroy(sl3dgpu_v3d* h) {
+  const LibraryCall inside;
+  delete h;
+}
 
 extern "C" int sl3dgpu_v3d_shape(const sl3dgpu_v3d* h, int* nodes, int* ntheta, int* nphi) {
   if (h == nullptr) {
@@ -3844,6 +3852,7 @@ extern "C" int sl3dgpu_v3d_scales(const sl3dgpu_v3d* h, double* length, double* 
 }
 
 extern "C" int sl3dgpu_v3d_set_delta(sl3dgpu_v3d* h, const double* samples, int on_device) {
+  const LibraryCall inside;
   if (h == nullptr || samples == nullptr) {
     SetError("v3d: null argument");
     return SL3DGPU_ERR_ARGUMENT;
@@ -3852,6 +3861,7 @@ extern "C" int sl3dgpu_v3d_set_delta(sl3dgpu_v3d* h, const double* samples, int 
 }
 
 extern "C" int sl3dgpu_v3d_zero_state(sl3dgpu_v3d* h, sl3dgpu_v3d_state** out) {
+  const LibraryCall inside;
   if (h == nullptr || out == nullptr) {
     SetError("v3d: null argument");
     return SL3DGPU_ERR_ARGUMENT;
@@ -3862,10 +3872,14 @@ extern "C" int sl3dgpu_v3d_zero_state(sl3dgpu_v3d* h, sl3dgpu_v3d_state** out) {
   return SL3DGPU_OK;
 }
 
-extern "C" void sl3dgpu_v3d_free_state(sl3dgpu_v3d_state* s) { delete s; }
+extern "C" void sl3dgpu_v3d_free_state(sl3dgpu_v3d_state* s) {
+  const LibraryCall inside;
+  delete s;
+}
 
 extern "C" int sl3dgpu_v3d_step(sl3dgpu_v3d* h, sl3dgpu_v3d_state* state, double dt, int scheme, const double* load0,
                                 const double* load1, sl3dgpu_step_info* info) {
+  const LibraryCall inside;
   if (h == nullptr || state == nullptr) {
     SetError("v3d: null argument");
     return SL3DGPU_ERR_ARGUMENT;
@@ -3875,6 +3889,7 @@ extern "C" int sl3dgpu_v3d_step(sl3dgpu_v3d* h, sl3dgpu_v3d_state* state, double
 
 extern "C" int sl3dgpu_v3d_step_device(sl3dgpu_v3d* h, sl3dgpu_v3d_state* state, double dt, int scheme,
                                        const double* load0, const double* load1, sl3dgpu_step_info* info) {
+  const LibraryCall inside;
   if (h == nullptr || state == nullptr) {
     SetError("v3d: null argument");
     return SL3DGPU_ERR_ARGUMENT;
@@ -3885,6 +3900,7 @@ extern "C" int sl3dgpu_v3d_step_device(sl3dgpu_v3d* h, sl3dgpu_v3d_state* state,
 extern "C" int sl3dgpu_v3d_step_tide(sl3dgpu_v3d* h, sl3dgpu_v3d_state* state, double dt, int scheme,
                                      const double* load0, const double* load1, const double* tide0,
                                      const double* tide1, int on_device, sl3dgpu_step_info* info) {
+  const LibraryCall inside;
   if (h == nullptr || state == nullptr) {
     SetError("v3d: null argument");
     return SL3DGPU_ERR_ARGUMENT;
@@ -3893,6 +3909,7 @@ extern "C" int sl3dgpu_v3d_step_tide(sl3dgpu_v3d* h, sl3dgpu_v3d_state* state, d
 }
 
 extern "C" int sl3dgpu_v3d_set_start(sl3dgpu_v3d* h, const double* coefficients, int on_device) {
+  const LibraryCall inside;
   if (h == nullptr) {
     SetError("v3d: null handle");
     return SL3DGPU_ERR_ARGUMENT;
@@ -3915,6 +3932,7 @@ extern "C" int sl3dgpu_v3d_state_coefficients(const sl3dgpu_v3d* h, const sl3dgp
 
 extern "C" int sl3dgpu_v3d_state_coefficients_copy(const sl3dgpu_v3d* h, const sl3dgpu_v3d_state* state,
                                                    double* device_out) {
+  const LibraryCall inside;
   if (h == nullptr || state == nullptr || device_out == nullptr || !state->st.hasCoeffs) {
     SetError("v3d: null argument or a state without strain coefficients");
     return SL3DGPU_ERR_ARGUMENT;
@@ -3926,6 +3944,7 @@ extern "C" int sl3dgpu_v3d_state_coefficients_copy(const sl3dgpu_v3d* h, const s
 }
 
 extern "C" int sl3dgpu_v3d_state_coefficients_host(const sl3dgpu_v3d* h, const sl3dgpu_v3d_state* state, double* out) {
+  const LibraryCall inside;
   if (h == nullptr || state == nullptr || out == nullptr || !state->st.hasCoeffs) {
     SetError("v3d: null argument or a state without strain coefficients");
     return SL3DGPU_ERR_ARGUMENT;
@@ -3949,6 +3968,7 @@ int NeedStepOperator(const sl3dgpu_v3d* h) {
 
 extern "C" int sl3dgpu_v3d_start_step(sl3dgpu_v3d* h, sl3dgpu_v3d_state* state, double dt, int scheme,
                                       const double* load0) {
+  const LibraryCall inside;
   SL3D_TRY(NeedStepOperator(h));
   if (state == nullptr) {
     SetError("v3d: null state");
@@ -3958,6 +3978,7 @@ extern "C" int sl3dgpu_v3d_start_step(sl3dgpu_v3d* h, sl3dgpu_v3d_state* state, 
 }
 
 extern "C" int sl3dgpu_v3d_step_start_strain(sl3dgpu_v3d* h, double* device_out) {
+  const LibraryCall inside;
   SL3D_TRY(NeedStepOperator(h));
   SL3D_TRY(h->op.OpenCheck());
   if (device_out == nullptr) {
@@ -3972,16 +3993,19 @@ extern "C" int sl3dgpu_v3d_step_start_strain(sl3dgpu_v3d* h, double* device_out)
 }
 
 extern "C" int sl3dgpu_v3d_step_respond(sl3dgpu_v3d* h, const double* strain) {
+  const LibraryCall inside;
   SL3D_TRY(NeedStepOperator(h));
   return h->op.OpenRespond(reinterpret_cast<const double2*>(strain));
 }
 
 extern "C" int sl3dgpu_v3d_step_add_channels(sl3dgpu_v3d* h, const double* load, const double* tide) {
+  const LibraryCall inside;
   SL3D_TRY(NeedStepOperator(h));
   return h->op.OpenChannels(load, tide);
 }
 
 extern "C" int sl3dgpu_v3d_step_strain_of(sl3dgpu_v3d* h, double* device_out) {
+  const LibraryCall inside;
   SL3D_TRY(NeedStepOperator(h));
   SL3D_TRY(h->op.OpenCheck());
   if (device_out == nullptr) {
@@ -3994,6 +4018,7 @@ extern "C" int sl3dgpu_v3d_step_strain_of(sl3dgpu_v3d* h, double* device_out) {
 
 extern "C" int sl3dgpu_v3d_step_converge(sl3dgpu_v3d* h, const double* load, const double* tide,
                                          double* device_strain, sl3dgpu_step_info* info) {
+  const LibraryCall inside;
   SL3D_TRY(NeedStepOperator(h));
   auto& op = h->op;
   SL3D_TRY(op.OpenConverge(load, tide, info));
@@ -4006,6 +4031,7 @@ extern "C" int sl3dgpu_v3d_step_converge(sl3dgpu_v3d* h, const double* load, con
 }
 
 extern "C" int sl3dgpu_v3d_step_forces(sl3dgpu_v3d* h, const double* load, const double* tide, double* out) {
+  const LibraryCall inside;
   SL3D_TRY(NeedStepOperator(h));
   if (out == nullptr) {
     SetError("v3d: null output");
@@ -4015,6 +4041,7 @@ extern "C" int sl3dgpu_v3d_step_forces(sl3dgpu_v3d* h, const double* load, const
 }
 
 extern "C" int sl3dgpu_v3d_step_apply(sl3dgpu_v3d* h, const double* x, double* out) {
+  const LibraryCall inside;
   SL3D_TRY(NeedStepOperator(h));
   if (x == nullptr || out == nullptr || x == out) {
     SetError("v3d: distinct device solutions and output");
@@ -4024,6 +4051,7 @@ extern "C" int sl3dgpu_v3d_step_apply(sl3dgpu_v3d* h, const double* x, double* o
 }
 
 extern "C" int sl3dgpu_v3d_step_solve(sl3dgpu_v3d* h, const double* forces, double* out, sl3dgpu_step_info* info) {
+  const LibraryCall inside;
   SL3D_TRY(NeedStepOperator(h));
   if (forces == nullptr) {
     SetError("v3d: null forces");
@@ -4033,11 +4061,13 @@ extern "C" int sl3dgpu_v3d_step_solve(sl3dgpu_v3d* h, const double* forces, doub
 }
 
 extern "C" int sl3dgpu_v3d_step_finish(sl3dgpu_v3d* h, const double* strain) {
+  const LibraryCall inside;
   SL3D_TRY(NeedStepOperator(h));
   return h->op.OpenFinish(reinterpret_cast<const double2*>(strain));
 }
 
 extern "C" int sl3dgpu_v3d_relative_change(sl3dgpu_v3d* h, const double* next, const double* now, double* out) {
+  const LibraryCall inside;
   SL3D_TRY(NeedStepOperator(h));
   if (next == nullptr || now == nullptr || out == nullptr) {
     SetError("v3d: null argument");
@@ -4076,6 +4106,7 @@ extern "C" int sl3dgpu_v3d_solution_layout(const sl3dgpu_v3d* h, int l, long lon
 
 extern "C" int sl3dgpu_v3d_synthesise_tensor(sl3dgpu_v3d* h, const double* spectral, double* c0, double* c1,
                                              double* r) {
+  const LibraryCall inside;
   SL3D_TRY(NeedStepOperator(h));
   if (spectral == nullptr || c0 == nullptr || c1 == nullptr || r == nullptr) {
     SetError("v3d: null argument");
@@ -4087,6 +4118,7 @@ extern "C" int sl3dgpu_v3d_synthesise_tensor(sl3dgpu_v3d* h, const double* spect
 
 extern "C" int sl3dgpu_v3d_analyse_tensor(sl3dgpu_v3d* h, const double* c0, const double* c1, const double* r,
                                           double* spectral) {
+  const LibraryCall inside;
   SL3D_TRY(NeedStepOperator(h));
   if (spectral == nullptr || c0 == nullptr || c1 == nullptr || r == nullptr) {
     SetError("v3d: null argument");
@@ -4098,6 +4130,7 @@ extern "C" int sl3dgpu_v3d_analyse_tensor(sl3dgpu_v3d* h, const double* c0, cons
 
 extern "C" int sl3dgpu_v3d_degree_forces(sl3dgpu_v3d* h, const double* spectral, double* spheroidal,
                                          double* toroidal) {
+  const LibraryCall inside;
   SL3D_TRY(NeedStepOperator(h));
   if (spectral == nullptr || spheroidal == nullptr || (toroidal == nullptr && h->op.rhsTorComplex > 0)) {
     SetError("v3d: null argument");
@@ -4109,6 +4142,7 @@ extern "C" int sl3dgpu_v3d_degree_forces(sl3dgpu_v3d* h, const double* spectral,
 
 extern "C" int sl3dgpu_v3d_strain_of_solutions(sl3dgpu_v3d* h, const double* spheroidal, const double* toroidal,
                                                double* spectral) {
+  const LibraryCall inside;
   SL3D_TRY(NeedStepOperator(h));
   if (spectral == nullptr || spheroidal == nullptr || (toroidal == nullptr && h->op.rhsTorComplex > 0)) {
     SetError("v3d: null argument");
@@ -4127,6 +4161,7 @@ extern "C" long long sl3dgpu_v3d_state_bytes(const sl3dgpu_v3d* h, const sl3dgpu
 }
 
 extern "C" int sl3dgpu_v3d_state_save(sl3dgpu_v3d* h, const sl3dgpu_v3d_state* state, void* out, long long capacity) {
+  const LibraryCall inside;
   if (h == nullptr || state == nullptr || out == nullptr) {
     SetError("v3d: null argument");
     return SL3DGPU_ERR_ARGUMENT;
@@ -4135,6 +4170,7 @@ extern "C" int sl3dgpu_v3d_state_save(sl3dgpu_v3d* h, const sl3dgpu_v3d_state* s
 }
 
 extern "C" int sl3dgpu_v3d_state_load(sl3dgpu_v3d* h, sl3dgpu_v3d_state* state, const void* in, long long bytes) {
+  const LibraryCall inside;
   if (h == nullptr || state == nullptr || in == nullptr) {
     SetError("v3d: null argument");
     return SL3DGPU_ERR_ARGUMENT;
@@ -4143,6 +4179,7 @@ extern "C" int sl3dgpu_v3d_state_load(sl3dgpu_v3d* h, sl3dgpu_v3d_state* state, 
 }
 
 extern "C" int sl3dgpu_v3d_set_ocean(sl3dgpu_v3d* h, const sl3dgpu_v3d_ocean* ocean) {
+  const LibraryCall inside;
   if (h == nullptr) {
     SetError("v3d: null handle");
     return SL3DGPU_ERR_ARGUMENT;
@@ -4151,6 +4188,7 @@ extern "C" int sl3dgpu_v3d_set_ocean(sl3dgpu_v3d* h, const sl3dgpu_v3d_ocean* oc
 }
 
 extern "C" int sl3dgpu_v3d_ocean_grid(sl3dgpu_v3d* h, int* ntheta, int* nphi, double* theta, double* weights) {
+  const LibraryCall inside;
   if (h == nullptr) {
     SetError("v3d: null handle");
     return SL3DGPU_ERR_ARGUMENT;
@@ -4175,6 +4213,7 @@ extern "C" int sl3dgpu_v3d_ocean_grid(sl3dgpu_v3d* h, int* ntheta, int* nphi, do
 
 extern "C" int sl3dgpu_v3d_step_ocean(sl3dgpu_v3d* h, sl3dgpu_v3d_state* state, double dt, int scheme,
                                       const double* load0, const double* load1, sl3dgpu_step_info* info) {
+  const LibraryCall inside;
   if (h == nullptr || state == nullptr) {
     SetError("v3d: null handle or state");
     return SL3DGPU_ERR_ARGUMENT;
@@ -4185,6 +4224,7 @@ extern "C" int sl3dgpu_v3d_step_ocean(sl3dgpu_v3d* h, sl3dgpu_v3d_state* state, 
 extern "C" int sl3dgpu_v3d_run_ocean(sl3dgpu_v3d* h, sl3dgpu_v3d_state* state, const double* times, int nodes,
                                      int scheme, const double* loads, double* u, double* phi, double* sea_level,
                                      double* angular_velocity, sl3dgpu_step_info* infos) {
+  const LibraryCall inside;
   if (h == nullptr || state == nullptr || times == nullptr || loads == nullptr || nodes < 0) {
     SetError("v3d: null argument or negative node count");
     return SL3DGPU_ERR_ARGUMENT;
@@ -4199,6 +4239,7 @@ extern "C" int sl3dgpu_v3d_run_ocean(sl3dgpu_v3d* h, sl3dgpu_v3d_state* state, c
 extern "C" int sl3dgpu_v3d_step_migrating(sl3dgpu_v3d* h, sl3dgpu_v3d_state* state, double dt, int scheme,
                                           const double* ice0, const double* ice1, const double* load0,
                                           const double* load1, sl3dgpu_step_info* info) {
+  const LibraryCall inside;
   if (h == nullptr || state == nullptr) {
     SetError("v3d: null handle or state");
     return SL3DGPU_ERR_ARGUMENT;
@@ -4210,6 +4251,7 @@ extern "C" int sl3dgpu_v3d_run_migrating(sl3dgpu_v3d* h, sl3dgpu_v3d_state* stat
                                          int scheme, const double* ice, const double* loads, double* u, double* phi,
                                          double* sea_level, double* angular_velocity, double* ocean_functions,
                                          sl3dgpu_step_info* infos) {
+  const LibraryCall inside;
   if (h == nullptr || state == nullptr || times == nullptr || ice == nullptr || nodes < 0) {
     SetError("v3d: null argument or negative node count");
     return SL3DGPU_ERR_ARGUMENT;
@@ -4219,6 +4261,7 @@ extern "C" int sl3dgpu_v3d_run_migrating(sl3dgpu_v3d* h, sl3dgpu_v3d_state* stat
 }
 
 extern "C" int sl3dgpu_v3d_ocean_function(sl3dgpu_v3d* h, double* out) {
+  const LibraryCall inside;
   if (h == nullptr || out == nullptr) {
     SetError("v3d: null handle or output");
     return SL3DGPU_ERR_ARGUMENT;
@@ -4228,6 +4271,7 @@ extern "C" int sl3dgpu_v3d_ocean_function(sl3dgpu_v3d* h, double* out) {
 
 extern "C" int sl3dgpu_v3d_sea_level(sl3dgpu_v3d* h, double* coefficients, double* angular_velocity,
                                      sl3dgpu_sle_result* result) {
+  const LibraryCall inside;
   if (h == nullptr) {
     SetError("v3d: null handle");
     return SL3DGPU_ERR_ARGUMENT;
@@ -4236,6 +4280,7 @@ extern "C" int sl3dgpu_v3d_sea_level(sl3dgpu_v3d* h, double* coefficients, doubl
 }
 
 extern "C" int sl3dgpu_v3d_effective_love(sl3dgpu_v3d* h, int scheme, double dt, double* out) {
+  const LibraryCall inside;
   if (h == nullptr || out == nullptr || scheme < 0 || scheme > 1 || !(dt >= 0.0) || h->op.staticMode) {
     SetError("v3d: effective Love numbers of a one-stage flavour (scheme 0 or 1, dt >= 0) of the step operator");
     return SL3DGPU_ERR_ARGUMENT;
@@ -4248,6 +4293,7 @@ extern "C" int sl3dgpu_v3d_effective_love(sl3dgpu_v3d* h, int scheme, double dt,
 
 extern "C" int sl3dgpu_v3d_run(sl3dgpu_v3d* h, sl3dgpu_v3d_state* state, const double* times, int nodes, int scheme,
                                const double* loads, double* u, double* phi, sl3dgpu_step_info* infos) {
+  const LibraryCall inside;
   if (h == nullptr || state == nullptr || times == nullptr || loads == nullptr || nodes < 0) {
     SetError("v3d: null argument or negative node count");
     return SL3DGPU_ERR_ARGUMENT;
@@ -4259,6 +4305,7 @@ extern "C" int sl3dgpu_v3d_adjoint_run(sl3dgpu_v3d* h, const double* times, int 
                                        const double* loads, const double* u_dual, const double* phi_dual,
                                        double* load_kernels, double* tide_kernels, double* delta_gradient,
                                        double* objective, sl3dgpu_step_info* infos) {
+  const LibraryCall inside;
   if (h == nullptr) {
     SetError("v3d adjoint: null operator");
     return SL3DGPU_ERR_ARGUMENT;
@@ -4271,6 +4318,7 @@ extern "C" int sl3dgpu_v3d_tangent_run(sl3dgpu_v3d* h, const double* times, int 
                                        const double* loads, const double* delta_direction,
                                        const double* load_directions, double* u, double* phi,
                                        sl3dgpu_step_info* infos) {
+  const LibraryCall inside;
   if (h == nullptr) {
     SetError("v3d tangent: null operator");
     return SL3DGPU_ERR_ARGUMENT;
@@ -4279,6 +4327,7 @@ extern "C" int sl3dgpu_v3d_tangent_run(sl3dgpu_v3d* h, const double* times, int 
 }
 
 extern "C" int sl3dgpu_v3d_sample_volumes(const sl3dgpu_v3d* h, double* out) {
+  const LibraryCall inside;
   if (h == nullptr || out == nullptr || h->op.staticMode) {
     SetError("v3d: null argument");
     return SL3DGPU_ERR_ARGUMENT;
@@ -4302,6 +4351,7 @@ extern "C" int sl3dgpu_v3d_run_many(int count, sl3dgpu_v3d* const* ops, sl3dgpu_
                                     const double* const* times, const int* nodes, int scheme,
                                     const double* const* loads, double* const* u, double* const* phi,
                                     sl3dgpu_step_info* const* infos, int threads, int* statuses) {
+  const LibraryCall inside;
   if (count < 0 || (count > 0 && (ops == nullptr || states == nullptr || times == nullptr || nodes == nullptr ||
                                   loads == nullptr || statuses == nullptr))) {
     SetError("v3d: run_many needs the operators, states, times, node counts, loads and statuses");
@@ -4317,8 +4367,7 @@ extern "C" int sl3dgpu_v3d_run_many(int count, sl3dgpu_v3d* const* ops, sl3dgpu_
   SL3D_CUDA(cudaGetDevice(&device));
   const int cores = std::max(1, static_cast<int>(std::thread::hardware_concurrency()));
   const int workers = std::max(1, std::min(count, threads > 0 ? threads : cores));
-  for (int i = 0; i < count; ++i)
-    if (ops[i] != nullptr) ops[i]->op.manyThreads = workers > 1;
+  const SeveralThreads several(workers > 1);  // until every worker is done
   std::vector<std::string> errors(count);
   std::atomic<int> next{0};
   auto work = [&] {
@@ -4334,8 +4383,6 @@ extern "C" int sl3dgpu_v3d_run_many(int count, sl3dgpu_v3d* const* ops, sl3dgpu_
   work();
   for (auto& t : pool) t.join();
   for (int i = 0; i < count; ++i)
-    if (ops[i] != nullptr) ops[i]->op.manyThreads = false;
-  for (int i = 0; i < count; ++i)
     if (statuses[i] != SL3DGPU_OK) {
       SetError("v3d: run " + std::to_string(i) + ": " + errors[i]);
       return statuses[i];
@@ -4345,6 +4392,7 @@ extern "C" int sl3dgpu_v3d_run_many(int count, sl3dgpu_v3d* const* ops, sl3dgpu_
 
 extern "C" int sl3dgpu_v3d_assembled_band(sl3dgpu_v3d* h, int scheme, double dt, int toroidal, int l, double* out,
                                           long long capacity, int* n, int* kd) {
+  const LibraryCall inside;
   if (h == nullptr) {
     SetError("v3d: null operator");
     return SL3DGPU_ERR_ARGUMENT;
@@ -4353,6 +4401,7 @@ extern "C" int sl3dgpu_v3d_assembled_band(sl3dgpu_v3d* h, int scheme, double dt,
 }
 
 extern "C" int sl3dgpu_v3d_inertia_moment(sl3dgpu_v3d* h, double* out) {
+  const LibraryCall inside;
   if (h == nullptr || out == nullptr) {
     SetError("v3d: null argument");
     return SL3DGPU_ERR_ARGUMENT;
@@ -4361,6 +4410,7 @@ extern "C" int sl3dgpu_v3d_inertia_moment(sl3dgpu_v3d* h, double* out) {
 }
 
 extern "C" int sl3dgpu_v3d_surface(sl3dgpu_v3d* h, int component, double* out) {
+  const LibraryCall inside;
   if (h == nullptr || out == nullptr) {
     SetError("v3d: null argument");
     return SL3DGPU_ERR_ARGUMENT;
@@ -4369,6 +4419,7 @@ extern "C" int sl3dgpu_v3d_surface(sl3dgpu_v3d* h, int component, double* out) {
 }
 
 extern "C" int sl3dgpu_v3d_surface_device(sl3dgpu_v3d* h, int component, double* device_out) {
+  const LibraryCall inside;
   if (h == nullptr || device_out == nullptr) {
     SetError("v3d: null argument");
     return SL3DGPU_ERR_ARGUMENT;
@@ -4377,6 +4428,7 @@ extern "C" int sl3dgpu_v3d_surface_device(sl3dgpu_v3d* h, int component, double*
 }
 
 extern "C" int sl3dgpu_v3d_state_strain(sl3dgpu_v3d* h, const sl3dgpu_v3d_state* state, double* out) {
+  const LibraryCall inside;
   if (h == nullptr || state == nullptr || out == nullptr) {
     SetError("v3d: null argument");
     return SL3DGPU_ERR_ARGUMENT;
@@ -4430,6 +4482,7 @@ struct sl3dgpu_ep3d {
 
 extern "C" int sl3dgpu_ep3d_create(const sl3dgpu_layer* layers, int nlayers, const sl3dgpu_ep3d_options* options,
                                    sl3dgpu_ep3d** out) {
+  const LibraryCall inside;
   if (layers == nullptr || options == nullptr || out == nullptr) {
     SetError("ep3d: null layers, options or output");
     return SL3DGPU_ERR_ARGUMENT;
@@ -4451,7 +4504,10 @@ extern "C" int sl3dgpu_ep3d_create(const sl3dgpu_layer* layers, int nlayers, con
   return SL3DGPU_OK;
 }
 
-extern "C" void sl3dgpu_ep3d_destroy(sl3dgpu_ep3d* h) { delete h; }
+extern "C" void sl3dgpu_ep3d_destroy(sl3dgpu_ep3d* h) {
+  const LibraryCall inside;
+  delete h;
+}
 
 extern "C" int sl3dgpu_ep3d_shape(const sl3dgpu_ep3d* h, int* nodes, int* ntheta, int* nphi) {
   if (h == nullptr) {
@@ -4501,6 +4557,7 @@ extern "C" int sl3dgpu_ep3d_scales(const sl3dgpu_ep3d* h, double* length, double
 }
 
 extern "C" int sl3dgpu_ep3d_set_moduli(sl3dgpu_ep3d* h, const double* d_mu, const double* d_kappa, int on_device) {
+  const LibraryCall inside;
   if (h == nullptr) {
     SetError("ep3d: null handle");
     return SL3DGPU_ERR_ARGUMENT;
@@ -4509,6 +4566,7 @@ extern "C" int sl3dgpu_ep3d_set_moduli(sl3dgpu_ep3d* h, const double* d_mu, cons
 }
 
 extern "C" int sl3dgpu_ep3d_solve_load(sl3dgpu_ep3d* h, const double* load) {
+  const LibraryCall inside;
   if (h == nullptr || load == nullptr) {
     SetError("ep3d: null handle or load");
     return SL3DGPU_ERR_ARGUMENT;
@@ -4517,6 +4575,7 @@ extern "C" int sl3dgpu_ep3d_solve_load(sl3dgpu_ep3d* h, const double* load) {
 }
 
 extern "C" int sl3dgpu_ep3d_respond(sl3dgpu_ep3d* h) {
+  const LibraryCall inside;
   if (h == nullptr) {
     SetError("ep3d: null handle");
     return SL3DGPU_ERR_ARGUMENT;
@@ -4535,6 +4594,7 @@ extern "C" int sl3dgpu_ep3d_layout(const sl3dgpu_ep3d* h, long long* spheroidal,
 }
 
 extern "C" int sl3dgpu_ep3d_force(sl3dgpu_ep3d* h, const double* x, double* out) {
+  const LibraryCall inside;
   if (h == nullptr || x == nullptr || out == nullptr || x == out) {
     SetError("ep3d: a handle and distinct device solutions and output");
     return SL3DGPU_ERR_ARGUMENT;
@@ -4543,6 +4603,7 @@ extern "C" int sl3dgpu_ep3d_force(sl3dgpu_ep3d* h, const double* x, double* out)
 }
 
 extern "C" int sl3dgpu_ep3d_apply(sl3dgpu_ep3d* h, const double* x, double* out) {
+  const LibraryCall inside;
   if (h == nullptr || x == nullptr || out == nullptr || x == out) {
     SetError("ep3d: a handle and distinct device solutions and output");
     return SL3DGPU_ERR_ARGUMENT;
@@ -4551,6 +4612,7 @@ extern "C" int sl3dgpu_ep3d_apply(sl3dgpu_ep3d* h, const double* x, double* out)
 }
 
 extern "C" int sl3dgpu_ep3d_load_forces(sl3dgpu_ep3d* h, const double* load, double* out) {
+  const LibraryCall inside;
   if (h == nullptr || load == nullptr || out == nullptr) {
     SetError("ep3d: null argument");
     return SL3DGPU_ERR_ARGUMENT;
@@ -4559,6 +4621,7 @@ extern "C" int sl3dgpu_ep3d_load_forces(sl3dgpu_ep3d* h, const double* load, dou
 }
 
 extern "C" int sl3dgpu_ep3d_solution(sl3dgpu_ep3d* h, double* out) {
+  const LibraryCall inside;
   if (h == nullptr || out == nullptr) {
     SetError("ep3d: null argument");
     return SL3DGPU_ERR_ARGUMENT;
@@ -4568,6 +4631,7 @@ extern "C" int sl3dgpu_ep3d_solution(sl3dgpu_ep3d* h, double* out) {
 
 extern "C" int sl3dgpu_ep3d_solve_lateral(sl3dgpu_ep3d* h, const double* load, double rtol, int max_iterations,
                                           sl3dgpu_step_info* info) {
+  const LibraryCall inside;
   if (h == nullptr || load == nullptr || !(rtol > 0.0) || max_iterations < 0) {
     SetError("ep3d: null handle or load, rtol > 0, max_iterations >= 0");
     return SL3DGPU_ERR_ARGUMENT;
@@ -4576,6 +4640,7 @@ extern "C" int sl3dgpu_ep3d_solve_lateral(sl3dgpu_ep3d* h, const double* load, d
 }
 
 extern "C" int sl3dgpu_ep3d_surface(sl3dgpu_ep3d* h, int component, double* out) {
+  const LibraryCall inside;
   if (h == nullptr || out == nullptr) {
     SetError("ep3d: null handle or output");
     return SL3DGPU_ERR_ARGUMENT;

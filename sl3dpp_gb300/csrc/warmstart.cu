@@ -38,6 +38,7 @@
 #include <random>
 #include <vector>
 
+#include "call_gate.cuh"
 #include "profile.cuh"
 #include "systems.cuh"
 #include "tc_gemm.cuh"
@@ -672,6 +673,7 @@ int BatchGradient(sl3dgpu_wsnet& n, int pairs, const float2* const* d2, const fl
 }  // namespace
 
 extern "C" int sl3dgpu_wsnet_create(int hidden, int depth, unsigned long long seed, sl3dgpu_wsnet** out) {
+  const LibraryCall inside;
   if (out == nullptr || hidden < 16 || hidden % 16 != 0 || depth < 1 || depth > 16) {
     SetError("wsnet: hidden a multiple of 16 (>= 16), 1..16 hidden layers");
     return SL3DGPU_ERR_ARGUMENT;
@@ -708,6 +710,7 @@ extern "C" int sl3dgpu_wsnet_create(int hidden, int depth, unsigned long long se
 }
 
 extern "C" void sl3dgpu_wsnet_destroy(sl3dgpu_wsnet* n) {
+  const LibraryCall inside;
   if (n == nullptr) return;
   if (n->stream) cudaStreamDestroy(n->stream);
   delete n;
@@ -716,6 +719,7 @@ extern "C" void sl3dgpu_wsnet_destroy(sl3dgpu_wsnet* n) {
 extern "C" long long sl3dgpu_wsnet_parameter_count(const sl3dgpu_wsnet* n) { return n ? n->count : -1; }
 
 extern "C" int sl3dgpu_wsnet_parameters(const sl3dgpu_wsnet* n, float* out) {
+  const LibraryCall inside;
   if (n == nullptr || out == nullptr) {
     SetError("wsnet: null argument");
     return SL3DGPU_ERR_ARGUMENT;
@@ -726,6 +730,7 @@ extern "C" int sl3dgpu_wsnet_parameters(const sl3dgpu_wsnet* n, float* out) {
 }
 
 extern "C" int sl3dgpu_wsnet_set_parameters(sl3dgpu_wsnet* n, const float* in) {
+  const LibraryCall inside;
   if (n == nullptr || in == nullptr) {
     SetError("wsnet: null argument");
     return SL3DGPU_ERR_ARGUMENT;
@@ -737,6 +742,7 @@ extern "C" int sl3dgpu_wsnet_set_parameters(sl3dgpu_wsnet* n, const float* in) {
 
 extern "C" int sl3dgpu_wsnet_bind(sl3dgpu_wsnet* n, int lmax, int lateral, const double* depth,
                                   const double* relax) {
+  const LibraryCall inside;
   if (n == nullptr || lmax < 2 || lateral < 1 || depth == nullptr || relax == nullptr) {
     SetError("wsnet: lmax >= 2, lateral nodes >= 1, depth and relaxation per lateral node");
     return SL3DGPU_ERR_ARGUMENT;
@@ -778,6 +784,7 @@ extern "C" int sl3dgpu_wsnet_bind(sl3dgpu_wsnet* n, int lmax, int lateral, const
 extern "C" int sl3dgpu_wsnet_gradient(sl3dgpu_wsnet* n, int pairs, const void* const* d2, const void* const* d1,
                                       const void* const* d0, const void* const* target, const float* ratio,
                                       const float* norm, float* grad, float* loss) {
+  const LibraryCall inside;
   if (n == nullptr || pairs < 1 || loss == nullptr) {
     SetError("wsnet: null network, no pairs or no loss");
     return SL3DGPU_ERR_ARGUMENT;
@@ -795,6 +802,7 @@ extern "C" int sl3dgpu_wsnet_gradient(sl3dgpu_wsnet* n, int pairs, const void* c
 extern "C" int sl3dgpu_wsnet_train_step(sl3dgpu_wsnet* n, int pairs, const void* const* d2, const void* const* d1,
                                         const void* const* d0, const void* const* target, const float* ratio,
                                         const float* norm, float lr, float* loss) {
+  const LibraryCall inside;
   SL3D_TRY(sl3dgpu_wsnet_gradient(n, pairs, d2, d1, d0, target, ratio, norm, nullptr, loss));
   ++n->step;
   const float b1 = 0.9f, b2 = 0.999f;
@@ -808,6 +816,7 @@ extern "C" int sl3dgpu_wsnet_train_step(sl3dgpu_wsnet* n, int pairs, const void*
 extern "C" int sl3dgpu_wsnet_predict(sl3dgpu_wsnet* n, int P, int lateral_first, const double* s_n,
                                      const double* s_nm1, const double* s_nm2, const double* s_nm3, double ratio,
                                      double* guess, void* stream) {
+  const LibraryCall inside;
   if (n == nullptr || n->L < 0 || s_n == nullptr || s_nm1 == nullptr || s_nm2 == nullptr || s_nm3 == nullptr ||
       guess == nullptr || lateral_first < 0 || lateral_first + n->lateral > P) {
     SetError("wsnet: a bound network, four snapshots, a guess buffer and the lateral range inside the nodes");
@@ -842,6 +851,7 @@ extern "C" int sl3dgpu_wsnet_predict(sl3dgpu_wsnet* n, int P, int lateral_first,
 // The network's products alone, for checking: C = A B^T for FP32 row-major
 // A (M x K) and B (N x K) on the tensor cores in BF16 (device pointers).
 extern "C" int sl3dgpu_wsnet_gemm(sl3dgpu_wsnet* n, const float* A, const float* B, int M, int N, int K, float* C) {
+  const LibraryCall inside;
   if (n == nullptr || A == nullptr || B == nullptr || C == nullptr || M < 0 || N < 0 || K < 1) {
     SetError("wsnet: null argument or negative size");
     return SL3DGPU_ERR_ARGUMENT;
