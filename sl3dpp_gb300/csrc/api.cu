@@ -15,14 +15,28 @@ thread_local std::string lastError;
 
 void SetError(const std::string& text) { lastError = text; }
 
+unsigned long long ContextId() {
+  using GetId = int (*)(void* context, unsigned long long* id);
+  static const GetId get = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult found{};
+    if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &f, 12000, cudaEnableDefault, &found) != cudaSuccess ||
+        found != cudaDriverEntryPointSuccess)
+      f = nullptr;
+    return reinterpret_cast<GetId>(f);
+  }();
+  unsigned long long id = 0;
+  return get != nullptr && get(nullptr, &id) == 0 ? id : 0;
+}
+
 cudaError_t AllowDynamicSmemOnce(const void* kernel) {
   static std::mutex lock;
-  static std::set<std::pair<int, const void*>> done;  // (device, kernel)
-  int device = 0;
-  if (const cudaError_t e = cudaGetDevice(&device); e != cudaSuccess) return e;
+  static std::set<std::pair<unsigned long long, const void*>> done;  // (context, kernel)
+  const unsigned long long context = ContextId();
   std::lock_guard<std::mutex> guard(lock);
-  if (done.count({device, kernel}) != 0) return cudaSuccess;
-  int optin = 0;
+  if (context != 0 && done.count({context, kernel}) != 0) return cudaSuccess;
+  int device = 0, optin = 0;
+  if (const cudaError_t e = cudaGetDevice(&device); e != cudaSuccess) return e;
   if (const cudaError_t e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
       e != cudaSuccess)
     return e;
@@ -32,7 +46,7 @@ cudaError_t AllowDynamicSmemOnce(const void* kernel) {
                                                  optin - static_cast<int>(a.sharedSizeBytes));
       e != cudaSuccess)
     return e;
-  done.insert({device, kernel});
+  if (context != 0) done.insert({context, kernel});
   return cudaSuccess;
 }
 

@@ -15,8 +15,8 @@
 // reads, so nothing needs clearing, and it keeps the last call's contents.
 // Calls that overlap on the GPU (on different streams, or from different
 // host threads) race on it and must be serialised by the caller.
+#include <map>
 #include <mutex>
-#include <vector>
 
 #include "call_gate.cuh"
 #include "common.cuh"
@@ -37,23 +37,23 @@ constexpr int kSolveColumns = 64;  // right-hand sides per work item of the batc
 
 static __device__ __align__(256) double gSolveScratch[kStaticDoubles];
 
-// The scratch's device address, found once per device (with that device
+// The scratch's device address, found once per context (with its device
 // current) by cudaGetSymbolAddress: in host code the array's name is only a
 // host-side stand-in, not a device address.
 std::mutex gAddressLock;
-std::vector<double*> gAddress;
+std::map<unsigned long long, double*> gAddress;
 
 int ScratchAddress(double** out) {
-  int device = 0;
-  SL3D_CUDA(cudaGetDevice(&device));
+  const unsigned long long context = ContextId();
   std::lock_guard<std::mutex> guard(gAddressLock);
-  if (static_cast<int>(gAddress.size()) <= device) gAddress.resize(device + 1, nullptr);
-  if (gAddress[device] == nullptr) {
-    void* ptr = nullptr;
-    SL3D_CUDA(cudaGetSymbolAddress(&ptr, gSolveScratch));
-    gAddress[device] = static_cast<double*>(ptr);
+  if (const auto found = gAddress.find(context); context != 0 && found != gAddress.end()) {
+    *out = found->second;
+    return SL3DGPU_OK;
   }
-  *out = gAddress[device];
+  void* ptr = nullptr;
+  SL3D_CUDA(cudaGetSymbolAddress(&ptr, gSolveScratch));
+  *out = static_cast<double*>(ptr);
+  if (context != 0) gAddress[context] = *out;
   return SL3DGPU_OK;
 }
 

@@ -56,12 +56,17 @@ inline cudaError_t ZeroIn(void* dst, size_t bytes) {
   return cudaStreamSynchronize(cudaStreamLegacy);
 }
 
+// The current context's id, new after a cudaDeviceReset: what the library keeps
+// of a context (kernel attributes, addresses of its device arrays) goes by it. 0
+// when the thread has no context yet; such a thing is then made again.
+unsigned long long ContextId();
+
 // Allow a kernel all the dynamic shared memory the device's opt-in limit
 // leaves beside its static shared memory. The attribute is global to the
 // function, so it takes one value for every caller: host threads driving
 // problems of different sizes would otherwise race between setting it and
 // launching. Occupancy follows each launch's actual dynamic size. Set once a
-// kernel and device: setting it at every launch cost two runtime calls each.
+// kernel and context: setting it at every launch cost two runtime calls each.
 cudaError_t AllowDynamicSmemOnce(const void* kernel);
 template <class F>
 inline cudaError_t AllowDynamicSmem(F* kernel) {
