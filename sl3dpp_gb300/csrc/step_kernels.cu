@@ -9,6 +9,7 @@
 #include <cmath>
 #include <type_traits>
 
+#include "divide.cuh"
 #include "host/lstsq.hpp"
 #include "profile.cuh"
 #include "step_kernels.cuh"
@@ -93,25 +94,6 @@ __device__ inline const double* Radii<double>(const Geometry& g) {
 template <>
 __device__ inline const float* Radii<float>(const Geometry& g) {
   return g.radii32;
-}
-
-// x / d rounded to nearest from d's rounded reciprocal y: a quotient and its
-// exact remainder, whose share corrects it (Markstein's division). A division
-// proper costs about ten instructions, six a point in the strain; FP64 ones
-// are 19 cycles an SM each. In FP64 one correction leaves the rounding wrong
-// for one value in 2^52; in FP32, where that would be one in 2^23, a second
-// leaves none. Zeros, subnormals and non-finite values as x y.
-__device__ inline double DivideBy(double x, double d, double y) {
-  const double q = x * y;
-  const uint32_t e = (static_cast<uint32_t>(__double2hiint(q)) >> 20) & 0x7FFu;
-  return e - 1u >= 0x7FEu ? q : fma(fma(-q, d, x), y, q);
-}
-__device__ inline float DivideBy(float x, float d, float y) {
-  float q = x * y;
-  const uint32_t e = (__float_as_uint(q) >> 23) & 0xFFu;
-  if (e - 1u >= 0xFEu) return q;
-  q = fmaf(fmaf(-q, d, x), y, q);
-  return fmaf(fmaf(-q, d, x), y, q);
 }
 
 template <class T2>
