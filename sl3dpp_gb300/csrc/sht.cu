@@ -1009,7 +1009,6 @@ int Grid::BatchFor(int N, bool real, bool analysis, int P, int p0, int count, co
     b.rowExps += g.M;
     b.colExps += g.N;
     b.maxNTiles64 = std::max(b.maxNTiles64, e.nTiles);
-    b.maxBTiles64 = std::max(b.maxBTiles64, e.nTiles * e.kSteps);
     b.tc64Host.push_back(e);
   }
   *out = &batches_.emplace(key, b).first->second;
@@ -1164,9 +1163,6 @@ int Grid::LegendreAnalysis(int N, bool real, const double* spectra, int P, int p
 }
 
 namespace {
-int LaunchRingWeightedF(Grid& g, int parts, bool real, const float* spectraIn, int count, const float* weight,
-                        float* spectraOut, cudaStream_t stream);
-
 // The most fields that count as a small batch (the FP64 units' rings).
 constexpr int kSmallBatch = 8;
 
@@ -1320,7 +1316,27 @@ int Grid::LegendreAnalysis3F(const float* spectra, int count, float* coeffs, cud
 
 int Grid::RingWeighted3F(const float* spectraIn, int count, const float* weight, float* spectraOut,
                          cudaStream_t stream) {
-  return LaunchRingWeightedF(*this, 3, false, spectraIn, count, weight, spectraOut, stream);
+  if (count == 0) return SL3DGPU_OK;
+  const SpinTable* t = nullptr;
+  if (int st = Table32(0, &t); st != SL3DGPU_OK) return st;  // makes the FP32 twiddles
+  int buffers = 2;
+  const RingFn<float2> kernel = RingKernelFor<float2>(nphi, &buffers);
+  const int rings = RingsPerCta<float2>(nphi, buffers);
+  SL3D_CUDA(AllowDynamicSmem(kernel));
+  RingParts p;  // real fields go two to a ring
+  p.blocks = (count + rings - 1) / rings;
+  p.stride = TripleStride(count);
+  const int blocks = 2 * p.blocks + (count + 2 * rings - 1) / (2 * rings);
+  // a real field's transform counts half a complex one
+  const double bytes = 2.0 * (2 * (2 * lmax + 1) + lmax + 1) * ntheta * count * 8.0 +
+                       3.0 * ntheta * nphi * count * 4.0;
+  const double flops = 5.0 * ntheta * count * 5.0 * nphi * std::log2(static_cast<double>(nphi));
+  prof::Scope scope(prof::kRing32, stream, flops, bytes);
+  kernel<<<dim3(blocks, ntheta), rings * kWarp, RingSmem<float2>(nphi, rings, buffers), stream>>>(
+      kRingWeighted, lmax, ntheta, count, false, plan, dTwiddle32, dWeights,
+      reinterpret_cast<const float2*>(spectraIn), nullptr, weight, nullptr, reinterpret_cast<float2*>(spectraOut), p);
+  SL3D_CHECK_LAUNCH();
+  return SL3DGPU_OK;
 }
 
 int Grid::RingSynthesis(bool real, const double* spectra, int count, double* fields,
@@ -1459,47 +1475,6 @@ int Grid::LegendreAnalysisF(int N, bool real, const float* spectra, int P, int p
   if (b == nullptr) return SL3DGPU_ERR_CUDA;
   return RunGemmF(N, real, *b, spectra, coeffs, accumulate, stream);
 }
-
-int Grid::RingWeightedF(bool real, const float* spectraIn, int count, const float* weight, float* spectraOut,
-                        cudaStream_t stream) {
-  return LaunchRingWeightedF(*this, 1, real, spectraIn, count, weight, spectraOut, stream);
-}
-
-namespace {
-// The FP32 weighted rings of one batch, or (parts 3) of a tensor's components.
-int LaunchRingWeightedF(Grid& g, int parts, bool real, const float* spectraIn, int count, const float* weight,
-                        float* spectraOut, cudaStream_t stream) {
-  if (count == 0) return SL3DGPU_OK;
-  const SpinTable* t = nullptr;
-  if (int st = g.Table32(0, &t); st != SL3DGPU_OK) return st;  // makes the FP32 twiddles
-  int buffers = 2;
-  const RingFn<float2> kernel = RingKernelFor<float2>(g.nphi, &buffers);
-  const int rings = RingsPerCta<float2>(g.nphi, buffers);
-  const size_t smem = RingSmem<float2>(g.nphi, rings, buffers);
-  SL3D_CUDA(AllowDynamicSmem(kernel));
-  auto blocks = [&](bool re) { return (count + (re ? 2 * rings : rings) - 1) / (re ? 2 * rings : rings); };
-  RingParts p{};
-  int x = blocks(real);
-  if (parts == 3) {
-    p.blocks = blocks(false);
-    p.stride = g.TripleStride(count);
-    x = 2 * p.blocks + blocks(true);
-  }
-  double flops = 0.0, bytes = 0.0;
-  for (int c = 0; c < parts; ++c) {
-    const bool re = parts == 3 ? c == 2 : real;
-    bytes += 2.0 * (re ? g.lmax + 1 : 2 * g.lmax + 1) * g.ntheta * count * 8.0 +
-             static_cast<double>(g.ntheta) * g.nphi * count * 4.0;
-    flops += (re ? 1.0 : 2.0) * g.ntheta * count * 5.0 * g.nphi * std::log2(static_cast<double>(g.nphi));
-  }
-  prof::Scope scope(prof::kRing32, stream, flops, bytes);
-  kernel<<<dim3(x, g.ntheta), rings * kWarp, smem, stream>>>(
-      kRingWeighted, g.lmax, g.ntheta, count, real, g.plan, g.dTwiddle32, g.dWeights,
-      reinterpret_cast<const float2*>(spectraIn), nullptr, weight, nullptr, reinterpret_cast<float2*>(spectraOut), p);
-  SL3D_CHECK_LAUNCH();
-  return SL3DGPU_OK;
-}
-}  // namespace
 
 namespace {
 dim3 PermuteGrid(long long rows, int count) {

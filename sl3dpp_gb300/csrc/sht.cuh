@@ -155,8 +155,6 @@ class Grid {
   int GiveUpFlag(int** flag);
   int LegendreAnalysisF(int N, bool real, const float* spectra, int P, int p0, int count, float* coeffs,
                         bool accumulate, cudaStream_t stream);
-  int RingWeightedF(bool real, const float* spectraIn, int count, const float* weight, float* spectraOut,
-                    cudaStream_t stream);
 
   // The same for a tensor's three components at once, spins -2 and -1 and the
   // real spin 0, in one launch each where the one-component calls would take
@@ -225,7 +223,7 @@ class Grid {
     // the FP64 slices' form: items (made on first use) and extents
     std::vector<Tc64Item> tc64Host;
     Tc64Item* tc64Items = nullptr;
-    int maxNTiles64 = 0, maxBTiles64 = 0;
+    int maxNTiles64 = 0;
     long long panel64 = 0, packed64 = 0;  // tiles of the panel and of the packed B
     long long rowExps = 0, colExps = 0;
   };
