@@ -73,7 +73,7 @@ def _rescale(lmax):
     LDELTA = max(2, lmax // 4)
 
 
-def workload_config(precision="mixed"):
+def workload_config(precision="mixed", cpu=False):
     return {"workload": f"3d_step_lmax{LMAX}_{precision}_sdirk2", "lmax": LMAX, "elements": ELEMENTS,
             "order": NGLL - 1, "delta_degree": LDELTA, "delta_rms": DELTA_RMS, "delta_seed": DELTA_SEED,
             "rheology": "maxwell", "cap_degrees": CAP_DEGREES, "cap_thickness_m": CAP_THICKNESS,
@@ -84,13 +84,17 @@ def workload_config(precision="mixed"):
             "warm_start": ("the previous step's strain, and the extrapolation 2 s_n - s_{n-1} of the last two "
                            "steps as the FP32 correction's start" if precision == "mixed" else
                            "the previous step's strain coefficients (the reference's plain warm start)"),
-            "fp64_contractions": ("the FP64 passes' Legendre contractions emulated on the tensor cores: 7 BF16 "
-                                  "slices a value under power-of-two row/column scales, exact FP32 slice products, "
-                                  "levels joined in FP64 (about 49 bits)" if precision == "mixed" else
-                                  "8 BF16 slices a value on the tensor cores (56 bits, the FP64 units' accuracy)"),
-            "fp64_ring_transforms": ("the FP64 passes' ring FFTs in double-float on the FP32 pipe (hi + lo FP32 "
-                                     "pairs, about 48 bits)" if precision == "mixed" else
-                                     "64-bit block fixed point (the FP64 transform's accuracy)"),
+            "fp64_contractions": {
+                "mixed": "the FP64 passes' Legendre contractions on the tensor cores: 7 BF16 slices a value under "
+                         "power-of-two row/column scales, exact FP32 slice products, levels joined exactly (about "
+                         "49 bits)",
+                "fp64": "8 BF16 slices a value on the tensor cores (56 bits below its row's and column's largest)",
+                "cpu": "FP64 sums on the host's cores"}["cpu" if cpu else precision],
+            "fp64_ring_transforms": {
+                "mixed": "the FP64 passes' ring FFTs in double-float on the FP32 pipe (hi + lo FP32 pairs, about 48 "
+                         "bits)",
+                "fp64": "64-bit block fixed point (the FP64 transform's accuracy)",
+                "cpu": "FP64 on the host's cores"}["cpu" if cpu else precision],
             "l2": "working set far above L2 (memory tensors ~3.3 GB per array)",
             "parallelism": "replicas (one independent operator per GPU)"}
 
@@ -180,24 +184,6 @@ def measured_peaks():
     if path.exists():
         return json.loads(path.read_text()), "measured"
     return {"hbm_gbs": 6800.0, "bf16_tflops": 1900.0, "bf16_tflops_sustained": 1700.0}, "fallback"
-
-
-# The committed ncu summary holding a kernel kind's DRAM bytes per launch.
-TRAFFIC_PROFILES = {"ring_fft": "ring_fft_df_3d_step_lmax256.md", "legendre_f32": "tcgemm_3d_step_lmax256_traffic.md"}
-
-
-def ncu_traffic(kernel: str):
-    """DRAM bytes per launch from the committed ncu summary of a kernel, if any."""
-    path = ROOT / "profiles" / TRAFFIC_PROFILES.get(kernel, f"{kernel}.md")
-    if not path.exists():
-        return None
-    for line in path.read_text().splitlines():
-        if line.strip().startswith("traffic_bytes_per_launch:"):
-            try:
-                return float(line.split(":", 1)[1].split()[0])
-            except ValueError:
-                return None
-    return None
 
 
 def build_operator(device, precision, emulation=None):
@@ -346,13 +332,15 @@ def gpu_arm(args, rank, world, device, precision, emulation=None, e2e=True, prof
 def roofline(prof, fp64_gflops, fp32_gflops, double_float_rings=False):
     """The dominant kernel kind against the bound of its work: the FP64
     Legendre GEMM, the FP64 ring FFTs and band solves against the FP64 FMA throughput
-    measured live, the emulated FP64 contraction against the measured BF16
-    tensor rate (algorithmic FP64 flops), the rest -- the 3xTF32 contraction
-    streaming its table panels included -- against the measured HBM copy
-    bandwidth with their algorithmic bytes. Under FP64 emulation the FP64
-    rings' transforms run in double-float on the FP32 pipe: their nominal
-    FFT flops are then FP64-equivalent work, still set against the FP64
-    FMA rate they replace (a fraction above 1 is possible), and said so."""
+    measured live, the sliced FP64 contraction against the measured BF16
+    tensor rate (algorithmic FP64 flops), the rest -- the 3xTF32 contraction,
+    with its table's two parts, its operand and its result counted once each,
+    included -- against the measured HBM copy bandwidth with their algorithmic
+    bytes. The FP64 rings' transforms run on other pipes, in double-float under
+    the emulation and in 64-bit integers without: their nominal FFT flops are
+    FP64-equivalent work, set against the FP64 FMA rate that they replace (a
+    fraction above 1 is possible), and said so. traffic is null: the forms of
+    the kernels under profiles/ are earlier ones."""
     kind = max(prof, key=lambda k: prof[k]["ms"])
     p = prof[kind]
     peaks, source = measured_peaks()
@@ -364,19 +352,20 @@ def roofline(prof, fp64_gflops, fp32_gflops, double_float_rings=False):
     if p["flops"] > 0 and kind in flops_bound:
         bound, peak = flops_bound[kind]
         achieved = p["flops"] / max(p["launches"], 1) / per_launch_s / 1e12
-        peak_source = (source + " (dense BF16; the 28 slice products a step are not counted)" if bound == "tensor"
-                       else "FP64 FMA throughput measured live by sl3dgpu_fp64_fma_peak (CUDA-core arithmetic: "
+        peak_source = (source + " (dense BF16; the slice products, 28 or 36 a step, are not counted)"
+                       if bound == "tensor" else "FP64 FMA throughput measured live by sl3dgpu_fp64_fma_peak (CUDA-core arithmetic: "
                             "MEASURED_PEAKS.json holds HBM and bf16 tensor figures only)")
-        if kind == "ring_fft" and double_float_rings:
+        if kind == "ring_fft":
             bound = "fp64-equivalent"
-            peak_source += ("; the transforms run in double-float on the FP32 pipe, their nominal 5 n log2 n FP64 "
-                            "flops set against the FP64 rate they replace")
+            peak_source += ("; the transforms run " + ("in double-float on the FP32 pipe" if double_float_rings else
+                                                       "in 64-bit integers") +
+                            ", their nominal 5 n log2 n FP64 flops set against the FP64 rate they replace")
         return {"kernel": kind, "bound": bound, "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
-                "frac": achieved / peak, "traffic": ncu_traffic(kind), "peak_source": peak_source,
+                "frac": achieved / peak, "traffic": None, "peak_source": peak_source,
                 "share_of_timed": share}
     achieved = p["bytes"] / max(p["launches"], 1) / per_launch_s / 1e9
     return {"kernel": kind, "bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
-            "frac": achieved / peaks["hbm_gbs"], "traffic": ncu_traffic(kind), "peak_source": source,
+            "frac": achieved / peaks["hbm_gbs"], "traffic": None, "peak_source": source,
             "share_of_timed": share}
 
 
@@ -850,7 +839,7 @@ def main():
         line = {"metric": METRIC, "value": value, "unit": "steps/s", "n_gpus": 0,
                 "steps": args.steps, "warmup": args.warmup, "ms_per_step": 1e3 / value,
                 "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f64",
-                "data": "synthetic", "config": workload_config("fp64"), "impl": "reference",
+                "data": "synthetic", "config": workload_config("fp64", cpu=True), "impl": "reference",
                 "extrapolated": True,
                 "timed_seconds": r["start_seconds"] + sum(r["pass_seconds"]),
                 "cpu_baseline": {"value": value, "unit": "steps/s", "cores": r["cores"], "kind": "port",
@@ -929,9 +918,8 @@ def main():
         mixed_surfaces = r["surfaces"]
         del r
         arms = {}
-        # the plain FP64 form at the reference's accuracy (eight slices, FP64 solves),
-        # and with its Legendre contractions emulated on the tensor cores and
-        # its ring transforms in double-float on the FP32 pipe
+        # the plain FP64 form (eight slices, fixed-point rings, FP64 solves), and the
+        # one at about 49 bits (seven slices, rings in double-float)
         for name, emulation in (("fp64_gpu", 0), ("fp64_gpu_tc_emulated", 1)):
             # timed with the kernel events on: a few ms of a 2-5 s step
             rr = gpu_arm(args, rank, world, device, "fp64", emulation=emulation, e2e=False, profile_apart=False)

@@ -950,6 +950,8 @@ int Grid::BatchFor(int N, bool real, bool analysis, int P, int p0, int count, co
       b.maxK = std::max(b.maxK, it.K);
       b.flops += 2.0 * it.M * it.N * it.K;
       b.outputs += static_cast<double>(it.M) * it.N;
+      b.inputs += static_cast<double>(it.K) * it.N;
+      b.tableValues += static_cast<double>(it.M) * it.K;
       items.push_back(it);
     }
     part.count = static_cast<int>(items.size()) - part.first;
@@ -1414,11 +1416,10 @@ int Grid::RunGemmF(int N, bool real, Batch& b, const float* B, float* C, bool ac
     LaunchPackB(items, b.count, b.maxBTiles, b.tileN, B, b.packed, stream);
     SL3D_CHECK_LAUNCH();
   }
-  // algorithmic traffic: the table panel once, B once per row tile (4 bytes
-  // a value read in the contraction; 8 from the packed tiles), C once
+  // algorithmic traffic: the table's two parts, B (its packed tiles with the
+  // separate pass) and C once each
   prof::Scope scope(prof::kLegendre32, stream, b.flops,
-                    4.0 * b.panelFloats + (separatePack ? 4.0 : 2.0) * b.packedFloats * b.maxMTiles +
-                        4.0 * b.outputs);
+                    8.0 * b.tableValues + 4.0 * (separatePack ? b.packedFloats : b.inputs) + 4.0 * b.outputs);
   return RunGemmTc(items, b.dTcTiles, static_cast<int>(b.tcTiles.size()), b.tileN, found->second, b.packed,
                    separatePack ? nullptr : B, C, accumulate, giveUp, stream);
 }

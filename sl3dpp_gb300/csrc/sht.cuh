@@ -209,7 +209,7 @@ class Grid {
     int count = 0, maxM = 0, maxN = 0;
     bool analysis = false;
     double flops = 0.0;    // 2 M N K summed over the items
-    double outputs = 0.0;  // M N summed over the items
+    double outputs = 0.0, inputs = 0.0, tableValues = 0.0;  // M N, K N and M K summed over the items
     // the tensor-core form (FP32): its items, tile width and extents, the
     // packed B (made on first use) and the key of its table panel
     std::vector<TcItemHost> tcHost;
