@@ -1056,8 +1056,7 @@ bool Grid::UseSlices64(const Batch& b) const {
 
 // The FP64 contraction as slice products on the tensor cores: the spin's
 // split panel for this direction made on first use, the batch's items on its
-// first use; then B split and packed into memory of this call, and the
-// contraction.
+// first use; then the contraction.
 int Grid::RunGemm64(int N, bool real, Batch& b, const double* B, double* C, bool accumulate,
                     cudaStream_t stream) {
   if (b.count == 0) return SL3DGPU_OK;
@@ -1081,7 +1080,8 @@ int Grid::RunGemm64(int N, bool real, Batch& b, const double* B, double* C, bool
   if (int st = Tables(b, &tables); st != SL3DGPU_OK) return st;
   const std::array<int, 4> key{N, real ? 1 : 0, b.analysis ? 1 : 0, slices};
   auto found = panels64_.find(key);
-  if (found == panels64_.end()) {
+  const bool made = found == panels64_.end();
+  if (made) {
     Tc64Panel panel;
     const size_t values = static_cast<size_t>(std::max<long long>(b.panel64, 1)) * slices * kTcTileM * kTcTileK;
     SL3D_CUDA(cudaMalloc(&panel.slices, values * sizeof(uint16_t)));
@@ -1092,11 +1092,18 @@ int Grid::RunGemm64(int N, bool real, Batch& b, const double* B, double* C, bool
                      b.maxATiles, tables.of[c], panel, stream);
       SL3D_CHECK_LAUNCH();
     }
-    // finished before a call on another stream can find it (once a panel, as Table waits)
-    SL3D_CUDA(cudaStreamSynchronize(stream));
     found = panels64_.emplace(key, panel).first;
   }
-  // this call's packed tiles, then its column exponents
+  const int status = Contract64(b, slices, tables, found->second, B, C, accumulate, giveUp, stream);
+  // a panel is finished before a call on another stream can find it (once each, as Table waits)
+  if (made) SL3D_CUDA(cudaStreamSynchronize(stream));
+  return status;
+}
+
+// B packed into memory of this call from the grid's pool, and the contraction.
+int Grid::Contract64(const Batch& b, int slices, const Tc64Tables& tables, const Tc64Panel& panel, const double* B,
+                     double* C, bool accumulate, int* giveUp, cudaStream_t stream) {
+  // the packed tiles, then the column exponents
   const size_t tileBytes = static_cast<size_t>(b.packed64) * slices * kTc64TileN * kTcTileK * sizeof(uint16_t);
   void* scratch = nullptr;
   SL3D_CUDA(cudaMallocFromPoolAsync(&scratch, tileBytes + std::max<long long>(b.colExps, 1) * sizeof(int), pool_,
@@ -1110,8 +1117,8 @@ int Grid::RunGemm64(int N, bool real, Batch& b, const double* B, double* C, bool
   }
   {
     prof::Scope scope(prof::kLegendre64Tc, stream, b.flops);
-    status = RunGemm64Tc(slices, b.items, b.tc64Items, b.count, b.maxMTiles, b.maxNTiles64, tables, found->second,
-                         B, packed, colExp, C, accumulate, giveUp, stream);
+    status = RunGemm64Tc(slices, b.items, b.tc64Items, b.count, b.maxMTiles, b.maxNTiles64, tables, panel, B, packed,
+                         colExp, C, accumulate, giveUp, stream);
   }
   SL3D_CUDA(cudaFreeAsync(scratch, stream));
   return status;
@@ -1390,7 +1397,8 @@ int Grid::RunGemmF(int N, bool real, Batch& b, const float* B, float* C, bool ac
   const auto* items = static_cast<const TcItem*>(b.tcItems);
   const std::array<int, 3> key{N, real ? 1 : 0, b.analysis ? 1 : 0};
   auto found = panels_.find(key);
-  if (found == panels_.end()) {
+  const bool made = found == panels_.end();
+  if (made) {
     Tc64Tables tables;
     if (int st = Tables(b, &tables); st != SL3DGPU_OK) return st;
     float* panel = nullptr;
@@ -1401,7 +1409,6 @@ int Grid::RunGemmF(int N, bool real, Batch& b, const float* B, float* C, bool ac
                    panel, stream);
       SL3D_CHECK_LAUNCH();
     }
-    SL3D_CUDA(cudaStreamSynchronize(stream));  // as RunGemm64's
     found = panels_.emplace(key, panel).first;
   }
   // B split and packed inside the contraction (B and C never overlap here:
@@ -1420,8 +1427,10 @@ int Grid::RunGemmF(int N, bool real, Batch& b, const float* B, float* C, bool ac
   // separate pass) and C once each
   prof::Scope scope(prof::kLegendre32, stream, b.flops,
                     8.0 * b.tableValues + 4.0 * (separatePack ? b.packedFloats : b.inputs) + 4.0 * b.outputs);
-  return RunGemmTc(items, b.dTcTiles, static_cast<int>(b.tcTiles.size()), b.tileN, found->second, b.packed,
-                   separatePack ? nullptr : B, C, accumulate, giveUp, stream);
+  const int status = RunGemmTc(items, b.dTcTiles, static_cast<int>(b.tcTiles.size()), b.tileN, found->second,
+                               b.packed, separatePack ? nullptr : B, C, accumulate, giveUp, stream);
+  if (made) SL3D_CUDA(cudaStreamSynchronize(stream));  // as RunGemm64's
+  return status;
 }
 
 Grid::Batch* Grid::MutableBatch(int N, bool real, bool analysis, int P, int p0, int count) {

@@ -240,6 +240,8 @@ class Grid {
     return component == 0 ? 0 : component == 1 ? SpinRows(-2) : SpinRows(-2) + SpinRows(-1);
   }
   int RunGemm64(int N, bool real, Batch& b, const double* B, double* C, bool accumulate, cudaStream_t stream);
+  int Contract64(const Batch& b, int slices, const Tc64Tables& tables, const Tc64Panel& panel, const double* B,
+                 double* C, bool accumulate, int* giveUp, cudaStream_t stream);
   // The table pre-tiled for the tensor cores per (spin, real, direction).
   std::map<std::array<int, 3>, float*> panels_;
   std::map<std::array<long long, 6>, Batch> batches_;

@@ -13,11 +13,15 @@ SHT = pathlib.Path(__file__).resolve().parent.parent / "sl3dpp_gb300" / "csrc" /
 
 
 @pytest.mark.parametrize("panels", ["panels64_", "panels_"])
-def test_a_panel_is_finished_before_it_can_be_found(panels):
+def test_a_panel_is_finished_before_another_call_can_find_it(panels):
+    """The wait comes after the call's launches, whatever their status, and
+    before the call returns (C calls hold the grid's lock until then)."""
     text = SHT.read_text()
-    end = text.index(f"found = {panels}.emplace(")
-    launch = max(text.rfind("LaunchPanelA64(", 0, end), text.rfind("LaunchPanelA(", 0, end))
-    assert "SL3D_CUDA(cudaStreamSynchronize(stream));" in text[launch:end]
+    made = text.index(f"found = {panels}.emplace(")
+    rest = text[made:text.index("\n}\n", made)]
+    after = rest[rest.index("const int status ="):]
+    assert "if (made) SL3D_CUDA(cudaStreamSynchronize(stream));" in after
+    assert "return" not in after[:after.index("if (made)")]
 
 
 @pytest.mark.gpu
