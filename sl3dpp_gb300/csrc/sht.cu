@@ -42,7 +42,10 @@ namespace {
 // -- Wigner table --------------------------------------------------------------------
 
 // The closed form at l0 = max(|m|, |N|) for N <= 0 (see the host oracle's
-// restatement of the same algorithm): a product recursion in |m|.
+// restatement of the same algorithm): a product recursion in |m|. kHigh: spins
+// above 2, whose orders below the spin take a product whose factors stay in
+// range; a kernel of its own, so that the compiler keeps the other's arithmetic.
+template <bool kHigh>
 __device__ double WignerStart(int N, int m, double c, double s) {
   const int M = abs(m), A = -N;
   if (M >= A) {
@@ -54,23 +57,25 @@ __device__ double WignerStart(int N, int m, double c, double s) {
     return v;
   }
   const int l = A;
-  double v = 1.0;
-  if (l <= 2) {
-    const double fact[5] = {1.0, 1.0, 2.0, 6.0, 24.0};
-    v = sqrt(fact[2 * l] / (fact[l + m] * fact[l - m]));
-    for (int k = 0; k < l - m; ++k) v *= c;
-    for (int k = 0; k < l + m; ++k) v *= s;
-  } else {
+  if constexpr (kHigh) {
     // sqrt(binomial(2 l, r)) (c s)^r factor by factor, then the rest of the larger power
     const int r = l - M, q = l + M;
+    double v = 1.0;
     for (int k = 1; k <= r; ++k) v *= sqrt((q + k) / static_cast<double>(k)) * c * s;
     for (int k = 0; k < 2 * M; ++k) v *= m > 0 ? s : c;
+    return (l + m) % 2 != 0 ? -v : v;
+  } else {
+    const double fact[5] = {1.0, 1.0, 2.0, 6.0, 24.0};
+    double v = sqrt(fact[2 * l] / (fact[l + m] * fact[l - m]));
+    for (int k = 0; k < l - m; ++k) v *= c;
+    for (int k = 0; k < l + m; ++k) v *= s;
+    if ((l + m) % 2 != 0) v = -v;
+    return v;
   }
-  if ((l + m) % 2 != 0) v = -v;
-  return v;
 }
 
 // One thread per (order, colatitude): the three-term recurrence in l.
+template <bool kHigh>
 __global__ void WignerTableKernel(int lmax, int N, int ntheta, const double* theta,
                                   const int* rowOffset, double* table) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
@@ -84,7 +89,7 @@ __global__ void WignerTableKernel(int lmax, int N, int ntheta, const double* the
   const double t = mirrored ? pi - theta[j] : theta[j];
   const double c = cos(0.5 * t), s = sin(0.5 * t);
   double* out = table + static_cast<long long>(rowOffset[m + lmax]) * ntheta + j;
-  double dprev = 0.0, d = WignerStart(Nr, m, c, s);
+  double dprev = 0.0, d = WignerStart<kHigh>(Nr, m, c, s);
   const double ct = cos(t);
   for (int l = l0; l <= lmax; ++l) {
     const double sign = mirrored && ((l + m) % 2 != 0) ? -1.0 : 1.0;
@@ -885,7 +890,8 @@ int Grid::Table(int N, const SpinTable** out) {
     SL3D_CUDA(CopyIn(t.dRowOffset, t.rowOffset.data(), t.rowOffset.size() * sizeof(int)));
     dim3 grid((ntheta + 127) / 128, 2 * lmax + 1);
     prof::Scope scope(prof::kOther, nullptr);
-    WignerTableKernel<<<grid, 128>>>(lmax, N, ntheta, dTheta, t.dRowOffset, t.values);
+    auto kernel = std::abs(N) > 2 ? WignerTableKernel<true> : WignerTableKernel<false>;
+    kernel<<<grid, 128>>>(lmax, N, ntheta, dTheta, t.dRowOffset, t.values);
     SL3D_CHECK_LAUNCH();
     SL3D_CUDA(cudaDeviceSynchronize());
     found = tables_.emplace(N, std::move(t)).first;
