@@ -140,10 +140,13 @@ int sl3dgpu_grid_lmax(const sl3dgpu_grid* grid);
 /* The grid's FP64 transforms. Both forms run the Legendre contractions on the
  * tensor cores (BF16 slices of each value under a power-of-two scale per row
  * and column, exact FP32 products, levels joined exactly): 0 with eight slices,
- * an error below the FP64 units' own rounding, and FP64-accurate rings; 1 with
- * seven (about 49 bits of each operand) and the rings in double-float. Depths
- * beyond 400 (448) and, in form 0, calls of up to eight fields stay on the
- * FP64 units. */
+ * an error below the FP64 units' own rounding in the norm, and rings in 64-bit
+ * fixed point, likewise; 1 with seven (about 49 bits of each operand) and the
+ * rings in double-float. In form 0 a value holds 56 bits below the largest of its
+ * column (one order's coefficients, or colatitudes, of a field's real or
+ * imaginary part) and of its table row, and 61 below its ring's sum: one far below
+ * them has fewer bits than the FP64 units' sums give it. Depths beyond 400 (448)
+ * and, in form 0, calls of up to eight fields stay on the FP64 units. */
 int sl3dgpu_grid_set_fp64_emulation(sl3dgpu_grid* grid, int on);
 /* Host copies of the colatitudes and their Gauss-Legendre weights. */
 int sl3dgpu_grid_colatitudes(const sl3dgpu_grid* grid, double* theta, double* weights);
@@ -325,7 +328,7 @@ typedef struct sl3dgpu_v3d_options {
   int warm_start;           /* 0: each step starts from the previous strain (the reference's start);
                                1: also guesses 2 s_n - s_{n-1}, the mixed form's FP32 correction
                                starting from it (the FP64 form tries it as a first pass) */
-  int fp64_emulation;       /* the FP64 transforms: 0 with the FP64 units' accuracy, 1 at about 49 bits
+  int fp64_emulation;       /* the FP64 transforms: 0 with the FP64 units' accuracy in the norm, 1 at about 49 bits
                                (sl3dgpu_grid_set_fp64_emulation) */
   int correction_memory;    /* mixed form: the FP32 correction's Anderson history, 0..16; 0 takes
                                anderson_memory */

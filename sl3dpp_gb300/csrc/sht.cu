@@ -8,11 +8,14 @@
 //  - analysis: G_m(theta_j) = (2 pi / nphi) w_j sum_k f e^{-i m phi_k}, then
 //    c_lm = sum_j Lambda^N_lm(theta_j) G_m(theta_j).
 // The contraction is one dense matrix product per (spin, order) with the
-// batch's fields as columns, run here as a batched FP64 register-tiled GEMM;
-// the FFT is a mixed-radix Stockham transform in shared memory, several rings
-// per CTA: FP64 values in block fixed point (ring_fixed.cu), in
-// double-float where the emulation was asked for (ring_df.cu), FP32 values
-// here, one warp per ring (warp-synchronous stages).
+// batch's fields as columns: FP64 as BF16 slices on the tensor cores
+// (tc_gemm64.cu), FP32 as three TF32 products (tc_gemm.cu), both in one launch
+// over the orders; up to eight FP64 fields, and depths beyond the slices', on
+// the FP64 units here. The FFT is a mixed-radix Stockham transform in shared
+// memory, several rings per CTA: FP64 values in block fixed point
+// (ring_fixed.cu), in double-float where the emulation was asked for
+// (ring_df.cu); FP32 values and few FP64 fields here, one warp per ring
+// (warp-synchronous stages).
 #include <algorithm>
 #include <cstdlib>
 #include <cmath>

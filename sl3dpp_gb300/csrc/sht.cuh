@@ -92,8 +92,8 @@ class Grid {
 
   int lmax = 0, nmax = 0, band = 0, ntheta = 0, nphi = 0;
   // The FP64 contractions run as slice products on the tensor cores
-  // (tc_gemm64.cu): eight slices, at least the FP64 units' accuracy, or, with
-  // this set, seven (about 49 bits) and the rings in double-float. Batches of
+  // (tc_gemm64.cu): eight slices, at least the FP64 units' accuracy in the norm,
+  // or, with this set, seven (about 49 bits) and the rings in double-float. Batches of
   // few columns and ones deeper than the slices' exactness bound keep the
   // FP64 units.
   bool emulateFp64 = false;

@@ -138,11 +138,8 @@ class Viscoelastic3DGpu {
   // mixer
   int mixerMemory = 0;
   Dev<double> xPrev, fPrev, gammaOut, mixPartial, mixSums;
-  // the Anderson least squares runs on the host: each mixer's Gram matrix,
-  // and pinned room for an update's sums (16) and gamma (9)
-  // the mixers' Gram matrices (memory x memory), on the device
+  // the mixers' Gram matrices (memory x memory) and their least squares, on the device
   Dev<double> gram64, gram32;
-  double* hostMix = nullptr;
   int MixerDeviceSolve(Dev<double>& gram, int m, int slot, int memory);
   std::vector<Dev<double>> dG, dF;
   Dev<double*> dGPtr, dFPtr;
@@ -329,7 +326,6 @@ class Viscoelastic3DGpu {
   ~Viscoelastic3DGpu() {
     for (auto& g : correctionGraphs) RetireGraph(g.exec);
     if (hostResult) cudaFreeHost(hostResult);
-    if (hostMix) cudaFreeHost(hostMix);
     if (stream) cudaStreamDestroy(stream);
   }
 
@@ -554,7 +550,6 @@ int Viscoelastic3DGpu::Create(const sl3dgpu_layer* layers, int nlayers, const sl
   }
   SL3D_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
   SL3D_CUDA(cudaMallocHost(&hostResult, 8 * sizeof(double)));
-  SL3D_CUDA(cudaMallocHost(&hostMix, 4 * kMixMaxMemory * sizeof(double)));  // sums, then gamma
   SL3D_CUDA(mixSums.Alloc(2 * kMixMaxMemory));
   SL3D_TRY(Grid::Create(opt.lmax, 2, opt.oversampling, grid));
   grid->emulateFp64 = opt.fp64_emulation == 1;

@@ -11,9 +11,11 @@
 // halves, and A_lo B_hi a second MMA into the first half: two MMAs per 8-deep
 // slice instead of three (an M = 128 MMA costs about the same below N = 128
 // as at N = 128, so the wide one is nearly free). The epilogue sums the
-// halves. Every wait has an iteration limit. The MMA lane sets the pace, four TF32
-// MMAs a step in about 1000 cycles: three spins of 55 fields at lmax 256 take
-// 199 us (260 while each role found its stage by a 64-bit remainder).
+// halves. Every wait has an iteration limit. A step takes about 1000 cycles, of
+// which its four TF32 MMAs account for some 400 to 500 by their measured costs;
+// what the MMA lane waits for in the rest has not been split up. Three spins of
+// 55 fields at lmax 256 take 199 us (260 while each role found its stage by a
+// 64-bit remainder).
 #include <cstdint>
 
 #include "profile.cuh"

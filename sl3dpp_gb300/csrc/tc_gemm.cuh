@@ -8,7 +8,7 @@
 // ready-made tiles: pre-tiled once per (spin, direction) into "panels" of
 // 128 x 16 tiles in the canonical K-major core-matrix layout, high part then
 // low part. B is split and packed the same way (tileN x 16 tiles) inside the
-// contraction, from its source, by two warps (or, the older form, by a
+// contraction, from its source, by six warps (or, the older form, by a
 // separate split-and-pack pass through HBM).
 #pragma once
 
@@ -97,9 +97,11 @@ int RunGemmTc(const TcItem* tcItems, const int4* tiles, int tileCount, int tileN
 // most 7 bits, x = sum_p s_p 2^{-7 (p + 1)} (the Ozaki splitting); the slice
 // products of each level d = p + q below the slice count are accumulated in
 // FP32 by tcgen05.mma kind::f16, exactly (integers below 2^24), and the levels
-// are joined in FP64. Seven slices carry about 49 bits of each value, eight
-// 56: with eight the result is at least as accurate as the FP64 units'
-// relative to (row maximum) x (column maximum) x K.
+// are joined exactly as integers and rounded once. Seven slices carry about 49
+// bits, eight 56, below the largest value of a row (of A) or column (of B): with
+// eight the result is at least as accurate as the FP64 units' in the norm,
+// relative to (row maximum) x (column maximum) x K. A value far below its row's
+// and column's largest keeps fewer bits than an FP64 sum would give it.
 constexpr int kTc64Slices = 7;       // a grid that asked for the emulation
 constexpr int kTc64SlicesFull = 8;   // the default FP64 contraction
 constexpr int kTc64TileN = 32;       // up to 8 accumulators of 32 columns in half of tensor memory

@@ -33,7 +33,7 @@ class SurfaceGrid:
     def __init__(self, lmax: int, nmax: int = 0, oversampling: float = 1.0, fp64_emulation: bool = False):
         """fp64_emulation: the Legendre contractions in seven BF16 slices a
         value (about 49 bits) and the rings in double-float, rather than with
-        the FP64 units' accuracy (eight slices, fixed-point rings)."""
+        the FP64 units' accuracy in the norm (eight slices, fixed-point rings)."""
         handle = c_void_p()
         check(lib().sl3dgpu_grid_create(lmax, nmax, float(oversampling), ctypes.byref(handle)))
         self._handle = handle
