@@ -229,12 +229,18 @@ __device__ __forceinline__ unsigned long long Bits(double v) {
   return static_cast<unsigned long long>(__double_as_longlong(v));
 }
 
-// A value's exponent among its ring's: 0 for zero alone, a subnormal value
+// The largest exponent of a thread's values: 0 for zeros alone, subnormal values
 // counting as 1, so that a ring (or its weights) of nothing larger takes the
-// FP64 form.
-__device__ __forceinline__ uint32_t RingExponent(unsigned long long bits) {
-  return max(static_cast<uint32_t>(FxExponent(bits)), (bits << 1) != 0 ? 1u : 0u);
-}
+// FP64 form. Kept as the largest upper word and the lower words together: two
+// instructions a value.
+struct LargestExponent {
+  uint32_t upper = 0, lower = 0;
+  __device__ __forceinline__ void See(unsigned long long bits) {
+    upper = max(upper, static_cast<uint32_t>(bits >> 32) & 0x7FFFFFFFu);
+    lower |= static_cast<uint32_t>(bits);
+  }
+  __device__ __forceinline__ uint32_t Exponent() const { return max(upper >> 20, (upper | lower) != 0 ? 1u : 0u); }
+};
 
 // Whether an exponent keeps a ring's scale inside the FP64 range (a ring of
 // zeros has none).
@@ -269,8 +275,8 @@ __global__ void __launch_bounds__(kFxThreads, 2) FxRingKernel(const __grid_const
   // The raw values: a complex field's order m at m (or n + m); a real pair's
   // order m at m and the second field's at n - m (order 0 of both at 0).
   // Only this thread's own entries until the transform.
-  uint32_t emax = 0;
-  auto seen = [&](unsigned long long bits) { emax = max(emax, RingExponent(bits)); };
+  LargestExponent largest;
+  auto seen = [&](unsigned long long bits) { largest.See(bits); };
   const bool synth = A.mode != kFxAnalyse;
   if (synth) {
     const double2* in = Q.spectraIn + static_cast<long long>(j) * A.count + fa;
@@ -321,7 +327,7 @@ __global__ void __launch_bounds__(kFxThreads, 2) FxRingKernel(const __grid_const
       seen(a.y);
     }
   }
-  emax = OverRing(emax, shared, G, Most);
+  const uint32_t emax = OverRing(largest.Exponent(), shared, G, Most);
   if (!FxCarries(emax)) fallback = 1;
   // The ring's sum of magnitudes, and its scale.
   uint32_t sum = 0;
@@ -418,13 +424,13 @@ __global__ void __launch_bounds__(kFxThreads, 2) FxRingKernel(const __grid_const
     // The weights under the ring's largest, in Q62 below 1; the products
     // (swapped for the analysis) and their sum of magnitudes; the rescale.
     Fx2* res = ring + at * n;
-    uint32_t wmax = 0;
+    LargestExponent weights;
     if (live)
       for (int k = lead; k < n; k += step) {
-        wmax = max(wmax, RingExponent(Bits(A.pointWeight[row0 + k])));
-        if (second) wmax = max(wmax, RingExponent(Bits(A.pointWeight[row1 + k])));
+        weights.See(Bits(A.pointWeight[row0 + k]));
+        if (second) weights.See(Bits(A.pointWeight[row1 + k]));
       }
-    wmax = OverRing(wmax, shared, G, Most);
+    const uint32_t wmax = OverRing(weights.Exponent(), shared, G, Most);
     if (!FxCarries(wmax) || (wmax > 0 && e0 > 0 && !FxCarries(static_cast<uint32_t>(max(1, e0 + static_cast<int>(wmax) - 1023)))))
       fallback = 1;
     const int wscale = 62 - (static_cast<int>(wmax) - 1022);  // |w| 2^wscale < 2^62
