@@ -864,6 +864,8 @@ Grid::~Grid() {
     cudaFree(b.tc64Items);
   }
   if (pool_ != nullptr) cudaMemPoolDestroy(pool_);
+  if (setup_ != nullptr) cudaStreamDestroy(setup_);
+  if (panelsMade_ != nullptr) cudaEventDestroy(panelsMade_);
   cudaFree(scratchSpectra_);
   cudaFree(scratchCoeffs_);
   for (auto& [N, t] : tables_) {
@@ -1089,24 +1091,61 @@ int Grid::RunGemm64(int N, bool real, Batch& b, const double* B, double* C, bool
   if (int st = Tables(b, &tables); st != SL3DGPU_OK) return st;
   const std::array<int, 4> key{N, real ? 1 : 0, b.analysis ? 1 : 0, slices};
   auto found = panels64_.find(key);
-  const bool made = found == panels64_.end();
-  if (made) {
+  if (found == panels64_.end()) {
+    if (int st = Setup(); st != SL3DGPU_OK) return st;
     Tc64Panel panel;
     const size_t values = static_cast<size_t>(std::max<long long>(b.panel64, 1)) * slices * kTcTileM * kTcTileK;
     SL3D_CUDA(cudaMalloc(&panel.slices, values * sizeof(uint16_t)));
     SL3D_CUDA(cudaMalloc(&panel.rowExp, std::max<long long>(b.rowExps, 1) * sizeof(int)));
     for (size_t c = 0; c < b.parts.size(); ++c) {
-      prof::Scope scope(prof::kOther, stream);
+      prof::Scope scope(prof::kOther, setup_);
       LaunchPanelA64(slices, b.items + b.parts[c].first, b.tc64Items + b.parts[c].first, b.parts[c].count, b.maxM,
-                     b.maxATiles, tables.of[c], panel, stream);
+                     b.maxATiles, tables.of[c], panel, setup_);
       SL3D_CHECK_LAUNCH();
     }
+    if (int st = PanelsLaunched(); st != SL3DGPU_OK) return st;
     found = panels64_.emplace(key, panel).first;
   }
-  const int status = Contract64(b, slices, tables, found->second, B, C, accumulate, giveUp, stream);
-  // a panel is finished before a call on another stream can find it (once each, as Table waits)
-  if (made) SL3D_CUDA(cudaStreamSynchronize(stream));
-  return status;
+  if (int st = AwaitPanels(stream); st != SL3DGPU_OK) return st;
+  return Contract64(b, slices, tables, found->second, B, C, accumulate, giveUp, stream);
+}
+
+// The grid's own stream for panels, and the event of the last one made.
+int Grid::Setup() {
+  if (setup_ != nullptr) return SL3DGPU_OK;
+  SL3D_CUDA(cudaEventCreateWithFlags(&panelsMade_, cudaEventDisableTiming));
+  SL3D_CUDA(cudaStreamCreateWithFlags(&setup_, cudaStreamNonBlocking));
+  return SL3DGPU_OK;
+}
+int Grid::PanelsLaunched() {
+  SL3D_CUDA(cudaEventRecord(panelsMade_, setup_));
+  panelsPending_ = true;
+  return SL3DGPU_OK;
+}
+int Grid::AwaitPanels(cudaStream_t stream) {
+  if (!panelsPending_) return SL3DGPU_OK;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  SL3D_CUDA(cudaStreamIsCapturing(stream, &capture));
+  if (capture != cudaStreamCaptureStatusNone) {
+    // a captured stream cannot wait for work outside its graph
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    SL3D_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+    const cudaError_t e = cudaEventSynchronize(panelsMade_);
+    SL3D_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+    SL3D_CUDA(e);
+    panelsPending_ = false;
+    return SL3DGPU_OK;
+  }
+  const cudaError_t e = cudaEventQuery(panelsMade_);
+  if (e == cudaSuccess) {
+    panelsPending_ = false;
+  } else if (e == cudaErrorNotReady) {
+    cudaGetLastError();  // not an error
+    SL3D_CUDA(cudaStreamWaitEvent(stream, panelsMade_, 0));
+  } else {
+    SL3D_CUDA(e);
+  }
+  return SL3DGPU_OK;
 }
 
 // B packed into memory of this call from the grid's pool, and the contraction.
@@ -1406,20 +1445,22 @@ int Grid::RunGemmF(int N, bool real, Batch& b, const float* B, float* C, bool ac
   const auto* items = static_cast<const TcItem*>(b.tcItems);
   const std::array<int, 3> key{N, real ? 1 : 0, b.analysis ? 1 : 0};
   auto found = panels_.find(key);
-  const bool made = found == panels_.end();
-  if (made) {
+  if (found == panels_.end()) {
+    if (int st = Setup(); st != SL3DGPU_OK) return st;
     Tc64Tables tables;
     if (int st = Tables(b, &tables); st != SL3DGPU_OK) return st;
     float* panel = nullptr;
     SL3D_CUDA(cudaMalloc(&panel, std::max<long long>(b.panelFloats, 1) * sizeof(float)));
     for (size_t c = 0; c < b.parts.size(); ++c) {
-      prof::Scope scope(prof::kOther, stream);
+      prof::Scope scope(prof::kOther, setup_);
       LaunchPanelA(b.items + b.parts[c].first, items + b.parts[c].first, b.parts[c].count, b.maxATiles, tables.of[c],
-                   panel, stream);
+                   panel, setup_);
       SL3D_CHECK_LAUNCH();
     }
+    if (int st = PanelsLaunched(); st != SL3DGPU_OK) return st;
     found = panels_.emplace(key, panel).first;
   }
+  if (int st = AwaitPanels(stream); st != SL3DGPU_OK) return st;
   // B split and packed inside the contraction (B and C never overlap here:
   // the packing warps read B while other CTAs' epilogues write C); with
   // SL3DGPU_PACKB=1 by the separate pass, through HBM
@@ -1436,10 +1477,8 @@ int Grid::RunGemmF(int N, bool real, Batch& b, const float* B, float* C, bool ac
   // separate pass) and C once each
   prof::Scope scope(prof::kLegendre32, stream, b.flops,
                     8.0 * b.tableValues + 4.0 * (separatePack ? b.packedFloats : b.inputs) + 4.0 * b.outputs);
-  const int status = RunGemmTc(items, b.dTcTiles, static_cast<int>(b.tcTiles.size()), b.tileN, found->second,
-                               b.packed, separatePack ? nullptr : B, C, accumulate, giveUp, stream);
-  if (made) SL3D_CUDA(cudaStreamSynchronize(stream));  // as RunGemm64's
-  return status;
+  return RunGemmTc(items, b.dTcTiles, static_cast<int>(b.tcTiles.size()), b.tileN, found->second, b.packed,
+                   separatePack ? nullptr : B, C, accumulate, giveUp, stream);
 }
 
 Grid::Batch* Grid::MutableBatch(int N, bool real, bool analysis, int P, int p0, int count) {

@@ -245,6 +245,15 @@ class Grid {
   // The table pre-tiled for the tensor cores per (spin, real, direction).
   std::map<std::array<int, 3>, float*> panels_;
   std::map<std::array<long long, 6>, Batch> batches_;
+  // Panels are made on a stream of the grid's own, under no capture of the
+  // caller's. A call waits for the last one made on its own stream (in a capture,
+  // on the host), until a call finds it finished.
+  cudaStream_t setup_ = nullptr;
+  cudaEvent_t panelsMade_ = nullptr;
+  bool panelsPending_ = false;
+  int Setup();
+  int PanelsLaunched();
+  int AwaitPanels(cudaStream_t stream);
   int BatchFor(int N, bool real, bool analysis, int P, int p0, int count, const Batch** out);
   Batch* MutableBatch(int N, bool real, bool analysis, int P, int p0, int count);
   double* scratchSpectra_ = nullptr;

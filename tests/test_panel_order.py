@@ -1,8 +1,8 @@
 """A grid's table panels (the Legendre tables split for the tensor cores,
-csrc/sht.cu) are made by the first call that wants one, on that call's stream.
-A call on another stream finds the panel made, so it must be finished by
-then: the waits are asserted on the source, and the second stream's results
-against the first's, whose stream made the panel, bit for bit."""
+csrc/sht.cu) are made by the first call that wants one, on a stream of the
+grid's own. Every call waits for them on its own stream: the waits are asserted
+on the source, the results of two streams' first calls against each other, and
+a capture right after the first call against the call itself, bit for bit."""
 
 import ctypes
 import pathlib
@@ -12,16 +12,16 @@ import pytest
 SHT = pathlib.Path(__file__).resolve().parent.parent / "sl3dpp_gb300" / "csrc" / "sht.cu"
 
 
-@pytest.mark.parametrize("panels", ["panels64_", "panels_"])
-def test_a_panel_is_finished_before_another_call_can_find_it(panels):
-    """The wait comes after the call's launches, whatever their status, and
-    before the call returns (C calls hold the grid's lock until then)."""
+@pytest.mark.parametrize("panels,launch,contract", [("panels64_", "LaunchPanelA64(", "Contract64("),
+                                                     ("panels_", "LaunchPanelA(", "RunGemmTc(")])
+def test_every_call_waits_for_the_panels(panels, launch, contract):
     text = SHT.read_text()
-    made = text.index(f"found = {panels}.emplace(")
-    rest = text[made:text.index("\n}\n", made)]
-    after = rest[rest.index("const int status ="):]
-    assert "if (made) SL3D_CUDA(cudaStreamSynchronize(stream));" in after
-    assert "return" not in after[:after.index("if (made)")]
+    body = text[text.index(f"auto found = {panels}.find(key);"):]
+    body = body[:body.index("\n}\n")]
+    call = body[body.index(launch):]
+    assert "setup_)" in call[:call.index(";")]
+    order = [body.index(t) for t in (launch, "PanelsLaunched()", f"{panels}.emplace(", "AwaitPanels(stream)", contract)]
+    assert order == sorted(order)
 
 
 @pytest.mark.gpu
@@ -51,3 +51,29 @@ def test_gpu_first_calls_on_two_streams(gpu, analysis, fp32, emulation):
     torch.cuda.synchronize()
     assert float(outs[0].abs().max()) > 0.0
     assert torch.equal(outs[0], outs[1])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("emulation", [False, True])
+def test_gpu_capture_after_the_first_call(gpu, emulation):
+    import torch
+
+    from sl3dpp_gb300.grid import SurfaceGrid
+
+    lmax, N, count = 48, -1, 12
+    grid = SurfaceGrid(lmax, 2, 1.5, fp64_emulation=emulation)
+    rng = torch.Generator(device=gpu).manual_seed(1)
+    c = torch.randn(count * grid.SpinCoefficientSize(N), dtype=torch.complex128, device=gpu, generator=rng)
+    later = torch.randn(c.shape, dtype=torch.complex128, device=gpu, generator=rng)
+    grid.ExpandSpinBatch(N, grid.SynthesiseSpinBatch(N, c, count), count)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        fields = grid.SynthesiseSpinBatch(N, c, count)
+        back = grid.ExpandSpinBatch(N, fields, count)
+    for values in (c.clone(), later):
+        c.copy_(values)
+        graph.replay()
+        torch.cuda.synchronize()
+        want = grid.SynthesiseSpinBatch(N, values, count)
+        assert torch.equal(fields, want)
+        assert torch.equal(back, grid.ExpandSpinBatch(N, want, count))
