@@ -864,7 +864,6 @@ Grid::~Grid() {
     cudaFree(b.tc64Items);
   }
   if (pool_ != nullptr) cudaMemPoolDestroy(pool_);
-  if (setup_ != nullptr) cudaStreamDestroy(setup_);
   if (panelsMade_ != nullptr) cudaEventDestroy(panelsMade_);
   cudaFree(scratchSpectra_);
   cudaFree(scratchCoeffs_);
@@ -1090,38 +1089,53 @@ int Grid::RunGemm64(int N, bool real, Batch& b, const double* B, double* C, bool
   Tc64Tables tables;
   if (int st = Tables(b, &tables); st != SL3DGPU_OK) return st;
   const std::array<int, 4> key{N, real ? 1 : 0, b.analysis ? 1 : 0, slices};
+  if (int st = AwaitPanels(stream); st != SL3DGPU_OK) return st;
   auto found = panels64_.find(key);
   if (found == panels64_.end()) {
-    if (int st = Setup(); st != SL3DGPU_OK) return st;
     Tc64Panel panel;
     const size_t values = static_cast<size_t>(std::max<long long>(b.panel64, 1)) * slices * kTcTileM * kTcTileK;
     SL3D_CUDA(cudaMalloc(&panel.slices, values * sizeof(uint16_t)));
     SL3D_CUDA(cudaMalloc(&panel.rowExp, std::max<long long>(b.rowExps, 1) * sizeof(int)));
-    for (size_t c = 0; c < b.parts.size(); ++c) {
-      prof::Scope scope(prof::kOther, setup_);
-      LaunchPanelA64(slices, b.items + b.parts[c].first, b.tc64Items + b.parts[c].first, b.parts[c].count, b.maxM,
-                     b.maxATiles, tables.of[c], panel, setup_);
-      SL3D_CHECK_LAUNCH();
-    }
-    if (int st = PanelsLaunched(); st != SL3DGPU_OK) return st;
+    const auto launch = [&](cudaStream_t s) -> int {
+      for (size_t c = 0; c < b.parts.size(); ++c) {
+        prof::Scope scope(prof::kOther, s);
+        LaunchPanelA64(slices, b.items + b.parts[c].first, b.tc64Items + b.parts[c].first, b.parts[c].count, b.maxM,
+                       b.maxATiles, tables.of[c], panel, s);
+        SL3D_CHECK_LAUNCH();
+      }
+      return SL3DGPU_OK;
+    };
+    if (int st = MakePanel(stream, launch); st != SL3DGPU_OK) return st;
     found = panels64_.emplace(key, panel).first;
   }
-  if (int st = AwaitPanels(stream); st != SL3DGPU_OK) return st;
   return Contract64(b, slices, tables, found->second, B, C, accumulate, giveUp, stream);
 }
 
-// The grid's own stream for panels, and the event of the last one made.
-int Grid::Setup() {
-  if (setup_ != nullptr) return SL3DGPU_OK;
-  SL3D_CUDA(cudaEventCreateWithFlags(&panelsMade_, cudaEventDisableTiming));
-  SL3D_CUDA(cudaStreamCreateWithFlags(&setup_, cudaStreamNonBlocking));
-  return SL3DGPU_OK;
+int Grid::MakePanel(cudaStream_t stream, const std::function<int(cudaStream_t)>& launch) {
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  SL3D_CUDA(cudaStreamIsCapturing(stream, &capture));
+  if (capture == cudaStreamCaptureStatusNone) {
+    if (panelsMade_ == nullptr) SL3D_CUDA(cudaEventCreateWithFlags(&panelsMade_, cudaEventDisableTiming));
+    if (int st = launch(stream); st != SL3DGPU_OK) return st;
+    SL3D_CUDA(cudaEventRecord(panelsMade_, stream));
+    panelsPending_ = true;
+    return SL3DGPU_OK;
+  }
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  SL3D_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+  cudaStream_t own = nullptr;
+  cudaError_t e = cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking);
+  int status = SL3DGPU_OK;
+  if (e == cudaSuccess) {
+    status = launch(own);
+    e = cudaStreamSynchronize(own);
+    cudaStreamDestroy(own);
+  }
+  SL3D_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+  SL3D_CUDA(e);
+  return status;
 }
-int Grid::PanelsLaunched() {
-  SL3D_CUDA(cudaEventRecord(panelsMade_, setup_));
-  panelsPending_ = true;
-  return SL3DGPU_OK;
-}
+
 int Grid::AwaitPanels(cudaStream_t stream) {
   if (!panelsPending_) return SL3DGPU_OK;
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
@@ -1444,23 +1458,25 @@ int Grid::RunGemmF(int N, bool real, Batch& b, const float* B, float* C, bool ac
   }
   const auto* items = static_cast<const TcItem*>(b.tcItems);
   const std::array<int, 3> key{N, real ? 1 : 0, b.analysis ? 1 : 0};
+  if (int st = AwaitPanels(stream); st != SL3DGPU_OK) return st;
   auto found = panels_.find(key);
   if (found == panels_.end()) {
-    if (int st = Setup(); st != SL3DGPU_OK) return st;
     Tc64Tables tables;
     if (int st = Tables(b, &tables); st != SL3DGPU_OK) return st;
     float* panel = nullptr;
     SL3D_CUDA(cudaMalloc(&panel, std::max<long long>(b.panelFloats, 1) * sizeof(float)));
-    for (size_t c = 0; c < b.parts.size(); ++c) {
-      prof::Scope scope(prof::kOther, setup_);
-      LaunchPanelA(b.items + b.parts[c].first, items + b.parts[c].first, b.parts[c].count, b.maxATiles, tables.of[c],
-                   panel, setup_);
-      SL3D_CHECK_LAUNCH();
-    }
-    if (int st = PanelsLaunched(); st != SL3DGPU_OK) return st;
+    const auto launch = [&](cudaStream_t s) -> int {
+      for (size_t c = 0; c < b.parts.size(); ++c) {
+        prof::Scope scope(prof::kOther, s);
+        LaunchPanelA(b.items + b.parts[c].first, items + b.parts[c].first, b.parts[c].count, b.maxATiles,
+                     tables.of[c], panel, s);
+        SL3D_CHECK_LAUNCH();
+      }
+      return SL3DGPU_OK;
+    };
+    if (int st = MakePanel(stream, launch); st != SL3DGPU_OK) return st;
     found = panels_.emplace(key, panel).first;
   }
-  if (int st = AwaitPanels(stream); st != SL3DGPU_OK) return st;
   // B split and packed inside the contraction (B and C never overlap here:
   // the packing warps read B while other CTAs' epilogues write C); with
   // SL3DGPU_PACKB=1 by the separate pass, through HBM

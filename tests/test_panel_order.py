@@ -1,8 +1,8 @@
 """A grid's table panels (the Legendre tables split for the tensor cores,
-csrc/sht.cu) are made by the first call that wants one, on a stream of the
-grid's own. Every call waits for them on its own stream: the waits are asserted
-on the source, the results of two streams' first calls against each other, and
-a capture right after the first call against the call itself, bit for bit."""
+csrc/sht.cu) are made by the first call that wants one, on its stream. Calls on
+other streams wait for them: the waits are asserted on the source, the results
+of two streams' first calls against each other, and a capture right after the
+first call against the call itself, bit for bit."""
 
 import ctypes
 import pathlib
@@ -16,12 +16,17 @@ SHT = pathlib.Path(__file__).resolve().parent.parent / "sl3dpp_gb300" / "csrc" /
                                                      ("panels_", "LaunchPanelA(", "RunGemmTc(")])
 def test_every_call_waits_for_the_panels(panels, launch, contract):
     text = SHT.read_text()
-    body = text[text.index(f"auto found = {panels}.find(key);"):]
+    wait = "if (int st = AwaitPanels(stream); st != SL3DGPU_OK) return st;"
+    find = text.index(f"auto found = {panels}.find(key);")
+    assert text[:find].rstrip().endswith(wait)
+    body = text[find:]
     body = body[:body.index("\n}\n")]
-    call = body[body.index(launch):]
-    assert "setup_)" in call[:call.index(";")]
-    order = [body.index(t) for t in (launch, "PanelsLaunched()", f"{panels}.emplace(", "AwaitPanels(stream)", contract)]
+    order = [body.index(t) for t in (launch, "MakePanel(stream, launch)", f"{panels}.emplace(", contract)]
     assert order == sorted(order)
+    made = text[text.index("int Grid::MakePanel("):]
+    made = made[:made.index("\n}\n")]
+    assert made.index("launch(stream)") < made.index("cudaEventRecord(panelsMade_, stream)") < made.index(
+        "panelsPending_ = true;")
 
 
 @pytest.mark.gpu
