@@ -1,4 +1,5 @@
 // Error text, version and the device-memory helpers of the sl3dgpu C ABI.
+#include <cstdint>
 #include <mutex>
 #include <set>
 #include <string>
@@ -32,9 +33,20 @@ unsigned long long ContextId() {
 cudaError_t AllowDynamicSmemOnce(const void* kernel) {
   static std::mutex lock;
   static std::set<std::pair<unsigned long long, const void*>> done;  // (context, kernel)
+  // what this thread last found done, by the kernel's address: no lock on most launches
+  struct Seen {
+    unsigned long long context = 0;
+    const void* kernel = nullptr;
+  };
+  thread_local Seen seen[64];
   const unsigned long long context = ContextId();
+  Seen& mine = seen[(reinterpret_cast<uintptr_t>(kernel) >> 4) % 64];
+  if (context != 0 && mine.context == context && mine.kernel == kernel) return cudaSuccess;
   std::lock_guard<std::mutex> guard(lock);
-  if (context != 0 && done.count({context, kernel}) != 0) return cudaSuccess;
+  if (context != 0 && done.count({context, kernel}) != 0) {
+    mine = Seen{context, kernel};
+    return cudaSuccess;
+  }
   int device = 0, optin = 0;
   if (const cudaError_t e = cudaGetDevice(&device); e != cudaSuccess) return e;
   if (const cudaError_t e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);

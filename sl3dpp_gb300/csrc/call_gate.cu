@@ -17,17 +17,20 @@ thread_local int aloneDepth = 0;  // its sections
 std::mutex retiredLock;
 std::vector<cudaGraphExec_t> retired;
 
+// The gate keeps calls apart in time; what they share has locks of its own (the
+// driver's, a grid's). So a call that ends does not order its stores: on Arm that
+// would wait for its launches' writes to the device.
 void Enter() {
-  for (int now = inside.load();;) {
+  for (int now = inside.load(std::memory_order_relaxed);;) {
     if ((now & kAlone) != 0) {
       inside.wait(now);
       now = inside.load();
-    } else if (inside.compare_exchange_weak(now, now + 1)) {
+    } else if (inside.compare_exchange_weak(now, now + 1, std::memory_order_acquire, std::memory_order_relaxed)) {
       return;
     }
   }
 }
-void Leave() { inside.fetch_sub(1); }
+void Leave() { inside.fetch_sub(1, std::memory_order_relaxed); }
 
 }  // namespace
 
