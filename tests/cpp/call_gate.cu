@@ -82,6 +82,7 @@ int main() {
           if (in.load() != 1) clash = true;
         }
         in.fetch_sub(1);
+        std::atomic_thread_fence(std::memory_order_seq_cst);  // what calls share orders itself
         if (t % 2) std::this_thread::yield();
       }
     });
