@@ -182,7 +182,7 @@ void Try(int status) {
 }
 
 template <class T>
-void Judge(const char* form, const Batch& b, int B, const std::vector<T> x[2], const std::vector<T> rhs[2]) {
+void CheckBound(const char* form, const Batch& b, int B, const std::vector<T> x[2], const std::vector<T> rhs[2]) {
   const double u = sizeof(T) == sizeof(double) ? std::ldexp(1.0, -53) : std::ldexp(1.0, -24);
   double worst = 0.0, ratio = 0.0;
   for (int which = 0; which < 2; ++which)
@@ -220,7 +220,7 @@ void Check(Batch& b, int expected, std::mt19937_64& rng) {
     Try(RunBlockSolver(solver, a.d.p, c.d.p, scales.d.p, nullptr));
     x[0] = a.Read();
     x[1] = c.Read();
-    Judge("FP64", b, solver.block, x, rhs);
+    CheckBound("FP64", b, solver.block, x, rhs);
     for (int w = 0; w < 2; ++w) {
       const auto& systems = w ? second : first;
       if (systems.empty()) continue;
@@ -232,7 +232,7 @@ void Check(Batch& b, int expected, std::mt19937_64& rng) {
                          bands.d.p, nullptr, (w ? rc : ra).d.p, scales.d.p, 0, nullptr));
       rows[w] = (w ? rc : ra).Read();
     }
-    Judge("FP64, row by row", b, solver.block, rows, rhs);
+    CheckBound("FP64, row by row", b, solver.block, rows, rhs);
   }
   // FP32 over windows: from the first row, from inside a block, one row, the
   // last row, and two empty ones (their right-hand sides all zero)
@@ -286,9 +286,9 @@ void Check(Batch& b, int expected, std::mt19937_64& rng) {
     }
     char name[32];
     std::snprintf(name, sizeof name, "FP32, windows %d", kind);
-    Judge(name, b, solver.block, x, rhs);
+    CheckBound(name, b, solver.block, x, rhs);
     std::snprintf(name, sizeof name, "FP32, windows %d, by rows", kind);
-    Judge(name, b, solver.block, rows, rhs);
+    CheckBound(name, b, solver.block, rows, rhs);
   }
 }
 
